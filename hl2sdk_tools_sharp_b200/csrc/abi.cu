@@ -75,19 +75,6 @@ cudaError_t ensure(void **buf, size_t *cap, size_t need) {
     return e;
 }
 
-int32_t check_overflow(vrad_ctx *ctx) {
-    uint32_t flag = 0;
-    cudaError_t e = cudaMemcpyAsync(&flag, ctx->status, sizeof flag, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = vrad::wait_stream(ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "reading the traversal status");
-    if (flag) {
-        cudaMemsetAsync(ctx->status, 0, sizeof(uint32_t), ctx->stream);
-        return fail(ctx, VRAD_ERR_CUDA, "traversal stack overflow (BVH deeper than %d)",
-                    vrad::kStackDepth);
-    }
-    return VRAD_OK;
-}
-
 int32_t upload(vrad_ctx *ctx, const vrad_triangle *tris, const vrad_kd_triangle *prep, int32_t n) {
     if (!ctx) return fail(nullptr, VRAD_ERR_ARG, "null context");
     if (n <= 0 || !tris)
@@ -149,8 +136,7 @@ int32_t upload(vrad_ctx *ctx, const vrad_triangle *tris, const vrad_kd_triangle 
 int32_t trace_device(vrad_ctx *ctx, const vrad_ray *d_rays, int64_t n,
                      const vrad_trace_options *opts, uint32_t *d_bits, vrad_hit *d_hits, int mode,
                      cudaStream_t stream) {
-    cudaError_t e = vrad::launch_trace(ctx->scene.view(), d_rays, n, params_of(opts, mode), d_bits,
-                                       d_hits, ctx->status, stream);
+    cudaError_t e = vrad::launch_trace(ctx->scene.view(), d_rays, n, params_of(opts, mode), d_bits, d_hits, stream);
     if (e == cudaSuccess) e = vrad::join_stream(ctx, stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "trace launch");
     return VRAD_OK;
@@ -374,7 +360,7 @@ int32_t vrad_trace_visibility(vrad_ctx *ctx, const vrad_ray *rays, int64_t n,
     e = cudaMemcpyAsync(hit_bits, ctx->d_out, 8 * words64, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = vrad::wait_stream(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "visibility trace");
-    return check_overflow(ctx);
+    return VRAD_OK;
 }
 
 int32_t vrad_trace_closest(vrad_ctx *ctx, const vrad_ray *rays, int64_t n,
@@ -400,7 +386,7 @@ int32_t vrad_trace_closest(vrad_ctx *ctx, const vrad_ray *rays, int64_t n,
                         ctx->stream);
     if (e == cudaSuccess) e = vrad::wait_stream(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "closest trace");
-    return check_overflow(ctx);
+    return VRAD_OK;
 }
 
 int32_t vrad_trace_visibility_device(vrad_ctx *ctx, const vrad_ray *d_rays, int64_t n,
@@ -449,8 +435,6 @@ int32_t vrad_trace_visibility_static(vrad_ctx *ctx, const vrad_ray *rays, int64_
     const int mode = (opts && opts->sky_does_not_block) ? vrad::kModeSkyPass : vrad::kModeAny;
     e = vrad::trace_visibility_static(ctx->scene.view(), ctx->device, ctx->stream, rays, n,
                                       params_of(opts, mode), hit_bits);
-    if (e == cudaErrorLaunchOutOfResources)
-        return fail(ctx, VRAD_ERR_CUDA, "traversal stack overflow (BVH deeper than %d)", vrad::kStackDepth);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "allocation-free visibility trace");
     return VRAD_OK;
 }

@@ -278,22 +278,49 @@ __device__ __forceinline__ float poly_to_diff(const BounceView &v, int s, float 
     return poly_to_diff_pts(v.points + w.x, w.y, area, o, n, open);
 }
 
+// MakeTransfer for an open pair (receiver p, source s): DiffToDiff(source,
+// receiver), the polygon form factor for a near source, trans = area *
+// scale > 1e-7; 0 for none.
+__device__ __forceinline__ float make_transfer(const BounceView &v, int p, int s, unsigned long long *open) {
+    const float4 so = __ldg(&v.origin[s]);
+    if (__ldg(&v.tree[s].w) != 0 || !(so.w > 0.0f)) return 0.0f;
+    const float4 po = __ldg(&v.origin[p]), pn = __ldg(&v.normal[p]), sn = __ldg(&v.normal[s]);
+    float scale = diff_to_diff(f3(so), f3(sn), f3(po), f3(pn));
+    if (scale <= 0.0f) return 0.0f;
+    const F3 dd = sub3(f3(po), f3(so));
+    const float threshold = (float)__dmul_rn(3.141592653589793 * 0.04, (double)dot3(dd, dd));
+    if (threshold < so.w) {
+        scale = poly_to_diff(v, s, so.w, f3(po), f3(pn), open);
+        if (scale <= 0.0f) return 0.0f;
+    }
+    const float trans = __fmul_rn(so.w, scale);
+    return (double)trans > 0.0000001 ? trans : 0.0f;
+}
+
+// Where each receiver's transfer rays start their walk.
+__global__ void k_starts(BounceView v, DeviceBvh opaque, int32_t *__restrict__ start) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= v.nreceivers) return;
+    const int p = __ldg(&v.recv[r]);
+    const F3 o = add3(f3(__ldg(&v.origin[p])), f3(__ldg(&v.normal[p])));
+    start[r] = start_node(opaque, o.x, o.y, o.z);
+}
+
 // One candidate pair: VisMatrix.TransferRay traced (StockExact: every
 // triangle blocks, t in (0, len)), then MakeTransfer.  cand_w = the
-// transfer, 0 for none.  Twelve CTAs per SM (40 registers, a few spilled
-// to L1): the walk is latency-bound, and the extra resident warps hide
-// more of it than the spills cost (measured 66 against 72 ms at 64
-// registers and 8 CTAs on the 8x8 map).
+// transfer, 0 for none, kBlocked for a blocked ray (which k_transfer_count
+// counts: an atomic per warp here would be 20 M on one address).  Twelve
+// CTAs per SM (40 registers, a few spilled to L1).
+constexpr float kBlocked = -1.0f;
+
 template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK, 12) k_transfer(BounceView v, DeviceScene sc, const int64_t *__restrict__ cand_off,
-                                                    const int32_t *__restrict__ cand_src, float *__restrict__ cand_w,
-                                                    int64_t ncand, unsigned long long *counters, uint32_t *overflow) {
+__global__ void __launch_bounds__(BLOCK, 12)
+    k_transfer(BounceView v, DeviceScene sc, const int64_t *__restrict__ cand_off, const int32_t *__restrict__ cand_src,
+               const int32_t *__restrict__ start_at, float *__restrict__ cand_w, int64_t ncand,
+               unsigned long long *open) {
     extern __shared__ int stack_mem[];  // sc.stack_depth() entries per thread
     int *stack = stack_mem + threadIdx.x;
     const int64_t q = (int64_t)blockIdx.x * BLOCK + threadIdx.x;
-    const bool live = q < ncand;
-    float w = 0.0f;
-    bool blocked = false;
     // The receiver whose run holds q: one binary search per warp, for its
     // first candidate, then each lane steps forward (a warp's 32
     // candidates seldom span more than one or two receivers).
@@ -309,7 +336,7 @@ __global__ void __launch_bounds__(BLOCK, 12) k_transfer(BounceView v, DeviceScen
         r0 = lo;
     }
     r0 = __shfl_sync(kFull, r0, 0);
-    if (live) {
+    if (q < ncand) {
         int lo = r0;
         while (__ldg(&cand_off[lo + 1]) <= q) lo++;
         const int p = __ldg(&v.recv[lo]);
@@ -322,53 +349,48 @@ __global__ void __launch_bounds__(BLOCK, 12) k_transfer(BounceView v, DeviceScen
         const float safe = len == 0.0f ? 1.1920929e-07f : len;
         const RayState ray = make_ray(start.x, start.y, start.z, __fdiv_rn(delta.x, safe), __fdiv_rn(delta.y, safe),
                                       __fdiv_rn(delta.z, safe));
-        float t;
+        float t, w = kBlocked;
         int32_t orig;
         uint32_t meta;
-        trace_ray<kModeAny, BLOCK>(sc, ray, 0.0f, len, -1, stack, overflow, blocked, t, orig, meta);
-        if (!blocked && __ldg(&v.tree[s].w) == 0 && so.w > 0.0f) {
-            // MakeTransfer: DiffToDiff(source, receiver), the polygon form
-            // factor for a near source, trans = area * scale > 1e-7.
-            float scale = diff_to_diff(f3(so), f3(sn), f3(po), f3(pn));
-            if (!(scale <= 0.0f)) {
-                const F3 dd = sub3(f3(po), f3(so));
-                const float threshold = (float)__dmul_rn(3.141592653589793 * 0.04, (double)dot3(dd, dd));
-                bool ok = true;
-                if (threshold < so.w) {
-                    scale = poly_to_diff(v, s, so.w, f3(po), f3(pn), &counters[2]);
-                    ok = !(scale <= 0.0f);
-                }
-                if (ok) {
-                    const float trans = __fmul_rn(so.w, scale);
-                    if ((double)trans > 0.0000001) w = trans;
-                }
-            }
+        bool blocked;
+        trace_ray<kModeAny, BLOCK, true>(sc, ray, 0.0f, len, -1, __ldg(&start_at[lo]), stack, blocked, t, orig, meta);
+        if (!blocked) {
+            // The pair's rows are read again here, not held across the walk:
+            // at 40 registers they would be spilled to L1, whose bandwidth
+            // bounds the walk (transfer build 53.9 -> 50.2 ms on the 8x8 map).
+            int64_t again = q;
+            asm volatile("" : "+r"(lo), "+l"(again));
+            w = make_transfer(v, __ldg(&v.recv[lo]), __ldg(&cand_src[again]), open);
         }
         cand_w[q] = w;
     }
-    // Ray counts: one warp add each.
-    const unsigned lane = threadIdx.x & 31;
-    const int nlive = __popc(__ballot_sync(kFull, live));
-    const int nblocked = __popc(__ballot_sync(kFull, live && blocked));
-    if (lane == 0) {
-        if (nlive) atomicAdd(&counters[0], (unsigned long long)nlive);
-        if (nblocked) atomicAdd(&counters[1], (unsigned long long)nblocked);
-    }
 }
 
-// MakeTransfers' count per receiver: accepted pairs, at most MaxPatches.
+// MakeTransfers' count per receiver: accepted pairs, at most MaxPatches;
+// and the blocked rays, added to *blocked.
 __global__ void k_transfer_count(int nrecv, const int64_t *__restrict__ cand_off, const float *__restrict__ cand_w,
-                                 int64_t *__restrict__ counts) {
+                                 int64_t *__restrict__ counts, unsigned long long *blocked) {
+    __shared__ unsigned long long part[kBounceBlock / 32];
     const int r = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const unsigned lane = threadIdx.x & 31;
-    if (r >= nrecv) return;
-    const int64_t a = cand_off[r], b = cand_off[r + 1];
-    int64_t n = 0;
-    for (int64_t base = a; base < b; base += 32) {
-        const int64_t q = base + lane;
-        n += __popc(__ballot_sync(kFull, q < b && cand_w[q] > 0.0f));
+    int64_t n = 0, shut = 0;
+    if (r < nrecv) {
+        const int64_t a = cand_off[r], b = cand_off[r + 1];
+        for (int64_t base = a; base < b; base += 32) {
+            const int64_t q = base + lane;
+            const float w = q < b ? cand_w[q] : 0.0f;
+            n += __popc(__ballot_sync(kFull, w > 0.0f));
+            shut += __popc(__ballot_sync(kFull, w == kBlocked));
+        }
+        if (lane == 0) counts[r] = n < kMaxTransfersPerReceiver ? n : kMaxTransfersPerReceiver;
     }
-    if (lane == 0) counts[r] = n < kMaxTransfersPerReceiver ? n : kMaxTransfersPerReceiver;
+    if (lane == 0) part[threadIdx.x >> 5] = (unsigned long long)shut;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long sum = 0;
+        for (int k = 0; k < kBounceBlock / 32; k++) sum += part[k];
+        if (sum) atomicAdd(blocked, sum);
+    }
 }
 
 // MakeTransfers' writes in candidate order (the first MaxPatches), then
@@ -692,7 +714,7 @@ unsigned blocks(int64_t n, int per) { return (unsigned)((n + per - 1) / per); }
 
 void BounceBuffers::release() {
     void *ptrs[] = {origin, normal, mins, maxs, refl, tree, wind, points, face_range, face_samples, face_plane,
-                    recv, row_off, row_faces, sample_area, cand_off, cand_src, cand_w, tr_off, tr, scan_tmp,
+                    recv, start, row_off, row_faces, sample_area, cand_off, cand_src, cand_w, tr_off, tr, scan_tmp,
                     acc, direct, total, emit[0], emit[1], shoot[0], shoot[1], sums, exact, counters, leaf_desc,
                     level_patch, leaf_rank, sell_key, sell_idx, sell_count, sell_order, sell_off, sell, sort_tmp,
                     first, guess, feat, pred,
@@ -747,11 +769,12 @@ cudaError_t launch_transfers(BounceBuffers &b, const DeviceScene &scene, uint32_
     }
     k_candidates<<<blocks(R, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, b.cand_off, nullptr, b.cand_src,
                                                                        overflow);
+    k_starts<<<blocks(R, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, scene.opaque, b.start);
     if (b.ncand > 0)
-        k_transfer<kBlock><<<blocks(b.ncand, kBlock), kBlock, sizeof(int) * scene.stack_depth() * kBlock, stream>>>(b.view, scene, b.cand_off, b.cand_src,
-                                                                           b.cand_w, b.ncand, b.counters, overflow);
-    k_transfer_count<<<blocks((int64_t)R * 32, kBounceBlock), kBounceBlock, 0, stream>>>(R, b.cand_off, b.cand_w,
-                                                                                         b.tr_off + 1);
+        k_transfer<kBlock><<<blocks(b.ncand, kBlock), kBlock, sizeof(int) * scene.stack_depth() * kBlock, stream>>>(
+            b.view, scene, b.cand_off, b.cand_src, b.start, b.cand_w, b.ncand, &b.counters[2]);
+    k_transfer_count<<<blocks((int64_t)R * 32, kBounceBlock), kBounceBlock, 0, stream>>>(
+        R, b.cand_off, b.cand_w, b.tr_off + 1, &b.counters[1]);
     e = cudaMemsetAsync(b.tr_off, 0, sizeof(int64_t), stream);
     if (e != cudaSuccess) return e;
     tmp = b.scan_tmp_bytes;

@@ -14,6 +14,8 @@
 //   face_plane[F] float4 (plane normal xyz, dist)
 //   recv[R]      int32  receiver order (VisMatrix.ReceiverOrder): cluster by
 //                       cluster, each cluster's leaf patches in index order
+//   start[R]     int32  the opaque BVH node where the receiver's transfer
+//                       rays start their walk (traverse.cuh:start_node)
 //   row_off / row_faces  per cluster, the faces its PVS row reaches, in
 //                       VisMatrix.FacesInRow order
 //   cand_off[R+1] int64, cand_src[Q] int32, cand_w[Q] float: each receiver's
@@ -73,7 +75,7 @@ struct BounceBuffers {
     int4 *face_range = nullptr;
     int2 *face_samples = nullptr;
     float4 *face_plane = nullptr;
-    int32_t *recv = nullptr, *row_off = nullptr, *row_faces = nullptr;
+    int32_t *recv = nullptr, *start = nullptr, *row_off = nullptr, *row_faces = nullptr;
     float *sample_area = nullptr;
     // Transfer build.
     int64_t *cand_off = nullptr;   // R + 1

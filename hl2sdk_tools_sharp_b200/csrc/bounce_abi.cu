@@ -279,7 +279,7 @@ cudaError_t run_bounce(vrad_ctx *ctx, cudaStream_t s, const float4 *sample_light
         cudaEventElapsedTime(&b.patch_light_ms, ev[0], ev[1]);
         cudaEventElapsedTime(&b.transfer_ms, ev[1], ev[2]);
         cudaEventElapsedTime(&b.bounce_ms, ev[2], ev[3]);
-        b.rays = counts[0];
+        b.rays = build_transfers ? (unsigned long long)b.ncand : 0;
         b.blocked = counts[1];
         b.open_ties = counts[2];
     } else {
@@ -550,6 +550,7 @@ extern "C" int32_t vrad_bounce_upload(vrad_ctx *ctx, const vrad_bounce_desc *d) 
     const size_t P1 = (size_t)(P ? P : 1), R1 = (size_t)R + 1, N1 = (size_t)(ncells ? ncells : 1);
     if (e == cudaSuccess) e = dev_alloc(&b.cand_off, sizeof(int64_t) * R1);
     if (e == cudaSuccess) e = dev_alloc(&b.tr_off, sizeof(int64_t) * R1);
+    if (e == cudaSuccess) e = dev_alloc(&b.start, sizeof(int32_t) * R1);
     for (float4 **q : {&b.acc, &b.direct, &b.total, &b.emit[0], &b.emit[1], &b.shoot[0], &b.shoot[1]})
         if (e == cudaSuccess) e = dev_alloc(q, sizeof(float4) * P1);
     if (e == cudaSuccess) e = dev_alloc(&b.sums, kSums * sizeof(double));

@@ -40,7 +40,7 @@ struct vrad_ctx {
     vrad::SceneBuffers scene;
     vrad::SceneBuildReport report;
     bool has_scene = false;
-    uint32_t *status = nullptr;   // [0] traversal stack overflow flag (sticky)
+    uint32_t *status = nullptr;   // [0] the candidate walk's overflow flag in a light pass (sticky)
     // Staging for the host-buffer entry points, grown on demand.
     void *d_rays = nullptr;
     size_t d_rays_cap = 0;

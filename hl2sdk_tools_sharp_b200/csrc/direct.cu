@@ -47,8 +47,7 @@ namespace {
 template <int BLOCK, bool DUAL>
 __global__ void __launch_bounds__(BLOCK) k_direct(DeviceScene sc, DeviceWorld w, float4 *__restrict__ out,
                                                   float4 *__restrict__ out_hdr,
-                                                  unsigned long long *__restrict__ counters,
-                                                  uint32_t *__restrict__ overflow) {
+                                                  unsigned long long *__restrict__ counters) {
     extern __shared__ int stack_mem[];  // sc.stack_depth() entries per thread
     int *stack = stack_mem + threadIdx.x;
     const int64_t slot = (int64_t)blockIdx.x * BLOCK + threadIdx.x;
@@ -71,13 +70,16 @@ __global__ void __launch_bounds__(BLOCK) k_direct(DeviceScene sc, DeviceWorld w,
     // One unit off the face (ComputeIlluminationPointAndNormals).
     const float px = __fadd_rn(sp.x, nx), py = __fadd_rn(sp.y, ny), pz = __fadd_rn(sp.z, nz);
 
-    unsigned long long vis_rays = 0, sky_rays = 0;
+    const int start = start_node(sc.opaque, px, py, pz);
+    if (real) w.start[si] = start;
+    uint32_t vis_rays = 0, sky_rays = 0;  // one point's rays
     float4 h;
     // The group's first sample (a face's groups start on lanes 0, 4, ...):
     // groups in sample order are ResolveGroup's order.
     const unsigned long long key_group = (unsigned long long)(uint32_t)__shfl_sync(kFull, si, lane & ~3) << 32;
     const float4 r = gather_point<BLOCK, DUAL>(sc, w, cluster, px, py, pz, nx, ny, nz, real, gmask, kAllLights,
-                                               stack, overflow, counters, vis_rays, sky_rays, &h, face, key_group);
+                                               start, stack, counters, vis_rays, sky_rays,
+                                               &h, face, key_group);
     if (real) {
         out[si] = r;
         if (DUAL) out_hdr[si] = h;
@@ -90,8 +92,8 @@ __global__ void __launch_bounds__(BLOCK) k_direct(DeviceScene sc, DeviceWorld w,
         sky_rays += __shfl_xor_sync(kFull, sky_rays, o);
     }
     if (lane == 0) {
-        atomicAdd(&counters[0], vis_rays);
-        atomicAdd(&counters[1], sky_rays);
+        atomicAdd(&counters[0], (unsigned long long)vis_rays);
+        atomicAdd(&counters[1], (unsigned long long)sky_rays);
     }
 }
 
@@ -115,6 +117,7 @@ void StyleState::release() {
 void WorldBuffers::release() {
     dev_free(slots);
     dev_free(sample_pos);
+    dev_free(start);
     dev_free(face_normal);
     dev_free(lights);
     dev_free(lights_hdr);
@@ -123,7 +126,7 @@ void WorldBuffers::release() {
     dev_free(dirs);
     dev_free(jitter);
     dev_free(counters);
-    slots = nullptr;
+    slots = start = nullptr;
     sample_pos = face_normal = lights = lights_hdr = dirs = jitter = nullptr;
     cl_off = cl_list = nullptr;
     counters = nullptr;
@@ -132,8 +135,7 @@ void WorldBuffers::release() {
 }
 
 cudaError_t launch_direct(const DeviceScene &scene, const DeviceWorld &world, float4 *out, float4 *out_hdr,
-                          unsigned long long *counters, uint32_t *overflow, cudaStream_t stream,
-                          int block) {
+                          unsigned long long *counters, cudaStream_t stream, int block) {
     if (world.nslots == 0) return cudaSuccess;
     if (out_hdr && !world.lights_hdr) return cudaErrorInvalidValue;
     const size_t smem = sizeof(int) * (size_t)scene.stack_depth();  // per thread
@@ -141,15 +143,15 @@ cudaError_t launch_direct(const DeviceScene &scene, const DeviceWorld &world, fl
                    g128 = (unsigned)((world.nslots + 127) / 128);
     if (out_hdr) {
         switch (block) {
-            case 32: k_direct<32, true><<<g32, 32, smem * 32, stream>>>(scene, world, out, out_hdr, counters, overflow); break;
-            case 64: k_direct<64, true><<<g64, 64, smem * 64, stream>>>(scene, world, out, out_hdr, counters, overflow); break;
-            default: k_direct<128, true><<<g128, 128, smem * 128, stream>>>(scene, world, out, out_hdr, counters, overflow); break;
+            case 32: k_direct<32, true><<<g32, 32, smem * 32, stream>>>(scene, world, out, out_hdr, counters); break;
+            case 64: k_direct<64, true><<<g64, 64, smem * 64, stream>>>(scene, world, out, out_hdr, counters); break;
+            default: k_direct<128, true><<<g128, 128, smem * 128, stream>>>(scene, world, out, out_hdr, counters); break;
         }
     } else {
         switch (block) {
-            case 32: k_direct<32, false><<<g32, 32, smem * 32, stream>>>(scene, world, out, nullptr, counters, overflow); break;
-            case 64: k_direct<64, false><<<g64, 64, smem * 64, stream>>>(scene, world, out, nullptr, counters, overflow); break;
-            default: k_direct<128, false><<<g128, 128, smem * 128, stream>>>(scene, world, out, nullptr, counters, overflow); break;
+            case 32: k_direct<32, false><<<g32, 32, smem * 32, stream>>>(scene, world, out, nullptr, counters); break;
+            case 64: k_direct<64, false><<<g64, 64, smem * 64, stream>>>(scene, world, out, nullptr, counters); break;
+            default: k_direct<128, false><<<g128, 128, smem * 128, stream>>>(scene, world, out, nullptr, counters); break;
         }
     }
     return cudaGetLastError();
@@ -347,6 +349,7 @@ extern "C" int32_t vrad_world_upload(vrad_ctx *ctx, const vrad_world_desc *w) {
                              ctx->styles.styles.end());
     if (e == cudaSuccess) e = vrad::stage_table(ctx->stager, ctx->stream, &wb.slots, slots);
     if (e == cudaSuccess) e = vrad::dma_table(&wb.sample_pos, pos, (size_t)w->nsamples, ctx->stream);
+    if (e == cudaSuccess) e = vrad::dev_alloc(&wb.start, sizeof(int32_t) * (size_t)(w->nsamples ? w->nsamples : 1));
     if (e == cudaSuccess) e = vrad::stage_table(ctx->stager, ctx->stream, &wb.face_normal, fnorm);
     if (e == cudaSuccess) e = vrad::stage_table(ctx->stager, ctx->stream, &wb.lights, lights);
     if (e == cudaSuccess && !lights_hdr.empty())
@@ -361,7 +364,7 @@ extern "C" int32_t vrad_world_upload(vrad_ctx *ctx, const vrad_world_desc *w) {
         wb.release();
         return vrad_cuda_fail(ctx, e, "world upload");
     }
-    wb.view = vrad::DeviceWorld{wb.slots, (int64_t)slots.size(), wb.sample_pos, wb.face_normal, wb.lights, nl,
+    wb.view = vrad::DeviceWorld{wb.slots, (int64_t)slots.size(), wb.sample_pos, wb.start, wb.face_normal, wb.lights, nl,
                                 wb.cl_off, wb.cl_list, w->nclusters, wb.dirs, w->nsky_directions, wb.jitter,
                                 w->nsun_jitter, w->sun_angular_extent, w->sun_samples, w->nsamples,
                                 wb.lights_hdr};
@@ -471,11 +474,11 @@ int32_t direct_on(vrad_ctx *ctx, float4 *ldr_out, float4 *hdr_out, cudaStream_t 
     cudaError_t e = cudaMemsetAsync(ctx->world.counters, 0, 3 * sizeof(unsigned long long), s);
     if (e == cudaSuccess) {
         if (ldr_out && hdr_out)
-            e = vrad::launch_direct(ctx->scene.view(), ctx->world.view, ldr_out, hdr_out, ctx->world.counters,
-                                    ctx->status, s, ctx->world.block);
+            e = vrad::launch_direct(ctx->scene.view(), ctx->world.view, ldr_out, hdr_out, ctx->world.counters, s,
+                                    ctx->world.block);
         else
             e = vrad::launch_direct(ctx->scene.view(), ldr_out ? ldr : hdr, ldr_out ? ldr_out : hdr_out, nullptr,
-                                    ctx->world.counters, ctx->status, s, ctx->world.block);
+                                    ctx->world.counters, s, ctx->world.block);
     }
     // The supersampling passes (FaceLightJob's rounds after the first),
     // per range.
@@ -485,7 +488,7 @@ int32_t direct_on(vrad_ctx *ctx, float4 *ldr_out, float4 *hdr_out, cudaStream_t 
         ctx->range_ss[r] = vrad::RangeSupersample{};
         if (!out || e != cudaSuccess) continue;
         e = vrad::run_supersample(ss, ctx->scene.view(), r == 0 ? ldr : hdr, ctx->final_pass.view, out,
-                                  ctx->world.counters, ctx->status, s);
+                                  ctx->world.counters, s);
         ctx->range_ss[r] = vrad::RangeSupersample{ss.passes_run, ss.supersampled, ss.ms};
     }
     if (e != cudaSuccess) return vrad_cuda_fail(ctx, e, "direct lighting launch");
@@ -557,21 +560,14 @@ extern "C" int32_t vrad_direct_lighting(vrad_ctx *ctx, vrad_lighting_value *out,
     }
     int32_t rc = direct_on(ctx, d_out, nullptr, ctx->stream);
     unsigned long long counts[2] = {0, 0};
-    uint32_t overflow = 0;
     if (rc == VRAD_OK) {
         e = cudaEventRecord(b, ctx->stream);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(out, d_out, sizeof(float4) * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(counts, ctx->world.counters, sizeof counts, cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(&overflow, ctx->status, sizeof overflow, cudaMemcpyDeviceToHost, ctx->stream);
         if (e == cudaSuccess) e = vrad::wait_stream(ctx->stream);
         if (e != cudaSuccess) rc = vrad_cuda_fail(ctx, e, "direct lighting");
-    }
-    if (rc == VRAD_OK && overflow) {
-        cudaMemsetAsync(ctx->status, 0, sizeof(uint32_t), ctx->stream);
-        rc = vrad_fail(ctx, VRAD_ERR_CUDA, "traversal stack overflow (BVH deeper than %d)", vrad::kStackDepth);
     }
     if (rc == VRAD_OK && stats) {
         float ms = 0.0f;
@@ -613,7 +609,7 @@ extern "C" int32_t vrad_direct_autotune(vrad_ctx *ctx, int32_t *chosen_block, fl
         e = cudaEventRecord(a, ctx->stream);
         if (e == cudaSuccess)
             e = vrad::launch_direct(ctx->scene.view(), dual ? ctx->world.view : vrad::range_view(ctx->world.view, false),
-                                    d_out, d_hdr, ctx->world.counters, ctx->status, ctx->stream, candidates[k]);
+                                    d_out, d_hdr, ctx->world.counters, ctx->stream, candidates[k]);
         if (e == cudaSuccess) e = cudaEventRecord(b, ctx->stream);
         if (e == cudaSuccess) e = cudaEventSynchronize(b);
         float ms = 0.0f;

@@ -11,6 +11,9 @@
 //                   adjacent lanes) and each cluster padded to whole warps,
 //                   so a warp's lanes share one light list.
 //   sample_pos[i]   float4 (position xyz, face index bits)
+//   start[i]        int32: the opaque BVH node where the sample's segments
+//                   start their walk (traverse.cuh:start_node); the gather
+//                   writes it, the supersampling passes read it
 //   face_normal[f]  float4 (plane normal xyz, cluster bits)
 //   lights[l]       5 x float4, the DirectLight fields:
 //                   (origin, type) (intensity, style) (normal, exponent)
@@ -37,6 +40,7 @@ struct DeviceWorld {
     const int32_t *slots;
     int64_t nslots;
     const float4 *sample_pos;
+    int32_t *start;
     const float4 *face_normal;
     const float4 *lights;
     int32_t nlights;
@@ -65,6 +69,7 @@ struct DeviceWorld {
 struct WorldBuffers {
     int32_t *slots = nullptr;
     float4 *sample_pos = nullptr;
+    int32_t *start = nullptr;
     float4 *face_normal = nullptr;
     float4 *lights = nullptr;
     float4 *lights_hdr = nullptr;
@@ -102,8 +107,7 @@ struct StyleState {
 // With out_hdr (and world.lights_hdr) one traversal lights both ranges:
 // out from world.lights, out_hdr from world.lights_hdr.
 cudaError_t launch_direct(const DeviceScene &scene, const DeviceWorld &world, float4 *out, float4 *out_hdr,
-                          unsigned long long *counters, uint32_t *overflow, cudaStream_t stream,
-                          int block);
+                          unsigned long long *counters, cudaStream_t stream, int block);
 
 // The world as one range sees it: lights = that range's table, no second.
 inline DeviceWorld range_view(const DeviceWorld &w, bool hdr) {

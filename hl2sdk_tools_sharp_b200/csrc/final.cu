@@ -662,8 +662,7 @@ int32_t ensure_style_layout(vrad_ctx *ctx, cudaStream_t s) {
         vrad::DeviceWorld v = vrad::range_view(ctx->world.view, false);
         v.style = st.styles[(size_t)i];
         v.face_key = st.keys + (size_t)i * nf;
-        e = vrad::launch_direct(ctx->scene.view(), v, st.light[0][(size_t)i], nullptr, scratch, ctx->status, s,
-                                ctx->world.block);
+        e = vrad::launch_direct(ctx->scene.view(), v, st.light[0][(size_t)i], nullptr, scratch, s, ctx->world.block);
     }
     std::vector<unsigned long long> keys((size_t)S * nf);
     if (e == cudaSuccess && nf)
@@ -751,16 +750,16 @@ int32_t pass_on(vrad_ctx *ctx, int32_t ranges, uint8_t *d_ldr, uint8_t *d_hdr, c
         float4 *lo = (ranges & VRAD_RANGE_LDR) ? st.light[0][i] : nullptr;
         float4 *hi = (ranges & VRAD_RANGE_HDR) ? st.light[1][i] : nullptr;
         if (lo && hi)
-            e = vrad::launch_direct(ctx->scene.view(), v, lo, hi, ctx->world.counters, ctx->status, s, ctx->world.block);
+            e = vrad::launch_direct(ctx->scene.view(), v, lo, hi, ctx->world.counters, s, ctx->world.block);
         else
             e = vrad::launch_direct(ctx->scene.view(), vrad::range_view(v, hi != nullptr), lo ? lo : hi, nullptr,
-                                    ctx->world.counters, ctx->status, s, ctx->world.block);
+                                    ctx->world.counters, s, ctx->world.block);
         for (int r = 0; r < 2 && e == cudaSuccess; r++) {
             float4 *out = r == 0 ? lo : hi;
             if (!out) continue;
             vrad::SupersampleBuffers &ss = ctx->supersample;
             e = vrad::run_supersample(ss, ctx->scene.view(), vrad::range_view(v, r == 1), fb.view, out,
-                                      ctx->world.counters, ctx->status, s);
+                                      ctx->world.counters, s);
             ctx->range_ss[r].supersampled += ss.supersampled;
             ctx->range_ss[r].ms += ss.ms;
         }
@@ -869,7 +868,7 @@ int32_t pass_host(vrad_ctx *ctx, int32_t ranges, uint8_t *ldr, int64_t ldr_capac
     }
     if (rc == VRAD_OK && overflow) {
         cudaMemsetAsync(ctx->status, 0, sizeof(uint32_t), s);
-        rc = vrad_fail(ctx, VRAD_ERR_CUDA, "traversal stack overflow (BVH deeper than %d)", vrad::kStackDepth);
+        rc = vrad_fail(ctx, VRAD_ERR_CUDA, "stack overflow in the candidate walk (flags %u)", overflow);
     }
     if (rc == VRAD_OK) {
         float final_ms[2] = {0.0f, 0.0f};

@@ -37,11 +37,6 @@ enum : int { kSurface = 0, kPoint = 1, kSpot = 2, kSkyLight = 3, kSkyAmbient = 4
 // LightConstants.DistEpsilon: how far a surface light's rays end off its patch.
 constexpr float kDistEpsilon = 0.03125f;
 
-// The any-hit walks' child order for the gather's segments: the farther
-// child first (measured faster for these rays than nearest first).
-constexpr bool kFarPoint = true;  // shadow segments to point and spot lights
-constexpr bool kFarSky = true;    // the opaque walk of the sun and sky tests
-
 __device__ __forceinline__ float maxps(float a, float b) { return a > b ? a : b; }
 __device__ __forceinline__ float minps(float a, float b) { return a < b ? a : b; }
 
@@ -56,16 +51,15 @@ __device__ __forceinline__ bool group_any(bool v, unsigned gmask) {
 // The segment start -> stop (LightRayLog.MakeRay: whole segment, reach 1).
 // Visibility blocks on any hit; a sky test blocks only when the first hit
 // is opaque.
-template <int MODE, int STRIDE, bool FAR_ANY>
+template <int MODE, int STRIDE>
 __device__ __forceinline__ bool segment_blocked(const DeviceScene &sc, float sx, float sy, float sz,
-                                                float ex, float ey, float ez, int *stack,
-                                                uint32_t *overflow) {
+                                                float ex, float ey, float ez, int start, int *stack) {
     const RayState r = make_ray(sx, sy, sz, __fsub_rn(ex, sx), __fsub_rn(ey, sy), __fsub_rn(ez, sz));
     bool hit;
     float t;
     int32_t orig;
     uint32_t meta;
-    trace_ray<MODE, STRIDE, FAR_ANY>(sc, r, 0.0f, 1.0f, -1, stack, overflow, hit, t, orig, meta);
+    trace_ray<MODE, STRIDE, true>(sc, r, 0.0f, 1.0f, -1, start, stack, hit, t, orig, meta);
     return hit;
 }
 
@@ -103,9 +97,9 @@ enum : int { kAllLights = 0, kAmbientOnly = 1, kDirectOnly = 2 };
 template <int BLOCK, bool DUAL = false>
 __device__ __forceinline__ float4 gather_point(const DeviceScene &sc, const DeviceWorld &w, int cluster, float px,
                                                float py, float pz, float nx, float ny, float nz, bool real,
-                                               unsigned gmask, int filter, int *stack, uint32_t *overflow,
-                                               unsigned long long *counters, unsigned long long &vis_rays,
-                                               unsigned long long &sky_rays, float4 *second = nullptr,
+                                               unsigned gmask, int filter, int start, int *stack,
+                                               unsigned long long *counters, uint32_t &vis_rays, uint32_t &sky_rays,
+                                               float4 *second = nullptr,
                                                int face = 0, unsigned long long key_group = 0) {
     float ax = 0.0f, ay = 0.0f, az = 0.0f, sun = 0.0f;
     float hx = 0.0f, hy = 0.0f, hz = 0.0f;
@@ -167,7 +161,7 @@ __device__ __forceinline__ float4 gather_point(const DeviceScene &sc, const Devi
             }
             if (real && dot != 0.0f && falloff != 0.0f) {
                 vis_rays++;
-                if (segment_blocked<kModeAny, BLOCK, kFarPoint>(sc, px, py, pz, A.x, A.y, A.z, stack, overflow)) dot = 0.0f;
+                if (segment_blocked<kModeAny, BLOCK>(sc, px, py, pz, A.x, A.y, A.z, start, stack)) dot = 0.0f;
             }
         } else if (type == kSurface) {
             // GatherSurfaceFour (DirectLightGatherer.cs:1452-1545): the
@@ -198,7 +192,7 @@ __device__ __forceinline__ float4 gather_point(const DeviceScene &sc, const Devi
                 const float ex = __fadd_rn(A.x, __fmul_rn(C.x, kDistEpsilon)),
                             ey = __fadd_rn(A.y, __fmul_rn(C.y, kDistEpsilon)),
                             ez = __fadd_rn(A.z, __fmul_rn(C.z, kDistEpsilon));
-                if (segment_blocked<kModeAny, BLOCK, kFarPoint>(sc, px, py, pz, ex, ey, ez, stack, overflow)) dot = 0.0f;
+                if (segment_blocked<kModeAny, BLOCK>(sc, px, py, pz, ex, ey, ez, start, stack)) dot = 0.0f;
             }
         } else if (type == kSkyLight) {
             // EmitSkyLight / ResolveSkyLight.
@@ -221,9 +215,9 @@ __device__ __forceinline__ float4 gather_point(const DeviceScene &sc, const Devi
                     float frac = 1.0f;
                     if (need && real) {
                         sky_rays++;
-                        if (segment_blocked<kModeSkyPass, BLOCK, kFarSky>(sc, px, py, pz, __fadd_rn(ex, px),
-                                                                 __fadd_rn(ey, py), __fadd_rn(ez, pz), stack,
-                                                                 overflow))
+                        if (segment_blocked<kModeSkyPass, BLOCK>(sc, px, py, pz, __fadd_rn(ex, px),
+                                                                 __fadd_rn(ey, py), __fadd_rn(ez, pz), start,
+                                                             stack))
                             frac = 0.0f;
                     }
                     total = __fadd_rn(total, frac);
@@ -248,16 +242,15 @@ __device__ __forceinline__ float4 gather_point(const DeviceScene &sc, const Devi
                 possible = __fadd_rn(valid ? 1.0f : 0.0f, possible);
                 float frac = 1.0f;
                 if (valid && real) {
-                    // surfacePos = points - anorm * -epsilon, epsilon 0;
-                    // stop = anorm * -MaxTraceLength + points.
-                    const float sx = __fsub_rn(px, __fmul_rn(an.x, -0.0f));
-                    const float sy = __fsub_rn(py, __fmul_rn(an.y, -0.0f));
-                    const float sz = __fsub_rn(pz, __fmul_rn(an.z, -0.0f));
+                    // surfacePos = points - anorm * -epsilon, epsilon 0, which
+                    // is the point but for the sign of a zero, and no sign
+                    // of a zero decides a hit; stop = anorm *
+                    // -MaxTraceLength + points.
                     const float ex = __fadd_rn(__fmul_rn(an.x, -kMaxTraceLength), px);
                     const float ey = __fadd_rn(__fmul_rn(an.y, -kMaxTraceLength), py);
                     const float ez = __fadd_rn(__fmul_rn(an.z, -kMaxTraceLength), pz);
                     sky_rays++;
-                    if (segment_blocked<kModeSkyPass, BLOCK, kFarSky>(sc, sx, sy, sz, ex, ey, ez, stack, overflow)) frac = 0.0f;
+                    if (segment_blocked<kModeSkyPass, BLOCK>(sc, px, py, pz, ex, ey, ez, start, stack)) frac = 0.0f;
                 }
                 ambient = __fadd_rn(ambient, __fmul_rn(frac, dv));
                 __syncwarp();

@@ -34,9 +34,8 @@ namespace {
 constexpr int64_t kMaxRays = VRAD_STATIC_MAX_RAYS;
 constexpr size_t kRayBytes = sizeof(vrad_ray) * (size_t)kMaxRays;
 constexpr size_t kBitBytes = 8 * (size_t)((kMaxRays + 63) / 64);
-// Layout: [rays | hit bits | status word (traversal stack overflow)].
-constexpr size_t kStatusOffset = kRayBytes + kBitBytes;
-constexpr size_t kScratchBytes = kStatusOffset + 256;
+// Layout: [rays | hit bits | 256 spare bytes].
+constexpr size_t kScratchBytes = kRayBytes + kBitBytes + 256;
 
 static_assert(kRayBytes % 256 == 0, "bits must start 256-byte aligned");
 static_assert(kScratchBytes == 1843456, "the size the header and the comment above state");
@@ -83,22 +82,16 @@ cudaError_t trace_visibility_static(const DeviceScene &scene, int device, cudaSt
     if (e != cudaSuccess) return e;
     vrad_ray *d_rays = reinterpret_cast<vrad_ray *>(base);
     uint32_t *d_bits = reinterpret_cast<uint32_t *>(base + kRayBytes);
-    uint32_t *d_status = reinterpret_cast<uint32_t *>(base + kStatusOffset);
     const size_t words64 = (size_t)((n + 63) / 64);
-    // The array keeps the previous call's contents: clear the status word
-    // and the bit words (the last one may belong to no warp).
-    e = cudaMemsetAsync(d_status, 0, sizeof(uint32_t), stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_bits, 0, 8 * words64, stream);
+    // The array keeps the previous call's contents: clear the bit words (the
+    // last one may belong to no warp).
+    e = cudaMemsetAsync(d_bits, 0, 8 * words64, stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d_rays, h_rays, sizeof(vrad_ray) * (size_t)n, cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess) e = launch_trace(scene, d_rays, n, p, d_bits, nullptr, d_status, stream);
+    if (e == cudaSuccess) e = launch_trace(scene, d_rays, n, p, d_bits, nullptr, stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(h_bits, d_bits, 8 * words64, cudaMemcpyDeviceToHost, stream);
-    uint32_t status = 0;
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&status, d_status, sizeof status, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    if (e == cudaSuccess && status != 0) return cudaErrorLaunchOutOfResources;  // stack overflow
     return e;
 }
 

@@ -38,7 +38,7 @@ namespace {
 __global__ void __launch_bounds__(kBlock) k_trace_flag(DeviceScene s, const vrad_ray *__restrict__ rays, int64_t n,
                                                        float tmin, int32_t skip_id, float margin,
                                                        uint32_t *__restrict__ bits, int32_t *__restrict__ flagged,
-                                                       int32_t *count, uint32_t *overflow) {
+                                                       int32_t *count) {
     extern __shared__ int stack_mem[];
     int *stack = stack_mem + threadIdx.x;
     const int lane = threadIdx.x & 31;
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kBlock) k_trace_flag(DeviceScene s, const vrad
         r.noy = -r.oy * r.iy;
         r.noz = -r.oz * r.iz;
         nc.thi = reach;
-        trace_ray_flagged(s, r, tmin, reach, skip_id, stack, overflow, hit, nc);
+        trace_ray_flagged(s, r, tmin, reach, skip_id, stack, hit, nc);
         if (nc.near) flagged[atomicAdd(count, 1)] = (int32_t)i;
     }
     const uint32_t word = __ballot_sync(kFull, hit);
@@ -213,7 +213,7 @@ extern "C" int32_t vrad_trace_visibility_recheck(vrad_ctx *ctx, const vrad_ray *
         const DeviceScene s = ctx->scene.view();
         const size_t smem = sizeof(int) * (size_t)s.stack_depth() * kBlock;
         k_trace_flag<<<(unsigned)((n + kBlock - 1) / kBlock), kBlock, smem, ctx->stream>>>(
-            s, d_rays, n, tmin, skip, flag_margin, d_bits, d_flagged, d_count, ctx->status);
+            s, d_rays, n, tmin, skip, flag_margin, d_bits, d_flagged, d_count);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(&nflagged, d_count, sizeof nflagged, cudaMemcpyDeviceToHost, ctx->stream);
@@ -239,15 +239,6 @@ extern "C" int32_t vrad_trace_visibility_recheck(vrad_ctx *ctx, const vrad_ray *
                     (void *)d_cls})
         dev_free(p);
     if (e != cudaSuccess) return vrad_cuda_fail(ctx, e, "visibility recheck");
-    uint32_t overflow = 0;
-    e = cudaMemcpyAsync(&overflow, ctx->status, sizeof overflow, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = wait_stream(ctx->stream);
-    if (e != cudaSuccess) return vrad_cuda_fail(ctx, e, "reading the traversal status");
-    if (overflow) {
-        cudaMemsetAsync(ctx->status, 0, sizeof(uint32_t), ctx->stream);
-        wait_stream(ctx->stream);
-        return vrad_fail(ctx, VRAD_ERR_CUDA, "traversal stack overflow");
-    }
     for (int64_t i = 0; i < n; i++) fp64_class[i] = -1;
     st.flagged = nflagged;
     for (int32_t k = 0; k < nflagged; k++) {

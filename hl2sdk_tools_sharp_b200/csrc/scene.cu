@@ -10,6 +10,7 @@
 //   k_bounds       scene bounds (one block, fixed-order reduction)
 //   host           boxes padded, SAH tree (two-child nodes of 64 B, leaf
 //                  references), uploaded
+//   k_octants      the nodes as a ray of each of the eight octants reads them
 //   k_gather       triangles into leaf order
 //
 // The tree's shape is free: no answer depends on it (the traversal tests
@@ -161,22 +162,72 @@ __global__ void k_bounds(const float *__restrict__ box, int n, float *__restrict
     }
 }
 
-// A one-triangle scene: a root whose second child is an empty box.
-__global__ void k_emit_single(const float *__restrict__ leaf_box, float4 *__restrict__ nodes) {
-    const float *b = leaf_box;
-    nodes[0] = make_float4(b[0], b[3], b[1], b[4]);
-    nodes[1] = make_float4(FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX);
-    nodes[2] = make_float4(b[2], b[5], FLT_MAX, -FLT_MAX);
-    nodes[3] = make_float4(__int_as_float(leaf_ref(0, 1)), __int_as_float(leaf_ref(0, 1)), 0.0f, 0.0f);
-}
-
-__global__ void k_pad_single(const float *__restrict__ tri_box, const float *__restrict__ bounds,
-                             float *__restrict__ leaf_box) {
-    const float pad = ldexpf(bounds[6], -16) + 1e-6f;
-    for (int a = 0; a < 3; a++) {
-        leaf_box[a] = tri_box[a] - pad;
-        leaf_box[3 + a] = tri_box[3 + a] + pad;
+// The eight octants' copies of the tree's nodes (vrad_internal.cuh's
+// layout) from its canonical ones: tree[4 i ..] = (c0.lo.x, c0.hi.x,
+// c0.lo.y, c0.hi.y), (c1 the same), (c0.lo.z, c0.hi.z, c1.lo.z, c1.hi.z),
+// (ref0, ref1, -, -); parent[i] = node i's parent (-1 the root's).  A node's
+// two children are ordered by their boxes' centres along the octant's
+// diagonal; a node that leads up keeps the nearer generation first.
+__global__ void k_octants(const float4 *__restrict__ tree, const int32_t *__restrict__ parent, int inner,
+                          float4 *__restrict__ nodes) {
+    const int id = blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= 16 * inner) return;
+    const int oct = id / (2 * inner), i = id - oct * 2 * inner;
+    float lo[2][3], hi[2][3];
+    int ref[2], next = -1;
+    auto child = [&](int node, int c, int to) {
+        const float4 *nd = tree + 4 * (size_t)node;
+        const float4 xy = nd[c], z = nd[2], r = nd[3];
+        lo[to][0] = xy.x;
+        hi[to][0] = xy.y;
+        lo[to][1] = xy.z;
+        hi[to][1] = xy.w;
+        lo[to][2] = c ? z.z : z.x;
+        hi[to][2] = c ? z.w : z.y;
+        ref[to] = __float_as_int(c ? r.y : r.x);
+    };
+    auto sibling = [&](int k, int to) {
+        const int p = k > 0 ? parent[k] : -1;
+        if (p >= 0) {
+            child(p, __float_as_int(tree[4 * (size_t)p + 3].x) == k ? 1 : 0, to);
+            return p;
+        }
+        for (int x = 0; x < 3; x++) {
+            lo[to][x] = FLT_MAX;
+            hi[to][x] = -FLT_MAX;
+        }
+        ref[to] = leaf_ref(0, 1);
+        return -1;
+    };
+    bool swap = false;
+    if (i < inner) {
+        child(i, 0, 0);
+        child(i, 1, 1);
+        float key[2] = {0.0f, 0.0f};
+        for (int c = 0; c < 2; c++)
+            for (int x = 0; x < 3; x++) {
+                const float mid = 0.5f * lo[c][x] + 0.5f * hi[c][x];
+                key[c] += (oct >> x) & 1 ? -mid : mid;
+            }
+        swap = key[1] < key[0];
+    } else {
+        const int p = sibling(i - inner, 0);
+        const int g = sibling(p, 1);
+        if (g > 0) next = inner + g;
     }
+    float near[2][3], far[2][3];
+    for (int c = 0; c < 2; c++)
+        for (int x = 0; x < 3; x++) {
+            const bool neg = (oct >> x) & 1;
+            near[c][x] = neg ? hi[c][x] : lo[c][x];
+            far[c][x] = neg ? lo[c][x] : hi[c][x];
+        }
+    const int p = swap ? 1 : 0, q = 1 - p;
+    float4 *o = nodes + 4 * (size_t)id;
+    o[0] = make_float4(near[p][0], near[p][1], far[p][0], far[p][1]);
+    o[1] = make_float4(near[q][0], near[q][1], far[q][0], far[q][1]);
+    o[2] = make_float4(near[p][2], far[p][2], near[q][2], far[q][2]);
+    o[3] = make_float4(__int_as_float(ref[p]), __int_as_float(ref[q]), __int_as_float(next), 0.0f);
 }
 
 __global__ void k_gather(const int32_t *__restrict__ order, int n, const float4 *__restrict__ s0,
@@ -219,13 +270,14 @@ cudaError_t build_bvh(BvhBuffers &sb, const vrad_triangle *h_tris,
     vrad_kd_triangle *d_prep = nullptr;
     int32_t *d_orig = nullptr;
     float4 *u0 = nullptr, *u1 = nullptr, *u2 = nullptr;
-    float *tri_box = nullptr, *d_bounds = nullptr, *leaf_box = nullptr;
-    int32_t *order = nullptr;
+    float *tri_box = nullptr, *d_bounds = nullptr;
+    float4 *d_tree = nullptr;
+    int32_t *order = nullptr, *d_parent = nullptr;
     int *d_stats = nullptr;
     int stats[4] = {0, 0, 0, 0};
     float bounds[7];
-    const int inner = n > 1 ? n - 1 : 1;
     SahTree tree;
+    std::vector<int32_t> parent;
 
     sb.release();
     if (n <= 0) return cudaSuccess;  // an empty subset: no BVH, never traversed
@@ -250,8 +302,6 @@ cudaError_t build_bvh(BvhBuffers &sb, const vrad_triangle *h_tris,
     VRAD_TRY(dev_alloc(&sb.tri0, sizeof(float4) * n));
     VRAD_TRY(dev_alloc(&sb.tri1, sizeof(float4) * n));
     VRAD_TRY(dev_alloc(&sb.tri2, sizeof(float4) * n));
-    VRAD_TRY(dev_alloc(&sb.nodes, sizeof(float4) * 4 * inner));
-    VRAD_TRY(dev_alloc(&leaf_box, sizeof(float) * 6 * n));
     VRAD_TRY(dev_alloc(&d_stats, sizeof(int) * 4));
     VRAD_TRY(cudaMemsetAsync(d_stats, 0, sizeof(int) * 4, stream));
 
@@ -262,19 +312,7 @@ cudaError_t build_bvh(BvhBuffers &sb, const vrad_triangle *h_tris,
     k_check_axes<<<blocks(n, 256), 256, 0, stream>>>(u2, n, d_stats);
     VRAD_TRY(cudaGetLastError());
 
-    if (n == 1) {
-        int32_t zero = 0;
-        VRAD_TRY(dev_alloc(&order, sizeof(int32_t)));
-        VRAD_TRY(cudaMemcpyAsync(order, &zero, sizeof(int32_t), cudaMemcpyHostToDevice, stream));
-        k_pad_single<<<1, 1, 0, stream>>>(tri_box, d_bounds, leaf_box);
-        k_emit_single<<<1, 1, 0, stream>>>(leaf_box, sb.nodes);
-        k_gather<<<1, 32, 0, stream>>>(order, 1, u0, u1, u2, sb.tri0, sb.tri1, sb.tri2);
-        VRAD_TRY(cudaGetLastError());
-        stats[0] = 1;
-        stats[1] = 1;
-        stats[2] = 1;
-        sb.depth = 1;
-    } else {
+    {
         // The boxes to the host, padded there as the walk's slab test needs
         // (a scene-relative margin), the SAH tree built, its nodes and leaf
         // order back.
@@ -288,17 +326,47 @@ cudaError_t build_bvh(BvhBuffers &sb, const vrad_triangle *h_tris,
                 box[6 * (size_t)i + a] -= pad;
                 box[6 * (size_t)i + 3 + a] += pad;
             }
-        build_sah(box.data(), n, tree);
+        if (n == 1) {
+            // A root whose second child is an empty box.
+            const int32_t leaf = leaf_ref(0, 1);
+            float r;
+            std::memcpy(&r, &leaf, 4);
+            tree.nodes = {make_float4(box[0], box[3], box[1], box[4]),
+                          make_float4(FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX),
+                          make_float4(box[2], box[5], FLT_MAX, -FLT_MAX), make_float4(r, r, 0.0f, 0.0f)};
+            tree.order = {0};
+            tree.inner = tree.leaves = tree.max_leaf = tree.depth = 1;
+        } else {
+            build_sah(box.data(), n, tree);
+        }
+        if (tree.depth > kStackDepth) {
+            err = cudaErrorInvalidValue;  // the builder's depth guard did not hold
+            goto fail;
+        }
+        parent.assign((size_t)tree.inner, -1);
+        for (int i = 0; i < tree.inner; i++)
+            for (int c = 0; c < 2; c++) {
+                int32_t r;
+                std::memcpy(&r, c ? &tree.nodes[4 * (size_t)i + 3].y : &tree.nodes[4 * (size_t)i + 3].x, 4);
+                if (r >= 0) parent[(size_t)r] = i;
+            }
         VRAD_TRY(dev_alloc(&order, sizeof(int32_t) * n));
+        VRAD_TRY(dev_alloc(&d_tree, sizeof(float4) * tree.nodes.size()));
+        VRAD_TRY(dev_alloc(&d_parent, sizeof(int32_t) * parent.size()));
+        VRAD_TRY(dev_alloc(&sb.nodes, sizeof(float4) * 16 * tree.nodes.size()));
         VRAD_TRY(cudaMemcpyAsync(order, tree.order.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, stream));
-        VRAD_TRY(cudaMemcpyAsync(sb.nodes, tree.nodes.data(), sizeof(float4) * tree.nodes.size(),
+        VRAD_TRY(cudaMemcpyAsync(d_tree, tree.nodes.data(), sizeof(float4) * tree.nodes.size(),
                                  cudaMemcpyHostToDevice, stream));
+        VRAD_TRY(cudaMemcpyAsync(d_parent, parent.data(), sizeof(int32_t) * parent.size(), cudaMemcpyHostToDevice,
+                                 stream));
+        k_octants<<<blocks(16 * tree.inner, 128), 128, 0, stream>>>(d_tree, d_parent, tree.inner, sb.nodes);
         k_gather<<<blocks(n, 256), 256, 0, stream>>>(order, n, u0, u1, u2, sb.tri0, sb.tri1, sb.tri2);
         VRAD_TRY(cudaGetLastError());
         stats[0] = tree.inner;
         stats[1] = tree.leaves;
         stats[2] = tree.max_leaf;
-        sb.depth = tree.depth > kStackDepth ? kStackDepth : tree.depth;  // deeper: walks report an overflow
+        sb.depth = tree.depth;
+        sb.inner = tree.inner;
     }
     {
         int dstats[4];
@@ -328,7 +396,7 @@ cudaError_t build_bvh(BvhBuffers &sb, const vrad_triangle *h_tris,
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, ev0, ev1);
         report->build_ms += ms;
-        report->device_bytes += (int64_t)n * 48 + (int64_t)inner * 64;
+        report->device_bytes += (int64_t)n * 48 + (int64_t)sb.inner * 16 * 64;
     }
 
 fail:
@@ -342,7 +410,8 @@ fail:
     dev_free(u2);
     dev_free(tri_box);
     dev_free(d_bounds);
-    dev_free(leaf_box);
+    dev_free(d_tree);
+    dev_free(d_parent);
     dev_free(order);
     dev_free(d_stats);
     if (ev0) cudaEventDestroy(ev0);
@@ -360,6 +429,7 @@ void BvhBuffers::release() {
     nodes = nullptr;
     ntris = 0;
     depth = 0;
+    inner = 0;
 }
 
 void SceneBuffers::release() {

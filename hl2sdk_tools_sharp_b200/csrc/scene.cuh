@@ -12,12 +12,13 @@ struct BvhBuffers {
     float4 *tri0 = nullptr;
     float4 *tri1 = nullptr;
     float4 *tri2 = nullptr;
-    float4 *nodes = nullptr;
+    float4 *nodes = nullptr;  // eight octants' copies, 2 inner nodes each
     int32_t ntris = 0;
     int32_t depth = 0;  // inner nodes on the longest root-to-leaf path
+    int32_t inner = 0;  // inner nodes
 
     void release();
-    DeviceBvh view() const { return DeviceBvh{tri0, tri1, tri2, nodes, ntris, depth}; }
+    DeviceBvh view() const { return DeviceBvh{tri0, tri1, tri2, nodes, ntris, depth, inner}; }
 };
 
 struct SceneBuffers {
@@ -53,7 +54,7 @@ cudaError_t build_bvh(BvhBuffers &bb, const vrad_triangle *h_tris,
 // Traversal launches (trace.cu).  d_bits is written as 32-bit words.
 cudaError_t launch_trace(const DeviceScene &scene, const vrad_ray *d_rays, int64_t n,
                          const TraceParams &p, uint32_t *d_bits, vrad_hit *d_hits,
-                         uint32_t *d_overflow, cudaStream_t stream);
+                         cudaStream_t stream);
 
 // Loads the visibility trace kernels' code on the current device (with lazy
 // module loading a kernel's code is otherwise placed on the device, which

@@ -188,8 +188,7 @@ __global__ void __launch_bounds__(BLOCK) k_resample(DeviceScene sc, DeviceWorld 
                                                     const int32_t *__restrict__ selected,
                                                     const float2 *__restrict__ origin_st, const int2 *__restrict__ wind,
                                                     const float4 *__restrict__ points, float4 *__restrict__ row_out,
-                                                    int32_t *__restrict__ row_bits, unsigned long long *counters,
-                                                    uint32_t *overflow) {
+                                                    int32_t *__restrict__ row_bits, unsigned long long *counters) {
     extern __shared__ int stack_mem[];  // sc.stack_depth() entries per thread
     int *stack = stack_mem + threadIdx.x;
     const int64_t tid = (int64_t)blockIdx.x * BLOCK + threadIdx.x;
@@ -213,11 +212,13 @@ __global__ void __launch_bounds__(BLOCK) k_resample(DeviceScene sc, DeviceWorld 
     const int code = __ldg(&rows[g]);
     float px = 0.0f, py = 0.0f, pz = 0.0f, nx = 0.0f, ny = 0.0f, nz = 1.0f;
     bool real = false, invalid = true;
+    int start = 0;
     if (code >= 0) {
         const int k = code / 5, row = code % 5;
         const int i = __ldg(&selected[k]);
         const int face = __float_as_int(__ldg(&w.sample_pos[i].w));
         const float4 fn = __ldg(&w.face_normal[face]);
+        start = w.start[i];  // the cell's points lie close to its sample
         nx = fn.x, ny = fn.y, nz = fn.z;
         const float4 o = __ldg(&fv.frames[5 * face]), ls = __ldg(&fv.frames[5 * face + 3]),
                      lt = __ldg(&fv.frames[5 * face + 4]);
@@ -251,9 +252,9 @@ __global__ void __launch_bounds__(BLOCK) k_resample(DeviceScene sc, DeviceWorld 
     bits |= __shfl_xor_sync(gmask, bits, 2);
     // A row whose four points all lie outside is not gathered.
     real = code >= 0 && bits != 0xFu;
-    unsigned long long vis_rays = 0, sky_rays = 0;
+    uint32_t vis_rays = 0, sky_rays = 0;  // one point's rays
     const float4 r = gather_point<BLOCK>(sc, w, cluster, px, py, pz, nx, ny, nz, real, gmask,
-                                         ambient ? kAmbientOnly : kDirectOnly, stack, overflow, counters, vis_rays,
+                                         ambient ? kAmbientOnly : kDirectOnly, start, stack, counters, vis_rays,
                                          sky_rays);
     if (code >= 0) {
         row_out[4 * (int64_t)code + l4] = r;
@@ -265,8 +266,8 @@ __global__ void __launch_bounds__(BLOCK) k_resample(DeviceScene sc, DeviceWorld 
         sky_rays += __shfl_xor_sync(kFull, sky_rays, o);
     }
     if (lane == 0) {
-        atomicAdd(&counters[0], vis_rays);
-        atomicAdd(&counters[1], sky_rays);
+        atomicAdd(&counters[0], (unsigned long long)vis_rays);
+        atomicAdd(&counters[1], (unsigned long long)sky_rays);
     }
 }
 
@@ -383,8 +384,7 @@ cudaError_t build_supersample(SupersampleBuffers &ss, const std::vector<vrad_fac
 }
 
 cudaError_t run_supersample(SupersampleBuffers &ss, const DeviceScene &scene, const DeviceWorld &world,
-                            const FinalView &fv, float4 *light, unsigned long long *counters, uint32_t *overflow,
-                            cudaStream_t s) {
+                            const FinalView &fv, float4 *light, unsigned long long *counters, cudaStream_t s) {
     ss.supersampled = 0;
     ss.passes_run = 0;
     ss.ms = 0.0f;
@@ -429,7 +429,7 @@ cudaError_t run_supersample(SupersampleBuffers &ss, const DeviceScene &scene, co
             k_resample<kSsBlock><<<grid_of(4 * (int64_t)g, kSsBlock), kSsBlock,
                                   sizeof(int) * scene.stack_depth() * kSsBlock, s>>>(
                 scene, world, fv, g, 2 * C + 1, ss.base, ss.rows, ss.selected, ss.origin_st, ss.wind, ss.points,
-                ss.row_out, ss.row_bits, counters, overflow);
+                ss.row_out, ss.row_bits, counters);
         if (e == cudaSuccess)
             k_ss_resolve<<<grid_of(nsel, 256), 256, 0, s>>>(nsel, ss.selected, ss.row_out, ss.row_bits, light,
                                                            ss.intensity, &counters[2]);

@@ -83,7 +83,6 @@ cudaError_t device_windings(SupersampleBuffers &ss, const RowStrips &rs, const F
 // The supersampling passes over `light` (the direct gather's output, one
 // float4 per sample), on `stream`.  Blocks once per pass.
 cudaError_t run_supersample(SupersampleBuffers &ss, const DeviceScene &scene, const DeviceWorld &world,
-                            const FinalView &fv, float4 *light, unsigned long long *counters, uint32_t *overflow,
-                            cudaStream_t stream);
+                            const FinalView &fv, float4 *light, unsigned long long *counters, cudaStream_t stream);
 
 }  // namespace vrad

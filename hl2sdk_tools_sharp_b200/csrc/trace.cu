@@ -27,8 +27,7 @@ namespace {
 template <int MODE>
 __global__ void __launch_bounds__(kBlock) k_trace(DeviceScene s, const vrad_ray *__restrict__ rays,
                                                   int64_t n, TraceParams p, uint32_t *__restrict__ bits,
-                                                  vrad_hit *__restrict__ hits,
-                                                  uint32_t *__restrict__ overflow) {
+                                                  vrad_hit *__restrict__ hits) {
     extern __shared__ int stack_mem[];  // sc.stack_depth() entries per thread
     int *stack = stack_mem + threadIdx.x;
     const int lane = threadIdx.x & 31;
@@ -54,8 +53,7 @@ __global__ void __launch_bounds__(kBlock) k_trace(DeviceScene s, const vrad_ray 
         r.nox = -r.ox * r.ix;
         r.noy = -r.oy * r.iy;
         r.noz = -r.oz * r.iz;
-        trace_ray<MODE>(s, r, p.tmin, reach, p.skip_id, stack, overflow, hit, best_t, best_orig,
-                        best_meta);
+        trace_ray<MODE>(s, r, p.tmin, reach, p.skip_id, 0, stack, hit, best_t, best_orig, best_meta);
     }
     if (MODE == kModeClosest) {
         if (i < n) {
@@ -79,20 +77,20 @@ __global__ void __launch_bounds__(kBlock) k_trace(DeviceScene s, const vrad_ray 
 
 cudaError_t launch_trace(const DeviceScene &scene, const vrad_ray *d_rays, int64_t n,
                          const TraceParams &p, uint32_t *d_bits, vrad_hit *d_hits,
-                         uint32_t *d_overflow, cudaStream_t stream) {
+                         cudaStream_t stream) {
     if (n <= 0) return cudaSuccess;
     const int64_t grid = (n + kBlock - 1) / kBlock;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
     const size_t smem = sizeof(int) * (size_t)scene.stack_depth() * kBlock;
     switch (p.mode) {
         case kModeAny:
-            k_trace<kModeAny><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits, d_hits, d_overflow);
+            k_trace<kModeAny><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits, d_hits);
             break;
         case kModeClosest:
-            k_trace<kModeClosest><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits, d_hits, d_overflow);
+            k_trace<kModeClosest><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits, d_hits);
             break;
         default:
-            k_trace<kModeSkyPass><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits, d_hits, d_overflow);
+            k_trace<kModeSkyPass><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits, d_hits);
             break;
     }
     return cudaGetLastError();

@@ -13,13 +13,23 @@
 //            meta = drop axis (bits 0-1) | sky (bit 2) | FCACHETRI flags << 8
 //   tri_id[orig]  int  the caller's id, read only for skip_id and outputs
 //
+// The nodes lie in eight copies, one per octant of a ray's direction (bit a
+// set: the direction's axis a is negative), 2 x `inner` nodes each; in a
+// copy every box is stored as the planes such a ray meets first (near) and
+// last (far), and child 0 is the child it meets first:
 //   node[k]  4 x float4 = 64 B, two child boxes and two child references:
-//            n0 = (c0.lo.x, c0.hi.x, c0.lo.y, c0.hi.y)
-//            n1 = (c1.lo.x, c1.hi.x, c1.lo.y, c1.hi.y)
-//            n2 = (c0.lo.z, c0.hi.z, c1.lo.z, c1.hi.z)
+//            n0 = child 0 (near.x, near.y, far.x, far.y)
+//            n1 = child 1 (near.x, near.y, far.x, far.y)
+//            n2 = (c0 near.z, c0 far.z, c1 near.z, c1 far.z)
 //            n3 = (ref0, ref1, -, -)
 //            ref >= 0 is an inner node; ref < 0 is a leaf, ~ref packing
 //            (first triangle << 3) | (count - 1), so a leaf holds 1..8.
+//            n3.z is -1.
+// Nodes inner .. 2 inner - 1 lead from a subtree up to the rest of the tree:
+// node inner + k has as its children the sibling of node k and the sibling
+// of k's parent (an empty box where there is none), and n3.z the node that
+// leads on from k's grandparent, -1 when the two children complete the
+// tree.
 #pragma once
 
 #include <cstdint>
@@ -40,7 +50,8 @@ struct DeviceBvh {
     const float4 *tri2;
     const float4 *nodes;
     int32_t ntris;  // 0: empty, never traversed
-    int32_t depth;  // stack entries a walk can need: the tree's depth in inner nodes
+    int32_t depth;  // inner nodes on the longest root-to-leaf path
+    int32_t inner;  // the tree's inner nodes: half of one octant's copy
 };
 
 struct DeviceScene {
@@ -48,10 +59,13 @@ struct DeviceScene {
     DeviceBvh sky;
     const int32_t *tri_id;
     // The traversal stack's entries per thread (kernels size their shared
-    // memory by it): the deeper tree's depth, at least 1, at most kStackDepth.
+    // memory by it).  A walk holds at most one entry per inner node of the
+    // path below the subtree it is in, and two more while it climbs: the
+    // deeper tree's depth plus two.  The build refuses a tree deeper than
+    // kStackDepth, so a walk needs no check of its own.
     __host__ __device__ int32_t stack_depth() const {
         const int32_t d = opaque.depth > sky.depth ? opaque.depth : sky.depth;
-        return d < 1 ? 1 : (d > kStackDepth ? kStackDepth : d);
+        return d + 2;
     }
 };
 

@@ -1,0 +1,56 @@
+"""The device's BVH walks against the oracle's brute force on triangle soups
+at the sizes where the tree's shape changes: one triangle (a root with an
+empty box), two, a leaf's most and one more, and trees of several levels;
+rays of every octant, along the axes (signed zeros in the direction) and in
+random directions, from inside and outside the soup.  Answers are the
+predicate's bits, so they are compared exactly."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from hl2sdk_tools_sharp_b200 import tracer as T
+
+pytestmark = pytest.mark.gpu
+
+
+def soup(n: int, sky: int, seed: int):
+    rng = np.random.default_rng([seed, n, sky])
+    c = rng.uniform(-500.0, 500.0, (n, 1, 3))
+    v = (c + rng.uniform(-120.0, 120.0, (n, 3, 3))).astype(np.float32).reshape(n, 9)
+    ids = np.full(n, 0x02000000, np.int32)
+    ids[:sky] = T.TRACE_ID_SKY
+    return v, ids
+
+
+def rays_for(seed: int, count: int = 4096):
+    rng = np.random.default_rng([seed, 7])
+    o = rng.uniform(-900.0, 900.0, (count, 3)).astype(np.float32)
+    d = rng.normal(size=(count, 3)).astype(np.float32)
+    axis = np.arange(count) % 8
+    for a in range(3):
+        only = axis == a
+        s = np.where(rng.uniform(size=only.sum()) < 0.5, 1.0, -1.0).astype(np.float32)
+        d[only] = np.where(rng.uniform(size=(only.sum(), 3)) < 0.5, np.float32(0.0), np.float32(-0.0))
+        d[only, a] = s
+    d *= rng.uniform(1.0, 1500.0, (count, 1)).astype(np.float32)
+    return T.make_rays(o, d, 1.0)
+
+
+@pytest.mark.parametrize("n,sky", [(1, 0), (1, 1), (2, 1), (8, 0), (9, 0), (33, 16), (1000, 100)])
+def test_soup_equals_brute_force(n, sky, oracle_mod):
+    O = oracle_mod
+    verts, ids = soup(n, sky, 11)
+    rays = rays_for(n)
+    tris = O.prepare_triangles(verts, ids)
+    flat = rays.view(np.float32).reshape(-1, 7)
+    with T.CudaRayTracer(T.make_triangles(verts, ids)) as tr:
+        for opts, flags in ((T.RayTraceOptions.stock_exact(), 0),
+                            (T.RayTraceOptions(0.0, sky_does_not_block=True), O.SKY_PASS)):
+            _, _, bits = O.brute_trace(tris, flat, flags=flags)
+            assert np.array_equal(tr.visibility(rays, opts), O.bits_to_bool(bits, len(rays)))
+        best, dist, _ = O.brute_trace(tris, flat, flags=O.CLOSEST)
+        got = tr.closest(rays)
+        assert np.array_equal(got["surface"], np.where(best >= 0, ids[np.maximum(best, 0)], -1))
+        hit = best >= 0
+        assert np.array_equal(got["fraction"][hit].view(np.uint32), dist[hit].astype(np.float32).view(np.uint32))
