@@ -9,9 +9,13 @@
 //                   surface order): lightmap offset, size, style slots,
 //                   sky flag, reflectivity, decoded tinted averages
 //   directions[i]   the 162 sample directions, float x 3
+//   by_octant[k]    float4: the directions grouped by octant, neighbouring
+//                   octants together, and each one's index in directions
+//   facing[j][q]    float2: for side j, the directions with a positive cosine
+//                   c with it, in table order: (index bits, c)
 //   power2n[k]      (float)(2^(k - 128) / 255), the RGBE decode table
-//   rad             scratch: each sample's 162 ray colours (float x 3),
-//                   for the samples of one chunk
+//   rad             scratch, for the samples of one chunk: rad[(3 i + c) *
+//                   rad_samples + s] = channel c of sample s's ray i
 #pragma once
 
 #include <cuda_runtime.h>
@@ -31,6 +35,10 @@ struct AmbientView {
     const vrad_ambient_face *faces;
     int32_t nfaces;
     const float *directions;
+    const float4 *by_octant;
+    const float2 *facing;       // 6 x 162
+    int32_t nfacing[kAmbientSides];
+    float inv[kAmbientSides];   // 1 / the cosines' sum in table order
     const float *power2n;
     float tan_theta;
     int32_t has_sky;
@@ -41,6 +49,8 @@ struct AmbientBuffers {
     uint8_t *light = nullptr;
     vrad_ambient_face *faces = nullptr;
     float *directions = nullptr;
+    float4 *by_octant = nullptr;
+    float2 *facing = nullptr;
     float *power2n = nullptr;
     float *rad = nullptr;          // chunk x 162 x 3
     int64_t rad_samples = 0;       // samples the scratch holds

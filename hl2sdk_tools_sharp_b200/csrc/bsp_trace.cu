@@ -25,9 +25,10 @@ namespace vrad {
 
 void BspBuffers::release() {
     for (void *p : {(void *)nodes, (void *)surfaces, (void *)node_faces, (void *)leaf_faces, (void *)leaf_run,
+                    (void *)node_surf, (void *)leaf_surf,
                     (void *)sky_points, (void *)sky_run})
         dev_free(p);
-    nodes = surfaces = sky_points = nullptr;
+    nodes = surfaces = sky_points = node_surf = leaf_surf = nullptr;
     node_faces = leaf_faces = nullptr;
     leaf_run = sky_run = nullptr;
     nnodes = nsurfaces = nleaves = 0;
@@ -43,8 +44,8 @@ __global__ void __launch_bounds__(kBspBlock) k_bsp_trace(DeviceBsp g, const vrad
                                                          float min_frac, vrad_hit *__restrict__ hits,
                                                          uint32_t *overflow) {
     const int64_t i = (int64_t)blockIdx.x * kBspBlock + threadIdx.x;
-    if (i >= n) return;
-    const float *r = reinterpret_cast<const float *>(rays + i);
+    const bool live = i < n;  // the walk takes whole warps
+    const float *r = reinterpret_cast<const float *>(rays + (live ? i : n - 1));
     bspwalk::Walk c;
     c.ox = __ldg(r + 0);
     c.oy = __ldg(r + 1);
@@ -57,7 +58,8 @@ __global__ void __launch_bounds__(kBspBlock) k_bsp_trace(DeviceBsp g, const vrad
     c.min_frac = min_frac;
     c.surface = -1;
     c.has_luxel = false;
-    const bool ok = bspwalk::walk(g, c);
+    const bool ok = bspwalk::walk(g, c, live);
+    if (!live) return;
     if (!ok) atomicOr(overflow, 1u);
     vrad_hit h;
     h.surface = ok ? c.surface : -1;
@@ -113,6 +115,15 @@ extern "C" int32_t vrad_bsp_upload(vrad_ctx *ctx, const vrad_bsp_geometry *b) {
     std::vector<float4> sky((size_t)(b->nsky_points ? b->nsky_points : 1));
     for (int32_t k = 0; k < b->nsky_points; k++)
         sky[(size_t)k] = make_float4(b->sky_points[3 * k], b->sky_points[3 * k + 1], b->sky_points[3 * k + 2], 0.0f);
+    // The faces' surfaces in each list's order.
+    const float4 *surfaces = reinterpret_cast<const float4 *>(b->surfaces);
+    auto in_order = [&](const int32_t *faces, int32_t n) {
+        std::vector<float4> out((size_t)4 * (n ? n : 1));
+        for (int32_t k = 0; k < n; k++) std::memcpy(&out[(size_t)4 * k], surfaces + 4 * (size_t)faces[k], 4 * sizeof(float4));
+        return out;
+    };
+    const std::vector<float4> node_surf = in_order(b->node_faces, b->nnode_faces),
+                              leaf_surf = in_order(b->leaf_faces, b->nleaf_faces);
     std::lock_guard<std::mutex> g(ctx->mu);
     vrad::settle_direct(ctx);
     cudaError_t e = cudaSetDevice(ctx->device);
@@ -128,6 +139,8 @@ extern "C" int32_t vrad_bsp_upload(vrad_ctx *ctx, const vrad_bsp_geometry *b) {
     if (e == cudaSuccess) e = up(&bb.surfaces, b->surfaces, sizeof(float) * 16 * (size_t)b->nsurfaces);
     if (e == cudaSuccess) e = up(&bb.node_faces, b->node_faces, sizeof(int32_t) * (size_t)b->nnode_faces);
     if (e == cudaSuccess) e = up(&bb.leaf_faces, b->leaf_faces, sizeof(int32_t) * (size_t)b->nleaf_faces);
+    if (e == cudaSuccess) e = up(&bb.node_surf, node_surf.data(), sizeof(float4) * 4 * (size_t)b->nnode_faces);
+    if (e == cudaSuccess) e = up(&bb.leaf_surf, leaf_surf.data(), sizeof(float4) * 4 * (size_t)b->nleaf_faces);
     if (e == cudaSuccess) e = up(&bb.leaf_run, leaf_run.data(), sizeof(int2) * (size_t)b->nleaves);
     if (e == cudaSuccess) e = up(&bb.sky_run, sky_run.data(), sizeof(int2) * (size_t)b->nsurfaces);
     if (e == cudaSuccess) e = up(&bb.sky_points, sky.data(), sizeof(float4) * (size_t)b->nsky_points);
@@ -139,7 +152,7 @@ extern "C" int32_t vrad_bsp_upload(vrad_ctx *ctx, const vrad_bsp_geometry *b) {
     bb.nnodes = b->nnodes;
     bb.nsurfaces = b->nsurfaces;
     bb.nleaves = b->nleaves;
-    bb.view = vrad::DeviceBsp{bb.nodes, bb.surfaces, bb.node_faces, bb.leaf_faces, bb.leaf_run, b->nleaves,
+    bb.view = vrad::DeviceBsp{bb.nodes, bb.surfaces, bb.node_faces, bb.leaf_faces, bb.node_surf, bb.leaf_surf, bb.leaf_run, b->nleaves,
                               bb.sky_points, bb.sky_run};
     bb.ready = true;
     return VRAD_OK;

@@ -9,6 +9,9 @@
 //                  (lightmap t, offset), (mins s, t, sizes s, t)
 //   node_faces     each node's candidate faces, lit then sky
 //   leaf_faces     each leaf's candidate faces; leaf_run[l] = (start, count)
+//   node_surf[q], leaf_surf[q]  surfaces[] of node_faces[q], leaf_faces[q]:
+//                  the walk streams a list's records without an index load
+//                  before each
 //   sky_points     the sky faces' windings (float4); sky_run[f] = (start, count)
 #pragma once
 
@@ -23,6 +26,8 @@ struct DeviceBsp {
     const float4 *surfaces;
     const int32_t *node_faces;
     const int32_t *leaf_faces;
+    const float4 *node_surf;
+    const float4 *leaf_surf;
     const int2 *leaf_run;
     int32_t nleaves;
     const float4 *sky_points;
@@ -34,6 +39,8 @@ struct BspBuffers {
     float4 *surfaces = nullptr;
     int32_t *node_faces = nullptr;
     int32_t *leaf_faces = nullptr;
+    float4 *node_surf = nullptr;
+    float4 *leaf_surf = nullptr;
     int2 *leaf_run = nullptr;
     float4 *sky_points = nullptr;
     int2 *sky_run = nullptr;

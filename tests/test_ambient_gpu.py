@@ -132,3 +132,20 @@ def test_device_form_and_errors(oracle_mod):
     with pytest.raises(RuntimeError):
         _oracle(oracle_mod, bad, r, pos)
 
+
+@pytest.mark.parametrize("n", [1, 31, 33, 256, 257, 2049])
+@pytest.mark.parametrize("spread", [8.0, 2000.0])
+def test_group_sizes_equal_the_oracle(n, spread, oracle_mod):
+    """Sample counts about the 32-sample groups and the few-sample limit;
+    points within one leaf's reach (a warp takes one direction of many
+    samples) and scattered over the map (many directions of one sample)."""
+    lumps = _lockdown_lumps()
+    rays, _, _, _ = F.lockdown_rays()
+    starts = rays[::162, :3]
+    rng = np.random.default_rng([n, int(spread)])
+    base = starts[:1] if spread < 100.0 else starts[rng.integers(0, len(starts), n)]
+    pos = (base + rng.uniform(-spread, spread, (n, 3)) * (1.0 if spread < 100.0 else 0.01)).astype(np.float32)
+    with A.CudaAmbientSampler(lumps) as s:
+        got = s.cubes(pos)
+    want = _oracle(oracle_mod, lumps, A.ambient_range(lumps, False), pos)
+    assert _same(got, want), int((got != want).any(axis=(1, 2)).sum())
