@@ -1,16 +1,15 @@
-// mlp.cu -- the learned warm start's network on the tensor cores: forward,
-// backward and Adam, each a kernel of this library.
+// mlp.cu -- the learned warm start's training on the tensor cores: the
+// gradient (forward, backward and weight gradients in one kernel) and Adam.
 //
 // Every matrix product is mma.sync.m16n8k16 with BF16 operands and FP32
 // accumulators.  The forward keeps a warp's 16 rows in registers through
 // all three layers: the accumulator fragments of one layer are, packed to
 // BF16, the A fragments of the next (the m16n8 C layout of two adjacent
-// n-tiles is the m16k16 A layout).  The backward does the same for the
-// activation gradients; the weight gradients are P^T Q reductions over the
-// rows, staged transposed in shared memory per 128-row tile, accumulated
-// in registers across tiles and added once per CTA.  Master weights and
-// Adam's moments are FP32; the BF16 operand copies are refreshed after
-// every step.
+// n-tiles is the m16k16 A layout); the backward does the same for the
+// activation gradients.  The weight gradients are P^T Q over a tile's rows,
+// both operands read transposed from the row-major tiles in shared memory
+// (ldmatrix.trans).  Master weights and Adam's moments are FP32; the BF16
+// operand copies are refreshed after every step.
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -50,56 +49,73 @@ __device__ __forceinline__ float bf_hi(uint32_t v) { return __uint_as_float(v & 
 
 __device__ __forceinline__ uint32_t ld32(const uint16_t *p) { return *reinterpret_cast<const uint32_t *>(p); }
 
-// The forward's weights in shared memory.
-struct FwdSmem {
-    uint16_t w1t[kMlpHidden * kMlpIn];
-    uint16_t w2t[kMlpHidden * kMlpHidden];
-    uint16_t w3t[kMlpOutPad * kMlpHidden];
+__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// Four 8 x 8 matrices of b16; lanes 8 i .. 8 i + 7 give matrix i's rows.
+__device__ __forceinline__ void ldsm4(uint32_t r[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t r[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+__device__ __forceinline__ void ldsm2_t(uint32_t r[2], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n"
+                 : "=r"(r[0]), "=r"(r[1])
+                 : "r"(addr)
+                 : "memory");
+}
+
+// Row strides in shared memory (b16): eight more than the row, so that the
+// eight rows of an ldmatrix fall into different banks.
+constexpr int kSx = kMlpIn + 8, kSh = kMlpHidden + 8;
+
+struct __align__(16) GradSmem {
+    uint16_t w1t[kMlpHidden * kSx];   // [128][32], output-major
+    uint16_t w2t[kMlpHidden * kSh];   // [128][128], output-major
+    uint16_t w3t[kMlpOutPad * kSh];   // [8][128], output-major
+    uint16_t w2[kMlpHidden * kSh];    // [128][128], input-major
+    uint16_t w3[kMlpHidden * kMlpOutPad];  // [128][8], input-major
+    uint16_t x[kTileRows * kSx];      // the tile's inputs
+    uint16_t h1[kTileRows * kSh];     // first hidden layer
+    uint16_t h2[kTileRows * kSh];     // second hidden layer, then dz1
+    uint16_t dz[kTileRows * kSh];     // dz2
+    uint16_t dy[kTileRows * kMlpOutPad];
     float b1[kMlpHidden], b2[kMlpHidden], b3[kMlpOutPad];
 };
+static_assert(sizeof(GradSmem) <= 227 * 1024, "one CTA's shared memory");
 
-__device__ void load_fwd(FwdSmem &s, const vrad_mlp &m) {
-    for (int i = threadIdx.x; i < kMlpHidden * kMlpIn / 2; i += blockDim.x)
-        reinterpret_cast<uint32_t *>(s.w1t)[i] = reinterpret_cast<const uint32_t *>(m.w1t)[i];
-    for (int i = threadIdx.x; i < kMlpHidden * kMlpHidden / 2; i += blockDim.x)
-        reinterpret_cast<uint32_t *>(s.w2t)[i] = reinterpret_cast<const uint32_t *>(m.w2t)[i];
-    for (int i = threadIdx.x; i < kMlpOutPad * kMlpHidden / 2; i += blockDim.x)
-        reinterpret_cast<uint32_t *>(s.w3t)[i] = reinterpret_cast<const uint32_t *>(m.w3t)[i];
-    for (int i = threadIdx.x; i < kMlpHidden; i += blockDim.x) {
-        s.b1[i] = m.master[kOffB1 + i];
-        s.b2[i] = m.master[kOffB2 + i];
-    }
-    if (threadIdx.x < kMlpOutPad) s.b3[threadIdx.x] = threadIdx.x < kMlpOut ? m.master[kOffB3 + threadIdx.x] : 0.0f;
+// acc[16 n-tiles] += A (16 x 16 KT) B, B from wt[n][k] with row stride S.
+template <int KT, int S>
+__device__ __forceinline__ void product(float acc[16][4], const uint32_t a[][4], const uint16_t *wt, int lane) {
+    const uint32_t at = smem_u32(wt + (lane & 7) * S + 8 * (lane >> 3));
+    // The sixteen accumulators' chains side by side.
+#pragma unroll
+    for (int kp = 0; kp < KT / 2; kp++)
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            uint32_t b[4];  // the n-tile's B fragments of two k-tiles
+            ldsm4(b, at + 2 * (8 * j * S + 32 * kp));
+            mma16816(acc[j], a[2 * kp], b);
+            mma16816(acc[j], a[2 * kp + 1], b + 2);
+        }
 }
 
-// One hidden layer: acc[16 n-tiles] = bias + A (16 x 16*KT) B, B from
-// output-major bf16 wt[n][k] with row stride K.
-template <int KT>
-__device__ __forceinline__ void layer(float acc[16][4], const uint32_t a[][4], const uint16_t *wt, const float *bias,
-                                      int g, int t) {
-    constexpr int K = 16 * KT;
+__device__ __forceinline__ void set_bias(float acc[16][4], const float *bias, int t) {
 #pragma unroll
     for (int j = 0; j < 16; j++) {
-        const float b0 = bias[8 * j + 2 * t], b1 = bias[8 * j + 2 * t + 1];
-        acc[j][0] = b0;
-        acc[j][1] = b1;
-        acc[j][2] = b0;
-        acc[j][3] = b1;
-#pragma unroll
-        for (int kt = 0; kt < KT; kt++) {
-            const uint16_t *row = wt + (8 * j + g) * K + 16 * kt + 2 * t;
-            const uint32_t b[2] = {ld32(row), ld32(row + 8)};
-            mma16816(acc[j], a[kt], b);
-        }
+        acc[j][0] = acc[j][2] = bias[8 * j + 2 * t];
+        acc[j][1] = acc[j][3] = bias[8 * j + 2 * t + 1];
     }
 }
 
-// ReLU, then the accumulators as the next layer's A fragments.
-__device__ __forceinline__ void relu_pack(float acc[16][4], uint32_t a[8][4]) {
-#pragma unroll
-    for (int j = 0; j < 16; j++)
-#pragma unroll
-        for (int q = 0; q < 4; q++) acc[j][q] = acc[j][q] > 0.0f ? acc[j][q] : 0.0f;
+// The accumulators as the next product's A fragments.
+__device__ __forceinline__ void pack(const float acc[16][4], uint32_t a[8][4]) {
 #pragma unroll
     for (int kt = 0; kt < 8; kt++) {
         a[kt][0] = pack2(acc[2 * kt][0], acc[2 * kt][1]);
@@ -109,222 +125,239 @@ __device__ __forceinline__ void relu_pack(float acc[16][4], uint32_t a[8][4]) {
     }
 }
 
-// Stores a warp's 16 x 128 bf16 activations from its A fragments.
-__device__ __forceinline__ void store_act(uint16_t *dst, const uint32_t a[8][4], int64_t r0, int64_t n, int g, int t) {
-    const int64_t ra = r0 + g, rb = r0 + g + 8;
+// ReLU, then pack; m = which of the 64 packed activations are above zero.
+__device__ __forceinline__ void relu_pack(float acc[16][4], uint32_t a[8][4], uint32_t m[2]) {
+#pragma unroll
+    for (int j = 0; j < 16; j++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) acc[j][q] = acc[j][q] > 0.0f ? acc[j][q] : 0.0f;
+    pack(acc, a);
+    m[0] = m[1] = 0;
+#pragma unroll
+    for (int kt = 0; kt < 8; kt++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int bit = 8 * (kt & 3) + 2 * q;
+            if (bf_lo(a[kt][q]) > 0.0f) m[kt >> 2] |= 1u << bit;
+            if (bf_hi(a[kt][q]) > 0.0f) m[kt >> 2] |= 2u << bit;
+        }
+}
+
+// Zero where the activation was not above zero, then pack.
+__device__ __forceinline__ void mask_pack(float acc[16][4], const uint32_t m[2], uint32_t a[8][4]) {
+#pragma unroll
+    for (int kt = 0; kt < 8; kt++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int bit = 8 * (kt & 3) + 2 * q, j = 2 * kt + (q >> 1), e = 2 * (q & 1);
+            if (!((m[kt >> 2] >> bit) & 1u)) acc[j][e] = 0.0f;
+            if (!((m[kt >> 2] >> bit) & 2u)) acc[j][e + 1] = 0.0f;
+        }
+    pack(acc, a);
+}
+
+// A warp's 16 x 128 tile from its A fragments into shared memory rows.
+__device__ __forceinline__ void store_tile(uint16_t *rows, const uint32_t a[8][4], int g, int t) {
+    uint16_t *p = rows + g * kSh + 2 * t;
 #pragma unroll
     for (int kt = 0; kt < 8; kt++) {
-        if (ra < n) {
-            *reinterpret_cast<uint32_t *>(dst + ra * kMlpHidden + 16 * kt + 2 * t) = a[kt][0];
-            *reinterpret_cast<uint32_t *>(dst + ra * kMlpHidden + 16 * kt + 8 + 2 * t) = a[kt][2];
-        }
-        if (rb < n) {
-            *reinterpret_cast<uint32_t *>(dst + rb * kMlpHidden + 16 * kt + 2 * t) = a[kt][1];
-            *reinterpret_cast<uint32_t *>(dst + rb * kMlpHidden + 16 * kt + 8 + 2 * t) = a[kt][3];
-        }
+        *reinterpret_cast<uint32_t *>(p + 16 * kt) = a[kt][0];
+        *reinterpret_cast<uint32_t *>(p + 8 * kSh + 16 * kt) = a[kt][1];
+        *reinterpret_cast<uint32_t *>(p + 16 * kt + 8) = a[kt][2];
+        *reinterpret_cast<uint32_t *>(p + 8 * kSh + 16 * kt + 8) = a[kt][3];
     }
 }
 
-__global__ void __launch_bounds__(kMlpThreads) k_mlp_forward(vrad_mlp m, const uint16_t *__restrict__ x, int64_t n,
-                                                             float *__restrict__ y, uint16_t *__restrict__ h1,
-                                                             uint16_t *__restrict__ h2) {
+// Adds a weight gradient's m16n8 tile at row m0, column n0 of grad.
+__device__ __forceinline__ void add_tile(float *grad, int stride, int ncols, int m0, int n0, const float c[4], int g,
+                                         int t) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int col = n0 + 2 * t + (q & 1);
+        if (col < ncols) atomicAdd(&grad[(m0 + g + 8 * (q >> 1)) * stride + col], c[q]);
+    }
+}
+
+// The mean squared error's gradient over n rows: m.grad += it, m.loss += the
+// loss.  A CTA of 8 warps takes tiles of 128 rows, 16 rows a warp for the
+// layers:
+//   forward, h1 and h2 into shared memory; dy = 2 (y - target) / 3n;
+//   dz2 = (dy W3^T) * [h2 > 0], dz1 = (dz2 W2^T) * [h1 > 0];
+// then the products over the tile's rows, split by output rows among the
+// warps and kept in registers from tile to tile: dW3 = h2^T dy, dW2 = h1^T
+// dz2, dW1 = x^T dz1, and the bias gradients as the same products with ones
+// for the left operand.
+// A minibatch is a few hundred tiles, so what counts is one tile's time and
+// what it sends to memory: nothing but x and the targets in, and one atomic
+// add per parameter and CTA out.  A tile takes 9.5 us, which is the rate of
+// mma.sync on this chip (sixteen warps, two to a row group, take as long),
+// and 32,768 rows 35 us.  As five kernels with the activations and their
+// gradients in HBM, shared memory operands read with up to eight-way bank
+// conflicts and transposed by 2-byte stores, they took 145 us.
+__global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_gradient(vrad_mlp m, const uint16_t *__restrict__ x,
+                                                                 const float *__restrict__ target, int64_t n, float inv) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    FwdSmem &s = *reinterpret_cast<FwdSmem *>(smem_raw);
-    load_fwd(s, m);
+    GradSmem &s = *reinterpret_cast<GradSmem *>(smem_raw);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    // The weights, eight at a time.
+    auto copy = [&](uint16_t *dst, const uint16_t *src, int rows, int cols, int stride) {
+        for (int i = tid; i < rows * cols / 8; i += kMlpThreads) {
+            const int r = i / (cols / 8), c = 8 * (i % (cols / 8));
+            *reinterpret_cast<uint4 *>(dst + r * stride + c) = *reinterpret_cast<const uint4 *>(src + r * cols + c);
+        }
+    };
+    copy(s.w1t, m.w1t, kMlpHidden, kMlpIn, kSx);
+    copy(s.w2t, m.w2t, kMlpHidden, kMlpHidden, kSh);
+    copy(s.w3t, m.w3t, kMlpOutPad, kMlpHidden, kSh);
+    copy(s.w2, m.w2, kMlpHidden, kMlpHidden, kSh);
+    copy(s.w3, m.w3, kMlpHidden, kMlpOutPad, kMlpOutPad);
+    for (int i = tid; i < kMlpHidden; i += kMlpThreads) {
+        s.b1[i] = m.master[kOffB1 + i];
+        s.b2[i] = m.master[kOffB2 + i];
+    }
+    if (tid < kMlpOutPad) s.b3[tid] = tid < kMlpOut ? m.master[kOffB3 + tid] : 0.0f;
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+
+    float g2[16][4] = {}, g1[4][4] = {}, g3[4] = {}, gb2[2][4] = {}, gb1[2][4] = {}, gb3[4] = {};
+    const uint32_t ones[4] = {0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u};
+    float loss = 0.0f;
+    uint16_t *xs = s.x + 16 * warp * kSx, *h1 = s.h1 + 16 * warp * kSh, *h2 = s.h2 + 16 * warp * kSh,
+             *dz = s.dz + 16 * warp * kSh, *dy = s.dy + 16 * warp * kMlpOutPad;
     for (int64_t tile = blockIdx.x; tile * kTileRows < n; tile += gridDim.x) {
-        const int64_t r0 = tile * kTileRows + 16 * warp;
-        if (r0 >= n) continue;
-        const int64_t ra = r0 + g, rb = r0 + g + 8;
-        uint32_t ax[2][4];
+        const int64_t ra = tile * kTileRows + 16 * warp + g, rb = ra + 8;
+        float acc[16][4];
+        uint32_t a[8][4], m1[2], m2[2];
 #pragma unroll
         for (int kt = 0; kt < 2; kt++) {
-            ax[kt][0] = ra < n ? ld32(x + ra * kMlpIn + 16 * kt + 2 * t) : 0u;
-            ax[kt][1] = rb < n ? ld32(x + rb * kMlpIn + 16 * kt + 2 * t) : 0u;
-            ax[kt][2] = ra < n ? ld32(x + ra * kMlpIn + 16 * kt + 8 + 2 * t) : 0u;
-            ax[kt][3] = rb < n ? ld32(x + rb * kMlpIn + 16 * kt + 8 + 2 * t) : 0u;
+            a[kt][0] = ra < n ? ld32(x + ra * kMlpIn + 16 * kt + 2 * t) : 0u;
+            a[kt][1] = rb < n ? ld32(x + rb * kMlpIn + 16 * kt + 2 * t) : 0u;
+            a[kt][2] = ra < n ? ld32(x + ra * kMlpIn + 16 * kt + 8 + 2 * t) : 0u;
+            a[kt][3] = rb < n ? ld32(x + rb * kMlpIn + 16 * kt + 8 + 2 * t) : 0u;
         }
-        float acc[16][4];
-        uint32_t ah[8][4];
-        layer<2>(acc, ax, s.w1t, s.b1, g, t);
-        relu_pack(acc, ah);
-        if (h1) store_act(h1, ah, r0, n, g, t);
-        layer<8>(acc, ah, s.w2t, s.b2, g, t);
-        relu_pack(acc, ah);
-        if (h2) store_act(h2, ah, r0, n, g, t);
+        // This row pair's targets, loaded ahead of the layers.
+        float want[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int c = 2 * t + (q & 1);
+            const int64_t r = q < 2 ? ra : rb;
+            want[q] = c < kMlpOut && r < n ? __ldg(&target[r * kMlpOut + c]) : 0.0f;
+        }
+#pragma unroll
+        for (int kt = 0; kt < 2; kt++) {
+            *reinterpret_cast<uint32_t *>(xs + g * kSx + 16 * kt + 2 * t) = a[kt][0];
+            *reinterpret_cast<uint32_t *>(xs + (g + 8) * kSx + 16 * kt + 2 * t) = a[kt][1];
+            *reinterpret_cast<uint32_t *>(xs + g * kSx + 16 * kt + 8 + 2 * t) = a[kt][2];
+            *reinterpret_cast<uint32_t *>(xs + (g + 8) * kSx + 16 * kt + 8 + 2 * t) = a[kt][3];
+        }
+        set_bias(acc, s.b1, t);
+        product<2, kSx>(acc, a, s.w1t, lane);
+        relu_pack(acc, a, m1);
+        store_tile(h1, a, g, t);
+        set_bias(acc, s.b2, t);
+        product<8, kSh>(acc, a, s.w2t, lane);
+        relu_pack(acc, a, m2);
+        store_tile(h2, a, g, t);
         float out[4] = {s.b3[2 * t], s.b3[2 * t + 1], s.b3[2 * t], s.b3[2 * t + 1]};
 #pragma unroll
-        for (int kt = 0; kt < 8; kt++) {
-            const uint16_t *row = s.w3t + g * kMlpHidden + 16 * kt + 2 * t;
-            const uint32_t b[2] = {ld32(row), ld32(row + 8)};
-            mma16816(out, ah[kt], b);
+        for (int kp = 0; kp < 4; kp++) {
+            uint32_t b[4];
+            ldsm4(b, smem_u32(s.w3t + (lane & 7) * kSh + 8 * (lane >> 3) + 32 * kp));
+            mma16816(out, a[2 * kp], b);
+            mma16816(out, a[2 * kp + 1], b + 2);
         }
-        // Output columns 2t, 2t + 1: the first three are the network's.
-        for (int q = 0; q < 2; q++) {
-            const int c = 2 * t + q;
-            if (c >= kMlpOut) continue;
-            if (ra < n) y[ra * kMlpOut + c] = out[q];
-            if (rb < n) y[rb * kMlpOut + c] = out[2 + q];
-        }
-    }
-}
-
-// The activation gradients of the mean squared error over n rows and three
-// outputs: dy = 2 (y - target) / 3n, dz2 = (dy W3^T) * [h2 > 0],
-// dz1 = (dz2 W2^T) * [h1 > 0], each stored as the bf16 the weight
-// gradients read; the loss summed into *loss.
-struct BwdSmem {
-    uint16_t w2[kMlpHidden * kMlpHidden];  // input-major
-    uint16_t w3[kMlpHidden * kMlpOutPad];  // input-major
-};
-
-__global__ void __launch_bounds__(kMlpThreads) k_mlp_backward(vrad_mlp m, const float *__restrict__ target, int64_t n,
-                                                              float inv) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    BwdSmem &s = *reinterpret_cast<BwdSmem *>(smem_raw);
-    for (int i = threadIdx.x; i < kMlpHidden * kMlpHidden / 2; i += blockDim.x)
-        reinterpret_cast<uint32_t *>(s.w2)[i] = reinterpret_cast<const uint32_t *>(m.w2)[i];
-    for (int i = threadIdx.x; i < kMlpHidden * kMlpOutPad / 2; i += blockDim.x)
-        reinterpret_cast<uint32_t *>(s.w3)[i] = reinterpret_cast<const uint32_t *>(m.w3)[i];
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    float loss = 0.0f;
-    for (int64_t tile = blockIdx.x; tile * kTileRows < n; tile += gridDim.x) {
-        const int64_t r0 = tile * kTileRows + 16 * warp;
-        if (r0 >= n) continue;
-        const int64_t ra = r0 + g, rb = r0 + g + 8;
-        // dy for columns 2t, 2t + 1 of rows ra, rb.
         float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        for (int q = 0; q < 2; q++) {
-            const int c = 2 * t + q;
-            if (c >= kMlpOut) continue;
-            if (ra < n) {
-                const float e = m.y[ra * kMlpOut + c] - target[ra * kMlpOut + c];
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (2 * t + (q & 1) < kMlpOut && (q < 2 ? ra : rb) < n) {
+                const float e = out[q] - want[q];
                 loss += e * e;
                 d[q] = 2.0f * e * inv;
             }
-            if (rb < n) {
-                const float e = m.y[rb * kMlpOut + c] - target[rb * kMlpOut + c];
-                loss += e * e;
-                d[2 + q] = 2.0f * e * inv;
-            }
-        }
-        const uint32_t dya = pack2(d[0], d[1]), dyb = pack2(d[2], d[3]);
-        if (ra < n) *reinterpret_cast<uint32_t *>(m.dy + ra * kMlpOutPad + 2 * t) = dya;
-        if (rb < n) *reinterpret_cast<uint32_t *>(m.dy + rb * kMlpOutPad + 2 * t) = dyb;
+        const uint32_t ady[4] = {pack2(d[0], d[1]), pack2(d[2], d[3]), 0u, 0u};
+        *reinterpret_cast<uint32_t *>(dy + g * kMlpOutPad + 2 * t) = ady[0];
+        *reinterpret_cast<uint32_t *>(dy + (g + 8) * kMlpOutPad + 2 * t) = ady[1];
         // dh2 = dy (16 x 8, k padded to 16 with zeros) W3^T.
-        const uint32_t ady[4] = {dya, dyb, 0u, 0u};
-        float acc[16][4];
-        uint32_t az[8][4];
 #pragma unroll
         for (int j = 0; j < 16; j++) {
             acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
             const uint32_t b[2] = {ld32(s.w3 + (8 * j + g) * kMlpOutPad + 2 * t), 0u};
             mma16816(acc[j], ady, b);
         }
-        // Mask by h2 > 0, pack, store dz2.
-        auto mask_pack = [&](const uint16_t *h, uint16_t *dz) {
-#pragma unroll
-            for (int j = 0; j < 16; j++) {
-                const uint32_t ha = ra < n ? ld32(h + ra * kMlpHidden + 8 * j + 2 * t) : 0u;
-                const uint32_t hb = rb < n ? ld32(h + rb * kMlpHidden + 8 * j + 2 * t) : 0u;
-                if (!(bf_lo(ha) > 0.0f)) acc[j][0] = 0.0f;
-                if (!(bf_hi(ha) > 0.0f)) acc[j][1] = 0.0f;
-                if (!(bf_lo(hb) > 0.0f)) acc[j][2] = 0.0f;
-                if (!(bf_hi(hb) > 0.0f)) acc[j][3] = 0.0f;
-            }
-#pragma unroll
-            for (int kt = 0; kt < 8; kt++) {
-                az[kt][0] = pack2(acc[2 * kt][0], acc[2 * kt][1]);
-                az[kt][1] = pack2(acc[2 * kt][2], acc[2 * kt][3]);
-                az[kt][2] = pack2(acc[2 * kt + 1][0], acc[2 * kt + 1][1]);
-                az[kt][3] = pack2(acc[2 * kt + 1][2], acc[2 * kt + 1][3]);
-            }
-            store_act(dz, az, r0, n, g, t);
-        };
-        mask_pack(m.h2, m.dz2);
+        mask_pack(acc, m2, a);
+        store_tile(dz, a, g, t);
         // dh1 = dz2 W2^T.
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-            acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+        for (int j = 0; j < 16; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+        product<8, kSh>(acc, a, s.w2, lane);
+        mask_pack(acc, m1, a);
+        __syncthreads();  // every warp's x, h1, h2, dy, dz2
+        // dW3 and dW2: this warp's 16 input rows.  A (m16 k16) of P^T from
+        // P's rows k: matrices (m, k) = (0, 0), (8, 0), (0, 8), (8, 8).
+        const int ka = (lane & 7) + 8 * (lane >> 4), ma = 16 * warp + 8 * ((lane >> 3) & 1);
+        // B (k16 n8) of two n-tiles: (k, n) = (0, 0), (8, 0), (0, 8), (8, 8).
+        const int kb = (lane & 7) + 8 * ((lane >> 3) & 1), nb = 8 * (lane >> 4);
 #pragma unroll
-            for (int kt = 0; kt < 8; kt++) {
-                const uint16_t *row = s.w2 + (8 * j + g) * kMlpHidden + 16 * kt + 2 * t;
-                const uint32_t b[2] = {ld32(row), ld32(row + 8)};
-                mma16816(acc[j], az[kt], b);
+        for (int kt = 0; kt < 8; kt++) {
+            uint32_t p[4], q[4];
+            ldsm4_t(p, smem_u32(s.h2 + (16 * kt + ka) * kSh + ma));
+            ldsm2_t(q, smem_u32(s.dy + (16 * kt + (lane & 15)) * kMlpOutPad));
+            mma16816(g3, p, q);
+            if (warp == 0) mma16816(gb3, ones, q);
+            ldsm4_t(p, smem_u32(s.h1 + (16 * kt + ka) * kSh + ma));
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                ldsm4_t(q, smem_u32(s.dz + (16 * kt + kb) * kSh + 16 * j + nb));
+                mma16816(g2[2 * j], p, q);
+                mma16816(g2[2 * j + 1], p, q + 2);
+                if (j == warp) {
+                    mma16816(gb2[0], ones, q);
+                    mma16816(gb2[1], ones, q + 2);
+                }
             }
         }
-        mask_pack(m.h1, m.dz1);
+        __syncthreads();  // h2 is read
+        store_tile(h2, a, g, t);  // dz1
+        __syncthreads();
+        // dW1: input rows 16 (warp & 1) .., columns 32 (warp >> 1) ..; db1:
+        // half of those columns each.
+#pragma unroll
+        for (int kt = 0; kt < 8; kt++) {
+            uint32_t p[4], q[4];
+            ldsm4_t(p, smem_u32(s.x + (16 * kt + ka) * kSx + 16 * (warp & 1) + 8 * ((lane >> 3) & 1)));
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                ldsm4_t(q, smem_u32(s.h2 + (16 * kt + kb) * kSh + 32 * (warp >> 1) + 16 * j + nb));
+                mma16816(g1[2 * j], p, q);
+                mma16816(g1[2 * j + 1], p, q + 2);
+                if (j == (warp & 1)) {
+                    mma16816(gb1[0], ones, q);
+                    mma16816(gb1[1], ones, q + 2);
+                }
+            }
+        }
+        __syncthreads();  // x and dz1 are read
+    }
+    // The CTA's sums.
+#pragma unroll
+    for (int j = 0; j < 16; j++) add_tile(m.grad + kOffW2, kMlpHidden, kMlpHidden, 16 * warp, 8 * j, g2[j], g, t);
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        add_tile(m.grad, kMlpHidden, kMlpHidden, 16 * (warp & 1), 32 * (warp >> 1) + 8 * j, g1[j], g, t);
+    add_tile(m.grad + kOffW3, kMlpOut, kMlpOut, 16 * warp, 0, g3, g, t);
+    if (g == 0) {  // every row of a product with ones is the column sums
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                atomicAdd(&m.grad[kOffB2 + 16 * warp + 8 * j + 2 * t + q], gb2[j][q]);
+                atomicAdd(&m.grad[kOffB1 + 32 * (warp >> 1) + 16 * (warp & 1) + 8 * j + 2 * t + q], gb1[j][q]);
+            }
+        if (warp == 0)
+            for (int q = 0; q < 2; q++)
+                if (2 * t + q < kMlpOut) atomicAdd(&m.grad[kOffB3 + 2 * t + q], gb3[q]);
     }
     for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
     if (lane == 0) atomicAdd(m.loss, loss * inv);
-}
-
-// grad[M][N] += P^T Q over n rows (P [n][M], Q [n][N], bf16), and
-// bias[N] += the column sums of Q, for one weight matrix.
-template <int M, int N>
-__global__ void __launch_bounds__(kMlpThreads) k_mlp_wgrad(const uint16_t *__restrict__ p, const uint16_t *__restrict__ q,
-                                                           int64_t n, int qstride, int ncols, float *__restrict__ grad,
-                                                           int gstride, float *__restrict__ bias) {
-    constexpr int R = kTileRows;       // rows per tile (the k extent)
-    constexpr int RS = R + 8;          // padded row of the transposed tiles
-    constexpr int TILES = (M / 16) * (N / 8);
-    constexpr int PER = (TILES + kMlpWarps - 1) / kMlpWarps;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    uint16_t *pt = reinterpret_cast<uint16_t *>(smem_raw);  // [M][RS]
-    uint16_t *qt = pt + M * RS;                             // [N][RS]
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    float acc[PER][4];
-#pragma unroll
-    for (int i = 0; i < PER; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
-    float colsum = 0.0f;  // thread c < N: column c's sum
-    for (int64_t tile = blockIdx.x; tile * R < n; tile += gridDim.x) {
-        const int64_t r0 = tile * R;
-        __syncthreads();
-        for (int i = threadIdx.x; i < R * M; i += blockDim.x) {
-            const int r = i / M, c = i % M;
-            pt[c * RS + r] = r0 + r < n ? p[(r0 + r) * M + c] : (uint16_t)0;
-        }
-        for (int i = threadIdx.x; i < R * N; i += blockDim.x) {
-            const int r = i / N, c = i % N;
-            qt[c * RS + r] = (r0 + r < n && c < ncols) ? q[(r0 + r) * qstride + c] : (uint16_t)0;
-        }
-        __syncthreads();
-        if (bias && threadIdx.x < N)
-            for (int r = 0; r < R; r++) colsum += __uint_as_float((uint32_t)qt[threadIdx.x * RS + r] << 16);
-#pragma unroll
-        for (int i = 0; i < PER; i++) {
-            const int tileid = warp + kMlpWarps * i;
-            if (tileid >= TILES) break;
-            const int mt = tileid / (N / 8), nt = tileid % (N / 8);
-#pragma unroll
-            for (int kt = 0; kt < R / 16; kt++) {
-                const uint16_t *a0 = pt + (16 * mt + g) * RS + 16 * kt + 2 * t;
-                const uint16_t *a1 = pt + (16 * mt + g + 8) * RS + 16 * kt + 2 * t;
-                const uint32_t a[4] = {ld32(a0), ld32(a1), ld32(a0 + 8), ld32(a1 + 8)};
-                const uint16_t *bq = qt + (8 * nt + g) * RS + 16 * kt + 2 * t;
-                const uint32_t b[2] = {ld32(bq), ld32(bq + 8)};
-                mma16816(acc[i], a, b);
-            }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < PER; i++) {
-        const int tileid = warp + kMlpWarps * i;
-        if (tileid >= TILES) break;
-        const int mt = tileid / (N / 8), nt = tileid % (N / 8);
-        const int m0 = 16 * mt + g, n0 = 8 * nt + 2 * t;
-        if (n0 < ncols) {
-            atomicAdd(&grad[m0 * gstride + n0], acc[i][0]);
-            atomicAdd(&grad[(m0 + 8) * gstride + n0], acc[i][2]);
-        }
-        if (n0 + 1 < ncols) {
-            atomicAdd(&grad[m0 * gstride + n0 + 1], acc[i][1]);
-            atomicAdd(&grad[(m0 + 8) * gstride + n0 + 1], acc[i][3]);
-        }
-    }
-    if (bias && threadIdx.x < ncols) atomicAdd(&bias[threadIdx.x], colsum);
 }
 
 // The BF16 operand copies of the master weights.
@@ -361,44 +394,14 @@ __global__ void k_mlp_adam(vrad_mlp m, float lr, float c1, float c2) {
     m.master[i] -= lr * (mm / c1) / (sqrtf(vv / c2) + 1e-8f);
 }
 
-unsigned blocks_for(int64_t n) {
-    const int64_t tiles = (n + kTileRows - 1) / kTileRows;
-    return (unsigned)(tiles < 4 * 148 ? (tiles > 0 ? tiles : 1) : 4 * 148);
-}
-
-cudaError_t grow(vrad_mlp &m, int64_t n) {
-    if (n <= m.scratch_rows) return cudaSuccess;
-    for (void *p : {(void *)m.h1, (void *)m.h2, (void *)m.dz1, (void *)m.dz2, (void *)m.dy, (void *)m.y}) cudaFree(p);
-    m.h1 = m.h2 = m.dz1 = m.dz2 = m.dy = nullptr;
-    m.y = nullptr;
-    m.scratch_rows = 0;
-    cudaError_t e = cudaMalloc(&m.h1, sizeof(uint16_t) * kMlpHidden * n);
-    if (e == cudaSuccess) e = cudaMalloc(&m.h2, sizeof(uint16_t) * kMlpHidden * n);
-    if (e == cudaSuccess) e = cudaMalloc(&m.dz1, sizeof(uint16_t) * kMlpHidden * n);
-    if (e == cudaSuccess) e = cudaMalloc(&m.dz2, sizeof(uint16_t) * kMlpHidden * n);
-    if (e == cudaSuccess) e = cudaMalloc(&m.dy, sizeof(uint16_t) * kMlpOutPad * n);
-    if (e == cudaSuccess) e = cudaMalloc(&m.y, sizeof(float) * kMlpOut * n);
-    if (e == cudaSuccess) m.scratch_rows = n;
-    return e;
-}
-
-// The MSE gradient into m.grad (and the loss into m.loss), on `s`.
+// The MSE gradient into m.grad (and the loss into m.loss, which lies just
+// behind it), on `s`.
 cudaError_t gradient(vrad_mlp &m, const uint16_t *x, const float *target, int64_t n, cudaStream_t s) {
-    cudaError_t e = grow(m, n);
-    if (e == cudaSuccess) e = cudaMemsetAsync(m.grad, 0, sizeof(float) * kMlpParams, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(m.loss, 0, sizeof(float), s);
+    cudaError_t e = cudaMemsetAsync(m.grad, 0, sizeof(float) * (kMlpParams + 1), s);
     if (e != cudaSuccess || n == 0) return e;
-    const unsigned nb = blocks_for(n);
-    k_mlp_forward<<<nb, kMlpThreads, sizeof(FwdSmem), s>>>(m, x, n, m.y, m.h1, m.h2);
-    k_mlp_backward<<<nb, kMlpThreads, sizeof(BwdSmem), s>>>(m, target, n, 1.0f / (3.0f * (float)n));
-    constexpr int RS = kTileRows + 8;
-    // dW3 = h2^T dy (+ db3), dW2 = h1^T dz2 (+ db2), dW1 = x^T dz1 (+ db1).
-    k_mlp_wgrad<kMlpHidden, kMlpOutPad><<<nb, kMlpThreads, sizeof(uint16_t) * RS * (kMlpHidden + kMlpOutPad), s>>>(
-        m.h2, m.dy, n, kMlpOutPad, kMlpOut, m.grad + kOffW3, kMlpOut, m.grad + kOffB3);
-    k_mlp_wgrad<kMlpHidden, kMlpHidden><<<nb, kMlpThreads, sizeof(uint16_t) * RS * (2 * kMlpHidden), s>>>(
-        m.h1, m.dz2, n, kMlpHidden, kMlpHidden, m.grad + kOffW2, kMlpHidden, m.grad + kOffB2);
-    k_mlp_wgrad<kMlpIn, kMlpHidden><<<nb, kMlpThreads, sizeof(uint16_t) * RS * (kMlpIn + kMlpHidden), s>>>(
-        x, m.dz1, n, kMlpHidden, kMlpHidden, m.grad, kMlpHidden, m.grad + kOffB1);
+    const int64_t tiles = (n + kTileRows - 1) / kTileRows;
+    k_mlp_gradient<<<(unsigned)(tiles < m.sms ? tiles : m.sms), kMlpThreads, sizeof(GradSmem), s>>>(
+        m, x, target, n, 1.0f / (3.0f * (float)n));
     return cudaGetLastError();
 }
 
@@ -408,13 +411,8 @@ std::mutex smem_mu;
 cudaError_t allow_smem(int device) {
     std::lock_guard<std::mutex> g(smem_mu);
     if (device >= 0 && device < 64 && smem_ready[device]) return cudaSuccess;
-    constexpr int RS = kTileRows + 8;
-    cudaError_t e = cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FwdSmem));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mlp_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BwdSmem));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mlp_wgrad<kMlpHidden, kMlpHidden>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(uint16_t) * RS * 2 * kMlpHidden));
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_mlp_gradient, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GradSmem));
     if (e == cudaSuccess && device >= 0 && device < 64) smem_ready[device] = true;
     return e;
 }
@@ -429,12 +427,46 @@ cudaError_t mlp_forward(const vrad_mlp &m, const uint16_t *x, int64_t n, float *
 
 namespace {
 
+// The pinned blocks that carry a network's gradient to the host: pinning one
+// takes 1 to 2.5 ms, several times what creating a network takes otherwise,
+// so a destroyed network's block serves the next one.  At most kSpareBlocks
+// (85 KB each) are kept.
+constexpr size_t kSpareBlocks = 8;
+std::mutex spare_mu;
+std::vector<float *> &spare_blocks() {
+    static std::vector<float *> *v = new std::vector<float *>;  // never destroyed: used from static destructors
+    return *v;
+}
+
+cudaError_t take_block(float **out) {
+    {
+        std::lock_guard<std::mutex> g(spare_mu);
+        if (!spare_blocks().empty()) {
+            *out = spare_blocks().back();
+            spare_blocks().pop_back();
+            return cudaSuccess;
+        }
+    }
+    return cudaHostAlloc(out, sizeof(float) * (vrad::kMlpParams + 1), cudaHostAllocPortable);
+}
+
+void give_block(float *p) {
+    if (!p) return;
+    {
+        std::lock_guard<std::mutex> g(spare_mu);
+        if (spare_blocks().size() < kSpareBlocks) {
+            spare_blocks().push_back(p);
+            return;
+        }
+    }
+    cudaFreeHost(p);
+}
+
 void release_mlp(vrad_mlp *m) {
     for (void *p : {(void *)m->master, (void *)m->adam_m, (void *)m->adam_v, (void *)m->grad, (void *)m->w1t,
-                    (void *)m->w2t, (void *)m->w3t, (void *)m->w2, (void *)m->w3, (void *)m->loss, (void *)m->flags,
-                    (void *)m->h1,
-                    (void *)m->h2, (void *)m->dz1, (void *)m->dz2, (void *)m->dy, (void *)m->y})
+                    (void *)m->w2t, (void *)m->w3t, (void *)m->w2, (void *)m->w3, (void *)m->flags})
         cudaFree(p);
+    give_block(m->host);
     delete m;
 }
 
@@ -453,10 +485,12 @@ extern "C" int32_t vrad_mlp_create(vrad_ctx *ctx, uint64_t seed, vrad_mlp **out)
     vrad_mlp *m = new vrad_mlp();
     m->device = ctx->device;
     for (float **p : {&m->master, &m->adam_m, &m->adam_v, &m->grad})
-        if (e == cudaSuccess) e = cudaMalloc(p, sizeof(float) * kMlpParams);
+        if (e == cudaSuccess) e = cudaMalloc(p, sizeof(float) * (kMlpParams + 1));
     for (uint16_t **p : {&m->w1t, &m->w2t, &m->w3t, &m->w2, &m->w3})
         if (e == cudaSuccess) e = cudaMalloc(p, sizeof(uint16_t) * kW2);
-    if (e == cudaSuccess) e = cudaMalloc(&m->loss, sizeof(float));
+    if (e == cudaSuccess) e = take_block(&m->host);
+    m->loss = m->grad ? m->grad + kMlpParams : nullptr;
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, ctx->device);
     if (e == cudaSuccess) e = cudaMalloc(&m->flags, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(m->flags, 0, sizeof(uint32_t));
     if (e == cudaSuccess) e = allow_smem(ctx->device);
@@ -518,10 +552,12 @@ extern "C" int32_t vrad_mlp_gradient_device(vrad_mlp *m, const uint16_t *x, cons
     cudaError_t e = cudaSetDevice(m->device);
     cudaStream_t s = (cudaStream_t)stream;
     if (e == cudaSuccess) e = vrad::gradient(*m, x, target, n, s);
-    if (e == cudaSuccess && grad)
-        e = cudaMemcpyAsync(grad, m->grad, sizeof(float) * vrad::kMlpParams, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess && loss) e = cudaMemcpyAsync(loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost, s);
+    // Gradient and loss in one copy, through pinned memory.
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(m->host, m->grad, sizeof(float) * (vrad::kMlpParams + 1), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess && grad) std::memcpy(grad, m->host, sizeof(float) * vrad::kMlpParams);
+    if (e == cudaSuccess && loss) *loss = m->host[vrad::kMlpParams];
     if (e != cudaSuccess) return vrad_cuda_fail(nullptr, e, "network gradient");
     return VRAD_OK;
 }

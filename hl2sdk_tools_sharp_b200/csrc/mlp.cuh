@@ -7,7 +7,7 @@
 //                  b1 [128], w2 [128][128], b2 [128], w3 [128][3], b3 [3]);
 //                  w[k][n] maps input k to output n
 //   adam_m, adam_v float  Adam's moments, same order
-//   grad   float   the gradient of the last step, same order
+//   grad   float   the gradient of the last step, same order, then the loss
 //   w1t [128][32], w2t [128][128], w3t [8][128] bf16: the forward's B
 //                  operands, output-major (rows 3..7 of w3t zero)
 //   w2 [128][128], w3 [128][8] bf16: the backward's B operands, input-major
@@ -39,12 +39,10 @@ struct vrad_mlp {
     int device = 0;
     float *master = nullptr, *adam_m = nullptr, *adam_v = nullptr, *grad = nullptr;
     uint16_t *w1t = nullptr, *w2t = nullptr, *w3t = nullptr, *w2 = nullptr, *w3 = nullptr;
-    float *loss = nullptr;        // device scalar of the last step
+    float *loss = nullptr;        // device scalar of the last step: grad[kMlpParams]
+    float *host = nullptr;        // pinned: the gradient and loss on their way to a caller
     uint32_t *flags = nullptr;    // device word: bit 0, a forward's MMA wait ran out (sticky)
-    // Training scratch, grown on demand: activations and their gradients.
-    uint16_t *h1 = nullptr, *h2 = nullptr, *dz1 = nullptr, *dz2 = nullptr, *dy = nullptr;
-    float *y = nullptr;
-    int64_t scratch_rows = 0;
+    int sms = 1;
     int64_t step = 0;
 };
 

@@ -56,6 +56,22 @@ def test_gradient_matches_oracle(net):
     assert _rel(g2, g) < 1e-5
 
 
+@pytest.mark.parametrize("rows", [1, 15, 17, 127, 128, 129, 148 * 128 + 1, 2 * 148 * 128 + 130])
+def test_gradient_at_tile_edges(net, rows):
+    """Row counts about a warp's 16 rows, a tile's 128 and the tiles the
+    chip's CTAs take in one and two turns; the tolerances are
+    test_gradient_matches_oracle's (BF16 activations and gradients)."""
+    from oracle import mlp_oracle as MO
+    n, torch = net
+    xt, bits, tt, t = _data(torch, rows, 3 + rows)
+    g, loss = n.gradient(xt, tt)
+    want, want_loss = MO.gradient(n.params(), bits, t)
+    assert abs(loss - want_loss) < 1e-3 * want_loss
+    gs, ws = LN.split(g), LN.split(want.astype(np.float32))
+    for name in ("w1", "b1", "w2", "b2", "w3", "b3"):
+        assert _rel(gs[name], ws[name]) < 1e-2, name
+
+
 def test_training_fits_a_function(net):
     import torch
     n, _ = net
