@@ -25,9 +25,11 @@
 //
 // Kernels of one light pass (after the direct gather):
 //   k_patch_samples   one thread per patch: the face's samples that overlap
-//                     it, in sample order (AddSampleToPatch)
-//   k_patch_tree      one thread per face: pushes, averages and area blends
-//                     over the face's patch list, then the move to emission
+//                     it, in sample order (AddSampleToPatch), averaged and
+//                     moved to emission
+//   k_parents         one block per face: the parents level by level, bottom
+//                     up (the direct light's area blends; after each bounce
+//                     CollectLight's; the warm start's)
 //   k_candidates      one thread per receiver: the candidate sources in the
 //                     enumerator's order (a counting and a writing launch)
 //   k_transfer        one thread per candidate: the transfer ray, traced
@@ -36,14 +38,12 @@
 //                     accepted pairs compacted in order, capped at
 //                     MaxPatches, and MakeScales' ordered sum
 //   k_sell_*          the transfer lists copied into slices of 32 receivers
-//                     sorted by count (SELL-32), once per pass
-//   k_gather          one thread per receiver (in count order): GatherLight's
-//                     ordered sum from its slice lane, then CollectLight's
-//                     leaf update
-//   k_collect_level   one thread per parent of one tree level: CollectLight's
-//                     parents, one launch per level, bottom up
-//   k_totals          fp64 sums of the light a bounce added, with absolute
-//                     sums that bound the reference's float sum
+//                     sorted by window and count (SELL-32), once per pass
+//   k_gather          one thread per receiver (in the slices' order):
+//                     GatherLight's ordered sum from its slice lane, then
+//                     CollectLight's leaf update, and fp64 sums of the light
+//                     the bounce added, with absolute sums that bound the
+//                     reference's float sum
 //   k_exact_total     one block: the reference's sequential float sum, run
 //                     only when the bound cannot settle the stop rule
 
@@ -63,6 +63,7 @@
 #include "bounce.cuh"
 #include "device_pool.h"
 #include "context.cuh"
+#include "final.cuh"
 #include "detmath.cuh"
 #include "mlp.cuh"
 #include "patches.h"
@@ -101,91 +102,231 @@ __device__ __forceinline__ F3 normalise3(F3 a, float &len) {
 
 // ---- the patches' direct light ----------------------------------------------
 
-// AddSampleToPatch for one patch over its face's samples, in sample order:
-// acc = (sample light * area summed, sample area summed).
-__global__ void k_patch_samples(BounceView v, const float4 *__restrict__ sample_light, float4 *__restrict__ acc) {
+// AddSampleToPatch for one leaf patch over its face's samples, in sample
+// order, then BuildPatchLights' average and MoveDirectLightToEmission: the
+// leaf's direct light, its emission and what it shoots; the bounced total
+// starts from zero.  The parents' sums that the reference pushes up are
+// replaced by the area blend of their children's averages before anything
+// reads them, so only that blend is built (k_parents).
+//
+// A face has hundreds of samples and a leaf a few cells of them, so where
+// the face's samples lie in cell order the leaf looks at the cells in
+// reach alone (box, k_patch_boxes): every sample that can pass the overlap
+// test lies there, and the cells come in sample order.  On the 8x8 grid of
+// rooms a pass takes 235 us, with all of the face's samples 3.1 ms.
+__global__ void k_patch_samples(BounceView v, const int4 *__restrict__ box, const int32_t *__restrict__ face_cells,
+                                const float4 *__restrict__ frames, const int32_t *__restrict__ cell_sample,
+                                const float4 *__restrict__ sample_light, float4 *__restrict__ direct,
+                                float4 *__restrict__ total, float4 *__restrict__ emit, float4 *__restrict__ shoot) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= v.npatches) return;
+    total[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const int4 tr = __ldg(&v.tree[p]);
+    if (tr.y != -1) return;
     float lx = 0.0f, ly = 0.0f, lz = 0.0f, area = 0.0f;
-    if (tr.y == -1 && tr.w == 0) {
+    if (tr.w == 0) {
         const float4 mn = __ldg(&v.mins[p]), mx = __ldg(&v.maxs[p]);
         const int f = __float_as_int(mn.w);
-        const int2 fs = __ldg(&v.face_samples[f]);
-        for (int k = fs.x; k < fs.x + fs.y; k++) {
+        auto sample = [&](int k) {
             const float4 L = __ldg(&sample_light[k]);
             // VectorAvg: a float divide by 3.
-            if (__fdiv_rn(__fadd_rn(__fadd_rn(L.x, L.y), L.z), 3.0f) < 1.0f) continue;
+            if (__fdiv_rn(__fadd_rn(__fadd_rn(L.x, L.y), L.z), 3.0f) < 1.0f) return;
             const float a = __ldg(&v.sample_area[k]);
             const float4 P = __ldg(&v.sample_pos[k]);
             const float radius = (float)__ddiv_rn((double)__fsqrt_rn(a), 2.0);
-            if (mn.x > __fadd_rn(P.x, radius) || mx.x < __fsub_rn(P.x, radius)) continue;
-            if (mn.y > __fadd_rn(P.y, radius) || mx.y < __fsub_rn(P.y, radius)) continue;
-            if (mn.z > __fadd_rn(P.z, radius) || mx.z < __fsub_rn(P.z, radius)) continue;
+            if (mn.x > __fadd_rn(P.x, radius) || mx.x < __fsub_rn(P.x, radius)) return;
+            if (mn.y > __fadd_rn(P.y, radius) || mx.y < __fsub_rn(P.y, radius)) return;
+            if (mn.z > __fadd_rn(P.z, radius) || mx.z < __fsub_rn(P.z, radius)) return;
             area = __fadd_rn(area, a);
             lx = __fadd_rn(lx, __fmul_rn(a, L.x));
             ly = __fadd_rn(ly, __fmul_rn(a, L.y));
             lz = __fadd_rn(lz, __fmul_rn(a, L.z));
+        };
+        const int4 bx = __ldg(&box[p]);
+        if (bx.x >= 0) {
+            const int base = __ldg(&face_cells[f]), w = __float_as_int(__ldg(&frames[5 * f].w));
+            for (int t = bx.y; t < bx.w; t++)
+                for (int s = bx.x; s < bx.z; s++) {
+                    const int k = __ldg(&cell_sample[base + s + t * w]);
+                    if (k >= 0) sample(k);
+                }
+        } else {
+            const int2 fs = __ldg(&v.face_samples[f]);
+            for (int k = fs.x; k < fs.x + fs.y; k++) sample(k);
         }
     }
-    acc[p] = make_float4(lx, ly, lz, area);
+    float4 e = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (area != 0.0f) {
+        const float scale = (float)__drcp_rn((double)area);
+        e = make_float4(__fadd_rn(0.0f, __fmul_rn(lx, scale)), __fadd_rn(0.0f, __fmul_rn(ly, scale)),
+                        __fadd_rn(0.0f, __fmul_rn(lz, scale)), 0.0f);
+    }
+    const float4 r = __ldg(&v.refl[p]);
+    direct[p] = e;
+    emit[p] = e;
+    shoot[p] = make_float4(__fmul_rn(e.x, r.x), __fmul_rn(e.y, r.y), __fmul_rn(e.z, r.z), 0.0f);
 }
 
-// The face's patch list (FacePatches after RebuildFaceLists): its
-// descendants in descending index order, then its root.
-struct FaceList {
-    int root, first, end;
-    __device__ __forceinline__ int count() const { return root < 0 ? 0 : end - first + 1; }
-    __device__ __forceinline__ int at(int k) const { return k < end - first ? end - 1 - k : root; }
+// A face's luxel coordinates in double: world to luxel (s, t) and how far a
+// box of half sizes h reaches in each.
+struct Luxels {
+    double ox, oy, oz, sx, sy, sz, tx, ty, tz;
+    int w, h, min_s, min_t;
+    __device__ __forceinline__ Luxels(const float4 *__restrict__ frames, int f) {
+        const float4 o = __ldg(&frames[5 * (int64_t)f]), a = __ldg(&frames[5 * (int64_t)f + 1]),
+                     b = __ldg(&frames[5 * (int64_t)f + 2]), c = __ldg(&frames[5 * (int64_t)f + 3]);
+        ox = o.x, oy = o.y, oz = o.z;
+        sx = a.x, sy = a.y, sz = a.z;
+        tx = b.x, ty = b.y, tz = b.z;
+        w = __float_as_int(o.w);
+        h = __float_as_int(a.w);
+        min_s = __float_as_int(b.w);
+        min_t = __float_as_int(c.w);
+    }
+    __device__ __forceinline__ double s(double x, double y, double z) const {
+        return (x - ox) * sx + (y - oy) * sy + (z - oz) * sz - (double)min_s;
+    }
+    __device__ __forceinline__ double t(double x, double y, double z) const {
+        return (x - ox) * tx + (y - oy) * ty + (z - oz) * tz - (double)min_t;
+    }
+    __device__ __forceinline__ double reach_s(double x, double y, double z) const {
+        return fabs(sx) * x + fabs(sy) * y + fabs(sz) * z;
+    }
+    __device__ __forceinline__ double reach_t(double x, double y, double z) const {
+        return fabs(tx) * x + fabs(ty) * y + fabs(tz) * z;
+    }
 };
 
-// BuildPatchLights after the samples (pushes to parents, averages, area
-// blends), then MoveDirectLightToEmission for the face's patches.
-__global__ void k_patch_tree(BounceView v, float4 *__restrict__ acc, float4 *__restrict__ direct,
-                             float4 *__restrict__ total, float4 *__restrict__ emit, float4 *__restrict__ shoot) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+// How a face's samples lie in its cells: (how far a sample's luxel
+// coordinates stray from its cell, s and t; the largest radius; 1 when the
+// samples are the cells' in cell order, and all of it is finite).  One warp
+// per face.
+__global__ void k_face_fit(BounceView v, const int32_t *__restrict__ face_cells, const float4 *__restrict__ frames,
+                           const int32_t *__restrict__ cell_sample, float4 *__restrict__ fit) {
+    const int f = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (f >= v.nfaces) return;
-    const int4 fr = __ldg(&v.face_range[f]);
-    const FaceList L{fr.x, fr.y, fr.z};
-    const int n = L.count();
-    for (int k = 0; k < n; k++) {
-        const int p = L.at(k);
-        const int parent = __ldg(&v.tree[p].x);
-        if (parent == -1) continue;
-        const float4 a = acc[p], b = acc[parent];
-        acc[parent] = make_float4(__fadd_rn(b.x, a.x), __fadd_rn(b.y, a.y), __fadd_rn(b.z, a.z), __fadd_rn(b.w, a.w));
-    }
-    for (int k = 0; k < n; k++) {
-        const int p = L.at(k);
-        const float4 a = acc[p];
-        float4 t = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (a.w != 0.0f) {
-            const float scale = (float)__drcp_rn((double)a.w);
-            t = make_float4(__fadd_rn(0.0f, __fmul_rn(a.x, scale)), __fadd_rn(0.0f, __fmul_rn(a.y, scale)),
-                            __fadd_rn(0.0f, __fmul_rn(a.z, scale)), 0.0f);
+    const int2 fs = __ldg(&v.face_samples[f]);
+    const Luxels lx(frames, f);
+    const int base = __ldg(&face_cells[f]), n = __ldg(&face_cells[f + 1]) - base;
+    double ds = 0.0, dt = 0.0, r = 0.0;
+    bool ok = true;
+    int last = fs.x - 1, found = 0;  // the last cell's sample so far, samples found
+    for (int c0 = 0; c0 < n; c0 += 32) {
+        const int c = c0 + lane, k = c < n ? __ldg(&cell_sample[base + c]) : -1;
+        const unsigned have = __ballot_sync(kFull, k >= 0), before = have & ((1u << lane) - 1u);
+        const int prev = __shfl_sync(kFull, k, before ? 31 - __clz(before) : 0);
+        if (k >= 0) {
+            ok = ok && k > (before ? prev : last) && k < fs.x + fs.y;
+            const float4 P = __ldg(&v.sample_pos[k]);
+            ds = fmax(ds, fabs(lx.s(P.x, P.y, P.z) - (double)(c % lx.w)));
+            dt = fmax(dt, fabs(lx.t(P.x, P.y, P.z) - (double)(c / lx.w)));
+            const double radius = sqrt((double)__ldg(&v.sample_area[k])) * 0.5;
+            r = fmax(r, radius);
+            ok = ok && isfinite(P.x) && isfinite(P.y) && isfinite(P.z) && isfinite(radius);
         }
-        total[p] = t;
-        direct[p] = t;
+        found += __popc(have);
+        if (have) last = __shfl_sync(kFull, k, 31 - __clz(have));
     }
-    for (int k = 0; k < n; k++) {
-        const int p = L.at(k);
-        const int4 tr = __ldg(&v.tree[p]);
-        if (tr.y == -1) continue;
-        const float a1 = __ldg(&v.origin[tr.y].w), a2 = __ldg(&v.origin[tr.z].w);
-        const float s1 = __fdiv_rn(a1, __fadd_rn(a1, a2)), s2 = __fdiv_rn(a2, __fadd_rn(a1, a2));
-        const float4 c1 = total[tr.y], c2 = total[tr.z];
-        const float4 t = make_float4(__fadd_rn(__fmul_rn(c1.x, s1), __fmul_rn(c2.x, s2)),
-                                     __fadd_rn(__fmul_rn(c1.y, s1), __fmul_rn(c2.y, s2)),
-                                     __fadd_rn(__fmul_rn(c1.z, s1), __fmul_rn(c2.z, s2)), 0.0f);
-        total[p] = t;
-        direct[p] = t;
+    for (int o = 16; o > 0; o >>= 1) {
+        ds = fmax(ds, __shfl_xor_sync(kFull, ds, o));
+        dt = fmax(dt, __shfl_xor_sync(kFull, dt, o));
+        r = fmax(r, __shfl_xor_sync(kFull, r, o));
     }
-    for (int k = 0; k < n; k++) {
-        const int p = L.at(k);
-        const float4 e = total[p], r = __ldg(&v.refl[p]);
-        emit[p] = e;
-        shoot[p] = make_float4(__fmul_rn(e.x, r.x), __fmul_rn(e.y, r.y), __fmul_rn(e.z, r.z), 0.0f);
-        total[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    ok = __all_sync(kFull, ok) && found == fs.y && ds < 1e6 && dt < 1e6 && r < 1e6;
+    // Rounded up: an upper bound is what is kept.
+    if (lane == 0) fit[f] = make_float4(__double2float_ru(ds), __double2float_ru(dt), __double2float_ru(r), ok ? 1.0f : 0.0f);
+}
+
+// Each leaf patch's cells in reach, [x, z) by [y, w): those whose sample
+// could pass the overlap test, that is, lie in the patch's bounds grown by
+// the face's largest radius.  The slack of 1e-3 units and 1e-6 of the
+// coordinates covers the test's float roundings (half an ulp is 6e-8 of
+// them), that of 0.01 luxels the sums here.  x = -1: the face's samples
+// don't lie in cell order or something isn't finite, and the patch looks at
+// all of them.
+__global__ void k_patch_boxes(BounceView v, const float4 *__restrict__ frames, const float4 *__restrict__ fit,
+                              int4 *__restrict__ box) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= v.npatches) return;
+    box[p] = make_int4(-1, 0, 0, 0);
+    const float4 mn = __ldg(&v.mins[p]), mx = __ldg(&v.maxs[p]);
+    const int f = __float_as_int(mn.w);
+    const float4 ft = __ldg(&fit[f]);
+    if (ft.w == 0.0f) return;
+    const Luxels lx(frames, f);
+    const double big = fmax(fmax(fmax(fabs((double)mn.x), fabs((double)mn.y)), fabs((double)mn.z)),
+                            fmax(fmax(fabs((double)mx.x), fabs((double)mx.y)), fabs((double)mx.z)));
+    const double grow = (double)ft.z + 1e-3 + 1e-6 * big;
+    const double cx = 0.5 * ((double)mn.x + mx.x), cy = 0.5 * ((double)mn.y + mx.y), cz = 0.5 * ((double)mn.z + mx.z);
+    const double hx = fmax(0.5 * ((double)mx.x - mn.x) + grow, 0.0), hy = fmax(0.5 * ((double)mx.y - mn.y) + grow, 0.0),
+                 hz = fmax(0.5 * ((double)mx.z - mn.z) + grow, 0.0);
+    const double s = lx.s(cx, cy, cz), t = lx.t(cx, cy, cz);
+    const double rs = lx.reach_s(hx, hy, hz) + ft.x + 0.01, rt = lx.reach_t(hx, hy, hz) + ft.y + 0.01;
+    if (!(fabs(s) + rs < 1e9 && fabs(t) + rt < 1e9)) return;
+    const int s0 = max((int)ceil(s - rs), 0), t0 = max((int)ceil(t - rt), 0);
+    box[p] = make_int4(s0, t0, min((int)floor(s + rs) + 1, lx.w), min((int)floor(t + rt) + 1, lx.h));
+}
+
+// ---- the parents -------------------------------------------------------------
+
+// The parents' records from their list.
+__global__ void k_parent_records(BounceView v, const int32_t *__restrict__ list, int n, int4 *__restrict__ parent,
+                                 float2 *__restrict__ share) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int p = __ldg(&list[i]);
+    const int4 tr = __ldg(&v.tree[p]);
+    const float a1 = __ldg(&v.origin[tr.y].w), a2 = __ldg(&v.origin[tr.z].w);
+    parent[i] = make_int4(p, tr.y, tr.z, tr.w);
+    share[i] = make_float2(__fdiv_rn(a1, __fadd_rn(a1, a2)), __fdiv_rn(a2, __fadd_rn(a1, a2)));
+}
+
+// One block per face: its parents level by level, bottom up, so that every
+// parent reads final children.  A level is a few loads that wait for one
+// another, so what it costs is launches and latency: a launch per level over
+// all faces took 93 us a bounce on the 8x8 grid of rooms and 45 on the 3x3
+// grid, and a thread per face 1.2 ms and 0.9 ms a pass for the direct light;
+// a block per face takes 39 and 16 us (32 to 128 threads: the same; 256: 10
+// us more).  OP per parent:
+//   kOpDirect   BuildPatchLights' area blend of the children's direct light,
+//               then MoveDirectLightToEmission
+//   kOpCollect  CollectLight's parents: the blend of the children's light
+//               and emission, shot on; nothing from a sky face
+//   kOpGuess    the blend of the warm start's guess
+enum : int { kOpDirect = 0, kOpCollect = 1, kOpGuess = 2 };
+constexpr int kFaceThreads = 64;
+
+__device__ __forceinline__ float4 blend(const float4 &a, const float4 &b, const float2 &s) {
+    return make_float4(__fadd_rn(__fmul_rn(a.x, s.x), __fmul_rn(b.x, s.y)),
+                       __fadd_rn(__fmul_rn(a.y, s.x), __fmul_rn(b.y, s.y)),
+                       __fadd_rn(__fmul_rn(a.z, s.x), __fmul_rn(b.z, s.y)), 0.0f);
+}
+
+template <int OP>
+__global__ void __launch_bounds__(kFaceThreads)
+    k_parents(BounceView v, const int32_t *__restrict__ face_level, const int32_t *__restrict__ level_off,
+              const int4 *__restrict__ parent, const float2 *__restrict__ share, float4 *light, float4 *emit,
+              float4 *shoot) {
+    const int f = blockIdx.x;
+    const int h1 = __ldg(&face_level[f + 1]) - 1;
+    for (int h = __ldg(&face_level[f]); h < h1; h++) {
+        const int end = __ldg(&level_off[h + 1]);
+        for (int i = __ldg(&level_off[h]) + threadIdx.x; i < end; i += kFaceThreads) {
+            const int4 p = __ldg(&parent[i]);
+            const float2 s = __ldg(&share[i]);
+            if (OP == kOpCollect && p.w) {
+                emit[p.x] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                shoot[p.x] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                continue;
+            }
+            const float4 t = blend(light[p.y], light[p.z], s);
+            light[p.x] = t;
+            if (OP == kOpGuess) continue;
+            const float4 e = OP == kOpDirect ? t : blend(emit[p.y], emit[p.z], s), r = __ldg(&v.refl[p.x]);
+            emit[p.x] = e;
+            shoot[p.x] = make_float4(__fmul_rn(e.x, r.x), __fmul_rn(e.y, r.y), __fmul_rn(e.z, r.z), 0.0f);
+        }
+        __syncthreads();
     }
 }
 
@@ -430,120 +571,69 @@ __global__ void k_transfer_write(int nrecv, const int64_t *__restrict__ cand_off
 
 // ---- bounces ---------------------------------------------------------------
 
-// The gather's slices (SELL-32) of the transfer lists: each receiver's
-// count and index for the sort by count.
-__global__ void k_sell_keys(int nrecv, const int64_t *__restrict__ tr_off, int32_t *__restrict__ key,
+// The gather's slices (SELL-32) of the transfer lists: each receiver's key
+// and index for the sort by window and count.
+__global__ void k_sell_keys(int nrecv, int window, const int64_t *__restrict__ tr_off, uint32_t *__restrict__ key,
                             int32_t *__restrict__ idx) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= nrecv) return;
-    key[r] = (int32_t)(tr_off[r + 1] - tr_off[r]);
+    key[r] = ((uint32_t)(r / window) << kCountBits) | (kCountMask - (uint32_t)(tr_off[r + 1] - tr_off[r]));
     idx[r] = r;
 }
 
+__device__ __forceinline__ int sell_count(uint32_t key) { return (int)(kCountMask - (key & kCountMask)); }
+
 // Slice s's size: 32 times its first (largest) count.
-__global__ void k_sell_width(int nrecv, int nslices, const int32_t *__restrict__ count, int64_t *__restrict__ width) {
+__global__ void k_sell_width(int nslices, const uint32_t *__restrict__ sorted, int64_t *__restrict__ width) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nslices) return;
-    width[s] = 32 * (int64_t)count[32 * s];
+    width[s] = 32 * (int64_t)sell_count(sorted[32 * s]);
 }
 
 // Copies each receiver's transfers into its lane of its slice.
-__global__ void k_sell_pack(int nrecv, const int32_t *__restrict__ order, const int32_t *__restrict__ count,
+__global__ void k_sell_pack(int nrecv, const int32_t *__restrict__ order, const uint32_t *__restrict__ sorted,
                             const int64_t *__restrict__ sell_off, const int64_t *__restrict__ tr_off,
                             const int2 *__restrict__ tr, int2 *__restrict__ sell) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nrecv) return;
-    const int r = order[i], n = count[i];
+    const int r = order[i], n = sell_count(sorted[i]);
     const int2 *src = tr + tr_off[r];
     int2 *dst = sell + sell_off[i >> 5] + (i & 31);
     for (int j = 0; j < n; j++) dst[32 * (int64_t)j] = __ldg(&src[j]);
 }
 
-// GatherLight for one receiver (the ordered sum over its transfers of the
-// sources' shoot times the weight), then CollectLight's update of that
-// leaf: the light added, emitted and shot on.  Thread i takes the i-th
-// receiver of the count order, its transfers from its lane of its slice.
-__global__ void k_gather(BounceView v, const int32_t *__restrict__ order, const int32_t *__restrict__ count,
-                         const int64_t *__restrict__ sell_off, const int2 *__restrict__ sell,
-                         const float4 *__restrict__ shoot_in, float4 *__restrict__ total,
-                         float4 *__restrict__ emit_out, float4 *__restrict__ shoot_out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= v.nreceivers) return;
-    const int p = __ldg(&v.recv[__ldg(&order[i])]);
-    const int n = __ldg(&count[i]);
-    const int2 *src = sell + __ldg(&sell_off[i >> 5]) + (i & 31);
-    float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-    for (int j = 0; j < n; j++) {
-        const int2 t = __ldg(&src[32 * (int64_t)j]);
-        const float w = __int_as_float(t.y);
-        const float4 s = __ldg(&shoot_in[t.x]);
-        sx = __fadd_rn(sx, __fmul_rn(s.x, w));
-        sy = __fadd_rn(sy, __fmul_rn(s.y, w));
-        sz = __fadd_rn(sz, __fmul_rn(s.z, w));
+// 32 times each window's largest candidate count, added up: what the slices'
+// padding can come to (a slice's padding is at most 32 times its first count
+// less its own transfers, and that first count at most the last of the
+// slice before).
+__global__ void k_sell_pad(int nrecv, int window, const int64_t *__restrict__ cand_off, unsigned long long *pad) {
+    __shared__ int largest;
+    if (threadIdx.x == 0) largest = 0;
+    __syncthreads();
+    int m = 0;
+    const int r0 = blockIdx.x * window;
+    for (int r = r0 + threadIdx.x; r < min(r0 + window, nrecv); r += blockDim.x) {
+        const int64_t n = cand_off[r + 1] - cand_off[r];
+        m = max(m, (int)(n < kMaxTransfersPerReceiver ? n : kMaxTransfersPerReceiver));
     }
-    if (__ldg(&v.tree[p].w)) {
-        emit_out[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        shoot_out[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        return;
-    }
-    const float4 t = total[p];
-    total[p] = make_float4(__fadd_rn(t.x, sx), __fadd_rn(t.y, sy), __fadd_rn(t.z, sz), 0.0f);
-    emit_out[p] = make_float4(sx, sy, sz, 0.0f);
-    const float4 rf = __ldg(&v.refl[p]);
-    shoot_out[p] = make_float4(__fmul_rn(sx, rf.x), __fmul_rn(sy, rf.y), __fmul_rn(sz, rf.z), 0.0f);
+    atomicMax(&largest, m);
+    __syncthreads();
+    if (threadIdx.x == 0) atomicAdd(pad, 32ull * (unsigned long long)largest);
 }
 
-// CollectLight's parents for one level of the patch trees: every parent
-// whose subtree is `level` deep, each the area blend of its children's
-// light and emission (the children, one level lower, are final).  Run for
-// levels 1, 2, ... this is CollectLight's bottom-up order within each face.
-__global__ void k_collect_level(BounceView v, const int32_t *__restrict__ parents, int n, float4 *__restrict__ total,
-                                float4 *__restrict__ emit_out, float4 *__restrict__ shoot_out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int p = __ldg(&parents[i]);
-    const int4 tr = __ldg(&v.tree[p]);
-    if (tr.w) {
-        emit_out[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        shoot_out[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        return;
-    }
-    const float a1 = __ldg(&v.origin[tr.y].w), a2 = __ldg(&v.origin[tr.z].w);
-    const float s1 = __fdiv_rn(a1, __fadd_rn(a1, a2)), s2 = __fdiv_rn(a2, __fadd_rn(a1, a2));
-    const float4 c1 = total[tr.y], c2 = total[tr.z];
-    total[p] = make_float4(__fadd_rn(__fmul_rn(c1.x, s1), __fmul_rn(c2.x, s2)),
-                           __fadd_rn(__fmul_rn(c1.y, s1), __fmul_rn(c2.y, s2)),
-                           __fadd_rn(__fmul_rn(c1.z, s1), __fmul_rn(c2.z, s2)), 0.0f);
-    const float4 e1 = emit_out[tr.y], e2 = emit_out[tr.z];
-    const float4 e = make_float4(__fadd_rn(__fmul_rn(e1.x, s1), __fmul_rn(e2.x, s2)),
-                                 __fadd_rn(__fmul_rn(e1.y, s1), __fmul_rn(e2.y, s2)),
-                                 __fadd_rn(__fmul_rn(e1.z, s1), __fmul_rn(e2.z, s2)), 0.0f);
-    emit_out[p] = e;
-    const float4 rf = __ldg(&v.refl[p]);
-    shoot_out[p] = make_float4(__fmul_rn(e.x, rf.x), __fmul_rn(e.y, rf.y), __fmul_rn(e.z, rf.z), 0.0f);
-}
-
-// The light a bounce added (the leaves' emission), in fp64, with two sums
-// that bound how far the reference's float sum (CollectLight's, in
-// leaf_desc order) can lie from it: the absolute values, and the absolute
-// values each weighted by the number of terms from it to the end of that
-// order (n - rank).  Recursive summation's error is at most
-// u * sum_k |partial sum k| <= u * sum_i |x_i| (n - rank_i), over 1 - n u.
-__global__ void k_totals(BounceView v, const float4 *__restrict__ emit, const int32_t *__restrict__ leaf_rank,
-                         int32_t nleaves, double *__restrict__ sums) {
+// The block's part of a bounce's totals: the light the bounce added (the
+// sky-free leaves' emission e), in fp64, with two sums that bound how far
+// the reference's float sum (CollectLight's, in leaf_desc order) can lie
+// from it: the absolute values, and the absolute values each weighted by the
+// number of terms from it to the end of that order (left = n - rank).
+// Recursive summation's error is at most u * sum_k |partial sum k| <=
+// u * sum_i |x_i| (n - rank_i), over 1 - n u.  The blocks add to kSumParts
+// parts, so that few meet on one address.
+__device__ __forceinline__ void add_totals(const F3 &e, double left, double *__restrict__ sums) {
     __shared__ double part[kSums][kBounceBlock / 32];
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    double s[kSums] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    if (p < v.npatches) {
-        const int4 tr = __ldg(&v.tree[p]);
-        if (tr.y == -1 && tr.w == 0) {
-            const float4 e = emit[p];
-            const double w = (double)(nleaves - __ldg(&leaf_rank[p]));
-            s[0] = e.x, s[1] = e.y, s[2] = e.z;
-            s[3] = fabs((double)e.x), s[4] = fabs((double)e.y), s[5] = fabs((double)e.z);
-            s[6] = s[3] * w, s[7] = s[4] * w, s[8] = s[5] * w;
-        }
-    }
+    double s[kSums] = {e.x, e.y, e.z, fabs((double)e.x), fabs((double)e.y), fabs((double)e.z)};
+    s[6] = s[3] * left, s[7] = s[4] * left, s[8] = s[5] * left;
+#pragma unroll
     for (int k = 0; k < kSums; k++)
         for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_down_sync(kFull, s[k], o);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -553,8 +643,82 @@ __global__ void k_totals(BounceView v, const float4 *__restrict__ emit, const in
     if (threadIdx.x < kSums) {
         double t = 0.0;
         for (int w = 0; w < kBounceBlock / 32; w++) t += part[threadIdx.x][w];
-        atomicAdd(&sums[threadIdx.x], t);
+        atomicAdd(&sums[kSums * (blockIdx.x % kSumParts) + threadIdx.x], t);
     }
+}
+
+// GatherLight for one receiver (the ordered sum over its transfers of the
+// sources' shoot times the weight), then CollectLight's update of that
+// leaf: the light added, emitted and shot on, and the bounce's totals.
+// Thread i takes the i-th receiver of the slices' order, its transfers from
+// its lane of its slice.
+//
+// Each sum is one chain in the reference's order, so the loads are what a
+// thread waits for: it asks for the next eight entries and for this eight's
+// sources before it adds.  The entries stream from HBM (8 B a transfer, once
+// a bounce); the sources are 16 B from anywhere in the light array, and a
+// window of neighbouring receivers, whose lists name much the same sources,
+// is what is sorted by count, not the whole map (whose slices then mix
+// receivers from everywhere).  With 214 M transfers a bounce (1.7 GB, 0.26
+// ms at the copy rate) took 0.66 ms one entry at a time, sorted as a whole,
+// with the totals and the parents' levels in launches of their own; 0.53
+// with windows of 1024 and those folded in (256 to 2048: the same; the whole
+// map: 0.62); 0.41 with eight ahead, of which the gather is 0.36.  Two,
+// four, twelve and sixteen ahead: 0.51, 0.51, 0.50 and 0.57.  With 35 k
+// receivers, 7 warps an SM, it is latency: 99 us a bounce, then 50.
+constexpr int kAhead = 8;
+
+__global__ void __launch_bounds__(kBounceBlock)
+    k_gather(BounceView v, const int32_t *__restrict__ order, const uint32_t *__restrict__ sorted,
+             const int64_t *__restrict__ sell_off, const int2 *__restrict__ sell, const float4 *__restrict__ shoot_in,
+             float4 *__restrict__ total, float4 *__restrict__ emit_out, float4 *__restrict__ shoot_out,
+             const int32_t *__restrict__ leaf_rank, int32_t nleaves, double *__restrict__ sums) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    F3 e = {0.0f, 0.0f, 0.0f};
+    double left = 0.0;
+    if (i < v.nreceivers) {
+        const int p = __ldg(&v.recv[__ldg(&order[i])]);
+        const int n = sell_count(__ldg(&sorted[i]));
+        const int2 *src = sell + __ldg(&sell_off[i >> 5]) + (i & 31);
+        float sx = 0.0f, sy = 0.0f, sz = 0.0f;
+        int2 t[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; k++)
+            if (k < n) t[k] = __ldcs(&src[32 * k]);
+        for (int j = 0; j < n; j += kAhead) {
+            float4 s[kAhead];
+            int2 next[kAhead];
+#pragma unroll
+            for (int k = 0; k < kAhead; k++)
+                if (j + k < n) s[k] = __ldg(&shoot_in[t[k].x]);
+#pragma unroll
+            for (int k = 0; k < kAhead; k++)
+                if (j + kAhead + k < n) next[k] = __ldcs(&src[32 * (int64_t)(j + kAhead + k)]);
+#pragma unroll
+            for (int k = 0; k < kAhead; k++)
+                if (j + k < n) {
+                    const float w = __int_as_float(t[k].y);
+                    sx = __fadd_rn(sx, __fmul_rn(s[k].x, w));
+                    sy = __fadd_rn(sy, __fmul_rn(s[k].y, w));
+                    sz = __fadd_rn(sz, __fmul_rn(s[k].z, w));
+                }
+#pragma unroll
+            for (int k = 0; k < kAhead; k++) t[k] = next[k];
+        }
+        if (__ldg(&v.tree[p].w)) {
+            emit_out[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            shoot_out[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        } else {
+            const float4 t = total[p];
+            total[p] = make_float4(__fadd_rn(t.x, sx), __fadd_rn(t.y, sy), __fadd_rn(t.z, sz), 0.0f);
+            emit_out[p] = make_float4(sx, sy, sz, 0.0f);
+            const float4 rf = __ldg(&v.refl[p]);
+            shoot_out[p] = make_float4(__fmul_rn(sx, rf.x), __fmul_rn(sy, rf.y), __fmul_rn(sz, rf.z), 0.0f);
+            e = {sx, sy, sz};
+            left = (double)(nleaves - __ldg(&leaf_rank[p]));
+        }
+    }
+    add_totals(e, left, sums);
 }
 
 // CollectLight's own total: the leaves' emission summed in float, in
@@ -659,31 +823,17 @@ __global__ void k_guess(BounceView v, const float *__restrict__ y, float4 *__res
     guess[p] = gv;
 }
 
-// A per-patch quantity of one level's parents as the area blend of their
-// children (as CollectLight blends the light); run level by level.
-__global__ void k_blend_level(BounceView v, const int32_t *__restrict__ parents, int n, float4 *__restrict__ a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int p = __ldg(&parents[i]);
-    const int4 tr = __ldg(&v.tree[p]);
-    const float a1 = __ldg(&v.origin[tr.y].w), a2 = __ldg(&v.origin[tr.z].w);
-    const float s1 = a1 / (a1 + a2), s2 = a2 / (a1 + a2);
-    const float4 c1 = a[tr.y], c2 = a[tr.z];
-    a[p] = make_float4(c1.x * s1 + c2.x * s2, c1.y * s1 + c2.y * s2, c1.z * s1 + c2.z * s2, 0.0f);
-}
-
 // The first warm step for each receiver (in count order, its transfers
 // from its slice lane): A = the transfers' gather of the guess's shot
 // light, then light = B1 + A (the Jacobi step from the guess), emission =
 // light - guess (the change, which later bounces carry on).
-__global__ void k_warm_combine(BounceView v, const int32_t *__restrict__ order, const int32_t *__restrict__ count,
-                               const int64_t *__restrict__ sell_off, const int2 *__restrict__ sell,
-                               const float4 *__restrict__ guess, const float4 *__restrict__ first,
-                               float4 *__restrict__ total, float4 *__restrict__ emit_out, float4 *__restrict__ shoot_out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= v.nreceivers) return;
-    const int p = __ldg(&v.recv[__ldg(&order[i])]);
-    const int n = __ldg(&count[i]);
+__device__ __forceinline__ F3 warm_combine(const BounceView &v, int i, const int32_t *__restrict__ order,
+                                           const uint32_t *__restrict__ sorted, const int64_t *__restrict__ sell_off,
+                                           const int2 *__restrict__ sell, const float4 *__restrict__ guess,
+                                           const float4 *__restrict__ first, float4 *__restrict__ total,
+                                           float4 *__restrict__ emit_out, float4 *__restrict__ shoot_out, int &p) {
+    p = __ldg(&v.recv[__ldg(&order[i])]);
+    const int n = sell_count(__ldg(&sorted[i]));
     const int2 *src = sell + __ldg(&sell_off[i >> 5]) + (i & 31);
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
     for (int j = 0; j < n; j++) {
@@ -697,7 +847,8 @@ __global__ void k_warm_combine(BounceView v, const int32_t *__restrict__ order, 
     if (__ldg(&v.tree[p].w)) {
         emit_out[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         shoot_out[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        return;
+        p = -1;
+        return {0.0f, 0.0f, 0.0f};
     }
     const float4 b1 = first[p], gv = guess[p];
     const float4 t = make_float4(b1.x + sx, b1.y + sy, b1.z + sz, 0.0f);
@@ -706,6 +857,20 @@ __global__ void k_warm_combine(BounceView v, const int32_t *__restrict__ order, 
     emit_out[p] = d;
     const float4 rf = __ldg(&v.refl[p]);
     shoot_out[p] = make_float4(d.x * rf.x, d.y * rf.y, d.z * rf.z, 0.0f);
+    return f3(d);
+}
+
+__global__ void __launch_bounds__(kBounceBlock)
+    k_warm_combine(BounceView v, const int32_t *__restrict__ order, const uint32_t *__restrict__ sorted,
+                   const int64_t *__restrict__ sell_off, const int2 *__restrict__ sell, const float4 *__restrict__ guess,
+                   const float4 *__restrict__ first, float4 *__restrict__ total, float4 *__restrict__ emit_out,
+                   float4 *__restrict__ shoot_out, const int32_t *__restrict__ leaf_rank, int32_t nleaves,
+                   double *__restrict__ sums) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    F3 e = {0.0f, 0.0f, 0.0f};
+    int p = -1;
+    if (i < v.nreceivers) e = warm_combine(v, i, order, sorted, sell_off, sell, guess, first, total, emit_out, shoot_out, p);
+    add_totals(e, p >= 0 ? (double)(nleaves - __ldg(&leaf_rank[p])) : 0.0, sums);
 }
 
 unsigned blocks(int64_t n, int per) { return (unsigned)((n + per - 1) / per); }
@@ -715,8 +880,9 @@ unsigned blocks(int64_t n, int per) { return (unsigned)((n + per - 1) / per); }
 void BounceBuffers::release() {
     void *ptrs[] = {origin, normal, mins, maxs, refl, tree, wind, points, face_range, face_samples, face_plane,
                     recv, start, row_off, row_faces, sample_area, cand_off, cand_src, cand_w, tr_off, tr, scan_tmp,
-                    acc, direct, total, emit[0], emit[1], shoot[0], shoot[1], sums, exact, counters, leaf_desc,
-                    level_patch, leaf_rank, sell_key, sell_idx, sell_count, sell_order, sell_off, sell, sort_tmp,
+                    direct, total, emit[0], emit[1], shoot[0], shoot[1], sums, exact, counters, leaf_desc,
+                    face_level, level_off, parent_list, parent, share, patch_box, leaf_rank,
+                    sell_key, sell_idx, sell_sorted, sell_order, sell_off, sell, sort_tmp,
                     first, guess, feat, pred,
                     pr_off, pr_patch, pr_box, pr_coord, prad_light, prad_weight};
     for (void *q : ptrs) dev_free(q);
@@ -724,26 +890,64 @@ void BounceBuffers::release() {
         if (g) cudaGraphExecDestroy(g);
     // The pinned stop-rule sums stay for the next upload (freeing pinned
     // memory can stall); free_pinned() frees them.
-    double *sums_h = h_sums;
+    double *parts_h = h_parts;
     float *exact_h = h_exact;
     *this = BounceBuffers();
-    h_sums = sums_h;
+    h_parts = parts_h;
     h_exact = exact_h;
 }
 
 void BounceBuffers::free_pinned() {
-    cudaFreeHost(h_sums);
+    cudaFreeHost(h_parts);
     cudaFreeHost(h_exact);
-    h_sums = nullptr;
+    h_parts = nullptr;
     h_exact = nullptr;
 }
 
-cudaError_t launch_patch_light(const BounceBuffers &b, const float4 *sample_light, cudaStream_t stream) {
-    if (b.npatches == 0) return cudaSuccess;
-    k_patch_samples<<<blocks(b.npatches, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, sample_light, b.acc);
-    k_patch_tree<<<blocks(b.nfaces, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, b.acc, b.direct, b.total,
-                                                                              b.emit[0], b.shoot[0]);
+template <int OP>
+static cudaError_t launch_parents(const BounceBuffers &b, float4 *light, float4 *emit, float4 *shoot,
+                                  cudaStream_t stream) {
+    if (b.nparents == 0) return cudaSuccess;
+    k_parents<OP><<<b.nfaces, kFaceThreads, 0, stream>>>(
+        b.view, b.face_level, b.level_off, b.parent, b.share, light, emit, shoot);
     return cudaGetLastError();
+}
+
+cudaError_t launch_bounce_tables(const BounceBuffers &b, const FinalView &fv, float4 *face_fit, cudaStream_t stream) {
+    if (b.nfaces)
+        k_face_fit<<<blocks((int64_t)b.nfaces * 32, kBounceBlock), kBounceBlock, 0, stream>>>(
+            b.view, fv.face_cells, fv.frames, fv.cell_sample, face_fit);
+    if (b.npatches)
+        k_patch_boxes<<<blocks(b.npatches, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, fv.frames, face_fit,
+                                                                                     b.patch_box);
+    if (b.nparents)
+        k_parent_records<<<blocks(b.nparents, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, b.parent_list, b.nparents,
+                                                                                        b.parent, b.share);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_sell_pad(const BounceBuffers &b, unsigned long long *d_pad, cudaStream_t stream) {
+    if (b.nreceivers == 0) return cudaSuccess;
+    k_sell_pad<<<blocks(b.nreceivers, b.sell_window), 256, 0, stream>>>(b.nreceivers, b.sell_window, b.cand_off, d_pad);
+    return cudaGetLastError();
+}
+
+cudaError_t sell_sort(BounceBuffers &b, int32_t window, void *tmp, size_t &bytes, cudaStream_t stream) {
+    const int nwindows = (int)blocks(b.nreceivers, window);
+    int bits = kCountBits;
+    while (bits < 32 && ((int64_t)nwindows - 1) >> (bits - kCountBits)) bits++;
+    return cub::DeviceRadixSort::SortPairs(tmp, bytes, b.sell_key, b.sell_sorted, b.sell_idx, b.sell_order, b.nreceivers,
+                                           0, bits, stream);
+}
+
+cudaError_t launch_patch_light(const BounceBuffers &b, const FinalView &fv, const float4 *sample_light,
+                               cudaStream_t stream) {
+    if (b.npatches == 0) return cudaSuccess;
+    k_patch_samples<<<blocks(b.npatches, kBounceBlock), kBounceBlock, 0, stream>>>(
+        b.view, b.patch_box, fv.face_cells, fv.frames, fv.cell_sample, sample_light, b.direct, b.total, b.emit[0],
+        b.shoot[0]);
+    const cudaError_t e = cudaGetLastError();
+    return e != cudaSuccess ? e : launch_parents<kOpDirect>(b, b.direct, b.emit[0], b.shoot[0], stream);
 }
 
 // The transfer build.  count_only: the candidate counts and offsets alone
@@ -784,39 +988,27 @@ cudaError_t launch_transfers(BounceBuffers &b, const DeviceScene &scene, uint32_
     k_transfer_write<<<blocks((int64_t)R * 32, kBounceBlock), kBounceBlock, 0, stream>>>(
         R, b.cand_off, b.cand_src, b.cand_w, b.tr_off, b.tr);
     e = cudaGetLastError();
-    return e != cudaSuccess ? e : launch_sell(b, stream);
+    return e != cudaSuccess ? e : launch_sell(b, b.sell_window, stream);
 }
 
 // The gather's slices (SELL-32) from the transfer lists tr_off / tr.
-cudaError_t launch_sell(BounceBuffers &b, cudaStream_t stream) {
+cudaError_t launch_sell(BounceBuffers &b, int32_t window, cudaStream_t stream) {
     const int R = b.nreceivers;
     if (R == 0) return cudaSuccess;
     cudaError_t e = cudaSuccess;
     size_t tmp = 0;
     const int nslices = (R + 31) / 32;
-    k_sell_keys<<<blocks(R, kBounceBlock), kBounceBlock, 0, stream>>>(R, b.tr_off, b.sell_key, b.sell_idx);
+    k_sell_keys<<<blocks(R, kBounceBlock), kBounceBlock, 0, stream>>>(R, window, b.tr_off, b.sell_key, b.sell_idx);
     tmp = b.sort_tmp_bytes;
-    e = cub::DeviceRadixSort::SortPairsDescending(b.sort_tmp, tmp, b.sell_key, b.sell_count, b.sell_idx, b.sell_order,
-                                                  R, 0, 20, stream);
+    e = sell_sort(b, window, b.sort_tmp, tmp, stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(b.sell_off, 0, sizeof(int64_t), stream);
     if (e != cudaSuccess) return e;
-    k_sell_width<<<blocks(nslices, kBounceBlock), kBounceBlock, 0, stream>>>(R, nslices, b.sell_count, b.sell_off + 1);
+    k_sell_width<<<blocks(nslices, kBounceBlock), kBounceBlock, 0, stream>>>(nslices, b.sell_sorted, b.sell_off + 1);
     tmp = b.scan_tmp_bytes;
     e = cub::DeviceScan::InclusiveSum(b.scan_tmp, tmp, b.sell_off + 1, b.sell_off + 1, nslices, stream);
     if (e != cudaSuccess) return e;
-    k_sell_pack<<<blocks(R, kBounceBlock), kBounceBlock, 0, stream>>>(R, b.sell_order, b.sell_count, b.sell_off,
+    k_sell_pack<<<blocks(R, kBounceBlock), kBounceBlock, 0, stream>>>(R, b.sell_order, b.sell_sorted, b.sell_off,
                                                                       b.tr_off, b.tr, b.sell);
-    return cudaGetLastError();
-}
-
-// CollectLight's parents, level by level.
-cudaError_t launch_collect(const BounceBuffers &b, float4 *emit_out, float4 *shoot_out, cudaStream_t stream) {
-    for (size_t h = 1; h + 1 < b.h_level_off.size(); h++) {
-        const int32_t a = b.h_level_off[h], n = b.h_level_off[h + 1] - a;
-        if (n > 0)
-            k_collect_level<<<blocks(n, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, b.level_patch + a, n, b.total,
-                                                                                  emit_out, shoot_out);
-    }
     return cudaGetLastError();
 }
 
@@ -824,17 +1016,16 @@ cudaError_t launch_collect(const BounceBuffers &b, float4 *emit_out, float4 *sho
 // other half, then the fp64 totals.
 cudaError_t launch_gather(BounceBuffers &b, int bounce, cudaStream_t stream) {
     const int in = bounce & 1, out = in ^ 1;
+    cudaError_t e = cudaMemsetAsync(b.sums, 0, kSumParts * kSums * sizeof(double), stream);
+    if (e != cudaSuccess) return e;
     if (b.nreceivers)
         k_gather<<<blocks(b.nreceivers, kBounceBlock), kBounceBlock, 0, stream>>>(
-            b.view, b.sell_order, b.sell_count, b.sell_off, b.sell, b.shoot[in], b.total, b.emit[out], b.shoot[out]);
-    cudaError_t e = launch_collect(b, b.emit[out], b.shoot[out], stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b.sums, 0, kSums * sizeof(double), stream);
-    if (e != cudaSuccess) return e;
-    if (b.npatches)
-        k_totals<<<blocks(b.npatches, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, b.emit[out], b.leaf_rank,
-                                                                                b.nleaves, b.sums);
+            b.view, b.sell_order, b.sell_sorted, b.sell_off, b.sell, b.shoot[in], b.total, b.emit[out], b.shoot[out],
+            b.leaf_rank, b.nleaves, b.sums);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = launch_parents<kOpCollect>(b, b.total, b.emit[out], b.shoot[out], stream);
     b.last_buffer = out;
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t launch_features(BounceBuffers &b, const DeviceWorld &w, cudaStream_t stream) {
@@ -854,21 +1045,17 @@ cudaError_t launch_warm_start(BounceBuffers &b, const DeviceWorld &w, const vrad
     if (e == cudaSuccess) e = cudaMemsetAsync(b.guess, 0, sizeof(float4) * (size_t)b.npatches, stream);
     if (e != cudaSuccess) return e;
     k_guess<<<blocks(b.nreceivers, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, b.pred, b.guess);
-    for (size_t h = 1; h + 1 < b.h_level_off.size(); h++) {
-        const int32_t a = b.h_level_off[h], n = b.h_level_off[h + 1] - a;
-        if (n > 0)
-            k_blend_level<<<blocks(n, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, b.level_patch + a, n, b.guess);
-    }
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = launch_parents<kOpGuess>(b, b.guess, nullptr, nullptr, stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(b.sums, 0, kSumParts * kSums * sizeof(double), stream);
+    if (e != cudaSuccess) return e;
     // Bounce 0 wrote half 1; the warm step writes half 0, as bounce 1 would.
     k_warm_combine<<<blocks(b.nreceivers, kBounceBlock), kBounceBlock, 0, stream>>>(
-        b.view, b.sell_order, b.sell_count, b.sell_off, b.sell, b.guess, b.first, b.total, b.emit[0], b.shoot[0]);
-    e = launch_collect(b, b.emit[0], b.shoot[0], stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b.sums, 0, kSums * sizeof(double), stream);
-    if (e != cudaSuccess) return e;
-    k_totals<<<blocks(b.npatches, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, b.emit[0], b.leaf_rank, b.nleaves,
-                                                                            b.sums);
+        b.view, b.sell_order, b.sell_sorted, b.sell_off, b.sell, b.guess, b.first, b.total, b.emit[0], b.shoot[0],
+        b.leaf_rank, b.nleaves, b.sums);
+    e = cudaGetLastError();
     b.last_buffer = 0;
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : launch_parents<kOpCollect>(b, b.total, b.emit[0], b.shoot[0], stream);
 }
 
 cudaError_t launch_bounce_graph(BounceBuffers &b, int bounce, cudaStream_t capture, cudaStream_t stream) {
@@ -879,7 +1066,8 @@ cudaError_t launch_bounce_graph(BounceBuffers &b, int bounce, cudaStream_t captu
         if (e != cudaSuccess) return e;
         cudaError_t inside = launch_gather(b, bounce, capture);
         if (inside == cudaSuccess)
-            inside = cudaMemcpyAsync(b.h_sums, b.sums, kSums * sizeof(double), cudaMemcpyDeviceToHost, capture);
+            inside = cudaMemcpyAsync(b.h_parts, b.sums, kSumParts * kSums * sizeof(double), cudaMemcpyDeviceToHost,
+                                     capture);
         e = cudaStreamEndCapture(capture, &g);
         if (e == cudaSuccess) e = inside;
         if (e == cudaSuccess) e = cudaGraphInstantiate(&b.bounce_graph[k], g, 0);

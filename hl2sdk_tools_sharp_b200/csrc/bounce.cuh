@@ -23,12 +23,12 @@
 //                       transfer each earns (0 when blocked or none)
 //   tr_off[R+1] int64, tr[T] int2 (source, weight bits): the transfer lists
 //                       (TransferSet), by receiver
-//   acc[P] float4 (sample light xyz, sample area); direct[P], total[P],
-//   emit[2][P], shoot[2][P] float4: PatchLighting and Radiosity state
+//   direct[P], total[P], emit[2][P], shoot[2][P] float4: PatchLighting and Radiosity state
 #pragma once
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -42,8 +42,19 @@ struct vrad_mlp;
 
 namespace vrad {
 
+struct FinalView;
+
 constexpr int64_t kMaxTransfersPerReceiver = 4 * 65536;  // VisMatrix.MaxPatches
-constexpr int kSums = 9;  // doubles in BounceBuffers::sums
+constexpr int kSums = 9;  // doubles in a part of BounceBuffers::sums
+constexpr int kSumParts = 64;
+constexpr int kCountBits = 20;  // of a SELL key: a receiver has at most 2^18 transfers
+constexpr uint32_t kCountMask = (1u << kCountBits) - 1;
+// Receivers to a window of the slices' sort, for `receivers` in all: 1024
+// (k_gather), or so many that the windows' numbers fit the key's other 12 bits.
+inline int32_t sell_window(int32_t receivers) {
+    const int64_t least = ((int64_t)receivers + 4095) / 4096;
+    return (int32_t)std::max<int64_t>(1024, (least + 31) / 32 * 32);
+}
 constexpr int kFeatures = 32;                            // the warm start network's inputs
 
 struct BounceView {
@@ -85,29 +96,38 @@ struct BounceBuffers {
     int2 *tr = nullptr;            // T
     void *scan_tmp = nullptr;
     size_t scan_tmp_bytes = 0;
-    // The transfers again, in slices for the gather (SELL-32): receivers
-    // sorted by transfer count, descending (stable), 32 to a slice; entry j
-    // of lane l of slice s at sell[sell_off[s] + 32 j + l], so a warp's
-    // loads of step j are one contiguous 256 B row.
-    int32_t *sell_key = nullptr, *sell_idx = nullptr;      // R: counts and receivers before the sort
-    int32_t *sell_count = nullptr, *sell_order = nullptr;  // R: after it
+    // The transfers again, in slices for the gather (SELL-32): each window of
+    // sell_window consecutive receivers sorted by transfer count, descending
+    // (stable), 32 receivers to a slice; entry j of lane l of slice s at
+    // sell[sell_off[s] + 32 j + l], so a warp's loads of step j are one
+    // contiguous 256 B row.  Keys: window << kCountBits | kCountMask - count.
+    uint32_t *sell_key = nullptr, *sell_sorted = nullptr;  // R: before and after the sort
+    int32_t *sell_idx = nullptr, *sell_order = nullptr;    // R: the receivers alike
+    int32_t sell_window = 0;  // a multiple of 32
+    int64_t sell_cap = 0;     // entries sell has room for
     int64_t *sell_off = nullptr;   // slices + 1
-    int2 *sell = nullptr;          // at most T + 32 * (the largest count) entries
+    int2 *sell = nullptr;          // at most T + 32 * (each window's largest count) entries
     void *sort_tmp = nullptr;
     size_t sort_tmp_bytes = 0;
     int64_t ncand = 0, ntransfers = 0;
     // Light state.
-    float4 *acc = nullptr, *direct = nullptr, *total = nullptr;
+    float4 *direct = nullptr, *total = nullptr;
     float4 *emit[2] = {nullptr, nullptr}, *shoot[2] = {nullptr, nullptr};
-    double *sums = nullptr;        // fp64 totals of a bounce (kSums): 3 sums, 3 absolute sums,
-                                   // 3 absolute sums weighted by the terms left in CollectLight's order
+    // fp64 totals of a bounce in kSumParts parts of kSums: 3 sums, 3 absolute
+    // sums, 3 absolute sums weighted by the terms left in CollectLight's order.
+    double *sums = nullptr;
     float *exact = nullptr;        // the sequential float total, when needed
     int32_t *leaf_desc = nullptr;  // the sky-free leaves, descending index (CollectLight's total order)
     int32_t *leaf_rank = nullptr;  // per patch: its position in leaf_desc, -1 off it
-    // CollectLight's parents by level (the depth of the subtree below):
-    // level h's are level_patch[h_level_off[h] .. h_level_off[h + 1]).
-    int32_t *level_patch = nullptr;
-    std::vector<int32_t> h_level_off;
+    // Each face's parents level by level, bottom up (a level: the depth of
+    // the subtree below): face f's level k are the entries level_off[face_level[f]
+    // + k] .. level_off[face_level[f] + k + 1] of parent (patch, its children,
+    // sky) and share (the children's shares of its area).
+    int32_t *face_level = nullptr, *level_off = nullptr, *parent_list = nullptr;
+    int4 *parent = nullptr;
+    float2 *share = nullptr;
+    int32_t nparents = 0;
+    int4 *patch_box = nullptr;     // per patch: its cells in reach (k_patch_boxes)
     // Learned warm start.
     float4 *first = nullptr;       // the first bounce's light per patch (bounce 0's total)
     float4 *guess = nullptr;       // the network's guess per patch
@@ -115,7 +135,8 @@ struct BounceBuffers {
     float *pred = nullptr;         // R x 3 outputs
     const vrad_mlp *model = nullptr;
     unsigned long long *counters = nullptr;  // [0] transfer rays, [1] blocked, [2] asin ties left open
-    double *h_sums = nullptr;      // pinned host copies
+    double *h_parts = nullptr;     // pinned host copy of the parts
+    double h_sums[9] = {};         // their sums (add_parts)
     float *h_exact = nullptr;
     // Final pass: each face's leaf patches whose radial box reaches it.
     int32_t *pr_off = nullptr;     // F + 1
@@ -131,8 +152,8 @@ struct BounceBuffers {
     int32_t max_bounces = 0;
     float threshold = 1.0f;
     int32_t last_buffer = 0;         // which emit/shoot half the last bounce wrote
-    // One bounce of each parity captured as a graph (gather, CollectLight's
-    // levels, the totals, their copy to h_sums), made on first use.
+    // One bounce of each parity captured as a graph (gather with the totals,
+    // CollectLight's parents, the totals' copy to h_parts), made on first use.
     cudaGraphExec_t bounce_graph[2] = {nullptr, nullptr};
     bool ready = false;
     // The transfer lists came from vrad_transfer_install: every light pass
@@ -146,20 +167,38 @@ struct BounceBuffers {
     float patch_light_ms = 0, transfer_ms = 0, bounce_ms = 0, final_ms = 0;
     unsigned long long rays = 0, blocked = 0, open_ties = 0;
 
+    // The last bounce's totals from the copied parts.
+    void add_parts() {
+        for (int k = 0; k < kSums; k++) {
+            h_sums[k] = 0.0;
+            for (int p = 0; p < kSumParts; p++) h_sums[k] += h_parts[kSums * p + k];
+        }
+    }
+
     void release();      // the device tables; the pinned sums stay
     void free_pinned();  // the pinned sums
 };
 
+// The tables the bounce's kernels read that follow from the uploaded patches
+// (the leaves' cells, the parents and their shares), once per upload;
+// face_fit: F float4 of scratch.
+cudaError_t launch_bounce_tables(const BounceBuffers &b, const FinalView &fv, float4 *face_fit, cudaStream_t stream);
+// How many entries the slices can need beyond the transfers, from the
+// candidate counts (cand_off), added to *d_pad.
+cudaError_t launch_sell_pad(const BounceBuffers &b, unsigned long long *d_pad, cudaStream_t stream);
+// The slices' sort: the bytes of its scratch (tmp == nullptr) or the sort.
+cudaError_t sell_sort(BounceBuffers &b, int32_t window, void *tmp, size_t &bytes, cudaStream_t stream);
 // Device phases of one bounce pass, all on `stream`.
-cudaError_t launch_patch_light(const BounceBuffers &b, const float4 *sample_light, cudaStream_t stream);
+cudaError_t launch_patch_light(const BounceBuffers &b, const FinalView &fv, const float4 *sample_light, cudaStream_t stream);
 cudaError_t launch_transfers(BounceBuffers &b, const DeviceScene &scene, uint32_t *overflow, cudaStream_t stream,
                              bool count_only);
 // The gather's slices from the transfer lists (the transfer build's last
-// step; also after the lists are installed from a cache).
-cudaError_t launch_sell(BounceBuffers &b, cudaStream_t stream);
+// step; also after the lists are installed from a cache), sorted within
+// windows of `window` receivers, a multiple of 32.
+cudaError_t launch_sell(BounceBuffers &b, int32_t window, cudaStream_t stream);
 cudaError_t launch_gather(BounceBuffers &b, int bounce, cudaStream_t stream);
 cudaError_t launch_exact_total(BounceBuffers &b, int bounce, cudaStream_t stream);
-// Bounce number `bounce` and the copy of its totals to h_sums as one graph
+// Bounce number `bounce` and the copy of its totals to h_parts as one graph
 // launch on `stream`; the graph of its parity is captured on `capture` (a
 // stream of the library's own) the first time.
 cudaError_t launch_bounce_graph(BounceBuffers &b, int bounce, cudaStream_t capture, cudaStream_t stream);

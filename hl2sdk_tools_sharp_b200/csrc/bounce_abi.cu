@@ -204,7 +204,7 @@ cudaError_t run_bounce(vrad_ctx *ctx, cudaStream_t s, const float4 *sample_light
     cudaError_t e = cudaSuccess;
     for (int k = 0; k < 4 && e == cudaSuccess; k++) e = cudaEventCreate(&ev[k]);
     if (e == cudaSuccess) e = cudaEventRecord(ev[0], s);
-    if (e == cudaSuccess) e = launch_patch_light(b, sample_light, s);
+    if (e == cudaSuccess) e = launch_patch_light(b, ctx->final_pass.view, sample_light, s);
     if (e == cudaSuccess) e = cudaEventRecord(ev[1], s);
     if (e == cudaSuccess) e = cudaMemsetAsync(b.counters, 0, 3 * sizeof(unsigned long long), s);
     if (e == cudaSuccess && build_transfers) e = launch_transfers(b, ctx->scene.view(), ctx->status, s, false);
@@ -212,7 +212,7 @@ cudaError_t run_bounce(vrad_ctx *ctx, cudaStream_t s, const float4 *sample_light
     b.bounces_run = 0;
     b.exact_totals = 0;
     // The float sum's error bound: u / (1 - n u) times the rank-weighted
-    // absolute sum (k_totals).
+    // absolute sum (add_totals).
     const double u = std::ldexp(1.0, -24);
     const double nu = (double)b.nleaves * u;
     const double scale = nu < 0.5 ? u / (1.0 - nu) : INFINITY;
@@ -227,10 +227,11 @@ cudaError_t run_bounce(vrad_ctx *ctx, cudaStream_t s, const float4 *sample_light
         if (e == cudaSuccess && i == 0)
             e = cudaMemcpyAsync(b.first, b.total, sizeof(float4) * (size_t)b.npatches, cudaMemcpyDeviceToDevice, s);
         if (e == cudaSuccess && !graph)
-            e = cudaMemcpyAsync(b.h_sums, b.sums, kSums * sizeof(double), cudaMemcpyDeviceToHost, s);
+            e = cudaMemcpyAsync(b.h_parts, b.sums, kSumParts * kSums * sizeof(double), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = vrad::wait_stream(s);
         if (e != cudaSuccess) break;
         b.bounces_run = i + 1;
+        b.add_parts();
         if (model) {
             // The warm iteration's changes can be negative: it stops on the
             // sum of their magnitudes.
@@ -474,42 +475,61 @@ extern "C" int32_t vrad_bounce_upload(vrad_ctx *ctx, const vrad_bounce_desc *d) 
     });
     // Each parent's level (1 + its deeper child's; leaves 0): a face's
     // tree is its root and its descendants, children numbered above their
-    // parent, so one descending pass per face, faces in parallel; then the
-    // parents grouped by level, index order within a level.
+    // parent, so one descending pass per face, faces in parallel; then each
+    // face's parents by level, descending index within a level.
     uvector<uint8_t> level((size_t)P, 0);
-    std::vector<int32_t> face_top((size_t)nf, 0);
-    parallel_for(nf, 16, [&](int64_t f) {
+    std::vector<int32_t> face_top((size_t)nf, 0), face_parents((size_t)nf, 0);
+    auto each_patch = [&](int64_t f, auto &&visit) {
         const int32_t root = tree.face_root[(size_t)f];
         if (root < 0) return;
-        int32_t top_f = 0;
-        auto visit = [&](int32_t i) {
+        for (int32_t i = tree.face_end[(size_t)f] - 1; i >= tree.face_first[(size_t)f]; i--) visit(i);
+        visit(root);
+    };
+    parallel_for(nf, 16, [&](int64_t f) {
+        int32_t top_f = 0, n = 0;
+        each_patch(f, [&](int32_t i) {
             const int4 t = tr[(size_t)i];
             if (t.y == -1) return;
             const int h = 1 + std::max(level[(size_t)t.y], level[(size_t)t.z]);
             level[(size_t)i] = (uint8_t)std::min(h, 255);
             top_f = std::max(top_f, h);
-        };
-        for (int32_t i = tree.face_end[(size_t)f] - 1; i >= tree.face_first[(size_t)f]; i--) visit(i);
-        visit(root);
+            n++;
+        });
         face_top[(size_t)f] = top_f;
+        face_parents[(size_t)f] = n;
     });
+    std::vector<int32_t> face_level((size_t)nf + 1, 0), first_parent((size_t)nf + 1, 0);
     int32_t top = 0;
-    for (int32_t f = 0; f < nf; f++) top = std::max(top, face_top[(size_t)f]);
+    for (int32_t f = 0; f < nf; f++) {
+        top = std::max(top, face_top[(size_t)f]);
+        face_level[(size_t)f + 1] = face_level[(size_t)f] + face_top[(size_t)f] + 1;
+        first_parent[(size_t)f + 1] = first_parent[(size_t)f] + face_parents[(size_t)f];
+    }
     if (top > 255) {
         vrad::wait_stream(rs);  // no DMA still reads the shelf or writes a released block
         b.release();
         return vrad_fail(ctx, VRAD_ERR_UNSUPPORTED, "a patch's subtree is deeper than 255 levels");
     }
-    std::vector<int32_t> level_off((size_t)top + 2, 0);
-    for (int32_t i = 0; i < P; i++)
-        if (level[(size_t)i]) level_off[(size_t)level[(size_t)i] + 1]++;
-    for (int32_t h = 0; h <= top; h++) level_off[(size_t)h + 1] += level_off[(size_t)h];
-    uvector<int32_t> level_patch((size_t)level_off[(size_t)top + 1]);
-    {
-        std::vector<int32_t> at(level_off.begin(), level_off.end() - 1);
-        for (int32_t i = 0; i < P; i++)
-            if (level[(size_t)i]) level_patch[(size_t)at[level[(size_t)i]]++] = i;
-    }
+    const int32_t nparents = first_parent[(size_t)nf];
+    uvector<int32_t> level_off((size_t)face_level[(size_t)nf]), parent_list((size_t)nparents);
+    parallel_for(nf, 16, [&](int64_t f) {
+        int32_t *off = level_off.data() + face_level[(size_t)f];
+        const int32_t n = face_top[(size_t)f];
+        int32_t at[256] = {};
+        each_patch(f, [&](int32_t i) {
+            if (level[(size_t)i]) at[level[(size_t)i] - 1]++;
+        });
+        int32_t o = first_parent[(size_t)f];
+        for (int32_t h = 0; h < n; h++) {
+            const int32_t c = at[h];
+            off[h] = at[h] = o;
+            o += c;
+        }
+        off[n] = o;
+        each_patch(f, [&](int32_t i) {
+            if (level[(size_t)i]) parent_list[(size_t)at[level[(size_t)i] - 1]++] = i;
+        });
+    });
     // FacesInRow: each visible cluster's faces, in face order (one leaf per
     // cluster, whose faces are the faces that lie in it).
     std::vector<std::vector<int32_t>> cluster_faces((size_t)C);
@@ -542,7 +562,9 @@ extern "C" int32_t vrad_bounce_upload(vrad_ctx *ctx, const vrad_bounce_desc *d) 
     if (e == cudaSuccess) e = stage_table(ctx->stager, ctx->stream, &b.recv, recv);
     if (e == cudaSuccess) e = stage_table(ctx->stager, ctx->stream, &b.leaf_desc, leaf_desc);
     if (e == cudaSuccess) e = stage_table(ctx->stager, ctx->stream, &b.leaf_rank, leaf_rank);
-    if (e == cudaSuccess) e = stage_table(ctx->stager, ctx->stream, &b.level_patch, level_patch);
+    if (e == cudaSuccess) e = stage_table(ctx->stager, ctx->stream, &b.face_level, face_level);
+    if (e == cudaSuccess) e = stage_table(ctx->stager, ctx->stream, &b.level_off, level_off);
+    if (e == cudaSuccess) e = stage_table(ctx->stager, ctx->stream, &b.parent_list, parent_list);
     if (e == cudaSuccess) e = stage_table(ctx->stager, ctx->stream, &b.row_off, row_off);
     if (e == cudaSuccess) e = stage_table(ctx->stager, ctx->stream, &b.row_faces, row_faces);
     if (e == cudaSuccess) e = stage_table(ctx->stager, ctx->stream, &b.sample_area, sample_area);
@@ -551,12 +573,16 @@ extern "C" int32_t vrad_bounce_upload(vrad_ctx *ctx, const vrad_bounce_desc *d) 
     if (e == cudaSuccess) e = dev_alloc(&b.cand_off, sizeof(int64_t) * R1);
     if (e == cudaSuccess) e = dev_alloc(&b.tr_off, sizeof(int64_t) * R1);
     if (e == cudaSuccess) e = dev_alloc(&b.start, sizeof(int32_t) * R1);
-    for (float4 **q : {&b.acc, &b.direct, &b.total, &b.emit[0], &b.emit[1], &b.shoot[0], &b.shoot[1]})
+    const size_t M1 = (size_t)(nparents ? nparents : 1);
+    if (e == cudaSuccess) e = dev_alloc(&b.parent, sizeof(int4) * M1);
+    if (e == cudaSuccess) e = dev_alloc(&b.share, sizeof(float2) * M1);
+    if (e == cudaSuccess) e = dev_alloc(&b.patch_box, sizeof(int4) * P1);
+    for (float4 **q : {&b.direct, &b.total, &b.emit[0], &b.emit[1], &b.shoot[0], &b.shoot[1]})
         if (e == cudaSuccess) e = dev_alloc(q, sizeof(float4) * P1);
-    if (e == cudaSuccess) e = dev_alloc(&b.sums, kSums * sizeof(double));
+    if (e == cudaSuccess) e = dev_alloc(&b.sums, kSumParts * kSums * sizeof(double));
     if (e == cudaSuccess) e = dev_alloc(&b.exact, 3 * sizeof(float));
     if (e == cudaSuccess) e = dev_alloc(&b.counters, 3 * sizeof(unsigned long long));
-    if (e == cudaSuccess && !b.h_sums) e = cudaMallocHost(&b.h_sums, kSums * sizeof(double));
+    if (e == cudaSuccess && !b.h_parts) e = cudaMallocHost(&b.h_parts, kSumParts * kSums * sizeof(double));
     if (e == cudaSuccess && !b.h_exact) e = cudaMallocHost(&b.h_exact, 3 * sizeof(float));
     if (e == cudaSuccess) e = dev_alloc(&b.first, sizeof(float4) * P1);
     if (e == cudaSuccess) e = dev_alloc(&b.guess, sizeof(float4) * P1);
@@ -565,23 +591,27 @@ extern "C" int32_t vrad_bounce_upload(vrad_ctx *ctx, const vrad_bounce_desc *d) 
     if (e == cudaSuccess) e = dev_alloc(&b.prad_light, sizeof(float4) * N1);
     if (e == cudaSuccess) e = dev_alloc(&b.prad_weight, sizeof(float) * N1);
     const int32_t nslices = (R + 31) / 32;
+    b.nreceivers = R;
+    b.sell_window = sell_window(R);
     if (e == cudaSuccess && R > 0) {
         // One scan buffer for the receiver scans and the slice scan; one
-        // sort buffer for the slices' count order.
+        // sort buffer for the slices' order.
         size_t need = 0, need2 = 0;
         e = cub::DeviceScan::InclusiveSum(nullptr, need, b.cand_off + 1, b.cand_off + 1, R);
         if (e == cudaSuccess) e = cub::DeviceScan::InclusiveSum(nullptr, need2, b.cand_off + 1, b.cand_off + 1, nslices);
         need = std::max(need, need2);
         if (e == cudaSuccess) e = dev_alloc(&b.scan_tmp, need ? need : 1);
         b.scan_tmp_bytes = need;
-        size_t sort = 0;
-        if (e == cudaSuccess)
-            e = cub::DeviceRadixSort::SortPairsDescending(nullptr, sort, (const int32_t *)nullptr, (int32_t *)nullptr,
-                                                          (const int32_t *)nullptr, (int32_t *)nullptr, R, 0, 20);
+        size_t sort = 0, all = 0;
+        if (e == cudaSuccess) e = sell_sort(b, b.sell_window, nullptr, sort, ctx->stream);
+        if (e == cudaSuccess) e = sell_sort(b, 32 * nslices, nullptr, all, ctx->stream);
+        sort = std::max(sort, all);
         if (e == cudaSuccess) e = dev_alloc(&b.sort_tmp, sort ? sort : 1);
         b.sort_tmp_bytes = sort;
     }
-    for (int32_t **q : {&b.sell_key, &b.sell_idx, &b.sell_count, &b.sell_order})
+    for (uint32_t **q : {&b.sell_key, &b.sell_sorted})
+        if (e == cudaSuccess) e = dev_alloc(q, sizeof(uint32_t) * (size_t)(R ? R : 1));
+    for (int32_t **q : {&b.sell_idx, &b.sell_order})
         if (e == cudaSuccess) e = dev_alloc(q, sizeof(int32_t) * (size_t)(R ? R : 1));
     if (e == cudaSuccess) e = dev_alloc(&b.sell_off, sizeof(int64_t) * ((size_t)nslices + 1));
     if (e != cudaSuccess) {
@@ -597,14 +627,18 @@ extern "C" int32_t vrad_bounce_upload(vrad_ctx *ctx, const vrad_bounce_desc *d) 
     b.max_bounces = d->bounces;
     b.threshold = d->threshold;
     b.h_recv = recv;
-    b.h_level_off = level_off;
+    b.nparents = nparents;
     b.view = BounceView{P, nf, R, b.origin, b.normal, b.mins, b.maxs, b.tree, b.refl, b.wind, b.points,
                         b.face_range, b.face_samples, b.face_plane, b.recv, b.row_off, b.row_faces, b.sample_area,
                         ctx->world.sample_pos};
     cudaStream_t s = ctx->stream;
+    float4 *face_fit = nullptr;
+    e = dev_alloc(&face_fit, sizeof(float4) * (size_t)(nf ? nf : 1));
+    if (e == cudaSuccess) e = launch_bounce_tables(b, ctx->final_pass.view, face_fit, s);
     // The final pass's patch tables over the smoothing neighbours, on the
-    // device from the uploaded patches.
-    e = radial_tables(b, ctx->final_pass.frames, nf, noff, nlist, ctx->stager, s);
+    // device from the uploaded patches (which waits for the stream).
+    if (e == cudaSuccess) e = radial_tables(b, ctx->final_pass.frames, nf, noff, nlist, ctx->stager, s);
+    dev_free(face_fit);
     if (e != cudaSuccess) {
         ctx->stager.finish(s);
         b.release();
@@ -618,7 +652,11 @@ extern "C" int32_t vrad_bounce_upload(vrad_ctx *ctx, const vrad_bounce_desc *d) 
     if (e == cudaSuccess) e = cudaMemsetAsync(walk_flag, 0, sizeof(uint32_t), s);
     if (e == cudaSuccess) e = launch_transfers(b, ctx->scene.view(), walk_flag, s, true);
     int64_t ncand = 0;
+    unsigned long long pad = 0;
+    if (e == cudaSuccess) e = cudaMemsetAsync(b.counters, 0, sizeof pad, s);
+    if (e == cudaSuccess) e = launch_sell_pad(b, b.counters, s);
     if (e == cudaSuccess && R > 0) e = cudaMemcpyAsync(&ncand, b.cand_off + R, sizeof ncand, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&pad, b.counters, sizeof pad, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = vrad::wait_stream(s);
     b.ncand = ncand;
     clock.mark("candidate count");
@@ -628,10 +666,11 @@ extern "C" int32_t vrad_bounce_upload(vrad_ctx *ctx, const vrad_bounce_desc *d) 
     // bound, so sizing needs no trace.
     uint32_t overflow = 0;
     if (e == cudaSuccess) e = dev_alloc(&b.tr, sizeof(int2) * (size_t)(ncand ? ncand : 1));
-    // The slices hold the transfers and at most 32 times the largest count
-    // of padding.
-    const int64_t sell_cap = ncand + 32 * std::min<int64_t>(kMaxTransfersPerReceiver, ncand);
-    if (e == cudaSuccess) e = dev_alloc(&b.sell, sizeof(int2) * (size_t)(sell_cap ? sell_cap : 1));
+    // The slices hold the transfers and at most, for each window, 32 times
+    // its largest count of padding; an installed set may have longer lists
+    // than candidates, and then takes one window (vrad_transfer_install).
+    b.sell_cap = ncand + std::max<int64_t>((int64_t)pad, 32 * std::min<int64_t>(kMaxTransfersPerReceiver, ncand));
+    if (e == cudaSuccess) e = dev_alloc(&b.sell, sizeof(int2) * (size_t)(b.sell_cap ? b.sell_cap : 1));
     if (e == cudaSuccess) e = cudaMemcpyAsync(&overflow, walk_flag, sizeof overflow, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = vrad::wait_stream(s);
     if (e != cudaSuccess) {

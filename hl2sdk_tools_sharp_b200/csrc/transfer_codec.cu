@@ -668,6 +668,17 @@ extern "C" int32_t vrad_transfer_install(vrad_ctx *ctx, const uint8_t *index, in
     // then the gather's slices.
     std::vector<int64_t> off((size_t)R + 1, 0);
     for (int32_t r = 0; r < R; r++) off[(size_t)r + 1] = off[(size_t)r] + set.counts[(size_t)b.h_recv[(size_t)r]];
+    // The slices' room was made for a set of this bounce's own candidates;
+    // one whose lists need more padding is sorted as one window, which needs
+    // 32 times the longest list at most.
+    int64_t room = set.total;
+    for (int32_t r0 = 0; r0 < R; r0 += b.sell_window) {
+        int64_t longest = 0;
+        for (int32_t r = r0; r < std::min(R, r0 + b.sell_window); r++)
+            longest = std::max(longest, off[(size_t)r + 1] - off[(size_t)r]);
+        room += 32 * longest;
+    }
+    const int32_t window = room <= b.sell_cap ? b.sell_window : (R + 31) / 32 * 32;
     cudaStream_t s = ctx->stream;
     int64_t *d_poff = nullptr;
     e = mem.get(&d_poff, sizeof(int64_t) * ((size_t)P + 1));
@@ -680,7 +691,7 @@ extern "C" int32_t vrad_transfer_install(vrad_ctx *ctx, const uint8_t *index, in
             R, b.recv, b.tr_off, d_poff, b.tr, set.arena);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = launch_sell(b, s);
+    if (e == cudaSuccess) e = launch_sell(b, window, s);
     if (e == cudaSuccess) e = wait_stream(s);
     if (e != cudaSuccess) {
         b.lists_ready = false;

@@ -158,6 +158,35 @@ def test_sample_runs_in_any_face_order_light_the_same_lump():
     assert np.array_equal(lumps[0], lumps[1])
 
 
+@pytest.mark.parametrize("samples", ["cell order", "reversed"])
+@pytest.mark.parametrize("chop", [2.0, 64.0], ids=["small", "large"])
+def test_patch_light_over_the_cells_in_reach(oracle_mod, samples, chop):
+    """The patches' direct light where a leaf looks at its own cells (the
+    samples in cell order) and where it looks at its whole face (they are
+    not), for leaves of a few samples and of many."""
+    w = rg.generate(rg.config_3x3(seed=2))
+    inp = L.prepare(w)
+    if samples == "reversed":
+        ff = inp.face_first
+        idx = np.concatenate([np.arange(ff[f], ff[f + 1])[::-1] for f in range(len(inp.faces))])
+        inp = L.LightingInputs(**{**inp.__dict__, "samples": inp.samples[idx].copy()})
+    off, lst = L.pvs_lists(w)
+    refl = L.face_reflectivity(w)
+    with L.LightingStage(w, inp) as st:
+        st.set_extra_passes(0)
+        st.upload_bounce(refl, off, lst, max_chop=chop, bounces=1)
+        st.light_pass()
+        total, direct = st.patch_light()
+        light = _sample_light(st)
+    ob = oracle_mod.Bounce(oracle_mod.kd_build(w.tri_verts, w.tri_ids), inp.faces, inp.verts, inp.samples,
+                           inp.face_first, refl, off, lst, max_chop=chop, bounces=1)
+    ob.transfers()
+    o_total, o_direct, _, _ = ob.run(light)
+    assert (direct > 0).any()
+    assert np.array_equal(_bits(direct), _bits(o_direct))
+    assert np.array_equal(_bits(total), _bits(o_total))
+
+
 def test_reupload_grows_the_patch_forest_ahead_and_keeps_the_lump():
     """A context that has bounced grows the next world's patch forest while
     the world uploads, with its last chop sizes; the bounce upload takes it

@@ -146,3 +146,44 @@ def test_a_set_of_another_patch_tree_is_refused_and_changes_nothing():
         lump, _, _ = st.light_pass()
         assert st.bounce_stats().transfers_cached == 0
     assert np.array_equal(lump, want)
+
+
+@pytest.mark.parametrize("lists", ["tails", "long"])
+def test_installed_lists_of_any_length_are_gathered_in_order(lists):
+    """One bounce over installed lists, each receiver's sum in its list's
+    order: lengths around the gather's batches, and a list in every 1024
+    receivers that is longer than the candidates the slices have room for."""
+    w = rg.generate(rg.config_3x3(seed=2))
+    inp = L.prepare(w)
+    patches, _ = L.build_patches(inp.faces, inp.verts, L.face_reflectivity(w))
+    pvs_off, pvs = L.pvs_lists(w)
+    rng = np.random.default_rng(3)
+    with L.LightingStage(w, inp) as st:
+        st.upload_bounce(L.face_reflectivity(w), pvs_off, pvs, bounces=1)
+        st.light_pass()
+        pairs = st.bounce_stats().transfer_rays
+        leaves = np.flatnonzero(patches["child1"] == -1)
+        leaves = leaves[np.argsort(patches["cluster"][leaves], kind="stable")]  # the receivers' order
+        counts = np.zeros(len(patches), np.int64)
+        counts[leaves] = rng.integers(0, 34, len(leaves)) if lists == "tails" else rng.integers(0, 3, len(leaves))
+        if lists == "long":
+            picks = leaves[::1024]
+            counts[picks] = 40000
+            assert counts.max() < 4 * 65536 and 32 * counts[picks].sum() > pairs + 32 * min(4 * 65536, pairs)
+        assert counts.sum() <= pairs
+        off = np.concatenate([[0], np.cumsum(counts)])
+        tr = np.zeros(off[-1], O.TRANSFER_DTYPE)
+        tr["patch"] = rng.integers(0, len(patches), len(tr))
+        tr["weight"] = rng.random(len(tr), np.float32) * np.float32(0.01)
+        sets = [tr[off[p]:off[p + 1]] for p in range(len(patches))]
+        assert C.install(st, O.index(sets), [C.pack(c) for c in O.chunks(sets, 1 << 20)])
+        st.light_pass()
+        # What each patch shoots is its direct light times its reflectivity.
+        total, direct = st.patch_light()
+    shoot = direct.astype(np.float32) * patches["reflectivity"]
+    term = shoot[tr["patch"]] * tr["weight"][:, None]
+    for p in leaves[::7] if lists == "tails" else leaves[::1024]:
+        want = np.add.accumulate(np.concatenate([np.zeros((1, 3), np.float32), term[off[p]:off[p + 1]]]), axis=0)[-1]
+        if patches["sky"][p]:
+            want = np.zeros(3, np.float32)
+        assert np.array_equal(total[p].view(np.uint32), want.astype(np.float32).view(np.uint32)), p
