@@ -30,8 +30,9 @@
 //   k_parents         one block per face: the parents level by level, bottom
 //                     up (the direct light's area blends; after each bounce
 //                     CollectLight's; the warm start's)
-//   k_candidates      one thread per receiver: the candidate sources in the
-//                     enumerator's order (a counting and a writing launch)
+//   k_candidates      one lane per receiver, one walk per warp: the candidate
+//                     sources in the enumerator's order (a counting launch
+//                     at the upload, a writing one)
 //   k_transfer        one thread per candidate: the transfer ray, traced
 //                     in-thread, and MakeTransfer for an open pair
 //   k_transfer_count / k_transfer_write  one warp per receiver: the
@@ -281,6 +282,26 @@ __global__ void k_parent_records(BounceView v, const int32_t *__restrict__ list,
     share[i] = make_float2(__fdiv_rn(a1, __fadd_rn(a1, a2)), __fdiv_rn(a2, __fadd_rn(a1, a2)));
 }
 
+// The faces' roots, as the candidate walk reads them.
+__global__ void k_roots(BounceView v, float4 *__restrict__ plane, float4 *__restrict__ origin,
+                        int4 *__restrict__ tree) {
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= v.nfaces) return;
+    const int root = __ldg(&v.face_range[f].x);
+    if (root < 0) {
+        tree[f] = make_int4(-1, -1, -1, f);
+        // No receiver lies in front of it.
+        plane[f] = make_float4(0.0f, 0.0f, 0.0f, FLT_MAX);
+        origin[f] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        return;
+    }
+    const int4 tr = __ldg(&v.tree[root]);
+    const float4 n = __ldg(&v.normal[root]);
+    plane[f] = make_float4(n.x, n.y, n.z, __double2float_rd((double)n.w + 0.01));
+    origin[f] = __ldg(&v.origin[root]);
+    tree[f] = make_int4(root, tr.y, tr.z, f);
+}
+
 // One block per face: its parents level by level, bottom up, so that every
 // parent reads final children.  A level is a few loads that wait for one
 // another, so what it costs is launches and latency: a launch per level over
@@ -335,55 +356,131 @@ __global__ void __launch_bounds__(kFaceThreads)
 // Enumerator.Run for one receiver: the faces of its cluster's PVS row
 // other than its own, each tested with TestPatchToFace, then its patch
 // tree walked as TestPatchToPatch recurses (child1's subtree before
-// child2's).  Counts (out == nullptr) or writes the candidates.
-__global__ void k_candidates(BounceView v, const int64_t *__restrict__ cand_off, int64_t *__restrict__ counts,
-                             int32_t *__restrict__ out, uint32_t *__restrict__ overflow) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= v.nreceivers) return;
-    const int p = __ldg(&v.recv[r]);
-    const F3 o = f3(__ldg(&v.origin[p]));
-    const float4 mn = __ldg(&v.mins[p]), mx = __ldg(&v.maxs[p]);
-    const int face = __float_as_int(mn.w), cluster = __float_as_int(mx.w);
-    const float4 pl = __ldg(&v.face_plane[face]);
-    const F3 me_n = {pl.x, pl.y, pl.z};
-    const double me_d = (double)__ldg(&v.normal[p].w) + 0.01;
-    int64_t n = 0;
-    int64_t at = out ? cand_off[r] : 0;
-    int stack[kEnumStack];
-    const int q0 = __ldg(&v.row_off[cluster]), q1 = __ldg(&v.row_off[cluster + 1]);
-    for (int q = q0; q < q1; q++) {
-        const int g = __ldg(&v.row_faces[q]);
-        if (g == face) continue;
-        const int root = __ldg(&v.face_range[g].x);
-        if (root < 0) continue;
-        const float4 rn = __ldg(&v.normal[root]);
-        if (!((double)dot3(o, f3(rn)) > (double)rn.w + 0.01)) continue;
-        int sp = 0;
-        stack[sp++] = root;
-        while (sp > 0) {
-            const int s = stack[--sp];
-            const int4 tr = __ldg(&v.tree[s]);
-            const float4 so = __ldg(&v.origin[s]);
-            if (tr.y != -1) {
-                const F3 d = sub3(o, f3(so));
-                if ((double)dot3(d, d) * 0.0625 < (double)so.w) {
+// child2's).  Counts, or writes the candidates.
+//
+// One lane per receiver, but one walk per warp: its receivers share the row
+// and lie beside each other, so nearly every node that one of them visits,
+// the others do.  A node is popped with the lanes that are to look at it,
+// loaded once for all, and its children are pushed with the lanes that
+// refine it; what a lane takes still comes in its own walk's order.  The
+// row's faces are staged 32 at a time in shared memory.
+//
+// The comparisons are the reference's, which widens to double, as float
+// comparisons that say the same: x > d of a float x and a double d is x > the
+// largest float up to d; x / 16 < a is x < 16 a, both products exact.
+//
+// What bounds it is the issue of the walk's steps, the union of 32 receivers'
+// (500 to 1700 nodes on the 3x3 grid of rooms), and for few receivers the
+// chain of one warp's, so then a row is cut into segments (row_segments) that
+// are warps of their own.  On the 8x8 grid (1 M receivers, 649 M candidates)
+// it takes 4.1 ms, a walk by each thread took 6.8; on the 3x3 grid (35 k,
+// 10 M) 0.24 ms in 16 segments, 0.40, 0.26 in 4 and 8, 0.59 in one, 0.66 by
+// each thread.  Candidates are held back until four make a 16 B store: one by
+// one the 8x8 grid takes 6.6 ms, by eight or in rows of 32 by warp 4.2.
+constexpr int kHold = 4;
+
+template <bool WRITE>
+__global__ void __launch_bounds__(kBounceBlock)
+    k_candidates(BounceView v, const float4 *__restrict__ root_plane, const float4 *__restrict__ root_origin,
+                 const int4 *__restrict__ root_tree, const int64_t *__restrict__ seg_off,
+                 int64_t *__restrict__ counts, int32_t *__restrict__ out, uint32_t *__restrict__ overflow) {
+    constexpr int kWarps = kBounceBlock / 32;
+    __shared__ float4 s_plane[kWarps][32], s_origin[kWarps][32];
+    __shared__ int4 s_tree[kWarps][32];
+    __shared__ int2 s_stack[kWarps][kEnumStack];
+    __shared__ int s_held[WRITE ? kHold : 1][kBounceBlock];
+    const int r = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool live = r < v.nreceivers;
+    const int seg = blockIdx.y, nseg = gridDim.y;
+    F3 o = {0.0f, 0.0f, 0.0f}, me_n = o;
+    float me_d = 0.0f;
+    int face = -1, cluster = -1;
+    int64_t first = 0;
+    if (live) {
+        const int p = __ldg(&v.recv[r]);
+        const float4 mn = __ldg(&v.mins[p]), mx = __ldg(&v.maxs[p]);
+        o = f3(__ldg(&v.origin[p]));
+        face = __float_as_int(mn.w);
+        cluster = __float_as_int(mx.w);
+        me_n = f3(__ldg(&v.face_plane[face]));
+        me_d = __double2float_rd((double)__ldg(&v.normal[p].w) + 0.01);
+        if (WRITE) first = seg_off[(int64_t)r * nseg + seg];
+    }
+    int64_t at = first;
+    auto take = [&](int s, const float4 &so) {
+        if (!(dot3(f3(so), me_n) > me_d)) return;
+        if (WRITE) {
+            s_held[at & (kHold - 1)][threadIdx.x] = s;
+            if ((at & (kHold - 1)) == kHold - 1) {
+                if (at - (kHold - 1) >= first)
+                    *(int4 *)(out + at - (kHold - 1)) = make_int4(s_held[0][threadIdx.x], s_held[1][threadIdx.x],
+                                                                  s_held[2][threadIdx.x], s_held[3][threadIdx.x]);
+                else
+                    for (int64_t q = first; q <= at; q++) out[q] = s_held[q & (kHold - 1)][threadIdx.x];
+            }
+        }
+        at++;
+    };
+    // Whether the lane refines the patch (takes its children instead).
+    auto refines = [&](const float4 &so, int child1) {
+        const F3 d = sub3(o, f3(so));
+        return child1 != -1 && dot3(d, d) < 16.0f * so.w;
+    };
+    unsigned todo = __ballot_sync(kFull, live);
+    while (todo) {
+        // The lanes of one cluster: all of them but where a warp straddles two.
+        const int c = __shfl_sync(kFull, cluster, __ffs(todo) - 1);
+        const bool mine = live && cluster == c;
+        todo &= ~__ballot_sync(kFull, mine);
+        const int row = __ldg(&v.row_off[c]), n = __ldg(&v.row_off[c + 1]) - row;
+        const int q0 = row + (int)((int64_t)n * seg / nseg), q1 = row + (int)((int64_t)n * (seg + 1) / nseg);
+        for (int q = q0; q < q1; q += 32) {
+            const int m = min(32, q1 - q);
+            __syncwarp();
+            if (lane < m) {
+                const int g = __ldg(&v.row_faces[q + lane]);
+                s_plane[warp][lane] = __ldg(&root_plane[g]);
+                s_origin[warp][lane] = __ldg(&root_origin[g]);
+                s_tree[warp][lane] = __ldg(&root_tree[g]);
+            }
+            __syncwarp();
+            for (int k = 0; k < m; k++) {
+                const int4 rt = s_tree[warp][k];
+                const float4 rp = s_plane[warp][k];
+                const bool pass = mine && rt.w != face && dot3(o, f3(rp)) > rp.w;
+                if (!__any_sync(kFull, pass)) continue;
+                const float4 ro = s_origin[warp][k];
+                const bool ref = pass && refines(ro, rt.y);
+                if (pass && !ref) take(rt.x, ro);
+                unsigned lanes = __ballot_sync(kFull, ref);
+                if (!lanes) continue;
+                int sp = 2;
+                if (lane < 2) s_stack[warp][lane] = make_int2(lane ? rt.y : rt.z, (int)lanes);
+                __syncwarp();
+                while (sp > 0) {
+                    const int2 top = s_stack[warp][--sp];
+                    const int4 tr = __ldg(&v.tree[top.x]);
+                    const float4 so = __ldg(&v.origin[top.x]);
+                    const bool in = ((unsigned)top.y >> lane) & 1u, refine = in && refines(so, tr.y);
+                    if (in && !refine) take(top.x, so);
+                    lanes = __ballot_sync(kFull, refine);
+                    if (!lanes) continue;
                     if (sp + 2 > kEnumStack) {
-                        atomicOr(overflow, 2u);
+                        if (lane == 0) atomicOr(overflow, 2u);
                         continue;
                     }
-                    stack[sp++] = tr.z;
-                    stack[sp++] = tr.y;
-                    continue;
+                    if (lane < 2) s_stack[warp][sp + lane] = make_int2(lane ? tr.y : tr.z, (int)lanes);
+                    sp += 2;
+                    __syncwarp();
                 }
-            }
-            if ((double)dot3(f3(so), me_n) > me_d) {
-                if (out) out[at] = s;
-                at++;
-                n++;
             }
         }
     }
-    if (!out) counts[r] = n;
+    if (!live) return;
+    if (!WRITE) counts[(int64_t)r * nseg + seg] = at - first;
+    if (WRITE)
+        for (int64_t q = max(first, at & ~(int64_t)(kHold - 1)); q < at; q++)
+            out[q] = s_held[q & (kHold - 1)][threadIdx.x];
 }
 
 // FormFactors.DiffToDiff(o1, n1, o2, n2): delta = normalise(o1 - o2), then
@@ -879,9 +976,9 @@ unsigned blocks(int64_t n, int per) { return (unsigned)((n + per - 1) / per); }
 
 void BounceBuffers::release() {
     void *ptrs[] = {origin, normal, mins, maxs, refl, tree, wind, points, face_range, face_samples, face_plane,
-                    recv, start, row_off, row_faces, sample_area, cand_off, cand_src, cand_w, tr_off, tr, scan_tmp,
+                    recv, start, row_off, row_faces, sample_area, cand_off, seg_off, cand_src, cand_w, tr_off, tr, scan_tmp,
                     direct, total, emit[0], emit[1], shoot[0], shoot[1], sums, exact, counters, leaf_desc,
-                    face_level, level_off, parent_list, parent, share, patch_box, leaf_rank,
+                    face_level, level_off, parent_list, parent, share, patch_box, root_plane, root_origin, root_tree, leaf_rank,
                     sell_key, sell_idx, sell_sorted, sell_order, sell_off, sell, sort_tmp,
                     first, guess, feat, pred,
                     pr_off, pr_patch, pr_box, pr_coord, prad_light, prad_weight};
@@ -917,6 +1014,9 @@ cudaError_t launch_bounce_tables(const BounceBuffers &b, const FinalView &fv, fl
     if (b.nfaces)
         k_face_fit<<<blocks((int64_t)b.nfaces * 32, kBounceBlock), kBounceBlock, 0, stream>>>(
             b.view, fv.face_cells, fv.frames, fv.cell_sample, face_fit);
+    if (b.nfaces)
+        k_roots<<<blocks(b.nfaces, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, b.root_plane, b.root_origin,
+                                                                             b.root_tree);
     if (b.npatches)
         k_patch_boxes<<<blocks(b.npatches, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, fv.frames, face_fit,
                                                                                      b.patch_box);
@@ -963,16 +1063,19 @@ cudaError_t launch_transfers(BounceBuffers &b, const DeviceScene &scene, uint32_
     size_t tmp = 0;
     if (count_only) {
         // Candidate counts into cand_off[1..R], then the exclusive scan.
-        k_candidates<<<blocks(R, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, nullptr, b.cand_off + 1, nullptr,
-                                                                           overflow);
-        e = cudaMemsetAsync(b.cand_off, 0, sizeof(int64_t), stream);
+        k_candidates<false><<<dim3(blocks(R, kBounceBlock), b.segments), kBounceBlock, 0, stream>>>(
+            b.view, b.root_plane, b.root_origin, b.root_tree, nullptr, b.seg_off + 1, nullptr, overflow);
+        e = cudaMemsetAsync(b.seg_off, 0, sizeof(int64_t), stream);
         if (e != cudaSuccess) return e;
         tmp = b.scan_tmp_bytes;
-        e = cub::DeviceScan::InclusiveSum(b.scan_tmp, tmp, b.cand_off + 1, b.cand_off + 1, R, stream);
+        e = cub::DeviceScan::InclusiveSum(b.scan_tmp, tmp, b.seg_off + 1, b.seg_off + 1, (int64_t)R * b.segments, stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpy2DAsync(b.cand_off, sizeof(int64_t), b.seg_off, sizeof(int64_t) * (size_t)b.segments,
+                                  sizeof(int64_t), (size_t)R + 1, cudaMemcpyDeviceToDevice, stream);
         return e != cudaSuccess ? e : cudaGetLastError();
     }
-    k_candidates<<<blocks(R, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, b.cand_off, nullptr, b.cand_src,
-                                                                       overflow);
+    k_candidates<true><<<dim3(blocks(R, kBounceBlock), b.segments), kBounceBlock, 0, stream>>>(
+        b.view, b.root_plane, b.root_origin, b.root_tree, b.seg_off, nullptr, b.cand_src, overflow);
     k_starts<<<blocks(R, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, scene.opaque, b.start);
     if (b.ncand > 0)
         k_transfer<kBlock><<<blocks(b.ncand, kBlock), kBlock, sizeof(int) * scene.stack_depth() * kBlock, stream>>>(

@@ -49,6 +49,12 @@ constexpr int kSums = 9;  // doubles in a part of BounceBuffers::sums
 constexpr int kSumParts = 64;
 constexpr int kCountBits = 20;  // of a SELL key: a receiver has at most 2^18 transfers
 constexpr uint32_t kCountMask = (1u << kCountBits) - 1;
+// Segments to a receiver's row in the candidate walk: as many as make 32 k
+// warps (seven rounds of the chip's 4736 resident ones, so that the last
+// round weighs little), up to 16 (k_candidates; about ten faces each then).
+inline int32_t row_segments(int32_t receivers) {
+    return (int32_t)std::min<int64_t>(16, std::max<int64_t>(1, 32 * 32768ll / std::max(receivers, 1)));
+}
 // Receivers to a window of the slices' sort, for `receivers` in all: 1024
 // (k_gather), or so many that the windows' numbers fit the key's other 12 bits.
 inline int32_t sell_window(int32_t receivers) {
@@ -90,6 +96,8 @@ struct BounceBuffers {
     float *sample_area = nullptr;
     // Transfer build.
     int64_t *cand_off = nullptr;   // R + 1
+    int64_t *seg_off = nullptr;    // R * segments + 1: the same by segment of the receiver's row
+    int32_t segments = 1;
     int32_t *cand_src = nullptr;   // Q
     float *cand_w = nullptr;       // Q
     int64_t *tr_off = nullptr;     // R + 1
@@ -127,6 +135,11 @@ struct BounceBuffers {
     int4 *parent = nullptr;
     float2 *share = nullptr;
     int32_t nparents = 0;
+    // Per face, what the candidate walk reads of its root: (normal, the
+    // largest float up to plane dist + 0.01), (origin, area), (patch, child1,
+    // child2, face).
+    float4 *root_plane = nullptr, *root_origin = nullptr;
+    int4 *root_tree = nullptr;
     int4 *patch_box = nullptr;     // per patch: its cells in reach (k_patch_boxes)
     // Learned warm start.
     float4 *first = nullptr;       // the first bounce's light per patch (bounce 0's total)

@@ -571,12 +571,18 @@ extern "C" int32_t vrad_bounce_upload(vrad_ctx *ctx, const vrad_bounce_desc *d) 
     clock.mark("tables copied");
     const size_t P1 = (size_t)(P ? P : 1), R1 = (size_t)R + 1, N1 = (size_t)(ncells ? ncells : 1);
     if (e == cudaSuccess) e = dev_alloc(&b.cand_off, sizeof(int64_t) * R1);
+    b.segments = row_segments(R);
+    if (e == cudaSuccess) e = dev_alloc(&b.seg_off, sizeof(int64_t) * ((size_t)R * (size_t)b.segments + 1));
     if (e == cudaSuccess) e = dev_alloc(&b.tr_off, sizeof(int64_t) * R1);
     if (e == cudaSuccess) e = dev_alloc(&b.start, sizeof(int32_t) * R1);
     const size_t M1 = (size_t)(nparents ? nparents : 1);
     if (e == cudaSuccess) e = dev_alloc(&b.parent, sizeof(int4) * M1);
     if (e == cudaSuccess) e = dev_alloc(&b.share, sizeof(float2) * M1);
     if (e == cudaSuccess) e = dev_alloc(&b.patch_box, sizeof(int4) * P1);
+    const size_t F1 = (size_t)(nf ? nf : 1);
+    if (e == cudaSuccess) e = dev_alloc(&b.root_plane, sizeof(float4) * F1);
+    if (e == cudaSuccess) e = dev_alloc(&b.root_origin, sizeof(float4) * F1);
+    if (e == cudaSuccess) e = dev_alloc(&b.root_tree, sizeof(int4) * F1);
     for (float4 **q : {&b.direct, &b.total, &b.emit[0], &b.emit[1], &b.shoot[0], &b.shoot[1]})
         if (e == cudaSuccess) e = dev_alloc(q, sizeof(float4) * P1);
     if (e == cudaSuccess) e = dev_alloc(&b.sums, kSumParts * kSums * sizeof(double));
@@ -597,7 +603,7 @@ extern "C" int32_t vrad_bounce_upload(vrad_ctx *ctx, const vrad_bounce_desc *d) 
         // One scan buffer for the receiver scans and the slice scan; one
         // sort buffer for the slices' order.
         size_t need = 0, need2 = 0;
-        e = cub::DeviceScan::InclusiveSum(nullptr, need, b.cand_off + 1, b.cand_off + 1, R);
+        e = cub::DeviceScan::InclusiveSum(nullptr, need, b.seg_off + 1, b.seg_off + 1, (int64_t)R * b.segments);
         if (e == cudaSuccess) e = cub::DeviceScan::InclusiveSum(nullptr, need2, b.cand_off + 1, b.cand_off + 1, nslices);
         need = std::max(need, need2);
         if (e == cudaSuccess) e = dev_alloc(&b.scan_tmp, need ? need : 1);
@@ -633,7 +639,7 @@ extern "C" int32_t vrad_bounce_upload(vrad_ctx *ctx, const vrad_bounce_desc *d) 
                         ctx->world.sample_pos};
     cudaStream_t s = ctx->stream;
     float4 *face_fit = nullptr;
-    e = dev_alloc(&face_fit, sizeof(float4) * (size_t)(nf ? nf : 1));
+    e = dev_alloc(&face_fit, sizeof(float4) * F1);
     if (e == cudaSuccess) e = launch_bounce_tables(b, ctx->final_pass.view, face_fit, s);
     // The final pass's patch tables over the smoothing neighbours, on the
     // device from the uploaded patches (which waits for the stream).

@@ -120,6 +120,34 @@ def test_8x8_transfers_sampled_and_bounce_bit_exact(oracle_mod):
     assert len(bad) == 0, f"{len(bad)} of {len(lump) // 4} RGBE words differ"
 
 
+@pytest.mark.parametrize("side,chop", [(1, 64.0), (2, 4.0), (4, 4.0), (5, 4.0)],
+                         ids=["few receivers", "16 segments", "9 segments", "2 segments"])
+def test_transfers_where_a_row_is_cut_into_segments(oracle_mod, side, chop):
+    """The candidate walk's split of a receiver's row: the transfers of
+    sampled receivers, the first and the last among them."""
+    w = rg.generate(rg.Config(side=side, seed=3, luxel_scale=32.0, pillars=(0, 3)))
+    inp = L.prepare(w)
+    off, lst = L.pvs_lists(w)
+    refl = L.face_reflectivity(w)
+    with L.LightingStage(w, inp) as st:
+        st.upload_bounce(refl, off, lst, max_chop=chop, bounces=1)
+        st.light_pass()
+        t_off, tr = st.transfers()
+    ob = oracle_mod.Bounce(oracle_mod.kd_build(w.tri_verts, w.tri_ids), inp.faces, inp.verts, inp.samples,
+                           inp.face_first, refl, off, lst, max_chop=chop, bounces=1)
+    patches, _ = ob.patches()
+    leaves = np.flatnonzero(patches["child1"] == -1)
+    pick = np.random.default_rng(7).choice(leaves, min(len(leaves), 300), replace=False)
+    sub = np.unique(np.concatenate([pick, leaves[[0, -1]]]))
+    o_off, o_src, o_w, _ = ob.transfers(sub)
+    assert o_off[-1] > 0
+    for p in sub:
+        a, b = t_off[p], t_off[p + 1]
+        c, d = o_off[p], o_off[p + 1]
+        assert np.array_equal(tr["patch"][a:b], o_src[c:d]), p
+        assert np.array_equal(_bits(tr["weight"][a:b]), _bits(o_w[c:d])), p
+
+
 def test_bounce_pass_is_repeatable_and_device_entry_matches():
     import torch
     w, inp, st = _stage(rg.config_3x3(seed=2))
