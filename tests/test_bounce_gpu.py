@@ -148,6 +148,29 @@ def test_transfers_where_a_row_is_cut_into_segments(oracle_mod, side, chop):
         assert np.array_equal(_bits(tr["weight"][a:b]), _bits(o_w[c:d])), p
 
 
+@pytest.mark.parametrize("luxel_scale", [200.0, 56.0, 24.0, 7.0])
+def test_lumps_of_faces_of_few_and_many_luxels(oracle_mod, luxel_scale):
+    """The final pass where a warp's cells are of many faces, of one and of a
+    part of one, and the medians of few and of many luxels."""
+    w = rg.generate(rg.Config(side=2, seed=5, luxel_scale=luxel_scale, pillars=(0, 4)))
+    inp = L.prepare(w)
+    off, lst = L.pvs_lists(w)
+    refl = L.face_reflectivity(w)
+    with L.LightingStage(w, inp) as st:
+        st.upload_bounce(refl, off, lst, bounces=2)
+        lump, lightofs, _ = st.light_pass()
+        t_off, tr = st.transfers()
+        light = _sample_light(st)
+    ob = oracle_mod.Bounce(oracle_mod.kd_build(w.tri_verts, w.tri_ids), inp.faces, inp.verts, inp.samples,
+                           inp.face_first, refl, off, lst, bounces=2)
+    ob.set_transfers(t_off, tr["patch"], tr["weight"])
+    ob.run(light)
+    want, want_ofs = ob.final(light)
+    assert np.array_equal(lightofs, want_ofs)
+    bad = np.flatnonzero(lump.view(np.uint32) != want.view(np.uint32))
+    assert len(bad) == 0, f"{len(bad)} of {len(lump) // 4} RGBE words differ"
+
+
 def test_bounce_pass_is_repeatable_and_device_entry_matches():
     import torch
     w, inp, st = _stage(rg.config_3x3(seed=2))
