@@ -45,8 +45,8 @@
 //                     CollectLight's leaf update, and fp64 sums of the light
 //                     the bounce added, with absolute sums that bound the
 //                     reference's float sum
-//   k_exact_total     one block: the reference's sequential float sum, run
-//                     only when the bound cannot settle the stop rule
+//   k_exact_*         the reference's sequential float sum, run only when
+//                     the bound cannot settle the stop rule
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -820,48 +820,127 @@ __global__ void __launch_bounds__(kBounceBlock)
 
 // CollectLight's own total: the leaves' emission summed in float, in
 // descending index order (leaf_desc lists the sky-free leaves that way).
-// The sum is one chain of dependent adds; one block keeps it fed: all of
-// its threads stage the next tile of values in shared memory while warp 0
-// adds up the current one, every lane of it the same chain.
-constexpr int kExactThreads = 1024;
-constexpr int kExactTile = 1024;  // two tiles of float4: 32 KB of shared memory
+// The sum is one chain of a million dependent, rounded adds, but while it
+// stays between two powers of two it is a whole number of ulps u, and adding
+// x >= 0 adds rint(x / u) of them, whatever the sum, unless x lies half way
+// between two ulps (then the sum's parity decides).  So the leaves are cut
+// into chunks:
+//   k_exact_sums   each chunk's sum in fp64
+//   k_exact_steps  each chunk's whole ulps, for the ulp at which the sums
+//                  before it say that it starts
+//   k_exact_walk   from chunk to chunk: a chunk whose start has that ulp,
+//                  that leaves it unchanged and that has no half way case
+//                  is one integer add; any other is added up value by value
+// A sum over 1 M leaves passes about twenty powers of two, so nearly every
+// chunk is one add: 0.5 ms, 5.0 as one chain of adds fed by a block.
+struct ExactStep {
+    long long ulps;
+    int32_t exponent;  // the biased exponent of the chunk's start
+    int32_t kind;      // kByValue, kByUlps, or kNothing: every value is zero
+};
+enum : int32_t { kByValue = 0, kByUlps = 1, kNothing = 2 };
+constexpr int kExactBlock = 128;
 
-__global__ void __launch_bounds__(kExactThreads) k_exact_total(const int32_t *__restrict__ leaf_desc, int32_t n,
-                                                               const float4 *__restrict__ emit, float *__restrict__ out) {
-    __shared__ float4 tile[2][kExactTile];
-    float x = 0.0f, y = 0.0f, z = 0.0f;
-    // Stages tile `buf` with threads [first, kExactThreads).
-    auto stage = [&](int buf, int base, int first) {
-        for (int k = (int)threadIdx.x - first; k < kExactTile; k += kExactThreads - first) {
-            const int i = base + k;
-            tile[buf][k] = i < n ? __ldg(&emit[__ldg(&leaf_desc[i])]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
-    };
-    stage(0, 0, 0);
+__device__ __forceinline__ float channel(const float4 &v, int c) { return c == 0 ? v.x : c == 1 ? v.y : v.z; }
+
+// The block's sum of x; every thread has it.
+template <typename T>
+__device__ __forceinline__ T block_sum(T x, T *part) {
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(kFull, x, o);
     __syncthreads();
-    for (int base = 0, buf = 0; base < n; base += kExactTile, buf ^= 1) {
-        if (threadIdx.x >= 32) {
-            stage(buf ^ 1, base + kExactTile, 32);
-        } else {
-            // The three chains of dependent adds; unrolled so the tile's
-            // loads run ahead of them.
-            const int m = min(kExactTile, n - base);
-            const float4 *t = tile[buf];
-#pragma unroll 16
-            for (int k = 0; k < m; k++) {
-                const float4 v = t[k];
-                x = __fadd_rn(x, v.x);
-                y = __fadd_rn(y, v.y);
-                z = __fadd_rn(z, v.z);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = x;
+    __syncthreads();
+    T t = part[0];
+    for (int w = 1; w < kExactBlock / 32; w++) t += part[w];
+    return t;
+}
+
+__global__ void __launch_bounds__(kExactBlock) k_exact_sums(const int32_t *__restrict__ leaf_desc, int32_t n, int per,
+                                                            int nchunks, const float4 *__restrict__ emit,
+                                                            double *__restrict__ sums) {
+    __shared__ double part[kExactBlock / 32];
+    double s[3] = {0.0, 0.0, 0.0};
+    const int64_t first = (int64_t)blockIdx.x * per, end = first + per < n ? first + per : n;
+    for (int64_t i = first + threadIdx.x; i < end; i += kExactBlock) {
+        const float4 v = __ldg(&emit[__ldg(&leaf_desc[i])]);
+        for (int c = 0; c < 3; c++) s[c] += (double)channel(v, c);
+    }
+    for (int c = 0; c < 3; c++) {
+        const double t = block_sum(s[c], part);
+        if (threadIdx.x == 0) sums[(int64_t)c * nchunks + blockIdx.x] = t;
+    }
+}
+
+__global__ void __launch_bounds__(kExactBlock) k_exact_steps(const int32_t *__restrict__ leaf_desc, int32_t n, int per,
+                                                             int nchunks, const float4 *__restrict__ emit,
+                                                             const double *__restrict__ sums,
+                                                             ExactStep *__restrict__ steps) {
+    __shared__ double part[kExactBlock / 32];
+    __shared__ long long ipart[kExactBlock / 32];
+    const int64_t first = (int64_t)blockIdx.x * per, end = first + per < n ? first + per : n;
+    for (int c = 0; c < 3; c++) {
+        double before = 0.0;
+        for (int k = threadIdx.x; k < (int)blockIdx.x; k += kExactBlock) before += __ldg(&sums[(int64_t)c * nchunks + k]);
+        const float start = (float)block_sum(before, part);
+        const int e = (int)(__float_as_uint(start) >> 23);
+        // 2^(150 - e), one over the ulp.
+        const double per_ulp = __longlong_as_double((long long)(1023 + 150 - e) << 52);
+        long long ulps = 0;
+        bool whole = e > 0 && e < 255, zero = true;
+        for (int64_t i = first + threadIdx.x; i < end; i += kExactBlock) {
+            const float x = channel(__ldg(&emit[__ldg(&leaf_desc[i])]), c);
+            zero = zero && x == 0.0f;
+            const double q = (double)x * per_ulp;
+            whole = whole && x >= 0.0f && q < 16777216.0 && q - floor(q) != 0.5;
+            if (whole) ulps += __double2ll_rn(q);
+        }
+        ulps = block_sum(ulps, ipart);
+        whole = __syncthreads_and(whole);
+        zero = __syncthreads_and(zero);
+        if (threadIdx.x == 0)
+            steps[(int64_t)c * nchunks + blockIdx.x] = {ulps, e, zero ? kNothing : whole ? kByUlps : kByValue};
+    }
+}
+
+// One warp per channel.
+__global__ void __launch_bounds__(96) k_exact_walk(const int32_t *__restrict__ leaf_desc, int32_t n, int per, int nchunks,
+                                                   const float4 *__restrict__ emit, const ExactStep *__restrict__ steps,
+                                                   float *__restrict__ out) {
+    const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto value = [&](int64_t i, int64_t end) {
+        return i < end ? channel(__ldg(&emit[__ldg(&leaf_desc[i])]), c) : 0.0f;
+    };
+    float s = 0.0f;
+    for (int base = 0; base < nchunks; base += 32) {
+        const int m = min(32, nchunks - base);
+        ExactStep mine = {0, 0, kNothing};
+        if (lane < m) mine = steps[(int64_t)c * nchunks + base + lane];
+        for (int j = 0; j < m; j++) {
+            const int kind = __shfl_sync(kFull, mine.kind, j);
+            const int e = __shfl_sync(kFull, mine.exponent, j);
+            const long long ulps = __shfl_sync(kFull, mine.ulps, j);
+            if (kind == kNothing) continue;
+            const uint32_t bits = __float_as_uint(s);
+            const long long k = (long long)((bits & 0x7FFFFFu) | 0x800000u) + ulps;
+            if (kind == kByUlps && (int)(bits >> 23) == e && k < 0x1000000) {
+                s = __uint_as_float(((uint32_t)e << 23) | ((uint32_t)k & 0x7FFFFFu));
+                continue;
+            }
+            const int64_t first = (int64_t)(base + j) * per, end = first + per < n ? first + per : n;
+            float next = value(first + lane, end);
+            for (int64_t i = first; i < end; i += 32) {
+                const float v = next;
+                next = value(i + 32 + lane, end);
+                if (i + 32 <= end) {
+#pragma unroll
+                    for (int l = 0; l < 32; l++) s = __fadd_rn(s, __shfl_sync(kFull, v, l));
+                } else {
+                    for (int l = 0; l < (int)(end - i); l++) s = __fadd_rn(s, __shfl_sync(kFull, v, l));
+                }
             }
         }
-        __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        out[0] = x;
-        out[1] = y;
-        out[2] = z;
-    }
+    if (lane == 0) out[c] = s;
 }
 
 // ---- the learned warm start --------------------------------------------------
@@ -977,7 +1056,7 @@ unsigned blocks(int64_t n, int per) { return (unsigned)((n + per - 1) / per); }
 void BounceBuffers::release() {
     void *ptrs[] = {origin, normal, mins, maxs, refl, tree, wind, points, face_range, face_samples, face_plane,
                     recv, start, row_off, row_faces, sample_area, cand_off, seg_off, cand_src, cand_w, tr_off, tr, scan_tmp,
-                    direct, total, emit[0], emit[1], shoot[0], shoot[1], sums, exact, counters, leaf_desc,
+                    direct, total, emit[0], emit[1], shoot[0], shoot[1], sums, exact, exact_sums, exact_steps, counters, leaf_desc,
                     face_level, level_off, parent_list, parent, share, patch_box, root_plane, root_origin, root_tree, leaf_rank,
                     sell_key, sell_idx, sell_sorted, sell_order, sell_off, sell, sort_tmp,
                     first, guess, feat, pred,
@@ -1184,8 +1263,29 @@ cudaError_t launch_bounce_graph(BounceBuffers &b, int bounce, cudaStream_t captu
     return cudaGraphLaunch(b.bounce_graph[k], stream);
 }
 
+cudaError_t alloc_exact(BounceBuffers &b) {
+    // Chunks of 512 leaves, or larger ones so that there are 4096 at most (a
+    // chunk's block adds up the sums before it).
+    b.exact_per = (int32_t)std::max<int64_t>(512, ((int64_t)b.nleaves + 4095) / 4096);
+    b.exact_chunks = (int32_t)(((int64_t)b.nleaves + b.exact_per - 1) / b.exact_per);
+    const size_t n = 3 * (size_t)std::max(b.exact_chunks, 1);
+    cudaError_t e = dev_alloc(&b.exact, 3 * sizeof(float));
+    if (e == cudaSuccess) e = dev_alloc(&b.exact_sums, n * sizeof(double));
+    if (e == cudaSuccess) e = dev_alloc(&b.exact_steps, n * sizeof(ExactStep));
+    return e;
+}
+
 cudaError_t launch_exact_total(BounceBuffers &b, int bounce, cudaStream_t stream) {
-    k_exact_total<<<1, kExactThreads, 0, stream>>>(b.leaf_desc, b.nleaves, b.emit[(bounce & 1) ^ 1], b.exact);
+    const float4 *emit = b.emit[(bounce & 1) ^ 1];
+    ExactStep *steps = (ExactStep *)b.exact_steps;
+    const int nchunks = b.exact_chunks;
+    if (nchunks) {
+        k_exact_sums<<<nchunks, kExactBlock, 0, stream>>>(b.leaf_desc, b.nleaves, b.exact_per, nchunks, emit,
+                                                          b.exact_sums);
+        k_exact_steps<<<nchunks, kExactBlock, 0, stream>>>(b.leaf_desc, b.nleaves, b.exact_per, nchunks, emit,
+                                                           b.exact_sums, steps);
+    }
+    k_exact_walk<<<1, 96, 0, stream>>>(b.leaf_desc, b.nleaves, b.exact_per, nchunks, emit, steps, b.exact);
     return cudaGetLastError();
 }
 

@@ -125,6 +125,9 @@ struct BounceBuffers {
     // sums, 3 absolute sums weighted by the terms left in CollectLight's order.
     double *sums = nullptr;
     float *exact = nullptr;        // the sequential float total, when needed
+    double *exact_sums = nullptr;  // per channel and chunk of exact_per leaves (k_exact_sums)
+    void *exact_steps = nullptr;   // alike (k_exact_steps)
+    int32_t exact_per = 0, exact_chunks = 0;
     int32_t *leaf_desc = nullptr;  // the sky-free leaves, descending index (CollectLight's total order)
     int32_t *leaf_rank = nullptr;  // per patch: its position in leaf_desc, -1 off it
     // Each face's parents level by level, bottom up (a level: the depth of
@@ -210,6 +213,8 @@ cudaError_t launch_transfers(BounceBuffers &b, const DeviceScene &scene, uint32_
 // windows of `window` receivers, a multiple of 32.
 cudaError_t launch_sell(BounceBuffers &b, int32_t window, cudaStream_t stream);
 cudaError_t launch_gather(BounceBuffers &b, int bounce, cudaStream_t stream);
+// The sequential total's buffers, for b.nleaves leaves.
+cudaError_t alloc_exact(BounceBuffers &b);
 cudaError_t launch_exact_total(BounceBuffers &b, int bounce, cudaStream_t stream);
 // Bounce number `bounce` and the copy of its totals to h_parts as one graph
 // launch on `stream`; the graph of its parity is captured on `capture` (a

@@ -586,7 +586,8 @@ extern "C" int32_t vrad_bounce_upload(vrad_ctx *ctx, const vrad_bounce_desc *d) 
     for (float4 **q : {&b.direct, &b.total, &b.emit[0], &b.emit[1], &b.shoot[0], &b.shoot[1]})
         if (e == cudaSuccess) e = dev_alloc(q, sizeof(float4) * P1);
     if (e == cudaSuccess) e = dev_alloc(&b.sums, kSumParts * kSums * sizeof(double));
-    if (e == cudaSuccess) e = dev_alloc(&b.exact, 3 * sizeof(float));
+    b.nleaves = nleaves;
+    if (e == cudaSuccess) e = alloc_exact(b);
     if (e == cudaSuccess) e = dev_alloc(&b.counters, 3 * sizeof(unsigned long long));
     if (e == cudaSuccess && !b.h_parts) e = cudaMallocHost(&b.h_parts, kSumParts * kSums * sizeof(double));
     if (e == cudaSuccess && !b.h_exact) e = cudaMallocHost(&b.h_exact, 3 * sizeof(float));

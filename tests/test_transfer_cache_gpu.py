@@ -187,3 +187,46 @@ def test_installed_lists_of_any_length_are_gathered_in_order(lists):
         if patches["sky"][p]:
             want = np.zeros(3, np.float32)
         assert np.array_equal(total[p].view(np.uint32), want.astype(np.float32).view(np.uint32)), p
+
+
+@pytest.mark.parametrize("values", ["wide", "half ways", "mostly zero", "negative", "infinite"])
+def test_the_total_is_the_sequential_sum(values):
+    """CollectLight's float total of one bounce: one installed transfer per
+    leaf makes its light any value, and the total is the sequential sum of
+    those, in descending order of the leaves, to the bit."""
+    w = rg.generate(rg.config_3x3(seed=2))
+    inp = L.prepare(w)
+    patches, _ = L.build_patches(inp.faces, inp.verts, L.face_reflectivity(w))
+    pvs_off, pvs = L.pvs_lists(w)
+    rng = np.random.default_rng(4)
+    leaves = np.flatnonzero((patches["child1"] == -1) & (patches["sky"] == 0))
+    n = len(leaves)
+    with L.LightingStage(w, inp) as st:
+        st.upload_bounce(L.face_reflectivity(w), pvs_off, pvs, bounces=1)
+        st.light_pass()
+        _, direct = st.patch_light()
+        shoot = direct.astype(np.float32) * patches["reflectivity"]
+        source = int(np.argmax(shoot.min(axis=1)))
+        c = shoot[source, 0]
+        want = {"wide": 2.0 ** rng.uniform(-20, 20, n), "half ways": rng.integers(1, 64, n) / 8.0,
+                "mostly zero": np.where(rng.random(n) < 0.01, rng.random(n), 0.0),
+                "negative": rng.normal(0, 1, n), "infinite": rng.random(n)}[values].astype(np.float32)
+        weight = want / c
+        for step in (-1, 1):      # the weight whose product is the value, where a neighbour is
+            near = (weight.view(np.int32) + step).view(np.float32)
+            weight = np.where((c * weight != want) & (c * near == want), near, weight)
+        if values == "infinite":
+            weight[n // 3] = np.float32(np.inf)
+        tr = np.zeros(n, O.TRANSFER_DTYPE)
+        tr["patch"], tr["weight"] = source, weight
+        sets = [np.zeros(0, O.TRANSFER_DTYPE)] * len(patches)
+        for i, p in enumerate(leaves):
+            sets[p] = tr[i:i + 1]
+        assert C.install(st, O.index(sets), [C.pack(k) for k in O.chunks(sets, 1 << 20)])
+        st.light_pass()
+        last = st.last_total()
+    x = (shoot[source][None, :] * weight[:, None]).astype(np.float32)[::-1]
+    if values == "half ways":
+        assert (x[:, 0] == want[::-1]).mean() > 0.5
+    total = np.add.accumulate(np.concatenate([np.zeros((1, 3), np.float32), x]), axis=0, dtype=np.float32)[-1]
+    assert np.array_equal(last.astype(np.float32).view(np.uint32), total.view(np.uint32))
