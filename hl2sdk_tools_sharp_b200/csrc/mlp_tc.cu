@@ -2,29 +2,36 @@
 // generation tensor cores: tcgen05.mma with the accumulators in TMEM.
 //
 // The network is 32 -> 128 -> 128 -> 3 (ReLU, BF16 weights and activations,
-// FP32 accumulation; mlp.cuh).  One CTA of 8 warps works on 128 rows at a
-// time and keeps the whole network in shared memory:
+// FP32 accumulation; mlp.cuh).  One CTA per SM keeps the whole network in
+// shared memory and has two row tiles of 128 rows in flight, one per group
+// of eight warps:
 //   w1 (N 128, K 32), w2 (N 128, K 128), w3 (N 16, K 128; rows 3..15 zero)
-//   as the MMAs' B operands and the row tile's x (K 32) and hidden layer h
-//   (K 128) as their A operands, all in the canonical K-major layout
-//   without swizzle: 8-row x 16-byte core matrices, each 128 contiguous
-//   bytes, core (row group g, K chunk k) at (k x row groups + g) x 128 B;
-// and 128 TMEM columns (128 lanes x 128 FP32) that each layer's
-// accumulator reuses.  Per tile:
-//   x -> shared memory (each thread 32 bytes of a row, loaded from global
-//     memory while the previous tile ran)
-//   layer 1: 2 x tcgen05.mma M128 N128 K16 -> TMEM, commit -> mbarrier
+//   as the MMAs' B operands and each group's x (K 32) as an A operand, in
+//   the canonical K-major layout without swizzle: 8-row x 16-byte core
+//   matrices, each 128 contiguous bytes, core (row group g, K chunk k) at
+//   (k x row groups + g) x 128 B;
+// and 256 TMEM columns per group (128 lanes x 32 bits each): 128 of the
+// hidden layers' accumulator, 64 of the hidden layer itself, two BF16 a
+// column, the A operand of layers 2 and 3, and 16 of layer 3's accumulator.
+// A group takes a tile through all layers on its own:
+//   layer 1: 2 x tcgen05.mma M128 N128 K16 over x, commit -> mbarrier
 //   epilogue: tcgen05.ld (warp w reads lanes 32 (w % 4) .., columns
-//     64 (w / 4) ..), + bias, ReLU, BF16 -> h in shared memory
-//   layer 2: 8 x M128 N128 K16 over h; the same epilogue into h
-//   layer 3: 8 x M128 N16 K16 over h; warps 0-3 add the bias and write
-//     the three outputs.
-// Thread 0 issues every MMA and the commit; everyone waits on the
-// mbarrier, each wait bounded by a clock limit after which the kernel
-// records the fault in the network's flags and every thread of the CTA
-// leaves together (the TMEM is freed on the way out).  Two CTAs share an
-// SM (87 KB of shared memory, 128 TMEM columns each), so one CTA's
-// epilogue overlaps the other's MMAs.
+//     64 (w / 4) ..), + bias, BF16, ReLU, tcgen05.st
+//   layer 2: 8 x M128 N128 K16 over the hidden layer; the same epilogue
+//   layer 3: 8 x M128 N16 K16 over it, and the next tile's layer 1 in the
+//     same commit; the outputs are written while the next layer 2 runs.
+// A group's first thread issues its MMAs and commits; its threads wait on
+// its mbarrier, each wait bounded by a clock limit after which the kernel
+// records the fault in the network's flags and the group leaves (the TMEM
+// is freed on the way out).
+//
+// What bounds it is shared memory: an M128 N128 K16 product of two operands
+// there reads 8 KB in the 64 cycles that it takes, and the epilogues wrote
+// and read 64 KB a tile besides.  With the hidden layers there 1 M rows took
+// 90 us (two CTAs of eight warps, the tensor pipe 24 % active), 79 us with
+// four tiles in flight; in TMEM, half of that traffic gone, 71 us.  TMEM then
+// holds two tiles, and what is left is their latency: of a tile's 4500
+// cycles the epilogues are 1900, the waits for MMAs 1400.
 //
 // The sums are the mma.sync forward's (mlp.cu) up to FP32 rounding: the
 // bias is added after the products here rather than before.
@@ -39,10 +46,13 @@
 namespace vrad {
 namespace {
 
-constexpr int kTcWarps = 8;
-constexpr int kTcThreads = 32 * kTcWarps;
-constexpr int kTcRows = 128;
-constexpr uint32_t kTmemCols = 128;
+constexpr int kTcRows = 128;   // rows of a tile
+constexpr int kTcGroups = 2;   // tiles in flight on an SM
+constexpr int kGroupThreads = 256;
+constexpr int kTcThreads = kGroupThreads * kTcGroups;
+constexpr uint32_t kTileCols = 256;                     // TMEM columns of a tile
+constexpr uint32_t kHiddenCol = 128, kOutCol = 192;     // where its hidden layer and its outputs begin
+constexpr uint32_t kTmemCols = kTileCols * kTcGroups;
 constexpr int kN3 = 16;                                 // layer 3's N, padded
 constexpr long long kWaitCycles = 2000000000LL;         // about a second at the B200's clocks
 constexpr uint32_t kFlagTimeout = 1;
@@ -51,13 +61,13 @@ struct __align__(1024) TcSmem {
     uint16_t w1[kMlpHidden * kMlpIn];
     uint16_t w2[kMlpHidden * kMlpHidden];
     uint16_t w3[kN3 * kMlpHidden];
-    uint16_t x[kTcRows * kMlpIn];
-    uint16_t h[kTcRows * kMlpHidden];
+    uint16_t x[kTcGroups][kTcRows * kMlpIn];
     float b1[kMlpHidden], b2[kMlpHidden], b3[kN3];
-    unsigned long long bar;
+    unsigned long long bar[kTcGroups];
     uint32_t tmem;
-    int abort;
+    int abort[kTcGroups];
 };
+static_assert(sizeof(TcSmem) <= 227 * 1024, "one CTA's shared memory");
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return (uint32_t)__cvta_generic_to_shared(p);
@@ -88,6 +98,16 @@ __device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
         "l"(a), "l"(b), "r"(id), "r"((uint32_t)acc)
+        : "memory");
+}
+
+// The same with A in TMEM.
+__device__ __forceinline__ void mma_t(uint32_t d, uint32_t a, uint64_t b, uint32_t id, bool acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d),
+        "r"(a), "l"(b), "r"(id), "r"((uint32_t)acc)
         : "memory");
 }
 
@@ -141,40 +161,69 @@ __device__ __forceinline__ void tmem_ld4(uint32_t addr, float v[4]) {
     for (int i = 0; i < 4; i++) v[i] = __uint_as_float(r[i]);
 }
 
+// 32 consecutive columns of this warp's 32 lanes.
+__device__ __forceinline__ void tmem_st32(uint32_t addr, const uint32_t r[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};\n" ::"r"(addr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
+        "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
+        "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        : "memory");
+}
+
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t *>(&v);
+// The group's threads (a named barrier each).
+__device__ __forceinline__ void group_sync(int group) {
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(kGroupThreads) : "memory");
 }
 
-// Bias, ReLU and BF16 of this thread's 64 accumulator columns of row r into h.
-// Both 32-column loads are in flight before the one wait.
-__device__ __forceinline__ void hidden_epilogue(TcSmem &s, uint32_t taddr, const float *bias, int r, int c0) {
-    float v[64];
-    tmem_ld32(taddr + (uint32_t)c0, v);
-    tmem_ld32(taddr + (uint32_t)(c0 + 32), v + 32);
+// Two FP32 sums, each rounded on its own.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    unsigned long long ra = *reinterpret_cast<unsigned long long *>(&a), rb = *reinterpret_cast<unsigned long long *>(&b);
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(ra) : "l"(rb));
+    return *reinterpret_cast<float2 *>(&ra);
+}
+
+// Bias, BF16 and ReLU of this thread's 64 accumulator columns from c0 into
+// the hidden layer's: the ReLU after the rounding, two at a time, which gives
+// the same bits (rounding keeps the order and the sign; a NaN gives 0 either
+// way).  The second 32 columns load while the first are worked on.
+__device__ __forceinline__ void hidden_epilogue(uint32_t taddr, const float *bias, int c0) {
+    const __nv_bfloat162 zero = __floats2bfloat162_rn(0.0f, 0.0f);
+    float v[2][32];
+    uint32_t w[32];
+    tmem_ld32(taddr + (uint32_t)c0, v[0]);
     tmem_wait_ld();
+    tmem_ld32(taddr + (uint32_t)(c0 + 32), v[1]);
 #pragma unroll
-    for (int q = 0; q < 8; q++) {
-        const int c = c0 + 8 * q;
-        uint4 w;
-        uint32_t *pw = reinterpret_cast<uint32_t *>(&w);
+    for (int half = 0; half < 2; half++) {
+        if (half) tmem_wait_ld();
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const float a = fmaxf(__fadd_rn(v[8 * q + 2 * e], bias[c + 2 * e]), 0.0f);
-            const float b = fmaxf(__fadd_rn(v[8 * q + 2 * e + 1], bias[c + 2 * e + 1]), 0.0f);
-            pw[e] = pack2(a, b);
+        for (int q = 0; q < 8; q++) {
+            const float4 b = *reinterpret_cast<const float4 *>(bias + c0 + 32 * half + 4 * q);
+            const float2 s0 = add2(make_float2(v[half][4 * q], v[half][4 * q + 1]), make_float2(b.x, b.y));
+            const float2 s1 = add2(make_float2(v[half][4 * q + 2], v[half][4 * q + 3]), make_float2(b.z, b.w));
+            const __nv_bfloat162 h0 = __hmax2(__floats2bfloat162_rn(s0.x, s0.y), zero);
+            const __nv_bfloat162 h1 = __hmax2(__floats2bfloat162_rn(s1.x, s1.y), zero);
+            w[16 * half + 2 * q] = *reinterpret_cast<const uint32_t *>(&h0);
+            w[16 * half + 2 * q + 1] = *reinterpret_cast<const uint32_t *>(&h1);
         }
-        *reinterpret_cast<uint4 *>(s.h + canon(r, c, kTcRows / 8)) = w;
     }
+    tmem_st32(taddr + kHiddenCol + (uint32_t)(c0 / 2), w);
+    tmem_wait_st();
 }
 
-__global__ void __launch_bounds__(kTcThreads) k_mlp_forward_tc(vrad_mlp m, const uint16_t *__restrict__ x, int64_t n,
+__global__ void __launch_bounds__(kTcThreads, 1) k_mlp_forward_tc(vrad_mlp m, const uint16_t *__restrict__ x, int64_t n,
                                                                float *__restrict__ y) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     TcSmem &s = *reinterpret_cast<TcSmem *>(smem_raw);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int group = tid / kGroupThreads, gt = tid % kGroupThreads;  // gt: the thread in its group
 
     // The network into shared memory, as B operands.
     for (int i = tid; i < kMlpHidden * kMlpIn / 8; i += kTcThreads) {
@@ -198,10 +247,12 @@ __global__ void __launch_bounds__(kTcThreads) k_mlp_forward_tc(vrad_mlp m, const
         s.b2[i] = m.master[kOffB2 + i];
     }
     if (tid < kN3) s.b3[tid] = tid < kMlpOut ? m.master[kOffB3 + tid] : 0.0f;
-    const uint32_t bar = smem_u32(&s.bar);
+    const uint32_t bar = smem_u32(&s.bar[group]);
     if (tid == 0) {
-        s.abort = 0;
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+        for (int g = 0; g < kTcGroups; g++) {
+            s.abort[g] = 0;
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s.bar[g])) : "memory");
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -214,40 +265,44 @@ __global__ void __launch_bounds__(kTcThreads) k_mlp_forward_tc(vrad_mlp m, const
     fence_before();
     __syncthreads();
     fence_after();
-    const uint32_t tmem = s.tmem;
-    // This warp's TMEM lanes and accumulator columns.
-    const int row = 32 * (warp & 3) + lane;
-    const int c0 = 64 * (warp >> 2);
+    // The group's accumulator; this warp's lanes of it.
+    const uint32_t tmem = s.tmem + kTileCols * (uint32_t)group;
     const uint32_t taddr = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-    const uint32_t ax = smem_u32(s.x), ah = smem_u32(s.h), bw1 = smem_u32(s.w1), bw2 = smem_u32(s.w2),
-                   bw3 = smem_u32(s.w3);
+    const int row = 32 * (warp & 3) + (tid & 31), c0 = 64 * (gt >> 7);
+    const uint32_t ax = smem_u32(s.x[group]), bw1 = smem_u32(s.w1), bw2 = smem_u32(s.w2), bw3 = smem_u32(s.w3);
     constexpr uint32_t kLboWide = 16 * 128, kLboW3 = 2 * 128, kSbo = 128;
+    // The operands' descriptors; two K chunks on, the start is 2 LBO / 16 more.
+    const uint64_t dx = sdesc(ax, kLboWide, kSbo), d1 = sdesc(bw1, kLboWide, kSbo), d2 = sdesc(bw2, kLboWide, kSbo),
+                   d3 = sdesc(bw3, kLboW3, kSbo);
+    constexpr uint64_t kStepWide = 2 * kLboWide / 16, kStepW3 = 2 * kLboW3 / 16;
     const bool x16 = ((uintptr_t)x & 15) == 0;
     uint32_t parity = 0;
-    bool ok = true;
 
-    // Waits for the MMAs just committed; every thread of the CTA returns
-    // the same answer.
-    auto wait_all = [&]() -> bool {
-        const bool mine = wait_bar(bar, parity);
+    // Waits for the MMAs just committed.  A thread that gave up says so, and
+    // the group agrees to leave at its next barrier (synced): until then its
+    // loads of an unfinished accumulator give values that nobody keeps.
+    auto wait_mma = [&] {
+        if (!wait_bar(bar, parity)) atomicOr(&s.abort[group], 1);
         parity ^= 1;
-        if (!mine) atomicOr(&s.abort, 1);
-        __syncthreads();
+        __syncwarp();
         fence_after();
-        return s.abort == 0;
+    };
+    auto synced = [&]() -> bool {
+        fence_before();
+        group_sync(group);
+        return *(volatile int *)&s.abort[group] == 0;
     };
 
-    // x: thread t holds half of row t / 2 (two 16-byte chunks) of a tile;
-    // the next tile's are loaded while this tile's layers run.
-    const int xr_row = tid >> 1, xr_kc = 2 * (tid & 1);
+    // x: a thread holds half of row gt / 2 (two 16-byte chunks) of a tile.
+    const int x_row = gt >> 1, x_kc = 2 * (gt & 1);
     uint4 xr[2];
     auto load_x = [&](int64_t tile) {
-        const int64_t gr = tile * kTcRows + xr_row;
+        const int64_t gr = tile * kTcRows + x_row;
 #pragma unroll
         for (int q = 0; q < 2; q++) {
             xr[q] = make_uint4(0, 0, 0, 0);
             if (gr < n) {
-                const uint16_t *src = x + gr * kMlpIn + 8 * (xr_kc + q);
+                const uint16_t *src = x + gr * kMlpIn + 8 * (x_kc + q);
                 if (x16) {
                     xr[q] = *reinterpret_cast<const uint4 *>(src);
                 } else {
@@ -257,76 +312,95 @@ __global__ void __launch_bounds__(kTcThreads) k_mlp_forward_tc(vrad_mlp m, const
             }
         }
     };
-    load_x(blockIdx.x);
-
-    for (int64_t tile = blockIdx.x; ok && tile * kTcRows < n; tile += gridDim.x) {
-        const int64_t r0 = tile * kTcRows;
+    auto store_x = [&] {
 #pragma unroll
-        for (int q = 0; q < 2; q++) *reinterpret_cast<uint4 *>(s.x + canon(xr_row, 8 * (xr_kc + q), kTcRows / 8)) = xr[q];
+        for (int q = 0; q < 2; q++)
+            *reinterpret_cast<uint4 *>(s.x[group] + canon(x_row, 8 * (x_kc + q), kTcRows / 8)) = xr[q];
         fence_async_smem();
-        __syncthreads();
-        if (tid == 0) {
-            fence_after();
+    };
+    auto layer1 = [&] {
 #pragma unroll
-            for (int k = 0; k < kMlpIn / 16; k++)
-                mma(tmem, sdesc(ax + 2 * k * kLboWide, kLboWide, kSbo), sdesc(bw1 + 2 * k * kLboWide, kLboWide, kSbo),
-                    idesc(kMlpHidden), k > 0);
+        for (int k = 0; k < kMlpIn / 16; k++)
+            mma(tmem, dx + k * kStepWide, d1 + k * kStepWide, idesc(kMlpHidden), k > 0);
+    };
+    auto write_out = [&](int64_t tile) {
+        if (gt >= kTcRows) return;  // whole warps
+        float v[4];
+        tmem_ld4(taddr + kOutCol, v);
+        tmem_wait_ld();
+        const int64_t gr = tile * kTcRows + row;
+        if (gr < n) {
+#pragma unroll
+            for (int c = 0; c < kMlpOut; c++) y[gr * kMlpOut + c] = __fadd_rn(v[c], s.b3[c]);
+        }
+    };
+    // Tiles by CTA first, then by group: few tiles are spread over the SMs.
+    const int64_t step = (int64_t)gridDim.x * kTcGroups;
+    int64_t tile = blockIdx.x + (int64_t)gridDim.x * group;
+    bool ok = true;
+    if (tile * kTcRows < n) {
+        load_x(tile);
+        store_x();
+        ok = synced();
+        if (ok && gt == 0) {
+            fence_after();
+            layer1();
             commit(bar);
         }
-        load_x(tile + gridDim.x);
-        if (!(ok = wait_all())) break;
-        hidden_epilogue(s, taddr, s.b1, row, c0);
-        fence_before();
-        fence_async_smem();
-        __syncthreads();
-        if (tid == 0) {
-            fence_after();
+        load_x(tile + step);
+        bool first = true;
+        while (ok) {
+            // This tile's layer 1, and the tile before's layer 3.
+            wait_mma();
+            hidden_epilogue(taddr, s.b1, c0);
+            if (!(ok = synced())) break;
+            if (gt == 0) {
+                fence_after();
 #pragma unroll
-            for (int k = 0; k < kMlpHidden / 16; k++)
-                mma(tmem, sdesc(ah + 2 * k * kLboWide, kLboWide, kSbo), sdesc(bw2 + 2 * k * kLboWide, kLboWide, kSbo),
-                    idesc(kMlpHidden), k > 0);
-            commit(bar);
-        }
-        if (!(ok = wait_all())) break;
-        hidden_epilogue(s, taddr, s.b2, row, c0);
-        fence_before();
-        fence_async_smem();
-        __syncthreads();
-        if (tid == 0) {
-            fence_after();
-#pragma unroll
-            for (int k = 0; k < kMlpHidden / 16; k++)
-                mma(tmem, sdesc(ah + 2 * k * kLboWide, kLboWide, kSbo), sdesc(bw3 + 2 * k * kLboW3, kLboW3, kSbo),
-                    idesc(kN3), k > 0);
-            commit(bar);
-        }
-        if (!(ok = wait_all())) break;
-        if (warp < 4) {
-            float v[4];
-            tmem_ld4(taddr, v);
-            tmem_wait_ld();
-            const int64_t gr = r0 + row;
-            if (gr < n) {
-#pragma unroll
-                for (int c = 0; c < kMlpOut; c++) y[gr * kMlpOut + c] = __fadd_rn(v[c], s.b3[c]);
+                for (int k = 0; k < kMlpHidden / 16; k++)
+                    mma_t(tmem, tmem + kHiddenCol + 8 * k, d2 + k * kStepWide, idesc(kMlpHidden), k > 0);
+                commit(bar);
             }
+            __syncwarp();
+            if (!first) write_out(tile - step);
+            first = false;
+            store_x();
+            wait_mma();
+            hidden_epilogue(taddr, s.b2, c0);
+            if (!(ok = synced())) break;
+            const bool more = (tile + step) * kTcRows < n;
+            if (gt == 0) {
+                fence_after();
+#pragma unroll
+                for (int k = 0; k < kMlpHidden / 16; k++)
+                    mma_t(tmem + kOutCol, tmem + kHiddenCol + 8 * k, d3 + k * kStepW3, idesc(kN3), k > 0);
+                if (more) layer1();
+                commit(bar);
+            }
+            __syncwarp();
+            if (!more) {
+                wait_mma();
+                write_out(tile);
+                break;
+            }
+            tile += step;
+            load_x(tile + step);
         }
-        fence_before();
-        __syncthreads();
-        fence_after();
     }
     // After a timeout: record it, and leave with no MMA in flight (the last
     // commit's phase waited for once more, bounded again), then free the
-    // TMEM.
-    if (!ok && tid == 0) {
-        atomicOr(m.flags, kFlagTimeout);
-        wait_bar(bar, parity ^ 1);
+    // TMEM.  A timeout of the last wait shows here too.
+    if (!ok || *(volatile int *)&s.abort[group]) {
+        if (gt == 0) {
+            atomicOr(m.flags, kFlagTimeout);
+            wait_bar(bar, parity ^ 1);
+        }
     }
     fence_before();
     __syncthreads();
     fence_after();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s.tmem), "r"(kTmemCols) : "memory");
 }
 
 std::mutex tc_mu;
@@ -355,7 +429,7 @@ cudaError_t mlp_forward_tc(const vrad_mlp &m, const uint16_t *x, int64_t n, floa
         }
     }
     const int64_t tiles = (n + kTcRows - 1) / kTcRows;
-    const int64_t grid = tiles < 2LL * sms ? tiles : 2LL * sms;
+    const int64_t grid = tiles < sms ? tiles : sms;
     k_mlp_forward_tc<<<(unsigned)grid, kTcThreads, sizeof(TcSmem), s>>>(m, x, n, y);
     return cudaGetLastError();
 }

@@ -117,3 +117,29 @@ def test_tcgen05_forward_at_scale_and_alignment(net):
     y2 = n.forward(view)
     torch.cuda.synchronize()
     assert torch.equal(y2, y[:4096])
+
+
+@pytest.mark.parametrize("rows", [1, 127, 128, 129, 148 * 128 + 1, 2 * 148 * 128, 5 * 148 * 128 - 1])
+def test_forward_at_tile_edges(net, rows):
+    """One tile, a part of one, as many as the SMs, as many as are in flight,
+    several rounds with a partial last one; a row of infinities and one of
+    NaNs stay in their rows."""
+    from oracle import mlp_oracle as MO
+    n, torch = net
+    g = torch.Generator(device="cuda")
+    g.manual_seed(rows)
+    x = torch.randn((rows, LN.INPUTS), device="cuda", generator=g).to(torch.bfloat16).contiguous()
+    y = n.forward(x)
+    torch.cuda.synchronize()
+    n.status()
+    assert y.shape == (rows, 3)
+    want, _, _ = MO.forward(n.params(), x.cpu().view(torch.int16).numpy().view(np.uint16))
+    assert _rel(y.cpu().numpy(), want) < 2e-3
+    bad = x.clone()
+    bad[rows // 2] = float("nan")
+    bad[rows - 1, 0] = float("inf")
+    y2 = n.forward(bad)
+    torch.cuda.synchronize()
+    keep = torch.ones(rows, dtype=torch.bool, device="cuda")
+    keep[rows // 2] = keep[rows - 1] = False
+    assert torch.equal(y2[keep], y[keep])
