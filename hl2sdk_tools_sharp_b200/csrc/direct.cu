@@ -327,6 +327,17 @@ extern "C" int32_t vrad_world_upload(vrad_ctx *ctx, const vrad_world_desc *w) {
     }
     std::vector<int32_t> cl_off(w->cluster_light_offsets, w->cluster_light_offsets + w->nclusters + 1);
     std::vector<int32_t> cl_list(w->cluster_lights, w->cluster_lights + total);
+    // The most segments one point's lights trace: one each, the sun's and the
+    // sky's directions.
+    int32_t max_rays = 0;
+    for (int32_t c = 0; c < w->nclusters; c++) {
+        int64_t rays = 0;
+        for (int32_t k = cl_off[(size_t)c]; k < cl_off[(size_t)c + 1]; k++) {
+            const int type = w->lights[w->cluster_lights[k]].type;
+            rays += type == vrad::kSkyLight ? w->sun_samples : type == vrad::kSkyAmbient ? w->nsky_directions : 1;
+        }
+        max_rays = (int32_t)std::min<int64_t>(std::max<int64_t>(max_rays, rays), INT32_MAX);
+    }
     std::vector<float4> dirs((size_t)w->nsky_directions), jit((size_t)w->nsun_jitter);
     for (int32_t d = 0; d < w->nsky_directions; d++)
         dirs[(size_t)d] = make_float4(w->sky_directions[3 * d], w->sky_directions[3 * d + 1], w->sky_directions[3 * d + 2], 0.0f);
@@ -368,6 +379,7 @@ extern "C" int32_t vrad_world_upload(vrad_ctx *ctx, const vrad_world_desc *w) {
                                 wb.cl_off, wb.cl_list, w->nclusters, wb.dirs, w->nsky_directions, wb.jitter,
                                 w->nsun_jitter, w->sun_angular_extent, w->sun_samples, w->nsamples,
                                 wb.lights_hdr};
+    wb.view.max_rays = max_rays;
     clock.mark("world buffers");
     // The final pass's tables, and the direct gather's output buffer.  A
     // new world drops the old bounce.
@@ -422,7 +434,7 @@ extern "C" int32_t vrad_world_upload(vrad_ctx *ctx, const vrad_world_desc *w) {
         bool have = false;
         e = vrad::build_supersample(ctx->supersample, ctx->h_faces, ctx->h_vertices, area_coord, w->nsamples,
                                     ctx->final_pass,
-                                    w->nclusters, ctx->stager, ctx->stream, have, why);
+                                    w->nclusters, max_rays, ctx->stager, ctx->stream, have, why);
         if (e != cudaSuccess) {
             ctx->stager.finish(ctx->stream);  // no copy in flight into a released block
         wb.release();

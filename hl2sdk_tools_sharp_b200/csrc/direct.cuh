@@ -64,6 +64,7 @@ struct DeviceWorld {
     int32_t style;
     unsigned long long *face_key;
     const int8_t *face_slot;
+    int32_t max_rays;  // the most segments that one point's lights (of any cluster) trace
 };
 
 struct WorldBuffers {

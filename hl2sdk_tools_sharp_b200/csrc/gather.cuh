@@ -87,6 +87,21 @@ __device__ __forceinline__ float inverse_quadratic(float d, float q, float l, fl
 // Which lights a gather takes.
 enum : int { kAllLights = 0, kAmbientOnly = 1, kDirectOnly = 2 };
 
+// How a gather's segments are traced.  kTrace: by the point's own thread,
+// one after the other.  Where a launch has too few points to fill the chip,
+// that chain is all it waits for (a few hundred segments of about 20 us with
+// a sky), and two launches take its place: kTraceShare, in which the blocks
+// of `nsplit` shares trace every nsplit-th segment each and leave who was
+// blocked in `words` (a bit per lane, by segment and warp), and kLookUp, the
+// gather itself, which reads them.  What is traced and added, and in which
+// order, is the same.
+enum : int { kTrace = 0, kTraceShare = 1, kLookUp = 2 };
+struct RayShare {
+    uint32_t *words;
+    int nwarps, warp;  // the launch's warps, this one
+    int nsplit, turn;  // shares; segments until this share's next
+};
+
 // The light of one point (px, py, pz already one unit off the face, flat
 // normal n): (lighting xyz, direct sun amount).  Lanes with real = false
 // follow the group's decisions but trace nothing and add nothing.  With
@@ -94,13 +109,37 @@ enum : int { kAllLights = 0, kAmbientOnly = 1, kDirectOnly = 2 };
 // value from w.lights_hdr's intensities (every decision and every traced
 // segment is the range-independent one, so each range gets its own pass's
 // bits).
-template <int BLOCK, bool DUAL = false>
+template <int BLOCK, bool DUAL = false, int VIS = kTrace>
 __device__ __forceinline__ float4 gather_point(const DeviceScene &sc, const DeviceWorld &w, int cluster, float px,
                                                float py, float pz, float nx, float ny, float nz, bool real,
                                                unsigned gmask, int filter, int start, int *stack,
                                                unsigned long long *counters, uint32_t &vis_rays, uint32_t &sky_rays,
                                                float4 *second = nullptr,
-                                               int face = 0, unsigned long long key_group = 0) {
+                                               int face = 0, unsigned long long key_group = 0,
+                                               RayShare share = RayShare()) {
+    int64_t word = share.warp;  // this segment's: segment * nwarps + warp
+    // Whether the lane's segment is blocked, for the lanes that trace one
+    // (cond).  All of the warp's lanes come here together.
+    auto is_blocked = [&](bool cond, auto &&trace) {
+        if constexpr (VIS == kTrace) {
+            return cond && trace();
+        } else if constexpr (VIS == kTraceShare) {
+            bool b = false;
+            if (share.turn == 0) {
+                b = cond && trace();
+                const unsigned bits = __ballot_sync(kFull, b);
+                if ((threadIdx.x & 31) == 0) share.words[word] = bits;
+                share.turn = share.nsplit;
+            }
+            share.turn--;
+            word += share.nwarps;
+            return b;
+        } else {
+            const uint32_t bits = __ldg(&share.words[word]);
+            word += share.nwarps;
+            return cond && ((bits >> (threadIdx.x & 31)) & 1u);
+        }
+    };
     float ax = 0.0f, ay = 0.0f, az = 0.0f, sun = 0.0f;
     float hx = 0.0f, hy = 0.0f, hz = 0.0f;
 
@@ -117,6 +156,11 @@ __device__ __forceinline__ float4 gather_point(const DeviceScene &sc, const Devi
         // lights apart (EmitResample); the filter is warp-uniform.
         if (filter == kAmbientOnly && type != kSkyAmbient) continue;
         if (filter == kDirectOnly && type == kSkyAmbient) continue;
+        if (VIS == kTraceShare && type != kSkyLight && type != kSkyAmbient && share.turn != 0) {
+            share.turn--;  // another share's one segment
+            word += share.nwarps;
+            continue;
+        }
         float dot = 0.0f, falloff = 0.0f, sun_amount = 0.0f;
 
         if (type == kPoint || type == kSpot) {
@@ -159,10 +203,10 @@ __device__ __forceinline__ float4 gather_point(const DeviceScene &sc, const Devi
                     falloff = f;
                 }
             }
-            if (real && dot != 0.0f && falloff != 0.0f) {
-                vis_rays++;
-                if (segment_blocked<kModeAny, BLOCK>(sc, px, py, pz, A.x, A.y, A.z, start, stack)) dot = 0.0f;
-            }
+            const bool cond = real && dot != 0.0f && falloff != 0.0f;
+            if (cond) vis_rays++;
+            if (is_blocked(cond, [&] { return segment_blocked<kModeAny, BLOCK>(sc, px, py, pz, A.x, A.y, A.z, start, stack); }))
+                dot = 0.0f;
         } else if (type == kSurface) {
             // GatherSurfaceFour (DirectLightGatherer.cs:1452-1545): the
             // patch's cosine over the squared distance, the segment to the
@@ -187,13 +231,15 @@ __device__ __forceinline__ float4 gather_point(const DeviceScene &sc, const Devi
             if (hard) f = __fmul_rn(fade(dist, E.y, __fsub_rn(E.z, E.y)), f);
             dot = live ? d : 0.0f;
             falloff = live ? f : 0.0f;
-            if (real && dot != 0.0f && falloff != 0.0f) {
-                vis_rays++;
-                const float ex = __fadd_rn(A.x, __fmul_rn(C.x, kDistEpsilon)),
-                            ey = __fadd_rn(A.y, __fmul_rn(C.y, kDistEpsilon)),
-                            ez = __fadd_rn(A.z, __fmul_rn(C.z, kDistEpsilon));
-                if (segment_blocked<kModeAny, BLOCK>(sc, px, py, pz, ex, ey, ez, start, stack)) dot = 0.0f;
-            }
+            const bool cond = real && dot != 0.0f && falloff != 0.0f;
+            if (cond) vis_rays++;
+            if (is_blocked(cond, [&] {
+                    const float ex = __fadd_rn(A.x, __fmul_rn(C.x, kDistEpsilon)),
+                                ey = __fadd_rn(A.y, __fmul_rn(C.y, kDistEpsilon)),
+                                ez = __fadd_rn(A.z, __fmul_rn(C.z, kDistEpsilon));
+                    return segment_blocked<kModeAny, BLOCK>(sc, px, py, pz, ex, ey, ez, start, stack);
+                }))
+                dot = 0.0f;
         } else if (type == kSkyLight) {
             // EmitSkyLight / ResolveSkyLight.
             float d = -__fadd_rn(__fadd_rn(__fmul_rn(nx, C.x), __fmul_rn(ny, C.y)), __fmul_rn(nz, C.z));
@@ -213,13 +259,13 @@ __device__ __forceinline__ float4 gather_point(const DeviceScene &sc, const Devi
                         ez = __fadd_rn(ez, __fmul_rn(j.z, jitter_scale));
                     }
                     float frac = 1.0f;
-                    if (need && real) {
-                        sky_rays++;
-                        if (segment_blocked<kModeSkyPass, BLOCK>(sc, px, py, pz, __fadd_rn(ex, px),
-                                                                 __fadd_rn(ey, py), __fadd_rn(ez, pz), start,
-                                                             stack))
-                            frac = 0.0f;
-                    }
+                    if (need && real) sky_rays++;
+                    if (is_blocked(need && real, [&] {
+                            return segment_blocked<kModeSkyPass, BLOCK>(sc, px, py, pz, __fadd_rn(ex, px),
+                                                                        __fadd_rn(ey, py), __fadd_rn(ez, pz), start,
+                                                                        stack);
+                        }))
+                        frac = 0.0f;
                     total = __fadd_rn(total, frac);
                     __syncwarp();
                 }
@@ -241,7 +287,8 @@ __device__ __forceinline__ float4 gather_point(const DeviceScene &sc, const Devi
                 sumdot = __fadd_rn(dv, sumdot);
                 possible = __fadd_rn(valid ? 1.0f : 0.0f, possible);
                 float frac = 1.0f;
-                if (valid && real) {
+                if (valid && real) sky_rays++;
+                if (is_blocked(valid && real, [&] {
                     // surfacePos = points - anorm * -epsilon, epsilon 0, which
                     // is the point but for the sign of a zero, and no sign
                     // of a zero decides a hit; stop = anorm *
@@ -249,9 +296,9 @@ __device__ __forceinline__ float4 gather_point(const DeviceScene &sc, const Devi
                     const float ex = __fadd_rn(__fmul_rn(an.x, -kMaxTraceLength), px);
                     const float ey = __fadd_rn(__fmul_rn(an.y, -kMaxTraceLength), py);
                     const float ez = __fadd_rn(__fmul_rn(an.z, -kMaxTraceLength), pz);
-                    sky_rays++;
-                    if (segment_blocked<kModeSkyPass, BLOCK>(sc, px, py, pz, ex, ey, ez, start, stack)) frac = 0.0f;
-                }
+                    return segment_blocked<kModeSkyPass, BLOCK>(sc, px, py, pz, ex, ey, ez, start, stack);
+                }))
+                    frac = 0.0f;
                 ambient = __fadd_rn(ambient, __fmul_rn(frac, dv));
                 __syncwarp();
             }

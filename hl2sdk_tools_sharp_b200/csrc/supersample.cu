@@ -47,6 +47,16 @@ namespace vrad {
 namespace {
 
 constexpr int kSsBlock = 128;
+// A resampling launch of fewer warps is split by segments into shares
+// (gather.cuh: kTraceShare) until it has this many, four rounds of the
+// chip's resident ones.  The later passes light a few hundred points each,
+// and one point's chain of segments took 0.2 ms alone: on the 3x3 grid of
+// rooms the four passes take 0.6 ms, unsplit 1.4, and the light pass 3.62 ms
+// (4096: 4.00, 8192: 3.79, 32768: 3.63, 65536: 3.75), unsplit 4.42; the 8x8
+// and 4x4 maps' last passes gain 1.3 and 1.5 ms in all.  A world whose points
+// trace more than kSplitRays segments (64 MB of words) is not split.
+constexpr int kSplitWarps = 16384;
+constexpr int kSplitRays = 1024;
 constexpr float kSupersampleGradient = 0.0625f;  // LightConstants.SupersampleGradient
 
 // DetMath.PowToSingle: x^y rounded to double, then to float.  CUDA's pow
@@ -181,14 +191,15 @@ __device__ bool point_outside(float x, float y, float z, const float4 *__restric
 // One point of a supersampled row: its position in the cell, the winding
 // test of its row of four, the gather (the sky ambient for row 0, the other
 // lights for rows 1-4) and its LightingValue.
-template <int BLOCK>
+template <int BLOCK, int VIS>
 __global__ void __launch_bounds__(BLOCK) k_resample(DeviceScene sc, DeviceWorld w, FinalView fv, int32_t ngroups,
                                                     int32_t nruns, const int32_t *__restrict__ base,
                                                     const int32_t *__restrict__ rows,
                                                     const int32_t *__restrict__ selected,
                                                     const float2 *__restrict__ origin_st, const int2 *__restrict__ wind,
                                                     const float4 *__restrict__ points, float4 *__restrict__ row_out,
-                                                    int32_t *__restrict__ row_bits, unsigned long long *counters) {
+                                                    int32_t *__restrict__ row_bits, unsigned long long *counters,
+                                                    uint32_t *words) {
     extern __shared__ int stack_mem[];  // sc.stack_depth() entries per thread
     int *stack = stack_mem + threadIdx.x;
     const int64_t tid = (int64_t)blockIdx.x * BLOCK + threadIdx.x;
@@ -253,9 +264,11 @@ __global__ void __launch_bounds__(BLOCK) k_resample(DeviceScene sc, DeviceWorld 
     // A row whose four points all lie outside is not gathered.
     real = code >= 0 && bits != 0xFu;
     uint32_t vis_rays = 0, sky_rays = 0;  // one point's rays
-    const float4 r = gather_point<BLOCK>(sc, w, cluster, px, py, pz, nx, ny, nz, real, gmask,
-                                         ambient ? kAmbientOnly : kDirectOnly, start, stack, counters, vis_rays,
-                                         sky_rays);
+    const float4 r = gather_point<BLOCK, false, VIS>(
+        sc, w, cluster, px, py, pz, nx, ny, nz, real, gmask, ambient ? kAmbientOnly : kDirectOnly, start, stack, counters,
+        vis_rays, sky_rays, nullptr, 0, 0,
+        {words, (ngroups + 7) / 8, (int)(tid >> 5), (int)gridDim.y, (int)blockIdx.y});
+    if (VIS == kTraceShare) return;
     if (code >= 0) {
         row_out[4 * (int64_t)code + l4] = r;
         if (l4 == 0) row_bits[code] = real ? (int32_t)bits : -1;
@@ -314,7 +327,8 @@ unsigned grid_of(int64_t n, int per) { return (unsigned)((n + per - 1) / per); }
 }  // namespace
 
 void SupersampleBuffers::release() {
-    void *ptrs[] = {origin_st, cell, wind, points, intensity, processed, selected, counts, base, rows, row_out, row_bits};
+    void *ptrs[] = {origin_st, cell, wind, points, intensity, processed, selected, counts, base, rows, row_out, row_bits,
+                    words};
     for (void *p : ptrs) dev_free(p);
     // The pinned counts stay for the next upload (freeing pinned memory
     // can stall for a good part of a second); free_pinned() frees them.
@@ -335,7 +349,7 @@ void SupersampleBuffers::free_pinned() {
 
 cudaError_t build_supersample(SupersampleBuffers &ss, const std::vector<vrad_face> &faces,
                               const std::vector<float> &vertices, const float4 *area_coord, int64_t nsamples,
-                              const FinalBuffers &fb, int32_t nclusters, Stager &stager, cudaStream_t stream,
+                              const FinalBuffers &fb, int32_t nclusters, int32_t max_rays, Stager &stager, cudaStream_t stream,
                               bool &have, std::string &why) {
     ss.release();
     have = false;
@@ -365,6 +379,11 @@ cudaError_t build_supersample(SupersampleBuffers &ss, const std::vector<vrad_fac
     if (e == cudaSuccess) e = dev_alloc(&ss.rows, sizeof(int32_t) * groups);
     if (e == cudaSuccess) e = dev_alloc(&ss.row_out, sizeof(float4) * 20 * S1);
     if (e == cudaSuccess) e = dev_alloc(&ss.row_bits, sizeof(int32_t) * 5 * S1);
+    if (max_rays > 0 && max_rays <= kSplitRays) {
+        if (e == cudaSuccess)
+            e = dev_alloc(&ss.words, sizeof(uint32_t) * kSplitWarps * (size_t)max_rays + 3 * sizeof(unsigned long long));
+        ss.max_rays = max_rays;
+    }
     if (e == cudaSuccess && ss.h_counts_cap < 1 + (size_t)nclusters) {
         ss.free_pinned();
         e = cudaMallocHost(&ss.h_counts, sizeof(int32_t) * (1 + (size_t)nclusters));
@@ -381,6 +400,32 @@ cudaError_t build_supersample(SupersampleBuffers &ss, const std::vector<vrad_fac
     ss.ready = true;
     have = true;
     return cudaSuccess;
+}
+
+// One pass's points.  A launch of few warps is split by segments (kLookUp)
+// into as many shares as make kSplitWarps warps; with more of its own it is
+// left as it is.
+static cudaError_t launch_resample(const SupersampleBuffers &ss, const DeviceScene &scene, const DeviceWorld &world,
+                                   const FinalView &fv, int32_t g, unsigned long long *counters, cudaStream_t s) {
+    const unsigned grid = grid_of(4 * (int64_t)g, kSsBlock);
+    const size_t stack = sizeof(int) * scene.stack_depth() * kSsBlock;
+    const int nwarps = (g + 7) / 8, runs = 2 * ss.nclusters + 1;
+    const int shares = ss.max_rays >= world.max_rays ? std::min(kSplitWarps / nwarps, world.max_rays) : 1;
+    if (shares < 2) {
+        k_resample<kSsBlock, kTrace><<<grid, kSsBlock, stack, s>>>(scene, world, fv, g, runs, ss.base, ss.rows,
+                                                                   ss.selected, ss.origin_st, ss.wind, ss.points,
+                                                                   ss.row_out, ss.row_bits, counters, nullptr);
+        return cudaGetLastError();
+    }
+    // The tracing launches' own counts (pow_cr's) go to the scratch counters.
+    unsigned long long *scratch = (unsigned long long *)(ss.words + (size_t)kSplitWarps * ss.max_rays);
+    k_resample<kSsBlock, kTraceShare><<<dim3(grid, (unsigned)shares), kSsBlock, stack, s>>>(
+        scene, world, fv, g, runs, ss.base, ss.rows, ss.selected, ss.origin_st, ss.wind, ss.points, ss.row_out,
+        ss.row_bits, scratch, ss.words);
+    k_resample<kSsBlock, kLookUp><<<grid, kSsBlock, 0, s>>>(scene, world, fv, g, runs, ss.base, ss.rows, ss.selected,
+                                                            ss.origin_st, ss.wind, ss.points, ss.row_out, ss.row_bits,
+                                                            counters, ss.words);
+    return cudaGetLastError();
 }
 
 cudaError_t run_supersample(SupersampleBuffers &ss, const DeviceScene &scene, const DeviceWorld &world,
@@ -426,10 +471,7 @@ cudaError_t run_supersample(SupersampleBuffers &ss, const DeviceScene &scene, co
         if (e == cudaSuccess)
             k_ss_place<<<grid_of(nsel, 256), 256, 0, s>>>(nsel, world, ss.selected, ss.base, ss.counts + 1 + C, ss.rows);
         if (e == cudaSuccess && g > 0)
-            k_resample<kSsBlock><<<grid_of(4 * (int64_t)g, kSsBlock), kSsBlock,
-                                  sizeof(int) * scene.stack_depth() * kSsBlock, s>>>(
-                scene, world, fv, g, 2 * C + 1, ss.base, ss.rows, ss.selected, ss.origin_st, ss.wind, ss.points,
-                ss.row_out, ss.row_bits, counters);
+            e = launch_resample(ss, scene, world, fv, g, counters, s);
         if (e == cudaSuccess)
             k_ss_resolve<<<grid_of(nsel, 256), 256, 0, s>>>(nsel, ss.selected, ss.row_out, ss.row_bits, light,
                                                            ss.intensity, &counters[2]);

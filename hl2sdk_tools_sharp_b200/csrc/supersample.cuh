@@ -46,6 +46,8 @@ struct SupersampleBuffers {
     int32_t *rows = nullptr;        // group capacity: 5 * S + 16 * C
     float4 *row_out = nullptr;
     int32_t *row_bits = nullptr;
+    uint32_t *words = nullptr;      // kSplitWarps x the world's max_rays words of who was blocked, then 3 scratch counters
+    int32_t max_rays = 0;           // what words has room for; 0: none (too many rays a point)
     int32_t *h_counts = nullptr;    // pinned, kept across uploads (h_counts_cap entries)
     size_t h_counts_cap = 0;
     int64_t nsamples = 0;
@@ -69,7 +71,7 @@ struct SupersampleBuffers {
 // samples must match (pinned host memory, nsamples entries).
 cudaError_t build_supersample(SupersampleBuffers &ss, const std::vector<vrad_face> &faces,
                               const std::vector<float> &vertices, const float4 *area_coord, int64_t nsamples,
-                              const FinalBuffers &fb, int32_t nclusters, Stager &stager, cudaStream_t stream,
+                              const FinalBuffers &fb, int32_t nclusters, int32_t max_rays, Stager &stager, cudaStream_t stream,
                               bool &have, std::string &why);
 
 // The partial cells' windings, the samples' luxel origins and cells,

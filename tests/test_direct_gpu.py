@@ -124,6 +124,28 @@ def test_3x3_supersampling_counts_and_noextra(oracle_mod):
     assert ss_stats.visibility_rays + ss_stats.sky_rays > plain_stats.visibility_rays + plain_stats.sky_rays
 
 
+@pytest.mark.parametrize("side,scale,lights,sky,sun", [(1, 40.0, 1, True, 1), (1, 16.0, 7, False, 5),
+                                                       (2, 24.0, 9, True, 30), (4, 8.0, 16, True, 1)])
+def test_resampling_of_few_and_many_points(oracle_mod, side, scale, lights, sky, sun):
+    """The supersampling passes where each launch's segments are split into
+    shares (from one warp's to thousands of warps') and where they are not:
+    point and spot lights, the sky's directions, the sun's."""
+    w = rg.generate(rg.Config(side=side, seed=6, luxel_scale=scale, pillars=(0, 3), lights=lights, spot_fraction=0.5,
+                              sky_ambient=sky, sun_spread=2.0 if sun > 1 else 0.0, sun_samples=sun))
+    inp = L.prepare(w)
+    assert inp.sun_samples == sun
+    with L.LightingStage(w, inp) as st:
+        got, stats = st.direct()
+    g = np.concatenate([got["lighting"], got["direct_sun_amount"][:, None]], 1)
+    assert stats.supersampled > 0
+    if side < 4:
+        want, index = oracle_direct(oracle_mod, w, inp), slice(None)
+    else:
+        want, index = oracle_direct(oracle_mod, w, inp, np.arange(0, len(inp.faces), 9))
+    diff = (bits(g[index]) != bits(want)).any(1)
+    assert not diff.any(), f"{int(diff.sum())} of {len(diff)} samples differ"
+
+
 @pytest.mark.parametrize("change", ["area", "coord", "mins", "position", "swap"])
 def test_supersampling_refuses_samples_not_the_builders(change):
     # Supersampling needs each partial sample's cell winding, which the
