@@ -61,6 +61,8 @@ inline int32_t sell_window(int32_t receivers) {
     const int64_t least = ((int64_t)receivers + 4095) / 4096;
     return (int32_t)std::max<int64_t>(1024, (least + 31) / 32 * 32);
 }
+constexpr int kGroup = 16;  // receivers of a transfer group (k_transfer_groups)
+constexpr int32_t kGroupedReceivers = 65536;
 constexpr int kFeatures = 32;                            // the warm start network's inputs
 
 struct BounceView {
@@ -98,6 +100,13 @@ struct BounceBuffers {
     int64_t *cand_off = nullptr;   // R + 1
     int64_t *seg_off = nullptr;    // R * segments + 1: the same by segment of the receiver's row
     int32_t segments = 1;
+    // The transfer rays' warps, by group of kGroup receivers
+    // (k_transfer_groups): group g's are group_off[g] .. group_off[g + 1].
+    int64_t *group_off = nullptr;
+    int32_t *warp_group = nullptr;  // per such warp, its group
+    int64_t transfer_warps = 0;
+    bool grouped() const { return nreceivers >= kGroupedReceivers; }
+    int32_t ngroups() const { return (nreceivers + kGroup - 1) / kGroup; }
     int32_t *cand_src = nullptr;   // Q
     float *cand_w = nullptr;       // Q
     int64_t *tr_off = nullptr;     // R + 1
@@ -199,6 +208,8 @@ struct BounceBuffers {
 // (the leaves' cells, the parents and their shares), once per upload;
 // face_fit: F float4 of scratch.
 cudaError_t launch_bounce_tables(const BounceBuffers &b, const FinalView &fv, float4 *face_fit, cudaStream_t stream);
+// The transfer warps' groups, once group_off is known and warp_group allocated.
+cudaError_t launch_warp_groups(const BounceBuffers &b, cudaStream_t stream);
 // How many entries the slices can need beyond the transfers, from the
 // candidate counts (cand_off), added to *d_pad.
 cudaError_t launch_sell_pad(const BounceBuffers &b, unsigned long long *d_pad, cudaStream_t stream);

@@ -571,8 +571,10 @@ extern "C" int32_t vrad_bounce_upload(vrad_ctx *ctx, const vrad_bounce_desc *d) 
     clock.mark("tables copied");
     const size_t P1 = (size_t)(P ? P : 1), R1 = (size_t)R + 1, N1 = (size_t)(ncells ? ncells : 1);
     if (e == cudaSuccess) e = dev_alloc(&b.cand_off, sizeof(int64_t) * R1);
+    b.nreceivers = R;
     b.segments = row_segments(R);
     if (e == cudaSuccess) e = dev_alloc(&b.seg_off, sizeof(int64_t) * ((size_t)R * (size_t)b.segments + 1));
+    if (e == cudaSuccess) e = dev_alloc(&b.group_off, sizeof(int64_t) * ((size_t)b.ngroups() + 1));
     if (e == cudaSuccess) e = dev_alloc(&b.tr_off, sizeof(int64_t) * R1);
     if (e == cudaSuccess) e = dev_alloc(&b.start, sizeof(int32_t) * R1);
     const size_t M1 = (size_t)(nparents ? nparents : 1);
@@ -598,7 +600,6 @@ extern "C" int32_t vrad_bounce_upload(vrad_ctx *ctx, const vrad_bounce_desc *d) 
     if (e == cudaSuccess) e = dev_alloc(&b.prad_light, sizeof(float4) * N1);
     if (e == cudaSuccess) e = dev_alloc(&b.prad_weight, sizeof(float) * N1);
     const int32_t nslices = (R + 31) / 32;
-    b.nreceivers = R;
     b.sell_window = sell_window(R);
     if (e == cudaSuccess && R > 0) {
         // One scan buffer for the receiver scans and the slice scan; one
@@ -662,11 +663,16 @@ extern "C" int32_t vrad_bounce_upload(vrad_ctx *ctx, const vrad_bounce_desc *d) 
     unsigned long long pad = 0;
     if (e == cudaSuccess) e = cudaMemsetAsync(b.counters, 0, sizeof pad, s);
     if (e == cudaSuccess) e = launch_sell_pad(b, b.counters, s);
+    if (e == cudaSuccess && b.grouped())
+        e = cudaMemcpyAsync(&b.transfer_warps, b.group_off + b.ngroups(), sizeof b.transfer_warps, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess && R > 0) e = cudaMemcpyAsync(&ncand, b.cand_off + R, sizeof ncand, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&pad, b.counters, sizeof pad, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = vrad::wait_stream(s);
     b.ncand = ncand;
     clock.mark("candidate count");
+    if (e == cudaSuccess)
+        e = dev_alloc(&b.warp_group, sizeof(int32_t) * (size_t)(b.transfer_warps ? b.transfer_warps : 1));
+    if (e == cudaSuccess) e = launch_warp_groups(b, s);
     if (e == cudaSuccess) e = dev_alloc(&b.cand_src, sizeof(int32_t) * (size_t)(ncand ? ncand : 1));
     if (e == cudaSuccess) e = dev_alloc(&b.cand_w, sizeof(float) * (size_t)(ncand ? ncand : 1));
     // Transfers are at most the candidates: the list array takes that

@@ -189,7 +189,7 @@ template <bool ANY, int STRIDE = kBlock, bool UP = false, bool FLAG = false>
 __device__ __forceinline__ bool walk(const DeviceBvh &s, const int32_t *__restrict__ tri_id,
                                      const RayState &r, float tmin, int32_t skip_id, int start, int *stack,
                                      float &thi, int32_t &best_orig, uint32_t &best_meta,
-                                     NearCheck *nc = nullptr) {
+                                     NearCheck *nc = nullptr, int *at = nullptr) {
     constexpr int kEnd = INT32_MIN;
     const float4 *nodes = s.nodes + 8 * (size_t)(r.octant() * s.inner);
     bool hit = false;
@@ -250,6 +250,7 @@ __device__ __forceinline__ bool walk(const DeviceBvh &s, const int32_t *__restri
             thi = t;
             best_orig = orig;
             best_meta = meta;
+            if (at) *at = k;
             if (ANY) return true;
         }
         if (sp == 0) return hit;
@@ -267,19 +268,21 @@ __device__ __forceinline__ bool walk(const DeviceBvh &s, const int32_t *__restri
 //                 its first acceptance.
 // start: where the opaque tree's walk starts (start_node of the ray's
 // origin, or 0).  The sky tree is small and flat: its walk starts at the
-// root.
+// root.  kModeAny leaves in *at (when given) the opaque triangle that was
+// hit, by its place in the tree's arrays; a sky hit leaves it as it is.
 template <int MODE, int STRIDE = kBlock, bool UP = false>
 __device__ __forceinline__ void trace_ray(const DeviceScene &s, const RayState &r, float tmin,
                                           float reach, int32_t skip_id, int start, int *stack,
                                           bool &hit, float &best_t,
-                                          int32_t &best_orig, uint32_t &best_meta) {
+                                          int32_t &best_orig, uint32_t &best_meta, int *at = nullptr) {
     best_t = reach;
     best_orig = -1;
     best_meta = 0;
     hit = false;
     if (MODE == kModeAny) {
         if (s.opaque.ntris)
-            hit = walk<true, STRIDE, UP>(s.opaque, s.tri_id, r, tmin, skip_id, start, stack, best_t, best_orig, best_meta);
+            hit = walk<true, STRIDE, UP>(s.opaque, s.tri_id, r, tmin, skip_id, start, stack, best_t, best_orig, best_meta,
+                                         nullptr, at);
         if (!hit && s.sky.ntris)
             hit = walk<true, STRIDE>(s.sky, s.tri_id, r, tmin, skip_id, 0, stack, best_t, best_orig, best_meta);
     } else if (MODE == kModeClosest) {

@@ -171,6 +171,50 @@ def test_lumps_of_faces_of_few_and_many_luxels(oracle_mod, luxel_scale):
     assert len(bad) == 0, f"{len(bad)} of {len(lump) // 4} RGBE words differ"
 
 
+@pytest.mark.parametrize("side,scale,seed", [(2, 8.0, 3), (4, 16.0, 12)])
+def test_transfers_traced_by_groups_of_receivers(oracle_mod, side, scale, seed):
+    """Every transfer of maps with more receivers than the line from which
+    their rays are traced by groups, each first against the triangle that
+    blocked the one before it.  A ray through a triangle's edge can slip past
+    the reference's KD walk (test_adversarial_rays.py): where the lists
+    differ, brute force over all triangles, the device's contract, has to say
+    that the pair is blocked."""
+    O = oracle_mod
+    w = rg.generate(rg.Config(side=side, seed=seed, luxel_scale=scale, pillars=(1, 6)))
+    inp = L.prepare(w)
+    off, lst = L.pvs_lists(w)
+    refl = L.face_reflectivity(w)
+    with L.LightingStage(w, inp) as st:
+        st.upload_bounce(refl, off, lst, bounces=1)
+        st.light_pass()
+        t_off, tr = st.transfers()
+        bs = st.bounce_stats()
+    assert bs.receivers >= 65536 and 0.2 * bs.transfer_rays < bs.blocked < bs.transfer_rays
+    ob = O.Bounce(O.kd_build(w.tri_verts, w.tri_ids), inp.faces, inp.verts, inp.samples, inp.face_first, refl, off, lst,
+                  bounces=1)
+    o_off, o_src, o_w, rays = ob.transfers()
+    assert bs.transfer_rays == rays
+    same = np.diff(t_off) == np.diff(o_off)
+    assert same.mean() > 0.999
+    keep_t, keep_o = np.repeat(same, np.diff(t_off)), np.repeat(same, np.diff(o_off))
+    assert np.array_equal(tr["patch"][keep_t], o_src[keep_o])
+    assert np.array_equal(_bits(tr["weight"][keep_t]), _bits(o_w[keep_o]))
+    patches, _ = ob.patches()
+    at = (patches["origin"] + patches["normal"]).astype(np.float32)
+    pairs = []
+    for p in np.flatnonzero(~same):
+        mine, theirs = tr["patch"][t_off[p]:t_off[p + 1]], o_src[o_off[p]:o_off[p + 1]]
+        assert np.array_equal(mine, theirs[np.isin(theirs, mine)])
+        pairs += [(p, s) for s in theirs[~np.isin(theirs, mine)]]
+    if pairs:
+        p, s = np.array(pairs).T
+        d = at[s] - at[p]
+        length = np.sqrt((d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1]) + d[:, 2] * d[:, 2])
+        rays = np.concatenate([at[p], d / length[:, None], length[:, None]], axis=1)
+        _, _, blocked = O.brute_trace(O.prepare_triangles(w.tri_verts, w.tri_ids), rays)
+        assert O.bits_to_bool(blocked, len(rays)).all()
+
+
 def test_bounce_pass_is_repeatable_and_device_entry_matches():
     import torch
     w, inp, st = _stage(rg.config_3x3(seed=2))
