@@ -780,7 +780,7 @@ def ambient_run(args, samples: int = 131072) -> dict:
     out.update({"ms": ms, "rays_per_s": out["rays"] / (ms / 1000.0), "samples_per_s": samples / (ms / 1000.0),
                 "e2e": {"s": e2e_s, "rays_per_s": out["rays"] / e2e_s, "h2d_bytes": int(pos.nbytes),
                         "d2h_bytes": int(host.nbytes)},
-                "gpu_launches_per_call": 2 * ((samples + 16383) // 16384)})
+                "gpu_launches_per_call": 2 * ((samples + 32767) // 32768)})
     if not args.no_cpu:
         from oracle import oracle as O
         geom = B.trace_geometry(lumps)
@@ -1115,13 +1115,14 @@ def main_stage(args):
             "phase_ms": {"direct_both_ranges": direct_ms, "patch_light": statistics.median([p[0] for p in phases]),
                          "transfers": transfer_ms, "bounces": statistics.median([p[2] for p in phases])},
             "e2e": e2e,
-            # Per step (the ncu launch list in profiles/): the two-range
-            # gather 1; per range its supersampling (1 + 4 per pass run),
-            # patch light 2, final 4, per bounce the gather, the 8 tree
-            # levels of CollectLight and the totals; the transfer build 16
-            # (candidates, rays, count, write, slices, their scans and sort).
+            # Per step, the library's own kernels (its sort and scans come on
+            # top): the two-range gather 1; per range its supersampling (1 +
+            # 4 per pass run, one more where a pass is split by segments),
+            # patch light 2, final 4, per bounce the gather and
+            # CollectLight's parents; the transfer build 8 (candidates,
+            # starts, rays, count, write, three of the slices).
             "gpu_launches": (1 + (1 + 4 * int(st_l.extra_passes_run)) + (1 + 4 * int(st_h.extra_passes_run))
-                             + 2 * (2 + 4) + 16 + 10 * (nb_l + nb_h)) * args.steps,
+                             + 2 * (2 + 4) + 8 + 2 * (nb_l + nb_h)) * args.steps,
             "roofline": roofline,
             "cpu_baseline": cpu,
             "clocks": clocks.summary(),
