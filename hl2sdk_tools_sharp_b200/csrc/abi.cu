@@ -119,7 +119,7 @@ int32_t upload(vrad_ctx *ctx, const vrad_triangle *tris, const vrad_kd_triangle 
     vrad::BvhBuffers *dst[2] = {&ctx->scene.opaque, &ctx->scene.sky};
     for (int k = 0; k < 2; k++) {
         e = vrad::build_bvh(*dst[k], part[k].data(), prep ? ppart[k].data() : nullptr, orig[k].data(),
-                            (int)part[k].size(), ctx->stream, &ctx->report);
+                            (int)part[k].size(), ctx->scene.one_copy() ? 1 : 8, ctx->stream, &ctx->report);
         if (e != cudaSuccess) {
             ctx->scene.release();
             if (e == cudaErrorInvalidValue && prep)

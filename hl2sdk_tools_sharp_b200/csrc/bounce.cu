@@ -552,7 +552,7 @@ __global__ void k_starts(BounceView v, DeviceBvh opaque, int32_t *__restrict__ s
 // CTAs per SM (40 registers, a few spilled to L1).
 constexpr float kBlocked = -1.0f;
 
-template <int BLOCK>
+template <bool ONE, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 12)
     k_transfer(BounceView v, DeviceScene sc, const int64_t *__restrict__ cand_off, const int32_t *__restrict__ cand_src,
                const int32_t *__restrict__ start_at, float *__restrict__ cand_w, int64_t ncand,
@@ -592,7 +592,8 @@ __global__ void __launch_bounds__(BLOCK, 12)
         int32_t orig;
         uint32_t meta;
         bool blocked;
-        trace_ray<kModeAny, BLOCK, true>(sc, ray, 0.0f, len, -1, __ldg(&start_at[lo]), stack, blocked, t, orig, meta);
+        trace_ray<ONE, kModeAny, BLOCK, true>(sc, ray, 0.0f, len, -1, ONE ? 0 : __ldg(&start_at[lo]), stack, blocked, t,
+                                              orig, meta);
         if (!blocked) {
             // The pair's rows are read again here, not held across the walk:
             // at 40 registers they would be spilled to L1, whose bandwidth
@@ -635,7 +636,7 @@ __global__ void k_warp_groups(int ngroups, const int64_t *__restrict__ group_off
 // 62 %) 9.2 and 11.0; with 76 k receivers 2.23 and 2.31, with 61 k 1.66 both
 // ways, with 36 k 1.07 and 1.03: few receivers make too few warps of 512 rays
 // each.  Ten CTAs an SM: twelve 36.4 ms, eight 36.1.
-template <int BLOCK>
+template <bool ONE, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 10)
     k_transfer_groups(BounceView v, DeviceScene sc, const int64_t *__restrict__ cand_off,
                       const int32_t *__restrict__ cand_src, const int32_t *__restrict__ start_at,
@@ -683,8 +684,8 @@ __global__ void __launch_bounds__(BLOCK, 10)
             uint32_t meta;
             int at = -1;
             bool blocked;
-            trace_ray<kModeAny, BLOCK, true>(sc, ray, 0.0f, len, -1, __ldg(&start_at[r]), stack, blocked, t, orig, meta,
-                                             &at);
+            trace_ray<ONE, kModeAny, BLOCK, true>(sc, ray, 0.0f, len, -1, ONE ? 0 : __ldg(&start_at[r]), stack, blocked, t,
+                                                  orig, meta, &at);
             // The pair's rows are read again here, not held across the walk.
             e = queue[n - m + lane];
             q = off[e >> 5] + chunk + (e & 31);
@@ -1285,14 +1286,18 @@ cudaError_t launch_transfers(BounceBuffers &b, const DeviceScene &scene, uint32_
     }
     k_candidates<true><<<dim3(blocks(R, kBounceBlock), b.segments), kBounceBlock, 0, stream>>>(
         b.view, b.root_plane, b.root_origin, b.root_tree, b.seg_off, nullptr, b.cand_src, overflow);
-    k_starts<<<blocks(R, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, scene.opaque, b.start);
-    if (!b.grouped() && b.ncand > 0)
-        k_transfer<kBlock><<<blocks(b.ncand, kBlock), kBlock, sizeof(int) * scene.stack_depth() * kBlock, stream>>>(
-            b.view, scene, b.cand_off, b.cand_src, b.start, b.cand_w, b.ncand, &b.counters[2]);
-    if (b.transfer_warps > 0)
-        k_transfer_groups<kBlock><<<blocks(32 * b.transfer_warps, kBlock), kBlock, sizeof(int) * scene.stack_depth() * kBlock,
-                             stream>>>(b.view, scene, b.cand_off, b.cand_src, b.start, b.group_off, b.warp_group,
-                                       b.transfer_warps, b.cand_w, &b.counters[2]);
+    if (!scene.one_copy) k_starts<<<blocks(R, kBounceBlock), kBounceBlock, 0, stream>>>(b.view, scene.opaque, b.start);
+    const size_t stack = sizeof(int) * scene.stack_depth() * kBlock;
+    by_copies(scene, [&](auto one) {
+        constexpr bool kOne = decltype(one)::value;
+        if (!b.grouped() && b.ncand > 0)
+            k_transfer<kOne, kBlock><<<blocks(b.ncand, kBlock), kBlock, stack, stream>>>(
+                b.view, scene, b.cand_off, b.cand_src, b.start, b.cand_w, b.ncand, &b.counters[2]);
+        if (b.transfer_warps > 0)
+            k_transfer_groups<kOne, kBlock><<<blocks(32 * b.transfer_warps, kBlock), kBlock, stack, stream>>>(
+                b.view, scene, b.cand_off, b.cand_src, b.start, b.group_off, b.warp_group, b.transfer_warps, b.cand_w,
+                &b.counters[2]);
+    });
     k_transfer_count<<<blocks((int64_t)R * 32, kBounceBlock), kBounceBlock, 0, stream>>>(
         R, b.cand_off, b.cand_w, b.tr_off + 1, &b.counters[1]);
     e = cudaMemsetAsync(b.tr_off, 0, sizeof(int64_t), stream);

@@ -44,7 +44,7 @@ namespace {
 // its SM slot as soon as its own warps are done.
 // DUAL: one traversal lights both ranges (out from w.lights, out_hdr from
 // w.lights_hdr).
-template <int BLOCK, bool DUAL>
+template <bool ONE, int BLOCK, bool DUAL>
 __global__ void __launch_bounds__(BLOCK) k_direct(DeviceScene sc, DeviceWorld w, float4 *__restrict__ out,
                                                   float4 *__restrict__ out_hdr,
                                                   unsigned long long *__restrict__ counters) {
@@ -70,14 +70,14 @@ __global__ void __launch_bounds__(BLOCK) k_direct(DeviceScene sc, DeviceWorld w,
     // One unit off the face (ComputeIlluminationPointAndNormals).
     const float px = __fadd_rn(sp.x, nx), py = __fadd_rn(sp.y, ny), pz = __fadd_rn(sp.z, nz);
 
-    const int start = start_node(sc.opaque, px, py, pz);
+    const int start = ONE ? 0 : start_node(sc.opaque, px, py, pz);
     if (real) w.start[si] = start;
     uint32_t vis_rays = 0, sky_rays = 0;  // one point's rays
     float4 h;
     // The group's first sample (a face's groups start on lanes 0, 4, ...):
     // groups in sample order are ResolveGroup's order.
     const unsigned long long key_group = (unsigned long long)(uint32_t)__shfl_sync(kFull, si, lane & ~3) << 32;
-    const float4 r = gather_point<BLOCK, DUAL>(sc, w, cluster, px, py, pz, nx, ny, nz, real, gmask, kAllLights,
+    const float4 r = gather_point<ONE, BLOCK, DUAL>(sc, w, cluster, px, py, pz, nx, ny, nz, real, gmask, kAllLights,
                                                start, stack, counters, vis_rays, sky_rays,
                                                &h, face, key_group);
     if (real) {
@@ -141,19 +141,22 @@ cudaError_t launch_direct(const DeviceScene &scene, const DeviceWorld &world, fl
     const size_t smem = sizeof(int) * (size_t)scene.stack_depth();  // per thread
     const unsigned g32 = (unsigned)((world.nslots + 31) / 32), g64 = (unsigned)((world.nslots + 63) / 64),
                    g128 = (unsigned)((world.nslots + 127) / 128);
-    if (out_hdr) {
-        switch (block) {
-            case 32: k_direct<32, true><<<g32, 32, smem * 32, stream>>>(scene, world, out, out_hdr, counters); break;
-            case 64: k_direct<64, true><<<g64, 64, smem * 64, stream>>>(scene, world, out, out_hdr, counters); break;
-            default: k_direct<128, true><<<g128, 128, smem * 128, stream>>>(scene, world, out, out_hdr, counters); break;
+    by_copies(scene, [&](auto one) {
+        constexpr bool kOne = decltype(one)::value;
+        if (out_hdr) {
+            switch (block) {
+                case 32: k_direct<kOne, 32, true><<<g32, 32, smem * 32, stream>>>(scene, world, out, out_hdr, counters); break;
+                case 64: k_direct<kOne, 64, true><<<g64, 64, smem * 64, stream>>>(scene, world, out, out_hdr, counters); break;
+                default: k_direct<kOne, 128, true><<<g128, 128, smem * 128, stream>>>(scene, world, out, out_hdr, counters); break;
+            }
+        } else {
+            switch (block) {
+                case 32: k_direct<kOne, 32, false><<<g32, 32, smem * 32, stream>>>(scene, world, out, nullptr, counters); break;
+                case 64: k_direct<kOne, 64, false><<<g64, 64, smem * 64, stream>>>(scene, world, out, nullptr, counters); break;
+                default: k_direct<kOne, 128, false><<<g128, 128, smem * 128, stream>>>(scene, world, out, nullptr, counters); break;
+            }
         }
-    } else {
-        switch (block) {
-            case 32: k_direct<32, false><<<g32, 32, smem * 32, stream>>>(scene, world, out, nullptr, counters); break;
-            case 64: k_direct<64, false><<<g64, 64, smem * 64, stream>>>(scene, world, out, nullptr, counters); break;
-            default: k_direct<128, false><<<g128, 128, smem * 128, stream>>>(scene, world, out, nullptr, counters); break;
-        }
-    }
+    });
     return cudaGetLastError();
 }
 

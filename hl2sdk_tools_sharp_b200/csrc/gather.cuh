@@ -51,7 +51,7 @@ __device__ __forceinline__ bool group_any(bool v, unsigned gmask) {
 // The segment start -> stop (LightRayLog.MakeRay: whole segment, reach 1).
 // Visibility blocks on any hit; a sky test blocks only when the first hit
 // is opaque.
-template <int MODE, int STRIDE>
+template <bool ONE, int MODE, int STRIDE>
 __device__ __forceinline__ bool segment_blocked(const DeviceScene &sc, float sx, float sy, float sz,
                                                 float ex, float ey, float ez, int start, int *stack) {
     const RayState r = make_ray(sx, sy, sz, __fsub_rn(ex, sx), __fsub_rn(ey, sy), __fsub_rn(ez, sz));
@@ -59,7 +59,7 @@ __device__ __forceinline__ bool segment_blocked(const DeviceScene &sc, float sx,
     float t;
     int32_t orig;
     uint32_t meta;
-    trace_ray<MODE, STRIDE, true>(sc, r, 0.0f, 1.0f, -1, start, stack, hit, t, orig, meta);
+    trace_ray<ONE, MODE, STRIDE, true, true>(sc, r, 0.0f, 1.0f, -1, start, stack, hit, t, orig, meta);
     return hit;
 }
 
@@ -109,7 +109,7 @@ struct RayShare {
 // value from w.lights_hdr's intensities (every decision and every traced
 // segment is the range-independent one, so each range gets its own pass's
 // bits).
-template <int BLOCK, bool DUAL = false, int VIS = kTrace>
+template <bool ONE, int BLOCK, bool DUAL = false, int VIS = kTrace>
 __device__ __forceinline__ float4 gather_point(const DeviceScene &sc, const DeviceWorld &w, int cluster, float px,
                                                float py, float pz, float nx, float ny, float nz, bool real,
                                                unsigned gmask, int filter, int start, int *stack,
@@ -205,7 +205,7 @@ __device__ __forceinline__ float4 gather_point(const DeviceScene &sc, const Devi
             }
             const bool cond = real && dot != 0.0f && falloff != 0.0f;
             if (cond) vis_rays++;
-            if (is_blocked(cond, [&] { return segment_blocked<kModeAny, BLOCK>(sc, px, py, pz, A.x, A.y, A.z, start, stack); }))
+            if (is_blocked(cond, [&] { return segment_blocked<ONE, kModeAny, BLOCK>(sc, px, py, pz, A.x, A.y, A.z, start, stack); }))
                 dot = 0.0f;
         } else if (type == kSurface) {
             // GatherSurfaceFour (DirectLightGatherer.cs:1452-1545): the
@@ -237,7 +237,7 @@ __device__ __forceinline__ float4 gather_point(const DeviceScene &sc, const Devi
                     const float ex = __fadd_rn(A.x, __fmul_rn(C.x, kDistEpsilon)),
                                 ey = __fadd_rn(A.y, __fmul_rn(C.y, kDistEpsilon)),
                                 ez = __fadd_rn(A.z, __fmul_rn(C.z, kDistEpsilon));
-                    return segment_blocked<kModeAny, BLOCK>(sc, px, py, pz, ex, ey, ez, start, stack);
+                    return segment_blocked<ONE, kModeAny, BLOCK>(sc, px, py, pz, ex, ey, ez, start, stack);
                 }))
                 dot = 0.0f;
         } else if (type == kSkyLight) {
@@ -261,7 +261,7 @@ __device__ __forceinline__ float4 gather_point(const DeviceScene &sc, const Devi
                     float frac = 1.0f;
                     if (need && real) sky_rays++;
                     if (is_blocked(need && real, [&] {
-                            return segment_blocked<kModeSkyPass, BLOCK>(sc, px, py, pz, __fadd_rn(ex, px),
+                            return segment_blocked<ONE, kModeSkyPass, BLOCK>(sc, px, py, pz, __fadd_rn(ex, px),
                                                                         __fadd_rn(ey, py), __fadd_rn(ez, pz), start,
                                                                         stack);
                         }))
@@ -296,7 +296,7 @@ __device__ __forceinline__ float4 gather_point(const DeviceScene &sc, const Devi
                     const float ex = __fadd_rn(__fmul_rn(an.x, -kMaxTraceLength), px);
                     const float ey = __fadd_rn(__fmul_rn(an.y, -kMaxTraceLength), py);
                     const float ez = __fadd_rn(__fmul_rn(an.z, -kMaxTraceLength), pz);
-                    return segment_blocked<kModeSkyPass, BLOCK>(sc, px, py, pz, ex, ey, ez, start, stack);
+                    return segment_blocked<ONE, kModeSkyPass, BLOCK>(sc, px, py, pz, ex, ey, ez, start, stack);
                 }))
                     frac = 0.0f;
                 ambient = __fadd_rn(ambient, __fmul_rn(frac, dv));

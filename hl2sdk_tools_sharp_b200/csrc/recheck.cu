@@ -35,6 +35,7 @@
 namespace vrad {
 namespace {
 
+template <bool ONE>
 __global__ void __launch_bounds__(kBlock) k_trace_flag(DeviceScene s, const vrad_ray *__restrict__ rays, int64_t n,
                                                        float tmin, int32_t skip_id, float margin,
                                                        uint32_t *__restrict__ bits, int32_t *__restrict__ flagged,
@@ -63,7 +64,7 @@ __global__ void __launch_bounds__(kBlock) k_trace_flag(DeviceScene s, const vrad
         r.noy = -r.oy * r.iy;
         r.noz = -r.oz * r.iz;
         nc.thi = reach;
-        trace_ray_flagged(s, r, tmin, reach, skip_id, stack, hit, nc);
+        trace_ray_flagged<ONE>(s, r, tmin, reach, skip_id, stack, hit, nc);
         if (nc.near) flagged[atomicAdd(count, 1)] = (int32_t)i;
     }
     const uint32_t word = __ballot_sync(kFull, hit);
@@ -212,8 +213,10 @@ extern "C" int32_t vrad_trace_visibility_recheck(vrad_ctx *ctx, const vrad_ray *
     if (e == cudaSuccess) {
         const DeviceScene s = ctx->scene.view();
         const size_t smem = sizeof(int) * (size_t)s.stack_depth() * kBlock;
-        k_trace_flag<<<(unsigned)((n + kBlock - 1) / kBlock), kBlock, smem, ctx->stream>>>(
-            s, d_rays, n, tmin, skip, flag_margin, d_bits, d_flagged, d_count);
+        by_copies(s, [&](auto one) {
+            k_trace_flag<decltype(one)::value><<<(unsigned)((n + kBlock - 1) / kBlock), kBlock, smem, ctx->stream>>>(
+                s, d_rays, n, tmin, skip, flag_margin, d_bits, d_flagged, d_count);
+        });
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(&nflagged, d_count, sizeof nflagged, cudaMemcpyDeviceToHost, ctx->stream);

@@ -11,6 +11,7 @@
 //   host           boxes padded, SAH tree (two-child nodes of 64 B, leaf
 //                  references), uploaded
 //   k_octants      the nodes as a ray of each of the eight octants reads them
+//                  (a large scene's as octant 0 does, for all rays)
 //   k_gather       triangles into leaf order
 //
 // The tree's shape is free: no answer depends on it (the traversal tests
@@ -162,17 +163,19 @@ __global__ void k_bounds(const float *__restrict__ box, int n, float *__restrict
     }
 }
 
-// The eight octants' copies of the tree's nodes (vrad_internal.cuh's
-// layout) from its canonical ones: tree[4 i ..] = (c0.lo.x, c0.hi.x,
+// The octants' copies of the tree's nodes (vrad_internal.cuh's layout), the
+// first n nodes of them, from its canonical ones: tree[4 i ..] = (c0.lo.x, c0.hi.x,
 // c0.lo.y, c0.hi.y), (c1 the same), (c0.lo.z, c0.hi.z, c1.lo.z, c1.hi.z),
 // (ref0, ref1, -, -); parent[i] = node i's parent (-1 the root's).  A node's
 // two children are ordered by their boxes' centres along the octant's
-// diagonal; a node that leads up keeps the nearer generation first.
+// diagonal; a node that leads up keeps the nearer generation first.  An
+// empty box is a point farther off than any hit, which no segment meets
+// whether its planes come ordered by octant or not.
 __global__ void k_octants(const float4 *__restrict__ tree, const int32_t *__restrict__ parent, int inner,
-                          float4 *__restrict__ nodes) {
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= 16 * inner) return;
-    const int oct = id / (2 * inner), i = id - oct * 2 * inner;
+                          int64_t n, float4 *__restrict__ nodes) {
+    const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= n) return;
+    const int oct = (int)(id / (2 * inner)), i = (int)(id - (int64_t)oct * 2 * inner);
     float lo[2][3], hi[2][3];
     int ref[2], next = -1;
     auto child = [&](int node, int c, int to) {
@@ -194,7 +197,7 @@ __global__ void k_octants(const float4 *__restrict__ tree, const int32_t *__rest
         }
         for (int x = 0; x < 3; x++) {
             lo[to][x] = FLT_MAX;
-            hi[to][x] = -FLT_MAX;
+            hi[to][x] = FLT_MAX;
         }
         ref[to] = leaf_ref(0, 1);
         return -1;
@@ -223,7 +226,7 @@ __global__ void k_octants(const float4 *__restrict__ tree, const int32_t *__rest
             far[c][x] = neg ? lo[c][x] : hi[c][x];
         }
     const int p = swap ? 1 : 0, q = 1 - p;
-    float4 *o = nodes + 4 * (size_t)id;
+    float4 *o = nodes + 4 * id;
     o[0] = make_float4(near[p][0], near[p][1], far[p][0], far[p][1]);
     o[1] = make_float4(near[q][0], near[q][1], far[q][0], far[q][1]);
     o[2] = make_float4(near[p][2], far[p][2], near[q][2], far[q][2]);
@@ -247,7 +250,7 @@ __global__ void k_check_axes(const float4 *__restrict__ t2, int n, int *__restri
     if ((__float_as_uint(t2[i].w) & 3u) == 3u) atomicAdd(&stats[3], 1);
 }
 
-inline int blocks(int n, int b) { return (n + b - 1) / b; }
+inline unsigned blocks(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
 
 }  // namespace
 
@@ -261,7 +264,7 @@ inline int blocks(int n, int b) { return (n + b - 1) / b; }
     } while (0)
 
 cudaError_t build_bvh(BvhBuffers &sb, const vrad_triangle *h_tris,
-                      const vrad_kd_triangle *h_prepared, const int32_t *h_orig, int n,
+                      const vrad_kd_triangle *h_prepared, const int32_t *h_orig, int n, int copies,
                       cudaStream_t stream, SceneBuildReport *report) {
     cudaError_t err = cudaSuccess;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -275,6 +278,7 @@ cudaError_t build_bvh(BvhBuffers &sb, const vrad_triangle *h_tris,
     int32_t *order = nullptr, *d_parent = nullptr;
     int *d_stats = nullptr;
     int stats[4] = {0, 0, 0, 0};
+    int64_t nnodes = 0;
     float bounds[7];
     SahTree tree;
     std::vector<int32_t> parent;
@@ -332,8 +336,8 @@ cudaError_t build_bvh(BvhBuffers &sb, const vrad_triangle *h_tris,
             float r;
             std::memcpy(&r, &leaf, 4);
             tree.nodes = {make_float4(box[0], box[3], box[1], box[4]),
-                          make_float4(FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX),
-                          make_float4(box[2], box[5], FLT_MAX, -FLT_MAX), make_float4(r, r, 0.0f, 0.0f)};
+                          make_float4(FLT_MAX, FLT_MAX, FLT_MAX, FLT_MAX),
+                          make_float4(box[2], box[5], FLT_MAX, FLT_MAX), make_float4(r, r, 0.0f, 0.0f)};
             tree.order = {0};
             tree.inner = tree.leaves = tree.max_leaf = tree.depth = 1;
         } else {
@@ -353,13 +357,14 @@ cudaError_t build_bvh(BvhBuffers &sb, const vrad_triangle *h_tris,
         VRAD_TRY(dev_alloc(&order, sizeof(int32_t) * n));
         VRAD_TRY(dev_alloc(&d_tree, sizeof(float4) * tree.nodes.size()));
         VRAD_TRY(dev_alloc(&d_parent, sizeof(int32_t) * parent.size()));
-        VRAD_TRY(dev_alloc(&sb.nodes, sizeof(float4) * 16 * tree.nodes.size()));
+        nnodes = (int64_t)tree.inner * (copies > 1 ? 2 * copies : 1);
+        VRAD_TRY(dev_alloc(&sb.nodes, sizeof(float4) * 4 * (size_t)nnodes));
         VRAD_TRY(cudaMemcpyAsync(order, tree.order.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, stream));
         VRAD_TRY(cudaMemcpyAsync(d_tree, tree.nodes.data(), sizeof(float4) * tree.nodes.size(),
                                  cudaMemcpyHostToDevice, stream));
         VRAD_TRY(cudaMemcpyAsync(d_parent, parent.data(), sizeof(int32_t) * parent.size(), cudaMemcpyHostToDevice,
                                  stream));
-        k_octants<<<blocks(16 * tree.inner, 128), 128, 0, stream>>>(d_tree, d_parent, tree.inner, sb.nodes);
+        k_octants<<<blocks(nnodes, 128), 128, 0, stream>>>(d_tree, d_parent, tree.inner, nnodes, sb.nodes);
         k_gather<<<blocks(n, 256), 256, 0, stream>>>(order, n, u0, u1, u2, sb.tri0, sb.tri1, sb.tri2);
         VRAD_TRY(cudaGetLastError());
         stats[0] = tree.inner;
@@ -396,7 +401,7 @@ cudaError_t build_bvh(BvhBuffers &sb, const vrad_triangle *h_tris,
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, ev0, ev1);
         report->build_ms += ms;
-        report->device_bytes += (int64_t)n * 48 + (int64_t)sb.inner * 16 * 64;
+        report->device_bytes += (int64_t)n * 48 + nnodes * 64;
     }
 
 fail:

@@ -12,7 +12,7 @@ struct BvhBuffers {
     float4 *tri0 = nullptr;
     float4 *tri1 = nullptr;
     float4 *tri2 = nullptr;
-    float4 *nodes = nullptr;  // eight octants' copies, 2 inner nodes each
+    float4 *nodes = nullptr;  // eight octants' copies of 2 inner nodes, or inner nodes
     int32_t ntris = 0;
     int32_t depth = 0;  // inner nodes on the longest root-to-leaf path
     int32_t inner = 0;  // inner nodes
@@ -27,8 +27,9 @@ struct SceneBuffers {
     int32_t *tri_id = nullptr;  // caller ids by original index
     int32_t ntris = 0;
 
+    bool one_copy() const { return ntris > kOctantTriangles; }
     void release();
-    DeviceScene view() const { return DeviceScene{opaque.view(), sky.view(), tri_id}; }
+    DeviceScene view() const { return DeviceScene{opaque.view(), sky.view(), tri_id, one_copy()}; }
 };
 
 struct SceneBuildReport {
@@ -45,10 +46,10 @@ struct SceneBuildReport {
 
 // Builds one BVH from n host triangles (and, optionally, their
 // intersection form); h_orig gives each triangle's original index in the
-// whole scene.  Synchronises `stream` before returning.  report is
-// accumulated into (counts added, bounds merged).
+// whole scene; copies of the nodes: 8 or 1.  Synchronises `stream` before
+// returning.  report is accumulated into (counts added, bounds merged).
 cudaError_t build_bvh(BvhBuffers &bb, const vrad_triangle *h_tris,
-                      const vrad_kd_triangle *h_prepared, const int32_t *h_orig, int n,
+                      const vrad_kd_triangle *h_prepared, const int32_t *h_orig, int n, int copies,
                       cudaStream_t stream, SceneBuildReport *report);
 
 // Traversal launches (trace.cu).  d_bits is written as 32-bit words.

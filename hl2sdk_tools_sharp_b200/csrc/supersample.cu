@@ -191,7 +191,7 @@ __device__ bool point_outside(float x, float y, float z, const float4 *__restric
 // One point of a supersampled row: its position in the cell, the winding
 // test of its row of four, the gather (the sky ambient for row 0, the other
 // lights for rows 1-4) and its LightingValue.
-template <int BLOCK, int VIS>
+template <bool ONE, int BLOCK, int VIS>
 __global__ void __launch_bounds__(BLOCK) k_resample(DeviceScene sc, DeviceWorld w, FinalView fv, int32_t ngroups,
                                                     int32_t nruns, const int32_t *__restrict__ base,
                                                     const int32_t *__restrict__ rows,
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(BLOCK) k_resample(DeviceScene sc, DeviceWorld 
     // A row whose four points all lie outside is not gathered.
     real = code >= 0 && bits != 0xFu;
     uint32_t vis_rays = 0, sky_rays = 0;  // one point's rays
-    const float4 r = gather_point<BLOCK, false, VIS>(
+    const float4 r = gather_point<ONE, BLOCK, false, VIS>(
         sc, w, cluster, px, py, pz, nx, ny, nz, real, gmask, ambient ? kAmbientOnly : kDirectOnly, start, stack, counters,
         vis_rays, sky_rays, nullptr, 0, 0,
         {words, (ngroups + 7) / 8, (int)(tid >> 5), (int)gridDim.y, (int)blockIdx.y});
@@ -412,17 +412,21 @@ static cudaError_t launch_resample(const SupersampleBuffers &ss, const DeviceSce
     const int nwarps = (g + 7) / 8, runs = 2 * ss.nclusters + 1;
     const int shares = ss.max_rays >= world.max_rays ? std::min(kSplitWarps / nwarps, world.max_rays) : 1;
     if (shares < 2) {
-        k_resample<kSsBlock, kTrace><<<grid, kSsBlock, stack, s>>>(scene, world, fv, g, runs, ss.base, ss.rows,
-                                                                   ss.selected, ss.origin_st, ss.wind, ss.points,
-                                                                   ss.row_out, ss.row_bits, counters, nullptr);
+        by_copies(scene, [&](auto one) {
+            k_resample<decltype(one)::value, kSsBlock, kTrace><<<grid, kSsBlock, stack, s>>>(
+                scene, world, fv, g, runs, ss.base, ss.rows, ss.selected, ss.origin_st, ss.wind, ss.points, ss.row_out,
+                ss.row_bits, counters, nullptr);
+        });
         return cudaGetLastError();
     }
     // The tracing launches' own counts (pow_cr's) go to the scratch counters.
     unsigned long long *scratch = (unsigned long long *)(ss.words + (size_t)kSplitWarps * ss.max_rays);
-    k_resample<kSsBlock, kTraceShare><<<dim3(grid, (unsigned)shares), kSsBlock, stack, s>>>(
-        scene, world, fv, g, runs, ss.base, ss.rows, ss.selected, ss.origin_st, ss.wind, ss.points, ss.row_out,
-        ss.row_bits, scratch, ss.words);
-    k_resample<kSsBlock, kLookUp><<<grid, kSsBlock, 0, s>>>(scene, world, fv, g, runs, ss.base, ss.rows, ss.selected,
+    by_copies(scene, [&](auto one) {
+        k_resample<decltype(one)::value, kSsBlock, kTraceShare><<<dim3(grid, (unsigned)shares), kSsBlock, stack, s>>>(
+            scene, world, fv, g, runs, ss.base, ss.rows, ss.selected, ss.origin_st, ss.wind, ss.points, ss.row_out,
+            ss.row_bits, scratch, ss.words);
+    });
+    k_resample<false, kSsBlock, kLookUp><<<grid, kSsBlock, 0, s>>>(scene, world, fv, g, runs, ss.base, ss.rows, ss.selected,
                                                             ss.origin_st, ss.wind, ss.points, ss.row_out, ss.row_bits,
                                                             counters, ss.words);
     return cudaGetLastError();

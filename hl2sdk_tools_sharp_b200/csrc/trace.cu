@@ -24,7 +24,7 @@ namespace vrad {
 
 namespace {
 
-template <int MODE>
+template <bool ONE, int MODE>
 __global__ void __launch_bounds__(kBlock) k_trace(DeviceScene s, const vrad_ray *__restrict__ rays,
                                                   int64_t n, TraceParams p, uint32_t *__restrict__ bits,
                                                   vrad_hit *__restrict__ hits) {
@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(kBlock) k_trace(DeviceScene s, const vrad_ray 
         r.nox = -r.ox * r.ix;
         r.noy = -r.oy * r.iy;
         r.noz = -r.oz * r.iz;
-        trace_ray<MODE>(s, r, p.tmin, reach, p.skip_id, 0, stack, hit, best_t, best_orig, best_meta);
+        trace_ray<ONE, MODE>(s, r, p.tmin, reach, p.skip_id, 0, stack, hit, best_t, best_orig, best_meta);
     }
     if (MODE == kModeClosest) {
         if (i < n) {
@@ -82,24 +82,29 @@ cudaError_t launch_trace(const DeviceScene &scene, const vrad_ray *d_rays, int64
     const int64_t grid = (n + kBlock - 1) / kBlock;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
     const size_t smem = sizeof(int) * (size_t)scene.stack_depth() * kBlock;
-    switch (p.mode) {
-        case kModeAny:
-            k_trace<kModeAny><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits, d_hits);
-            break;
-        case kModeClosest:
-            k_trace<kModeClosest><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits, d_hits);
-            break;
-        default:
-            k_trace<kModeSkyPass><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits, d_hits);
-            break;
-    }
+    by_copies(scene, [&](auto one) {
+        constexpr bool kOne = decltype(one)::value;
+        switch (p.mode) {
+            case kModeAny:
+                k_trace<kOne, kModeAny><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits, d_hits);
+                break;
+            case kModeClosest:
+                k_trace<kOne, kModeClosest><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits, d_hits);
+                break;
+            default:
+                k_trace<kOne, kModeSkyPass><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits, d_hits);
+                break;
+        }
+    });
     return cudaGetLastError();
 }
 
 cudaError_t load_visibility_kernels() {
     cudaFuncAttributes a;
-    cudaError_t e = cudaFuncGetAttributes(&a, k_trace<kModeAny>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_trace<kModeSkyPass>);
+    cudaError_t e = cudaFuncGetAttributes(&a, k_trace<false, kModeAny>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_trace<false, kModeSkyPass>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_trace<true, kModeAny>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_trace<true, kModeSkyPass>);
     return e;
 }
 

@@ -20,7 +20,7 @@ struct RayState {
     float ox, oy, oz, dx, dy, dz;
     float ix, iy, iz;      // 1/d with zeros saturated to +-2^60
     float nox, noy, noz;   // -o/d, for the FMA slab test
-    // The direction's octant: the copy of the nodes the walk reads.
+    // The direction's octant: the copy of the nodes the walk reads (of eight).
     __device__ __forceinline__ int octant() const {
         return (int)((__float_as_uint(ix) >> 31) | ((__float_as_uint(iy) >> 31) << 1) |
                      ((__float_as_uint(iz) >> 31) << 2));
@@ -128,6 +128,16 @@ __device__ __forceinline__ bool box_hit(const float4 &p, float zn, float zf, con
     return fmaxf(fmaxf(fmaxf(n.x, n.y), z.x), lo) <= fminf(fminf(fminf(f.x, f.y), z.y), hi);
 }
 
+// The same for planes as they lie (low, high), and where the segment enters.
+__device__ __forceinline__ bool box_meet(const float4 &p, float zl, float zh, const RayState &r, float lo, float hi,
+                                         float &enter) {
+    const float2 ixy = make_float2(r.ix, r.iy), nxy = make_float2(r.nox, r.noy);
+    const float2 a = fma2(make_float2(p.x, p.y), ixy, nxy), b = fma2(make_float2(p.z, p.w), ixy, nxy);
+    const float2 z = fma2(make_float2(zl, zh), make_float2(r.iz, r.iz), make_float2(r.noz, r.noz));
+    enter = fmaxf(fmaxf(fminf(a.x, b.x), fminf(a.y, b.y)), fmaxf(fminf(z.x, z.y), lo));
+    return enter <= fminf(fminf(fmaxf(a.x, b.x), fmaxf(a.y, b.y)), fminf(fmaxf(z.x, z.y), hi));
+}
+
 // The deepest inner node whose box, and every box above it, holds the point
 // (of two children that do, the one with the smaller box): where walk()
 // best starts for segments from there.
@@ -154,13 +164,44 @@ __device__ inline int start_node(const DeviceBvh &s, float x, float y, float z) 
     }
 }
 
-// One walk of one BVH.  Accepts a triangle hit (t, orig) when
-// t >= tmin and (t, orig) is lexicographically below the current best
-// (thi, best_orig); best_orig = -1 makes the window half-open, [tmin, thi).
-// ANY stops at the first acceptance; otherwise the best is kept and the
-// box window shrinks to [tmin, thi].  Returns whether anything was accepted.
-// Of two children the segment meets, the one nearer along its octant's
-// diagonal is entered first.
+// The triangles of the leaf `ref`.  Accepts a hit (t, orig) when t >= tmin and
+// (t, orig) is lexicographically below the current best (thi, best_orig);
+// best_orig = -1 makes the window half-open, [tmin, thi).  ANY stops at the
+// first acceptance; otherwise the best is kept.  Returns whether anything was
+// accepted.
+template <bool ANY, bool FLAG>
+__device__ __forceinline__ bool test_leaf(const DeviceBvh &s, const int32_t *__restrict__ tri_id, const RayState &r,
+                                          float tmin, int32_t skip_id, int ref, float &thi, int32_t &best_orig,
+                                          uint32_t &best_meta, NearCheck *nc, int *at) {
+    const int packed = ~ref;
+    const int first = packed >> 3;
+    const int count = (packed & 7) + 1;
+    bool hit = false;
+    for (int k = first; k < first + count; k++) {
+        float t;
+        uint32_t meta;
+        int32_t orig;
+        if (!kd_hit<FLAG>(s, k, r, t, meta, orig, nc)) continue;
+        if (!(t >= tmin)) continue;
+        if (!(t < thi || (t == thi && orig < best_orig))) continue;
+        if (skip_id != -1 && __ldg(&tri_id[orig]) == skip_id) continue;
+        hit = true;
+        thi = t;
+        best_orig = orig;
+        best_meta = meta;
+        if (at) *at = k;
+        if (ANY) return true;
+    }
+    return hit;
+}
+
+// One walk of one BVH: the leaves whose boxes the segment meets within
+// [tmin, thi], which shrinks with every hit that is kept.  Returns whether
+// anything was accepted.
+//
+// walk_octants, for scenes of up to kOctantTriangles triangles: of two
+// children the segment meets, the one nearer along its octant's diagonal is
+// entered first.
 //
 // UP: the walk starts with the subtree of inner node `start`, then takes the
 // nodes that lead up from it (vrad_internal.cuh), each holding the next two
@@ -186,7 +227,7 @@ __device__ inline int start_node(const DeviceBvh &s, float x, float y, float z) 
 // gave 57.8 ms for the transfer build, one 32-byte load for two 16-byte
 // ones nothing.
 template <bool ANY, int STRIDE = kBlock, bool UP = false, bool FLAG = false>
-__device__ __forceinline__ bool walk(const DeviceBvh &s, const int32_t *__restrict__ tri_id,
+__device__ __forceinline__ bool walk_octants(const DeviceBvh &s, const int32_t *__restrict__ tri_id,
                                      const RayState &r, float tmin, int32_t skip_id, int start, int *stack,
                                      float &thi, int32_t &best_orig, uint32_t &best_meta,
                                      NearCheck *nc = nullptr, int *at = nullptr) {
@@ -235,28 +276,92 @@ __device__ __forceinline__ bool walk(const DeviceBvh &s, const int32_t *__restri
             }
         }
         if (ref == kEnd) return hit;
-        const int packed = ~ref;
-        const int first = packed >> 3;
-        const int count = (packed & 7) + 1;
-        for (int k = first; k < first + count; k++) {
-            float t;
-            uint32_t meta;
-            int32_t orig;
-            if (!kd_hit<FLAG>(s, k, r, t, meta, orig, nc)) continue;
-            if (!(t >= tmin)) continue;
-            if (!(t < thi || (t == thi && orig < best_orig))) continue;
-            if (skip_id != -1 && __ldg(&tri_id[orig]) == skip_id) continue;
+        if (test_leaf<ANY, FLAG>(s, tri_id, r, tmin, skip_id, ref, thi, best_orig, best_meta, nc, at)) {
             hit = true;
-            thi = t;
-            best_orig = orig;
-            best_meta = meta;
-            if (at) *at = k;
             if (ANY) return true;
         }
         if (sp == 0) return hit;
         sp--;
         ref = stack[sp * STRIDE];
     }
+}
+
+// The same walk from the root over one copy of the nodes, for scenes of more
+// than kOctantTriangles triangles: of two children the segment meets, the one
+// that it enters first, or with FAR the other (the gather's segments, measured
+// below).
+//
+// What bounds it: the nodes come from L2, and a ray visits thirty and more of
+// them.  Eight copies leave L1 little to keep, and past 100 k triangles fill
+// the L2; and where a ray seldom meets a triangle, lanes that wait for one
+// another's leaves cost more than tests at part of the warp.  Triangle soups
+// (2 M rays, ms; octants, then this, any hit and closest; rays in random
+// directions, then warps of neighbouring rays):
+//   10 k   1.07 1.13, 0.94 1.03;   0.39 0.40, 0.37 0.39
+//   20 k   1.26 1.33, 1.13 1.24;   0.50 0.51, 0.49 0.52
+//   100 k  1.67 1.82, 1.55 1.74;   0.90 0.97, 0.82 0.92
+//   400 k  2.52 2.89, 1.96 2.21;   1.56 1.73, 1.28 1.44
+//   1.5 M  3.93 4.36, 2.68 3.18;   2.00 2.34, 1.75 2.05
+// Light passes of the room grids with so many small triangles added: 4x4 grid,
+// 5 k in all 44.8 and 46.4 ms, 18 k 92.1 and 81.8, 102 k 130 and 108, 1.5 M
+// 504 and 355; 8x8 grid, 9 k 84.4 and 99.9, 17 k 133 and 146, 29 k 179 and
+// 180.  Started from the origin's leaf as walk_octants' UP, the 1.5 M took 444
+// with the nearer child first and 452 with the farther.
+template <bool ANY, int STRIDE, bool FAR, bool FLAG>
+__device__ __forceinline__ bool walk_one(const DeviceBvh &s, const int32_t *__restrict__ tri_id, const RayState &r,
+                                         float tmin, int32_t skip_id, int *stack, float &thi, int32_t &best_orig,
+                                         uint32_t &best_meta, NearCheck *nc, int *at) {
+    bool hit = false;
+    int sp = 0;
+    int ref = 0;
+    while (true) {
+        if (ref >= 0) {
+            const float4 *nd = s.nodes + 4 * (size_t)ref;
+            const float4 a = __ldg(nd), b = __ldg(nd + 1), c = __ldg(nd + 2);
+            const int2 child = __ldg(reinterpret_cast<const int2 *>(nd + 3));
+            float lo = tmin, hi = thi, e0, e1;
+            if constexpr (FLAG) {
+                // The recheck also wants the triangles just past either end.
+                const float tm = nc->m * fmaxf(1.0f, fabsf(thi));
+                lo -= tm;
+                hi += tm;
+            }
+            const bool h0 = box_meet(a, c.x, c.y, r, lo, hi, e0), h1 = box_meet(b, c.z, c.w, r, lo, hi, e1);
+            if (h0 && h1) {
+                const bool second = FAR ? e1 > e0 : e1 < e0;
+                stack[sp * STRIDE] = second ? child.x : child.y;
+                sp++;
+                ref = second ? child.y : child.x;
+                continue;
+            }
+            if (h0) {
+                ref = child.x;
+                continue;
+            }
+            if (h1) {
+                ref = child.y;
+                continue;
+            }
+        } else if (test_leaf<ANY, FLAG>(s, tri_id, r, tmin, skip_id, ref, thi, best_orig, best_meta, nc, at)) {
+            hit = true;
+            if (ANY) return true;
+        }
+        if (sp == 0) return hit;
+        sp--;
+        ref = stack[sp * STRIDE];
+    }
+}
+
+// UP and start are walk_octants', FAR walk_one's.
+template <bool ONE, bool ANY, int STRIDE = kBlock, bool UP = false, bool FLAG = false, bool FAR = false>
+__device__ __forceinline__ bool walk(const DeviceBvh &s, const int32_t *__restrict__ tri_id, const RayState &r, float tmin,
+                                     int32_t skip_id, int start, int *stack, float &thi, int32_t &best_orig,
+                                     uint32_t &best_meta, NearCheck *nc = nullptr, int *at = nullptr) {
+    if constexpr (ONE)
+        return walk_one<ANY, STRIDE, FAR, FLAG>(s, tri_id, r, tmin, skip_id, stack, thi, best_orig, best_meta, nc, at);
+    else
+        return walk_octants<ANY, STRIDE, UP, FLAG>(s, tri_id, r, tmin, skip_id, start, stack, thi, best_orig, best_meta,
+                                                   nc, at);
 }
 
 // One ray against the scene.  Modes:
@@ -270,7 +375,8 @@ __device__ __forceinline__ bool walk(const DeviceBvh &s, const int32_t *__restri
 // origin, or 0).  The sky tree is small and flat: its walk starts at the
 // root.  kModeAny leaves in *at (when given) the opaque triangle that was
 // hit, by its place in the tree's arrays; a sky hit leaves it as it is.
-template <int MODE, int STRIDE = kBlock, bool UP = false>
+// FAR: which child the opaque any-hit walk over one copy enters first.
+template <bool ONE, int MODE, int STRIDE = kBlock, bool UP = false, bool FAR = false>
 __device__ __forceinline__ void trace_ray(const DeviceScene &s, const RayState &r, float tmin,
                                           float reach, int32_t skip_id, int start, int *stack,
                                           bool &hit, float &best_t,
@@ -281,28 +387,28 @@ __device__ __forceinline__ void trace_ray(const DeviceScene &s, const RayState &
     hit = false;
     if (MODE == kModeAny) {
         if (s.opaque.ntris)
-            hit = walk<true, STRIDE, UP>(s.opaque, s.tri_id, r, tmin, skip_id, start, stack, best_t, best_orig, best_meta,
+            hit = walk<ONE, true, STRIDE, UP, false, FAR>(s.opaque, s.tri_id, r, tmin, skip_id, start, stack, best_t, best_orig, best_meta,
                                          nullptr, at);
         if (!hit && s.sky.ntris)
-            hit = walk<true, STRIDE>(s.sky, s.tri_id, r, tmin, skip_id, 0, stack, best_t, best_orig, best_meta);
+            hit = walk<ONE, true, STRIDE>(s.sky, s.tri_id, r, tmin, skip_id, 0, stack, best_t, best_orig, best_meta);
     } else if (MODE == kModeClosest) {
         if (s.opaque.ntris)
-            hit = walk<false, STRIDE, UP>(s.opaque, s.tri_id, r, tmin, skip_id, start, stack, best_t, best_orig, best_meta);
+            hit = walk<ONE, false, STRIDE, UP>(s.opaque, s.tri_id, r, tmin, skip_id, start, stack, best_t, best_orig, best_meta);
         if (s.sky.ntris)
-            hit |= walk<false, STRIDE>(s.sky, s.tri_id, r, tmin, skip_id, 0, stack, best_t, best_orig, best_meta);
+            hit |= walk<ONE, false, STRIDE>(s.sky, s.tri_id, r, tmin, skip_id, 0, stack, best_t, best_orig, best_meta);
     } else {
         if (s.sky.ntris)
-            walk<false, STRIDE>(s.sky, s.tri_id, r, tmin, skip_id, 0, stack, best_t, best_orig, best_meta);
+            walk<ONE, false, STRIDE>(s.sky, s.tri_id, r, tmin, skip_id, 0, stack, best_t, best_orig, best_meta);
         // Blocked iff an opaque hit sorts before the nearest sky hit.
         if (s.opaque.ntris)
-            hit = walk<true, STRIDE, UP>(s.opaque, s.tri_id, r, tmin, skip_id, start, stack, best_t, best_orig, best_meta);
+            hit = walk<ONE, true, STRIDE, UP, false, FAR>(s.opaque, s.tri_id, r, tmin, skip_id, start, stack, best_t, best_orig, best_meta);
     }
 }
 
 
 // kModeAny with the FP64 recheck's flag: the same walks and answer as
 // trace_ray<kModeAny>, every box widened by the margin at both ends.
-template <int STRIDE = kBlock>
+template <bool ONE, int STRIDE = kBlock>
 __device__ __forceinline__ void trace_ray_flagged(const DeviceScene &s, const RayState &r, float tmin, float reach,
                                                   int32_t skip_id, int *stack, bool &hit, NearCheck &nc) {
     float best_t = reach;
@@ -310,10 +416,10 @@ __device__ __forceinline__ void trace_ray_flagged(const DeviceScene &s, const Ra
     uint32_t best_meta = 0;
     hit = false;
     if (s.opaque.ntris)
-        hit = walk<true, STRIDE, false, true>(s.opaque, s.tri_id, r, tmin, skip_id, 0, stack, best_t, best_orig, best_meta,
+        hit = walk<ONE, true, STRIDE, false, true>(s.opaque, s.tri_id, r, tmin, skip_id, 0, stack, best_t, best_orig, best_meta,
                                        &nc);
     if (!hit && s.sky.ntris)
-        hit = walk<true, STRIDE, false, true>(s.sky, s.tri_id, r, tmin, skip_id, 0, stack, best_t, best_orig, best_meta, &nc);
+        hit = walk<ONE, true, STRIDE, false, true>(s.sky, s.tri_id, r, tmin, skip_id, 0, stack, best_t, best_orig, best_meta, &nc);
 }
 
 __device__ __forceinline__ RayState make_ray(float ox, float oy, float oz, float dx, float dy, float dz) {

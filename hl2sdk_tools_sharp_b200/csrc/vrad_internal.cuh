@@ -13,10 +13,13 @@
 //            meta = drop axis (bits 0-1) | sky (bit 2) | FCACHETRI flags << 8
 //   tri_id[orig]  int  the caller's id, read only for skip_id and outputs
 //
-// The nodes lie in eight copies, one per octant of a ray's direction (bit a
-// set: the direction's axis a is negative), 2 x `inner` nodes each; in a
-// copy every box is stored as the planes such a ray meets first (near) and
-// last (far), and child 0 is the child it meets first:
+// The nodes of a scene of up to kOctantTriangles triangles lie in eight
+// copies, one per octant of a ray's direction (bit a set: the direction's
+// axis a is negative), 2 x `inner` nodes each (1 KB an inner node); in a copy
+// every box is stored as the planes such a ray meets first (near) and last
+// (far), and child 0 is the child it meets first.  A larger scene has the
+// first `inner` nodes of octant 0's copy alone (64 B an inner node), near the
+// low planes and far the high ones:
 //   node[k]  4 x float4 = 64 B, two child boxes and two child references:
 //            n0 = child 0 (near.x, near.y, far.x, far.y)
 //            n1 = child 1 (near.x, near.y, far.x, far.y)
@@ -25,7 +28,7 @@
 //            ref >= 0 is an inner node; ref < 0 is a leaf, ~ref packing
 //            (first triangle << 3) | (count - 1), so a leaf holds 1..8.
 //            n3.z is -1.
-// Nodes inner .. 2 inner - 1 lead from a subtree up to the rest of the tree:
+// Of eight copies, nodes inner .. 2 inner - 1 lead from a subtree up to the rest of the tree:
 // node inner + k has as its children the sibling of node k and the sibling
 // of k's parent (an empty box where there is none), and n3.z the node that
 // leads on from k's grandparent, -1 when the two children complete the
@@ -33,6 +36,7 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 
 #include "../../include/vrad_cuda.h"
 
@@ -43,6 +47,9 @@ constexpr int kStackDepth = 64;
 constexpr uint32_t kTraceIdSky = 0x01000000u;   // TraceId.Sky (MapTools/Rad/TraceId.cs)
 constexpr float kKdEps = 1.0e-10f;              // KdRayTracer.cs:1209-1230
 constexpr float kKdHuge = 1.0e23f;              // KdRayTracer.cs:985
+// Scenes of more triangles keep one copy of the nodes: where the two walks
+// take as long for warps of neighbouring rays (walk_one's table).
+constexpr int32_t kOctantTriangles = 20000;
 
 struct DeviceBvh {
     const float4 *tri0;
@@ -51,13 +58,14 @@ struct DeviceBvh {
     const float4 *nodes;
     int32_t ntris;  // 0: empty, never traversed
     int32_t depth;  // inner nodes on the longest root-to-leaf path
-    int32_t inner;  // the tree's inner nodes: half of one octant's copy
+    int32_t inner;  // the tree's inner nodes
 };
 
 struct DeviceScene {
     DeviceBvh opaque;
     DeviceBvh sky;
     const int32_t *tri_id;
+    bool one_copy;  // of the nodes: the kernels' ONE
     // The traversal stack's entries per thread (kernels size their shared
     // memory by it).  A walk holds at most one entry per inner node of the
     // path below the subtree it is in, and two more while it climbs: the
@@ -68,6 +76,13 @@ struct DeviceScene {
         return d + 2;
     }
 };
+
+// f(std::true_type or std::false_type): a launch of the kernel for the scene's
+// copies of the nodes.
+template <typename F>
+auto by_copies(const DeviceScene &s, F &&f) {
+    return s.one_copy ? f(std::true_type{}) : f(std::false_type{});
+}
 
 enum TraceMode : int { kModeAny = 0, kModeClosest = 1, kModeSkyPass = 2 };
 

@@ -5,6 +5,8 @@ FinalLightFace.BuildPatchRadial.
 The bar is bit-exact: every transfer (source and weight bits), every
 patch's direct and bounced light, the number of bounces the stop rule runs,
 and the LIGHTING lump's bytes."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -341,3 +343,33 @@ def test_direct_gather_queued_at_the_world_upload_lights_the_same_lump():
     st.upload_bounce(refl, off, lst)
     assert np.array_equal(st.light_pass()[0], noextra)
     st.close()
+
+
+@pytest.mark.parametrize("side,scale", [(2, 16.0), (4, 8.0)])
+def test_triangles_out_of_reach_light_the_same_lumps(side, scale):
+    """A scene of more than 20,000 triangles walks one copy of its nodes, in
+    the gather, the resampling and the transfers (by ray on the small map, by
+    groups of receivers on the large one).  The same map with as many
+    triangles far below it, which no segment reaches, is lit bit for bit as
+    the map alone."""
+    w = rg.generate(dataclasses.replace(rg.config_8x8(seed=4), side=side, luxel_scale=scale, lights=side * side,
+                                        sky_ambient=True))
+    inp = L.prepare(w, hdr=True)
+    off, lst = L.pvs_lists(w)
+    rng = np.random.default_rng(6)
+    far = rng.uniform(-8000.0, 8000.0, (20000, 1, 3)) + rng.uniform(-50.0, 50.0, (20000, 3, 3))
+    far[:, :, 2] -= 300000.0
+    verts = np.concatenate([np.asarray(w.tri_verts, np.float32).reshape(-1, 9), far.reshape(-1, 9).astype(np.float32)])
+    ids = np.concatenate([w.tri_ids, np.full(len(far), w.tri_ids[0], w.tri_ids.dtype)])
+    with L.LightingStage(w, inp) as st:
+        st.upload_bounce(L.face_reflectivity(w), off, lst, threshold=1.0)
+        want_ldr, want_hdr, *_ = st.light_pass_ranges()
+        bounces = st.bounce_stats().bounces
+        t_off, t_rec = st.transfers()
+        st.tracer.upload_scene(T.make_triangles(verts, ids))
+        ldr, hdr, *_ = st.light_pass_ranges()
+        assert want_ldr.any() and want_hdr.any() and len(t_rec)
+        assert np.array_equal(ldr, want_ldr) and np.array_equal(hdr, want_hdr)
+        assert st.bounce_stats().bounces == bounces
+        o2, r2 = st.transfers()
+        assert np.array_equal(o2, t_off) and np.array_equal(r2, t_rec)

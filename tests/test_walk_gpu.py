@@ -54,3 +54,34 @@ def test_soup_equals_brute_force(n, sky, oracle_mod):
         assert np.array_equal(got["surface"], np.where(best >= 0, ids[np.maximum(best, 0)], -1))
         hit = best >= 0
         assert np.array_equal(got["fraction"][hit].view(np.uint32), dist[hit].astype(np.float32).view(np.uint32))
+
+
+@pytest.mark.parametrize("n,sky", [(20000, 1), (20001, 1), (20001, 20000), (30000, 3000)])
+def test_soup_of_many_triangles_equals_brute_force(n, sky, oracle_mod):
+    """About the size from which a scene keeps one copy of its nodes (one of
+    the trees may still be a single triangle): the same answers from every
+    entry that walks, and no more than a node's own 64 bytes for each."""
+    O = oracle_mod
+    verts, ids = soup(n, sky, 12)
+    verts = verts.reshape(n, 3, 3)
+    verts = (verts.mean(1, keepdims=True) + 0.1 * (verts - verts.mean(1, keepdims=True))).reshape(n, 9)
+    rays = rays_for(n, 2048)
+    tris = O.prepare_triangles(verts, ids)
+    flat = rays.view(np.float32).reshape(-1, 7)
+    with T.CudaRayTracer(T.make_triangles(verts, ids)) as tr:
+        info = tr.scene_info()
+        if n > 20000:
+            assert info.device_bytes <= 52 * n + 64 * info.bvh_nodes
+        _, _, bits = O.brute_trace(tris, flat)
+        want = O.bits_to_bool(bits, len(rays))
+        assert want.any() and not want.all()
+        assert np.array_equal(tr.visibility(rays, T.RayTraceOptions.stock_exact()), want)
+        assert np.array_equal(tr.visibility_recheck(rays, T.RayTraceOptions.stock_exact())[0], want)
+        _, _, bits = O.brute_trace(tris, flat, flags=O.SKY_PASS)
+        got = tr.visibility(rays, T.RayTraceOptions(0.0, sky_does_not_block=True))
+        assert np.array_equal(got, O.bits_to_bool(bits, len(rays)))
+        best, dist, _ = O.brute_trace(tris, flat, flags=O.CLOSEST)
+        got = tr.closest(rays)
+        hit = best >= 0
+        assert np.array_equal(got["surface"], np.where(hit, ids[np.maximum(best, 0)], -1))
+        assert np.array_equal(got["fraction"][hit].view(np.uint32), dist[hit].astype(np.float32).view(np.uint32))
