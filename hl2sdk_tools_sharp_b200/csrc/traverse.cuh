@@ -422,6 +422,14 @@ __device__ __forceinline__ void trace_ray_flagged(const DeviceScene &s, const Ra
         hit = walk<ONE, true, STRIDE, false, true>(s.sky, s.tri_id, r, tmin, skip_id, 0, stack, best_t, best_orig, best_meta, &nc);
 }
 
+// How many octants the directions of the warp's `live` lanes lie in.
+__device__ __forceinline__ int octants_of(unsigned live, const RayState &r) {
+    const int oct = r.octant();
+    if (__all_sync(live, oct == __shfl_sync(live, oct, __ffs(live) - 1))) return 1;
+    const unsigned same = __match_any_sync(live, oct);
+    return __popc(__ballot_sync(live, (same & ((1u << (threadIdx.x & 31)) - 1u)) == 0));
+}
+
 __device__ __forceinline__ RayState make_ray(float ox, float oy, float oz, float dx, float dy, float dz) {
     RayState r;
     r.ox = ox;

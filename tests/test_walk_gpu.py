@@ -85,3 +85,30 @@ def test_soup_of_many_triangles_equals_brute_force(n, sky, oracle_mod):
         hit = best >= 0
         assert np.array_equal(got["surface"], np.where(hit, ids[np.maximum(best, 0)], -1))
         assert np.array_equal(got["fraction"][hit].view(np.uint32), dist[hit].astype(np.float32).view(np.uint32))
+
+
+@pytest.mark.parametrize("octants", [1, 4, 5, 8])
+@pytest.mark.parametrize("count", [1, 31, 33, 1000])
+def test_warps_of_few_and_many_octants(octants, count, oracle_mod):
+    """Each warp's rays lie in so many octants (the last warp's in as many as
+    it has rays for): either walk gives the brute force's answers."""
+    O = oracle_mod
+    verts, ids = soup(500, 50, 21)
+    rng = np.random.default_rng([octants, count])
+    o = rng.uniform(-900.0, 900.0, (count, 3)).astype(np.float32)
+    d = np.abs(rng.normal(size=(count, 3))).astype(np.float32) * np.float32(900.0)
+    which = (np.arange(count) % octants + 3) % 8
+    d *= np.where((which[:, None] >> np.arange(3)) & 1, np.float32(-1.0), np.float32(1.0))
+    rays = T.make_rays(o, d, 1.0)
+    tris = O.prepare_triangles(verts, ids)
+    flat = rays.view(np.float32).reshape(-1, 7)
+    with T.CudaRayTracer(T.make_triangles(verts, ids)) as tr:
+        for opts, flags in ((T.RayTraceOptions.stock_exact(), 0),
+                            (T.RayTraceOptions(0.0, sky_does_not_block=True), O.SKY_PASS)):
+            _, _, bits = O.brute_trace(tris, flat, flags=flags)
+            assert np.array_equal(tr.visibility(rays, opts), O.bits_to_bool(bits, len(rays)))
+        best, dist, _ = O.brute_trace(tris, flat, flags=O.CLOSEST)
+        got = tr.closest(rays)
+        hit = best >= 0
+        assert np.array_equal(got["surface"], np.where(hit, ids[np.maximum(best, 0)], -1))
+        assert np.array_equal(got["fraction"][hit].view(np.uint32), dist[hit].astype(np.float32).view(np.uint32))
