@@ -8,7 +8,8 @@
 // n-tiles is the m16k16 A layout); the backward does the same for the
 // activation gradients.  The weight gradients are P^T Q over a tile's rows,
 // both operands read transposed from the row-major tiles in shared memory
-// (ldmatrix.trans).  Master weights and Adam's moments are FP32; the BF16
+// (ldmatrix.trans), and the tiles' products and the bias gradients are FP32
+// sums.  Master weights and Adam's moments are FP32; the BF16
 // operand copies are refreshed after every step.
 
 #include <cuda_bf16.h>
@@ -87,7 +88,9 @@ struct __align__(16) GradSmem {
     uint16_t dz[kTileRows * kSh];     // dz2
     uint16_t dy[kTileRows * kMlpOutPad];
     float b1[kMlpHidden], b2[kMlpHidden], b3[kMlpOutPad];
+    float b3part[kMlpWarps][kMlpOutPad];
 };
+static_assert(kMlpThreads == 2 * kMlpHidden, "a thread per hidden bias");
 static_assert(sizeof(GradSmem) <= 227 * 1024, "one CTA's shared memory");
 
 // acc[16 n-tiles] += A (16 x 16 KT) B, B from wt[n][k] with row stride S.
@@ -168,6 +171,27 @@ __device__ __forceinline__ void store_tile(uint16_t *rows, const uint32_t a[8][4
     }
 }
 
+__device__ __forceinline__ void add4(float to[4], const float from[4]) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) to[q] += from[q];
+}
+
+// Adds a tile's column sums to c: the thread's two columns, 2 (tid & 63) and
+// the next, over its quarter of the rows.
+__device__ __forceinline__ void add_columns(float c[2], const uint16_t *rows, int tid) {
+    constexpr int kRows = kTileRows / (kMlpThreads / 64);
+    const uint16_t *p = rows + (tid >> 6) * kRows * kSh + 2 * (tid & 63);
+    float lo = 0.0f, hi = 0.0f;
+#pragma unroll
+    for (int r = 0; r < kRows; r++) {
+        const uint32_t v = ld32(p + r * kSh);
+        lo += bf_lo(v);
+        hi += bf_hi(v);
+    }
+    c[0] += lo;
+    c[1] += hi;
+}
+
 // Adds a weight gradient's m16n8 tile at row m0, column n0 of grad.
 __device__ __forceinline__ void add_tile(float *grad, int stride, int ncols, int m0, int n0, const float c[4], int g,
                                          int t) {
@@ -184,9 +208,12 @@ __device__ __forceinline__ void add_tile(float *grad, int stride, int ncols, int
 //   forward, h1 and h2 into shared memory; dy = 2 (y - target) / 3n;
 //   dz2 = (dy W3^T) * [h2 > 0], dz1 = (dz2 W2^T) * [h1 > 0];
 // then the products over the tile's rows, split by output rows among the
-// warps and kept in registers from tile to tile: dW3 = h2^T dy, dW2 = h1^T
-// dz2, dW1 = x^T dz1, and the bias gradients as the same products with ones
-// for the left operand.
+// warps: dW3 = h2^T dy, dW2 = h1^T dz2, dW1 = x^T dz1; and the bias gradients,
+// the columns' sums.  What is summed over tiles is summed by FP32 adds, in
+// registers: the tensor cores' accumulators cut off what the sum's last place
+// does not hold, and over the tiles of a CTA that adds up (a million rows,
+// against 64 bits: dW3 off by 2.4e-5 accumulated there, by 2.9e-7 so; 65,536
+// rows 6.9e-7 and 3.9e-7).
 // A minibatch is a few hundred tiles, so what counts is one tile's time and
 // what it sends to memory: nothing but x and the targets in, and one atomic
 // add per parameter and CTA out.  A tile takes 9.5 us, which is the rate of
@@ -218,8 +245,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_gradient(vrad_mlp m, con
     if (tid < kMlpOutPad) s.b3[tid] = tid < kMlpOut ? m.master[kOffB3 + tid] : 0.0f;
     __syncthreads();
 
-    float g2[16][4] = {}, g1[4][4] = {}, g3[4] = {}, gb2[2][4] = {}, gb1[2][4] = {}, gb3[4] = {};
-    const uint32_t ones[4] = {0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u};
+    float g2[16][4] = {}, g1[4][4] = {}, g3[4] = {}, gb2[2] = {}, gb1[2] = {}, gb3[2] = {};
     float loss = 0.0f;
     uint16_t *xs = s.x + 16 * warp * kSx, *h1 = s.h1 + 16 * warp * kSh, *h2 = s.h2 + 16 * warp * kSh,
              *dz = s.dz + 16 * warp * kSh, *dy = s.dy + 16 * warp * kMlpOutPad;
@@ -276,6 +302,8 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_gradient(vrad_mlp m, con
         const uint32_t ady[4] = {pack2(d[0], d[1]), pack2(d[2], d[3]), 0u, 0u};
         *reinterpret_cast<uint32_t *>(dy + g * kMlpOutPad + 2 * t) = ady[0];
         *reinterpret_cast<uint32_t *>(dy + (g + 8) * kMlpOutPad + 2 * t) = ady[1];
+        gb3[0] += bf_lo(ady[0]) + bf_lo(ady[1]);
+        gb3[1] += bf_hi(ady[0]) + bf_hi(ady[1]);
         // dh2 = dy (16 x 8, k padded to 16 with zeros) W3^T.
 #pragma unroll
         for (int j = 0; j < 16; j++) {
@@ -297,29 +325,32 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_gradient(vrad_mlp m, con
         // B (k16 n8) of two n-tiles: (k, n) = (0, 0), (8, 0), (0, 8), (8, 8).
         const int kb = (lane & 7) + 8 * ((lane >> 3) & 1), nb = 8 * (lane >> 4);
 #pragma unroll
+        for (int j = 0; j < 16; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+        float one[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
         for (int kt = 0; kt < 8; kt++) {
             uint32_t p[4], q[4];
             ldsm4_t(p, smem_u32(s.h2 + (16 * kt + ka) * kSh + ma));
             ldsm2_t(q, smem_u32(s.dy + (16 * kt + (lane & 15)) * kMlpOutPad));
-            mma16816(g3, p, q);
-            if (warp == 0) mma16816(gb3, ones, q);
+            mma16816(one, p, q);
             ldsm4_t(p, smem_u32(s.h1 + (16 * kt + ka) * kSh + ma));
 #pragma unroll
             for (int j = 0; j < 8; j++) {
                 ldsm4_t(q, smem_u32(s.dz + (16 * kt + kb) * kSh + 16 * j + nb));
-                mma16816(g2[2 * j], p, q);
-                mma16816(g2[2 * j + 1], p, q + 2);
-                if (j == warp) {
-                    mma16816(gb2[0], ones, q);
-                    mma16816(gb2[1], ones, q + 2);
-                }
+                mma16816(acc[2 * j], p, q);
+                mma16816(acc[2 * j + 1], p, q + 2);
             }
         }
+#pragma unroll
+        for (int j = 0; j < 16; j++) add4(g2[j], acc[j]);
+        add4(g3, one);
+        add_columns(gb2, s.dz, tid);
         __syncthreads();  // h2 is read
         store_tile(h2, a, g, t);  // dz1
         __syncthreads();
-        // dW1: input rows 16 (warp & 1) .., columns 32 (warp >> 1) ..; db1:
-        // half of those columns each.
+        // dW1: input rows 16 (warp & 1) .., columns 32 (warp >> 1) ...
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
 #pragma unroll
         for (int kt = 0; kt < 8; kt++) {
             uint32_t p[4], q[4];
@@ -327,14 +358,13 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_gradient(vrad_mlp m, con
 #pragma unroll
             for (int j = 0; j < 2; j++) {
                 ldsm4_t(q, smem_u32(s.h2 + (16 * kt + kb) * kSh + 32 * (warp >> 1) + 16 * j + nb));
-                mma16816(g1[2 * j], p, q);
-                mma16816(g1[2 * j + 1], p, q + 2);
-                if (j == (warp & 1)) {
-                    mma16816(gb1[0], ones, q);
-                    mma16816(gb1[1], ones, q + 2);
-                }
+                mma16816(acc[2 * j], p, q);
+                mma16816(acc[2 * j + 1], p, q + 2);
             }
         }
+#pragma unroll
+        for (int j = 0; j < 4; j++) add4(g1[j], acc[j]);
+        add_columns(gb1, s.h2, tid);
         __syncthreads();  // x and dz1 are read
     }
     // The CTA's sums.
@@ -344,17 +374,23 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_gradient(vrad_mlp m, con
     for (int j = 0; j < 4; j++)
         add_tile(m.grad, kMlpHidden, kMlpHidden, 16 * (warp & 1), 32 * (warp >> 1) + 8 * j, g1[j], g, t);
     add_tile(m.grad + kOffW3, kMlpOut, kMlpOut, 16 * warp, 0, g3, g, t);
-    if (g == 0) {  // every row of a product with ones is the column sums
+    // The bias gradients' parts first within the CTA: row quarters, warps.
+    float(*part)[2 * kMlpHidden + 2] = reinterpret_cast<float(*)[2 * kMlpHidden + 2]>(s.dz);
 #pragma unroll
-        for (int j = 0; j < 2; j++)
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                atomicAdd(&m.grad[kOffB2 + 16 * warp + 8 * j + 2 * t + q], gb2[j][q]);
-                atomicAdd(&m.grad[kOffB1 + 32 * (warp >> 1) + 16 * (warp & 1) + 8 * j + 2 * t + q], gb1[j][q]);
-            }
-        if (warp == 0)
-            for (int q = 0; q < 2; q++)
-                if (2 * t + q < kMlpOut) atomicAdd(&m.grad[kOffB3 + 2 * t + q], gb3[q]);
+    for (int q = 0; q < 2; q++) {
+        const int col = 2 * (tid & 63) + q;
+        part[tid >> 6][col] = gb1[q];
+        part[tid >> 6][kMlpHidden + col] = gb2[q];
+        for (int o = 16; o > 2; o >>= 1) gb3[q] += __shfl_xor_sync(0xffffffffu, gb3[q], o);  // the rows g
+        if (g == 0) s.b3part[warp][2 * t + q] = gb3[q];
+    }
+    __syncthreads();
+    const float b = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
+    atomicAdd(&m.grad[tid < kMlpHidden ? kOffB1 + tid : kOffB2 + tid - kMlpHidden], b);
+    if (tid < kMlpOut) {
+        float b3 = 0.0f;
+        for (int w = 0; w < kMlpWarps; w++) b3 += s.b3part[w][tid];
+        atomicAdd(&m.grad[kOffB3 + tid], b3);
     }
     for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
     if (lane == 0) atomicAdd(m.loss, loss * inv);

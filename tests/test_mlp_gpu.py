@@ -143,3 +143,35 @@ def test_forward_at_tile_edges(net, rows):
     keep = torch.ones(rows, dtype=torch.bool, device="cuda")
     keep[rows // 2] = keep[rows - 1] = False
     assert torch.equal(y2[keep], y[keep])
+
+
+def test_gradient_of_a_million_rows_is_summed_in_fp32(net):
+    """Against 64-bit products of the same BF16 activations and gradients.
+    A tile's 128 rows may lose an ulp (2^-23) a product step, eight steps;
+    the tiles' sums are FP32 adds, 55 a CTA and an atomic add per CTA, whose
+    roundings are as often up as down (2^-24 sqrt(203)); and an activation
+    that FP32 and 64 bits round to different BF16 values moves a sum by some
+    1e-6 at most.  1e-6 + 1e-6 + 2e-6 together."""
+    n, torch = net
+    rows = 1 << 20
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    x = torch.rand((rows, LN.INPUTS), device="cuda", generator=g).to(torch.bfloat16).contiguous()
+    target = (6.0 * x[:, :LN.OUTPUTS].float() + torch.rand((rows, LN.OUTPUTS), device="cuda", generator=g)).contiguous()
+
+    def bf(v):
+        return v.float().to(torch.bfloat16).double()
+
+    p = {k: torch.from_numpy(np.asarray(v, np.float32)).cuda() for k, v in LN.split(n.params()).items()}
+    p = {k: bf(v) if k[0] == "w" else v.double() for k, v in p.items()}
+    xd = x.double()
+    h1 = bf(torch.relu(xd @ p["w1"] + p["b1"]))
+    h2 = bf(torch.relu(h1 @ p["w2"] + p["b2"]))
+    e = h2 @ p["w3"] + p["b3"] - target.double()
+    dy = bf(2.0 * e / e.numel())
+    dz2 = bf((dy @ p["w3"].T) * (h2 > 0))
+    dz1 = bf((dz2 @ p["w2"].T) * (h1 > 0))
+    want = {"w1": xd.T @ dz1, "b1": dz1.sum(0), "w2": h1.T @ dz2, "b2": dz2.sum(0), "w3": h2.T @ dy, "b3": dy.sum(0)}
+    got, _ = n.gradient(x, target)
+    off = {k: _rel(np.asarray(v, np.float64).ravel(), want[k].cpu().numpy().ravel()) for k, v in LN.split(got).items()}
+    assert all(v < 4e-6 for v in off.values()), off
