@@ -463,23 +463,21 @@ cudaError_t mlp_forward(const vrad_mlp &m, const uint16_t *x, int64_t n, float *
 
 namespace {
 
-// The pinned blocks that carry a network's gradient to the host: pinning one
-// takes 1 to 2.5 ms, several times what creating a network takes otherwise,
-// so a destroyed network's block serves the next one.  At most kSpareBlocks
-// (85 KB each) are kept.
-constexpr size_t kSpareBlocks = 8;
+// The pinned blocks that carry a gradient to the host.  A call of
+// vrad_mlp_gradient_device takes one and gives it back: pinning one takes 1
+// to 2.5 ms where the driver maps new memory for it, several times what
+// creating a network takes, and a network that is only run forward or trained
+// needs none.  At most kSpareBlocks (85 KB each) are kept.
+constexpr int kSpareBlocks = 8;
 std::mutex spare_mu;
-std::vector<float *> &spare_blocks() {
-    static std::vector<float *> *v = new std::vector<float *>;  // never destroyed: used from static destructors
-    return *v;
-}
+float *spare_blocks[kSpareBlocks];
+int nspare = 0;
 
 cudaError_t take_block(float **out) {
     {
         std::lock_guard<std::mutex> g(spare_mu);
-        if (!spare_blocks().empty()) {
-            *out = spare_blocks().back();
-            spare_blocks().pop_back();
+        if (nspare > 0) {
+            *out = spare_blocks[--nspare];
             return cudaSuccess;
         }
     }
@@ -490,8 +488,8 @@ void give_block(float *p) {
     if (!p) return;
     {
         std::lock_guard<std::mutex> g(spare_mu);
-        if (spare_blocks().size() < kSpareBlocks) {
-            spare_blocks().push_back(p);
+        if (nspare < kSpareBlocks) {
+            spare_blocks[nspare++] = p;
             return;
         }
     }
@@ -502,7 +500,6 @@ void release_mlp(vrad_mlp *m) {
     for (void *p : {(void *)m->master, (void *)m->adam_m, (void *)m->adam_v, (void *)m->grad, (void *)m->w1t,
                     (void *)m->w2t, (void *)m->w3t, (void *)m->w2, (void *)m->w3, (void *)m->flags})
         cudaFree(p);
-    give_block(m->host);
     delete m;
 }
 
@@ -524,7 +521,6 @@ extern "C" int32_t vrad_mlp_create(vrad_ctx *ctx, uint64_t seed, vrad_mlp **out)
         if (e == cudaSuccess) e = cudaMalloc(p, sizeof(float) * (kMlpParams + 1));
     for (uint16_t **p : {&m->w1t, &m->w2t, &m->w3t, &m->w2, &m->w3})
         if (e == cudaSuccess) e = cudaMalloc(p, sizeof(uint16_t) * kW2);
-    if (e == cudaSuccess) e = take_block(&m->host);
     m->loss = m->grad ? m->grad + kMlpParams : nullptr;
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, ctx->device);
     if (e == cudaSuccess) e = cudaMalloc(&m->flags, sizeof(uint32_t));
@@ -589,11 +585,16 @@ extern "C" int32_t vrad_mlp_gradient_device(vrad_mlp *m, const uint16_t *x, cons
     cudaStream_t s = (cudaStream_t)stream;
     if (e == cudaSuccess) e = vrad::gradient(*m, x, target, n, s);
     // Gradient and loss in one copy, through pinned memory.
+    float *host = nullptr;
+    if (e == cudaSuccess) e = take_block(&host);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(m->host, m->grad, sizeof(float) * (vrad::kMlpParams + 1), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess && grad) std::memcpy(grad, m->host, sizeof(float) * vrad::kMlpParams);
-    if (e == cudaSuccess && loss) *loss = m->host[vrad::kMlpParams];
+        e = cudaMemcpyAsync(host, m->grad, sizeof(float) * (vrad::kMlpParams + 1), cudaMemcpyDeviceToHost, s);
+    // No copy may be in flight into a block that goes back.
+    const cudaError_t done = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = done;
+    if (e == cudaSuccess && grad) std::memcpy(grad, host, sizeof(float) * vrad::kMlpParams);
+    if (e == cudaSuccess && loss) *loss = host[vrad::kMlpParams];
+    give_block(host);
     if (e != cudaSuccess) return vrad_cuda_fail(nullptr, e, "network gradient");
     return VRAD_OK;
 }

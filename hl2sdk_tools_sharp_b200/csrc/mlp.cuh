@@ -40,7 +40,6 @@ struct vrad_mlp {
     float *master = nullptr, *adam_m = nullptr, *adam_v = nullptr, *grad = nullptr;
     uint16_t *w1t = nullptr, *w2t = nullptr, *w3t = nullptr, *w2 = nullptr, *w3 = nullptr;
     float *loss = nullptr;        // device scalar of the last step: grad[kMlpParams]
-    float *host = nullptr;        // pinned: the gradient and loss on their way to a caller
     uint32_t *flags = nullptr;    // device word: bit 0, a forward's MMA wait ran out (sticky)
     int sms = 1;
     int64_t step = 0;

@@ -175,3 +175,32 @@ def test_gradient_of_a_million_rows_is_summed_in_fp32(net):
     got, _ = n.gradient(x, target)
     off = {k: _rel(np.asarray(v, np.float64).ravel(), want[k].cpu().numpy().ravel()) for k, v in LN.split(got).items()}
     assert all(v < 4e-6 for v in off.values()), off
+
+
+def test_gradients_from_several_threads(net):
+    """More networks than pinned blocks are kept, their gradients taken at
+    once from a thread each, on a stream each: every caller gets its own."""
+    import threading
+    n, torch = net
+    tr = T.CudaRayTracer(T.make_triangles(np.zeros((1, 9), np.float32), np.zeros(1, np.int32)))
+    nets = [LN.Network(tr, seed=s) for s in range(12)]
+    data = [_data(torch, 300 + 7 * k, k) for k in range(len(nets))]
+    torch.cuda.synchronize()
+    want = [m.gradient(d[0], d[2]) for m, d in zip(nets, data)]
+    got = [None] * len(nets)
+
+    def work(k):
+        stream = torch.cuda.Stream()
+        for _ in range(20):
+            got[k] = nets[k].gradient(data[k][0], data[k][2], stream=stream.cuda_stream)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(nets))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for (g, loss), (w, wl) in zip(got, want):
+        assert _rel(g, w) < 1e-5 and abs(loss - wl) < 1e-5 * wl
+    for m in nets:
+        m.close()
+    tr.close()
