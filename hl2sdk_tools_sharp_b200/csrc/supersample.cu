@@ -379,10 +379,16 @@ cudaError_t build_supersample(SupersampleBuffers &ss, const std::vector<vrad_fac
     if (e == cudaSuccess) e = dev_alloc(&ss.rows, sizeof(int32_t) * groups);
     if (e == cudaSuccess) e = dev_alloc(&ss.row_out, sizeof(float4) * 20 * S1);
     if (e == cudaSuccess) e = dev_alloc(&ss.row_bits, sizeof(int32_t) * 5 * S1);
-    if (max_rays > 0 && max_rays <= kSplitRays) {
-        if (e == cudaSuccess)
-            e = dev_alloc(&ss.words, sizeof(uint32_t) * kSplitWarps * (size_t)max_rays + 3 * sizeof(unsigned long long));
-        ss.max_rays = max_rays;
+    if (e == cudaSuccess && max_rays > 0 && max_rays <= kSplitRays) {
+        // Only makes small launches faster: where there is no room for it,
+        // none is split.
+        e = dev_alloc(&ss.words, sizeof(uint32_t) * kSplitWarps * (size_t)max_rays + 3 * sizeof(unsigned long long));
+        if (e == cudaSuccess) {
+            ss.max_rays = max_rays;
+        } else if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();  // clear the recorded error
+            e = cudaSuccess;
+        }
     }
     if (e == cudaSuccess && ss.h_counts_cap < 1 + (size_t)nclusters) {
         ss.free_pinned();

@@ -47,7 +47,7 @@ struct SupersampleBuffers {
     float4 *row_out = nullptr;
     int32_t *row_bits = nullptr;
     uint32_t *words = nullptr;      // kSplitWarps x the world's max_rays words of who was blocked, then 3 scratch counters
-    int32_t max_rays = 0;           // what words has room for; 0: none (too many rays a point)
+    int32_t max_rays = 0;           // what words has room for; 0: none (too many rays a point, or no memory)
     int32_t *h_counts = nullptr;    // pinned, kept across uploads (h_counts_cap entries)
     size_t h_counts_cap = 0;
     int64_t nsamples = 0;
