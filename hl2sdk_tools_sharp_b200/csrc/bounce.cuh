@@ -120,7 +120,7 @@ struct BounceBuffers {
     // contiguous 256 B row.  Keys: window << kCountBits | kCountMask - count.
     uint32_t *sell_key = nullptr, *sell_sorted = nullptr;  // R: before and after the sort
     int32_t *sell_idx = nullptr, *sell_order = nullptr;    // R: the receivers alike
-    int32_t sell_window = 0;  // a multiple of 32
+    int32_t sell_window = 0;  // a multiple of 32; all receivers where memory is short
     int64_t sell_cap = 0;     // entries sell has room for
     int64_t *sell_off = nullptr;   // slices + 1
     int2 *sell = nullptr;          // at most T + 32 * (each window's largest count) entries

@@ -681,9 +681,18 @@ extern "C" int32_t vrad_bounce_upload(vrad_ctx *ctx, const vrad_bounce_desc *d) 
     if (e == cudaSuccess) e = dev_alloc(&b.tr, sizeof(int2) * (size_t)(ncand ? ncand : 1));
     // The slices hold the transfers and at most, for each window, 32 times
     // its largest count of padding; an installed set may have longer lists
-    // than candidates, and then takes one window (vrad_transfer_install).
-    b.sell_cap = ncand + std::max<int64_t>((int64_t)pad, 32 * std::min<int64_t>(kMaxTransfersPerReceiver, ncand));
+    // than candidates, and then takes one window (vrad_transfer_install).  The
+    // windows only make the gather faster: where there is no room for their
+    // padding (with a million receivers some hundred MB), there is one.
+    const int64_t one = 32 * std::min<int64_t>(kMaxTransfersPerReceiver, ncand);
+    b.sell_cap = ncand + std::max<int64_t>((int64_t)pad, one);
     if (e == cudaSuccess) e = dev_alloc(&b.sell, sizeof(int2) * (size_t)(b.sell_cap ? b.sell_cap : 1));
+    if (e == cudaErrorMemoryAllocation && !b.sell && b.sell_cap > ncand + one && b.tr) {
+        cudaGetLastError();  // clear the recorded error
+        b.sell_cap = ncand + one;
+        b.sell_window = 32 * nslices;
+        e = dev_alloc(&b.sell, sizeof(int2) * (size_t)b.sell_cap);
+    }
     if (e == cudaSuccess) e = cudaMemcpyAsync(&overflow, walk_flag, sizeof overflow, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = vrad::wait_stream(s);
     if (e != cudaSuccess) {
