@@ -278,11 +278,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_forward_tc(vrad_mlp m, co
     const bool x16 = ((uintptr_t)x & 15) == 0;
     uint32_t parity = 0;
 
-    // Waits for the MMAs just committed.  A thread that gave up says so, and
-    // the group agrees to leave at its next barrier (synced): until then its
-    // loads of an unfinished accumulator give values that nobody keeps.
+    // Waits for the MMAs just committed.  A thread that gave up records it for
+    // the host, whoever else did not, and for the group, which agrees to leave
+    // at its next barrier (synced): until then its loads of an unfinished
+    // accumulator give values that nobody keeps, or after the last wait
+    // outputs that the record disowns.
     auto wait_mma = [&] {
-        if (!wait_bar(bar, parity)) atomicOr(&s.abort[group], 1);
+        if (!wait_bar(bar, parity)) {
+            atomicOr(m.flags, kFlagTimeout);
+            atomicOr(&s.abort[group], 1);
+        }
         parity ^= 1;
         __syncwarp();
         fence_after();
@@ -387,15 +392,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_forward_tc(vrad_mlp m, co
             load_x(tile + step);
         }
     }
-    // After a timeout: record it, and leave with no MMA in flight (the last
-    // commit's phase waited for once more, bounded again), then free the
-    // TMEM.  A timeout of the last wait shows here too.
-    if (!ok || *(volatile int *)&s.abort[group]) {
-        if (gt == 0) {
-            atomicOr(m.flags, kFlagTimeout);
-            wait_bar(bar, parity ^ 1);
-        }
-    }
+    // After a timeout: leave with no MMA in flight (the last commit's phase
+    // waited for once more, bounded again), then free the TMEM.  The first
+    // thread sees its own timeout of the last wait; where only others gave up
+    // there, its MMAs are done.
+    if (gt == 0 && (!ok || *(volatile int *)&s.abort[group])) wait_bar(bar, parity ^ 1);
     fence_before();
     __syncthreads();
     fence_after();
