@@ -26,7 +26,6 @@
 
 #include <algorithm>
 #include <atomic>
-#include <cfloat>
 #include <climits>
 #include <cstring>
 #include <vector>
@@ -360,9 +359,6 @@ __global__ void __launch_bounds__(96) k_median(FinalView v, const float4 *__rest
         const uint32_t y = x | (1u << bit);
         if (below(y) <= rank) x = y;
     }
-    // Infinite: the sort of kMedianMax values, padded with the largest
-    // float, has the padding before the infinities.
-    if (x == 0x7F800000u && rank - below(x) < kMedianMax - count) x = __float_as_uint(FLT_MAX);
     if (lane == 0) mid[c] = count ? __uint_as_float(x) : 0.0f;
     __syncthreads();
     // Before lightofs, in reverse style order.

@@ -2,6 +2,8 @@
 LIGHTING lump's bytes against the oracle's restatement of FinalLightFace
 over the oracle's own direct gather.  The bar is byte-identical: every
 RGBE word of every luxel and every per-face median."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -53,3 +55,30 @@ def test_light_pass_device_matches_host():
         st.light_pass_device(d)
         torch.cuda.synchronize()
     assert np.array_equal(d.cpu().numpy(), lump)
+
+
+def test_a_face_whose_median_is_infinite(oracle_mod):
+    """Light that overflows FP32: the median of a face most of whose luxels
+    are infinite is infinite.  Where a channel is infinite its byte is not
+    compared (an infinity's conversion to a whole number is undefined in the
+    oracle's language), the shared exponent is, and so is every other word."""
+    w = rg.generate(rg.config_3x3(seed=2))
+    inp = L.prepare(w)
+    lights = inp.lights.copy()
+    point = np.flatnonzero(lights["type"] == L.EMIT_POINT)[:2]
+    lights["intensity"][point] = np.float32(3e38)
+    lights["constant_attn"][point] = np.float32(0.25)
+    lights["linear_attn"][point] = lights["quadratic_attn"][point] = np.float32(0.0)
+    inp = dataclasses.replace(inp, lights=lights)
+    with L.LightingStage(w, inp) as st:
+        lump, lightofs, _ = st.light_pass()
+        samples, _ = st.direct()
+    light = np.concatenate([samples["lighting"], samples["direct_sun_amount"][:, None]], 1)
+    want, want_ofs = oracle_mod.final(inp.faces, inp.verts, inp.samples, inp.face_first, light)
+    assert np.array_equal(lightofs, want_ofs)
+    got, want = lump.reshape(-1, 4), want.reshape(-1, 4)
+    assert np.array_equal(got[:, 3], want[:, 3])
+    infinite = want[:, 3] == 255 - (7 + 127)
+    medians = lightofs // 4 - 1
+    assert infinite[medians].any() and not infinite[medians].all() and infinite.sum() > infinite[medians].sum()
+    assert np.array_equal(got[~infinite], want[~infinite])
