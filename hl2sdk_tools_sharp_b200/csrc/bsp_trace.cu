@@ -24,11 +24,11 @@
 namespace vrad {
 
 void BspBuffers::release() {
-    for (void *p : {(void *)nodes, (void *)surfaces, (void *)node_faces, (void *)leaf_faces, (void *)leaf_run,
+    for (void *p : {(void *)nodes, (void *)node_faces, (void *)leaf_faces, (void *)leaf_run,
                     (void *)node_surf, (void *)leaf_surf,
                     (void *)sky_points, (void *)sky_run})
         dev_free(p);
-    nodes = surfaces = sky_points = node_surf = leaf_surf = nullptr;
+    nodes = sky_points = node_surf = leaf_surf = nullptr;
     node_faces = leaf_faces = nullptr;
     leaf_run = sky_run = nullptr;
     nnodes = nsurfaces = nleaves = 0;
@@ -136,7 +136,6 @@ extern "C" int32_t vrad_bsp_upload(vrad_ctx *ctx, const vrad_bsp_geometry *b) {
         return r;
     };
     if (e == cudaSuccess) e = up(&bb.nodes, b->nodes, sizeof(float) * 8 * (size_t)b->nnodes);
-    if (e == cudaSuccess) e = up(&bb.surfaces, b->surfaces, sizeof(float) * 16 * (size_t)b->nsurfaces);
     if (e == cudaSuccess) e = up(&bb.node_faces, b->node_faces, sizeof(int32_t) * (size_t)b->nnode_faces);
     if (e == cudaSuccess) e = up(&bb.leaf_faces, b->leaf_faces, sizeof(int32_t) * (size_t)b->nleaf_faces);
     if (e == cudaSuccess) e = up(&bb.node_surf, node_surf.data(), sizeof(float4) * 4 * (size_t)b->nnode_faces);
@@ -152,7 +151,7 @@ extern "C" int32_t vrad_bsp_upload(vrad_ctx *ctx, const vrad_bsp_geometry *b) {
     bb.nnodes = b->nnodes;
     bb.nsurfaces = b->nsurfaces;
     bb.nleaves = b->nleaves;
-    bb.view = vrad::DeviceBsp{bb.nodes, bb.surfaces, bb.node_faces, bb.leaf_faces, bb.node_surf, bb.leaf_surf, bb.leaf_run, b->nleaves,
+    bb.view = vrad::DeviceBsp{bb.nodes, bb.node_faces, bb.leaf_faces, bb.node_surf, bb.leaf_surf, bb.leaf_run, b->nleaves,
                               bb.sky_points, bb.sky_run};
     bb.ready = true;
     return VRAD_OK;

@@ -5,11 +5,11 @@
 //   nodes[n]       2 x float4: (plane normal, dist), (child0, child1, first
 //                  node face, packed) -- the last four as int bits; packed =
 //                  lit face count | sky face count << 15 | axis << 30
-//   surfaces[f]    4 x float4: (plane normal, dist), (lightmap s, offset),
-//                  (lightmap t, offset), (mins s, t, sizes s, t)
 //   node_faces     each node's candidate faces, lit then sky
 //   leaf_faces     each leaf's candidate faces; leaf_run[l] = (start, count)
-//   node_surf[q], leaf_surf[q]  surfaces[] of node_faces[q], leaf_faces[q]:
+//   node_surf[q], leaf_surf[q]  the surfaces of node_faces[q], leaf_faces[q],
+//                  4 x float4 each: (plane normal, dist), (lightmap s,
+//                  offset), (lightmap t, offset), (mins s, t, sizes s, t);
 //                  the walk streams a list's records without an index load
 //                  before each
 //   sky_points     the sky faces' windings (float4); sky_run[f] = (start, count)
@@ -23,7 +23,6 @@ namespace vrad {
 
 struct DeviceBsp {
     const float4 *nodes;
-    const float4 *surfaces;
     const int32_t *node_faces;
     const int32_t *leaf_faces;
     const float4 *node_surf;
@@ -36,7 +35,6 @@ struct DeviceBsp {
 
 struct BspBuffers {
     float4 *nodes = nullptr;
-    float4 *surfaces = nullptr;
     int32_t *node_faces = nullptr;
     int32_t *leaf_faces = nullptr;
     float4 *node_surf = nullptr;
