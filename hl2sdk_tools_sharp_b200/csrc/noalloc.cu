@@ -9,11 +9,11 @@
 // cudaMalloc, cudaFree or other allocating call.
 //
 // The array is a file-scope __device__ variable: every GPU that loads the
-// library holds it (sizeof(vrad_ray) x VRAD_STATIC_MAX_RAYS for the rays,
-// 8 KiB for the bits and 256 B for a status word: 1,843,456 bytes) until
-// the process exits.  Host code cannot use its name as a device address;
-// its address on each device is looked up by cudaGetSymbolAddress, with
-// that device current, and that pointer is what the kernel is given.
+// library holds it (sizeof(vrad_ray) x VRAD_STATIC_MAX_RAYS for the rays and
+// 8 KiB for the bits: 1,843,200 bytes) until the process exits.  Host code
+// cannot use its name as a device address; its address on each device is
+// looked up by cudaGetSymbolAddress, with that device current, and that
+// pointer is what the kernel is given.
 //
 // With lazy module loading (the CUDA 12 default) the array and the trace
 // kernels' code are placed on a device only when first used, and placing
@@ -34,11 +34,11 @@ namespace {
 constexpr int64_t kMaxRays = VRAD_STATIC_MAX_RAYS;
 constexpr size_t kRayBytes = sizeof(vrad_ray) * (size_t)kMaxRays;
 constexpr size_t kBitBytes = 8 * (size_t)((kMaxRays + 63) / 64);
-// Layout: [rays | hit bits | 256 spare bytes].
-constexpr size_t kScratchBytes = kRayBytes + kBitBytes + 256;
+// Layout: [rays | hit bits].
+constexpr size_t kScratchBytes = kRayBytes + kBitBytes;
 
 static_assert(kRayBytes % 256 == 0, "bits must start 256-byte aligned");
-static_assert(kScratchBytes == 1843456, "the size the header and the comment above state");
+static_assert(kScratchBytes == 1843200, "the size the header and the comment above state");
 
 __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 

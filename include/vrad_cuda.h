@@ -729,10 +729,10 @@ int32_t vrad_bounce_features_device(vrad_ctx *ctx, uint16_t *x, float *target, i
  * that freeing device memory can bring.  No counterpart in the
  * reference.  Same arguments, answers and errors as vrad_trace_visibility,
  * but rays and bits are staged through one fixed array inside the library
- * (1,843,456 bytes: sizeof(vrad_ray) x VRAD_STATIC_MAX_RAYS for the rays,
- * 8 KiB for the bits, 256 B for a status word), held on every GPU that
- * loads the library until the process exits, instead of buffers grown with
- * cudaMalloc, so the call makes no allocation.
+ * (1,843,200 bytes: sizeof(vrad_ray) x VRAD_STATIC_MAX_RAYS for the rays,
+ * 8 KiB for the bits), held on every GPU that loads the library until the
+ * process exits, instead of buffers grown with cudaMalloc, so the call makes
+ * no allocation.
  * n above VRAD_STATIC_MAX_RAYS is refused with VRAD_ERR_ARG.
  *
  * vrad_create places the array and the trace kernels on its device and
