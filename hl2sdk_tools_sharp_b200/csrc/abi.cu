@@ -125,6 +125,8 @@ int32_t upload(vrad_ctx *ctx, const vrad_triangle *tris, const vrad_kd_triangle 
             if (e == cudaErrorInvalidValue && prep)
                 return fail(ctx, VRAD_ERR_ARG,
                             "a supplied triangle's projection axes are not the successors of its drop axis");
+            if (e == cudaErrorNotSupported)
+                return fail(ctx, VRAD_ERR_UNSUPPORTED, "the scene's BVH is deeper than %d", vrad::kStackDepth);
             return cuda_fail(ctx, e, "scene build");
         }
     }

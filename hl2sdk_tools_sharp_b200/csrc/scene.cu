@@ -344,7 +344,7 @@ cudaError_t build_bvh(BvhBuffers &sb, const vrad_triangle *h_tris,
             build_sah(box.data(), n, tree);
         }
         if (tree.depth > kStackDepth) {
-            err = cudaErrorInvalidValue;  // the builder's depth guard did not hold
+            err = cudaErrorNotSupported;  // the builder's depth guard did not hold
             goto fail;
         }
         parent.assign((size_t)tree.inner, -1);

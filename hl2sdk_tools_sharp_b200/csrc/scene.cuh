@@ -48,6 +48,8 @@ struct SceneBuildReport {
 // intersection form); h_orig gives each triangle's original index in the
 // whole scene; copies of the nodes: 8 or 1.  Synchronises `stream` before
 // returning.  report is accumulated into (counts added, bounds merged).
+// cudaErrorInvalidValue: a supplied form's axes; cudaErrorNotSupported: a tree
+// deeper than kStackDepth.
 cudaError_t build_bvh(BvhBuffers &bb, const vrad_triangle *h_tris,
                       const vrad_kd_triangle *h_prepared, const int32_t *h_orig, int n, int copies,
                       cudaStream_t stream, SceneBuildReport *report);
