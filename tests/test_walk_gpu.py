@@ -112,3 +112,76 @@ def test_warps_of_few_and_many_octants(octants, count, oracle_mod):
         hit = best >= 0
         assert np.array_equal(got["surface"], np.where(hit, ids[np.maximum(best, 0)], -1))
         assert np.array_equal(got["fraction"][hit].view(np.uint32), dist[hit].astype(np.float32).view(np.uint32))
+
+
+def skewed(n, base=0.01, factor=1.4):
+    """Triangles in a row, each larger than the one before: a tree that takes
+    the large ones off one after the other."""
+    k = np.arange(n)
+    size = base * factor ** k
+    corner = np.stack([4.0 * size, 0.3 * size, -0.2 * size], 1)[:, None, :]
+    shape = np.array([[0.0, 0.0, 0.0], [1.0, 0.2, 0.1], [0.1, 1.0, -0.3]])[None]
+    return (corner + shape * size[:, None, None]).astype(np.float32).reshape(n, 9)
+
+
+@pytest.mark.parametrize("n", [20, 66])
+def test_skewed_scene_equals_brute_force(n, oracle_mod):
+    """A tree deeper than a balanced one: the stacks hold its depth."""
+    O = oracle_mod
+    verts = skewed(n)
+    ids = np.full(n, 0x02000000, np.int32)
+    ids[::7] = T.TRACE_ID_SKY
+    rng = np.random.default_rng(n)
+    at = verts.reshape(n, 3, 3)[rng.integers(0, n, 4096)].mean(1)
+    o = (at + rng.normal(size=at.shape) * np.linalg.norm(at, axis=1, keepdims=True)).astype(np.float32)
+    rays = T.make_rays(o, ((at - o) * rng.uniform(0.5, 3.0, (4096, 1))).astype(np.float32), 1.0)
+    tris = O.prepare_triangles(verts, ids)
+    flat = rays.view(np.float32).reshape(-1, 7)
+    with T.CudaRayTracer(T.make_triangles(verts, ids)) as tr:
+        assert tr.scene_info().bvh_depth > np.ceil(np.log2(n))
+        for opts, flags in ((T.RayTraceOptions.stock_exact(), 0),
+                            (T.RayTraceOptions(0.0, sky_does_not_block=True), O.SKY_PASS)):
+            _, _, bits = O.brute_trace(tris, flat, flags=flags)
+            assert np.array_equal(tr.visibility(rays, opts), O.bits_to_bool(bits, len(rays)))
+        best, dist, _ = O.brute_trace(tris, flat, flags=O.CLOSEST)
+        got = tr.closest(rays)
+        hit = best >= 0
+        assert hit.any() and np.array_equal(got["surface"], np.where(hit, ids[np.maximum(best, 0)], -1))
+        assert np.array_equal(got["fraction"][hit].view(np.uint32), dist[hit].astype(np.float32).view(np.uint32))
+
+
+@pytest.mark.parametrize("casters", ["skewed", "one opaque", "sky alone"])
+def test_walks_that_start_at_the_origins_leaf(casters):
+    """The light gather's segments and the transfer rays start their walk near
+    their origin and climb; with 20,000 triangles out of their reach added they
+    start at the root of one copy of the nodes.  Same lumps: over a map with a
+    skewed row of triangles in it, over one opaque triangle, over no opaque
+    triangle at all."""
+    import dataclasses
+    from hl2sdk_tools_sharp_b200 import lighting as L, roomgrid as rg
+    w = rg.generate(dataclasses.replace(rg.config_3x3(seed=2), side=2, lights=4, sky_ambient=True))
+    off, lst = L.pvs_lists(w)
+    verts, ids = np.asarray(w.tri_verts, np.float32).reshape(-1, 9), np.asarray(w.tri_ids)
+    sky = (ids & T.TRACE_ID_SKY) != 0
+    assert sky.any()
+    row = skewed(24, 0.05).reshape(-1, 3, 3) + verts.reshape(-1, 3)[~np.repeat(sky, 3)].mean(0)
+    row = row.astype(np.float32).reshape(-1, 9)
+    if casters == "skewed":
+        verts, ids = np.concatenate([verts, row]), np.concatenate([ids, np.full(len(row), ids[~sky][0], ids.dtype)])
+    elif casters == "one opaque":
+        verts, ids = np.concatenate([verts[sky], row[-1:]]), np.concatenate([ids[sky], ids[~sky][:1]])
+    else:
+        verts, ids = verts[sky], ids[sky]
+    rng = np.random.default_rng(8)
+    far = rng.uniform(-8000.0, 8000.0, (20000, 1, 3)) + rng.uniform(-50.0, 50.0, (20000, 3, 3))
+    far[:, :, 2] -= 300000.0
+    far = far.reshape(-1, 9).astype(np.float32)
+    lumps = []
+    with L.LightingStage(w) as st:
+        st.upload_bounce(L.face_reflectivity(w), off, lst, threshold=1.0)
+        for add in (0, len(far)):
+            both = np.concatenate([verts, far[:add]])
+            st.tracer.upload_scene(T.make_triangles(both, np.concatenate([ids, np.full(add, T.TRACE_ID_SKY, ids.dtype)])))
+            lump, _, _ = st.light_pass()
+            lumps.append(lump)
+    assert lumps[0].any() and np.array_equal(lumps[0], lumps[1])
