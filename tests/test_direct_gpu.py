@@ -146,6 +146,20 @@ def test_resampling_of_few_and_many_points(oracle_mod, side, scale, lights, sky,
     assert not diff.any(), f"{int(diff.sum())} of {len(diff)} samples differ"
 
 
+def test_resampling_of_points_with_more_segments_than_are_split(oracle_mod):
+    """A point that traces more than 1,024 segments: its launches stay whole,
+    however few points they have."""
+    w = rg.generate(rg.Config(side=1, seed=6, luxel_scale=40.0, pillars=(0, 3), lights=1, spot_fraction=0.5,
+                              sky_ambient=True, sun_spread=2.0, sun_samples=1100))
+    inp = L.prepare(w)
+    with L.LightingStage(w, inp) as st:
+        got, stats = st.direct()
+    g = np.concatenate([got["lighting"], got["direct_sun_amount"][:, None]], 1)
+    assert stats.supersampled > 0
+    diff = (bits(g) != bits(oracle_direct(oracle_mod, w, inp))).any(1)
+    assert not diff.any(), f"{int(diff.sum())} of {len(diff)} samples differ"
+
+
 @pytest.mark.parametrize("change", ["area", "coord", "mins", "position", "swap"])
 def test_supersampling_refuses_samples_not_the_builders(change):
     # Supersampling needs each partial sample's cell winding, which the
