@@ -68,12 +68,12 @@ constexpr int kRayBlock = 128;
 constexpr int kProjectBlock = 32 * kAmbientSides * 3;
 constexpr int64_t kChunkSamples = 32768;  // at most 63.7 MB of ray colours
 // A group's points are close together within this many units along each
-// axis: 100 k samples 3.90 ms at 256, 3.57 at 512, 3.38 at 1024, 5.61 when
-// no group is.
+// axis: 100 k samples of dm_lockdown 3.90 ms at 256, 3.57 at 512, 3.38 at
+// 1024, the largest that was tried, 5.61 when no group is.
 constexpr float kCompact = 1024.0f;
 // At most this many samples take four rays a warp: 100 samples 111 us
 // against 152 with 32, 300 samples 146 against 160, 768 samples 228 against
-// 184.
+// 184.  The two cross somewhere between the last two; the line lies below.
 constexpr int64_t kFewSamples = 256;
 constexpr float kRayLength = 32768.0f * 1.74f;
 constexpr uint32_t kFlagStack = 1, kFlagBadAverage = 2, kFlagOutsideLump = 4;

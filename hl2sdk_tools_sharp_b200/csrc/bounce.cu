@@ -1256,7 +1256,7 @@ cudaError_t launch_patch_light(const BounceBuffers &b, const FinalView &fv, cons
 // (at upload: they size the buffers, and they depend only on the patch
 // tree and the PVS rows, so they stay valid until the next upload).
 // Otherwise, with those offsets, the candidates written, their rays and
-// form factors, and the transfer lists; counters[0..1] are added to.
+// form factors, and the transfer lists; counters[1..2] are added to.
 cudaError_t launch_transfers(BounceBuffers &b, const DeviceScene &scene, uint32_t *overflow, cudaStream_t stream,
                              bool count_only) {
     const int R = b.nreceivers;

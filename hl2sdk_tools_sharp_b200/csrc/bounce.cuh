@@ -159,7 +159,9 @@ struct BounceBuffers {
     uint16_t *feat = nullptr;      // R x 32 BF16 inputs
     float *pred = nullptr;         // R x 3 outputs
     const vrad_mlp *model = nullptr;
-    unsigned long long *counters = nullptr;  // [0] transfer rays, [1] blocked, [2] asin ties left open
+    // [0] the slices' padding, at the upload; [1] blocked transfer rays, [2]
+    // asin ties left open, of a transfer build.
+    unsigned long long *counters = nullptr;
     double *h_parts = nullptr;     // pinned host copy of the parts
     double h_sums[9] = {};         // their sums (add_parts)
     float *h_exact = nullptr;

@@ -216,11 +216,13 @@ __device__ __forceinline__ void add_tile(float *grad, int stride, int ncols, int
 // rows 6.9e-7 and 3.9e-7).
 // A minibatch is a few hundred tiles, so what counts is one tile's time and
 // what it sends to memory: nothing but x and the targets in, and one atomic
-// add per parameter and CTA out.  A tile takes 9.5 us, which is the rate of
-// mma.sync on this chip (sixteen warps, two to a row group, take as long),
-// and 32,768 rows 35 us.  As five kernels with the activations and their
+// add per parameter and CTA out.  A tile takes 8.2 us, near the rate of
+// mma.sync on this chip (sixteen warps, two to a row group, take as long), and
+// what is around the tiles, the weights in and the gradients out, 16 us for
+// one CTA and 24 for 148: 128 rows 24 us, 18,944 (a tile a CTA) 32, 32,768 35,
+// 151,552 (eight) 90.  As five kernels with the activations and their
 // gradients in HBM, shared memory operands read with up to eight-way bank
-// conflicts and transposed by 2-byte stores, they took 145 us.
+// conflicts and transposed by 2-byte stores, 32,768 rows took 145 us.
 __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_gradient(vrad_mlp m, const uint16_t *__restrict__ x,
                                                                  const float *__restrict__ target, int64_t n, float inv) {
     extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -29,7 +29,7 @@
 // there reads 8 KB in the 64 cycles that it takes, and the epilogues wrote
 // and read 64 KB a tile besides.  With the hidden layers there 1 M rows took
 // 90 us (two CTAs of eight warps, the tensor pipe 24 % active), 79 us with
-// four tiles in flight; in TMEM, half of that traffic gone, 71 us.  TMEM then
+// four tiles in flight; in TMEM, half of that traffic gone, 74 us.  TMEM then
 // holds two tiles, and what is left is their latency: of a tile's 4500
 // cycles the epilogues are 1900, the waits for MMAs 1400.
 //

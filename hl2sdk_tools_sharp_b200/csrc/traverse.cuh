@@ -220,12 +220,12 @@ __device__ __forceinline__ bool test_leaf(const DeviceBvh &s, const int32_t *__r
 // its order (six packed FMAs and eight min/max a visit; no swap of planes,
 // no order to compare), and an inner loop that takes all lanes through
 // nodes until each has a leaf or is done, so that the triangle test runs
-// once for the warp.  Against a walk of canonical nodes from the root, on
-// the 8x8 map: direct gather and supersampling 35.2 -> 25.7 ms by the
-// octants and the loop, 22.6 ms with UP; transfer build 62.4 -> 54.3 -> 47.6
-// ms; 4.2 M closest hits 375 -> 291 us.  Four-wide nodes of the same layout
-// gave 57.8 ms for the transfer build, one 32-byte load for two 16-byte
-// ones nothing.
+// once for the warp.  Against a walk of canonical nodes from the root: the
+// 8x8 room grid's transfer build 62.4 -> 54.3 ms by the octants and the loop,
+// 47.6 ms with UP; the 4x4 grid's direct light with a soft sun 40.5 -> 23.9
+// ms with all three; 4.2 M closest hits 375 -> 291 us.  Four-wide nodes of the
+// same layout gave 57.8 ms for the transfer build, one 32-byte load for two
+// 16-byte ones nothing.
 template <bool ANY, int STRIDE = kBlock, bool UP = false, bool FLAG = false>
 __device__ __forceinline__ bool walk_octants(const DeviceBvh &s, const int32_t *__restrict__ tri_id,
                                      const RayState &r, float tmin, int32_t skip_id, int start, int *stack,
