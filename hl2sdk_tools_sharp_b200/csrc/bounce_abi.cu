@@ -653,6 +653,12 @@ extern "C" int32_t vrad_bounce_upload(vrad_ctx *ctx, const vrad_bounce_desc *d) 
         return vrad_cuda_fail(ctx, e, "patch radial tables");
     }
     clock.mark("patch radial tables");
+    // Until a pass bounces (with no bounces none does) there is no bounced or
+    // direct patch light and there are no transfers to report: the blocks hold
+    // what their last user left.
+    if (e == cudaSuccess) e = cudaMemsetAsync(b.total, 0, sizeof(float4) * P1, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(b.direct, 0, sizeof(float4) * P1, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(b.tr_off, 0, sizeof(int64_t) * R1, s);
     // Size the candidate and transfer arrays by one build.  The walk's
     // overflow flag is a status word of its own (status[1]): a direct
     // gather queued ahead may be running beside this upload.

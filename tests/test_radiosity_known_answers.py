@@ -254,3 +254,25 @@ def test_device_transfer_lists(oracle_mod):
     o = _oracle(oracle_mod, world, inp, refl, bounces=1)
     assert np.array_equal(d["off"], o["off"]) and np.array_equal(d["src"], o["src"])
     assert np.array_equal(d["w"].view(np.uint32), o["w"].view(np.uint32))
+
+
+@pytest.mark.gpu
+def test_device_without_bounces_reports_nothing_of_the_upload_before():
+    """No bounces after many, on one context, whose blocks are used again: no
+    bounced light, no patch light and no transfers, before and after the
+    pass."""
+    world, inp, refl = _box()
+    with L.LightingStage(world, inp) as st:
+        st.upload_bounce(refl, *PVS, bounces=100, threshold=1.0)
+        st.light_pass()
+        total, direct = st.patch_light()
+        off, tr = st.transfers()
+        assert total.any() and direct.any() and len(tr)
+        for _ in range(2):
+            st.upload_bounce(refl, *PVS, bounces=0, threshold=1.0)
+            for lit in (False, True):
+                if lit:
+                    st.light_pass()
+                total, direct = st.patch_light()
+                off, tr = st.transfers()
+                assert not total.any() and not direct.any() and not off.any() and len(tr) == 0
