@@ -705,12 +705,11 @@ def batched_run(args, device_index: int, rank: int = 0, world: int = 1) -> dict:
     return out
 
 
-# Per launch DRAM traffic of the dominant kernels, from one ncu capture each
-# (dram__bytes_read.sum + dram__bytes_write.sum over the units that launch
-# processed), scaled by the units a full launch processes.  The captures
-# and their commands: profiles/k_transfer_4x4_roomgrid.md,
-# profiles/k_direct_4x4_roomgrid.md.
-TRAFFIC_PER_TRANSFER_RAY = (92441088 + 49963008) / 19922134.0
+# DRAM traffic of the transfer rays' kernel, from one ncu capture
+# (dram__bytes_read.sum + dram__bytes_write.sum over the rays that launch
+# traced), scaled by the rays a full launch traces.  The capture and its
+# command: profiles/light_pass_4x4_roomgrid.md.
+TRAFFIC_PER_TRANSFER_RAY = (659467520 + 614478080) / 153232710.0
 
 
 def lockdown_ambient_lumps(seed: int = 3) -> dict:
@@ -1075,16 +1074,16 @@ def main_stage(args):
         traffic = None
     else:
         alg_bytes = 28.0 * transfer_rays + 8.0 * bst[0].transfers
-        kernel, kernel_ms = "transfer build (k_candidates + k_transfer + compaction)", transfer_ms
+        kernel, kernel_ms = "transfer build (k_candidates + k_transfer_groups + compaction)", transfer_ms
         alg_note = "28 B per candidate ray + 8 B per transfer written"
         traffic = TRAFFIC_PER_TRANSFER_RAY * transfer_rays
     achieved = alg_bytes / (kernel_ms / 1000.0) / 1e9
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": traffic, "kernel": kernel, "kernel_ms": kernel_ms, "algorithmic_bytes": alg_note,
                 "algorithmic_bytes_per_launch": alg_bytes,
-                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_transfer launch on "
-                                  "the 4x4 map (profiles/k_transfer_4x4_roomgrid.md), per transfer ray, times this "
-                                  "launch's transfer rays",
+                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_transfer_groups launch "
+                                  "on the 4x4 map (profiles/light_pass_4x4_roomgrid.md), per transfer ray, times "
+                                  "this launch's transfer rays",
                 "peak_source": "measured" if "hbm_gbs" in peaks else "fallback",
                 "direct_ms": direct_ms, "transfer_build_ms": transfer_ms}
     nb_l = int(statistics.median([p[3] for p in phases]))
