@@ -40,7 +40,13 @@ __device__ __forceinline__ RayState load_ray(const vrad_ray *__restrict__ ray, f
 // (a target straight ahead), take as long as before, 4.2 M closest hits on the
 // 8x8 room grid 300 us against 299.  A call of its own, so that the walk by
 // octants keeps its registers.
+//
+// Not for a batch that leaves the chip part idle, whose time is its longest
+// ray's: by octants that has fewer instructions a node.  1 k triangles, by
+// octants and so: 1,024 rays 31.4 and 35.4 us, 32,768 36.6 and 39.5, 65,536
+// 41.7 and 40.6, 131,072 53.6 and 49.6.
 constexpr int kTogether = 4;
+constexpr int64_t kApartRays = 65536;
 
 template <int MODE>
 __device__ __noinline__ int4 trace_apart(const DeviceScene &s, const vrad_ray *ray, const TraceParams &p, int *stack) {
@@ -53,7 +59,8 @@ __device__ __noinline__ int4 trace_apart(const DeviceScene &s, const vrad_ray *r
     return make_int4(hit ? 1 : 0, __float_as_int(best_t), best_orig, 0);
 }
 
-template <bool ONE, int MODE>
+// APART: the batch is large enough for trace_apart.
+template <bool ONE, bool APART, int MODE>
 __global__ void __launch_bounds__(kBlock) k_trace(const __grid_constant__ DeviceScene s,
                                                   const vrad_ray *__restrict__ rays, int64_t n,
                                                   const __grid_constant__ TraceParams p, uint32_t *__restrict__ bits,
@@ -72,7 +79,7 @@ __global__ void __launch_bounds__(kBlock) k_trace(const __grid_constant__ Device
         const RayState r = load_ray(rays + i, reach);
         if (ONE) {
             trace_ray<true, MODE>(s, r, p.tmin, reach, p.skip_id, 0, stack, hit, best_t, best_orig, best_meta);
-        } else if (octants_of(live, r) > kTogether) {
+        } else if (APART && octants_of(live, r) > kTogether) {
             const int4 h = trace_apart<MODE>(s, rays + i, p, stack);
             hit = h.x != 0;
             best_t = __int_as_float(h.y);
@@ -108,29 +115,36 @@ cudaError_t launch_trace(const DeviceScene &scene, const vrad_ray *d_rays, int64
     const int64_t grid = (n + kBlock - 1) / kBlock;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
     const size_t smem = sizeof(int) * (size_t)scene.stack_depth() * kBlock;
-    by_copies(scene, [&](auto one) {
-        constexpr bool kOne = decltype(one)::value;
+    auto launch = [&](auto one, auto apart) {
+        constexpr bool kOne = decltype(one)::value, kApart = decltype(apart)::value;
         switch (p.mode) {
             case kModeAny:
-                k_trace<kOne, kModeAny><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits, d_hits);
+                k_trace<kOne, kApart, kModeAny><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits, d_hits);
                 break;
             case kModeClosest:
-                k_trace<kOne, kModeClosest><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits, d_hits);
+                k_trace<kOne, kApart, kModeClosest><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits,
+                                                                                            d_hits);
                 break;
             default:
-                k_trace<kOne, kModeSkyPass><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits, d_hits);
+                k_trace<kOne, kApart, kModeSkyPass><<<(unsigned)grid, kBlock, smem, stream>>>(scene, d_rays, n, p, d_bits,
+                                                                                            d_hits);
                 break;
         }
-    });
+    };
+    if (scene.one_copy) launch(std::true_type{}, std::false_type{});
+    else if (n > kApartRays) launch(std::false_type{}, std::true_type{});
+    else launch(std::false_type{}, std::false_type{});
     return cudaGetLastError();
 }
 
+static_assert(VRAD_STATIC_MAX_RAYS <= kApartRays, "the allocation-free entry launches no kernel that is not loaded here");
+
 cudaError_t load_visibility_kernels() {
     cudaFuncAttributes a;
-    cudaError_t e = cudaFuncGetAttributes(&a, k_trace<false, kModeAny>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_trace<false, kModeSkyPass>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_trace<true, kModeAny>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_trace<true, kModeSkyPass>);
+    cudaError_t e = cudaFuncGetAttributes(&a, k_trace<false, false, kModeAny>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_trace<false, false, kModeSkyPass>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_trace<true, false, kModeAny>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_trace<true, false, kModeSkyPass>);
     return e;
 }
 

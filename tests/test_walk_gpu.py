@@ -88,7 +88,7 @@ def test_soup_of_many_triangles_equals_brute_force(n, sky, oracle_mod):
 
 
 @pytest.mark.parametrize("octants", [1, 4, 5, 8])
-@pytest.mark.parametrize("count", [1, 31, 33, 1000])
+@pytest.mark.parametrize("count", [1, 31, 33, 1000, 65536, 65537, 70001])
 def test_warps_of_few_and_many_octants(octants, count, oracle_mod):
     """Each warp's rays lie in so many octants (the last warp's in as many as
     it has rays for): either walk gives the brute force's answers."""
