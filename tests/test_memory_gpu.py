@@ -3,6 +3,7 @@ left out, and the pass gives the same lump.  A process of its own fills the
 device, so that no other test's cached blocks count."""
 from __future__ import annotations
 
+import os
 import pathlib
 import subprocess
 import sys
@@ -80,8 +81,10 @@ with L.LightingStage(small, L.prepare(small)) as st:   # the kernels' code is on
 
 
 def python(code, *args):
+    # Each tensor an allocation of its own size, so that the room left is exact.
+    env = dict(os.environ, PYTORCH_NO_CUDA_MEMORY_CACHING="1")
     run = subprocess.run([sys.executable, "-c", code, *map(str, args)], cwd=ROOT, capture_output=True, text=True,
-                         timeout=300)
+                         timeout=300, env=env)
     assert run.returncode == 0, run.stdout + run.stderr
     return run.stdout.split()
 
